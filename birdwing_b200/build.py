@@ -11,8 +11,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libbirdwing.so")
-SOURCES = ["bw_core.cu", "bw_noalloc.cu", "bw_batch.cu", "bw_server.cu", "bw_probe.cu"]
-HEADERS = ["bw_arith.cuh", "bw_kernels.cuh", "bw_host.h", "bw_internal.h"]
+SOURCES = ["bw_core.cu", "bw_tr_p32.cu", "bw_tr_p32w.cu", "bw_tr_p64.cu", "bw_tr_f64_0.cu", "bw_tr_f64_1.cu",
+           "bw_noalloc.cu", "bw_batch.cu",
+           "bw_server.cu", "bw_probe.cu"]
+HEADERS = ["bw_arith.cuh", "bw_kernels.cuh", "bw_host.h", "bw_internal.h", "bw_transform.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -17,6 +17,7 @@
 // src/crt_gpu.cu:47-67), which is a software division on the GPU.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 namespace bw {
 
@@ -29,6 +30,7 @@ struct alignas(2 * sizeof(T)) Tw {
 struct Ar32 {
     using T = uint32_t;
     static constexpr int BITS = 32;
+    static constexpr bool kF64 = false;
     uint32_t p;
     uint32_t p2;    // 2p
     uint32_t pinv;  // -p^-1 mod 2^32
@@ -81,6 +83,10 @@ struct Ar32 {
     __device__ __forceinline__ T inv_out(T a) const { return red1(a); }
     // x * w for a twiddle applied between transform passes, in [0, 2p)
     __device__ __forceinline__ T mulc(T x, T w, T wq) const { return shoup(x, w, wq); }
+    // a 16- or 32-bit coefficient as a residue
+    static __device__ __forceinline__ T from_u32(uint32_t x) { return (T)x; }
+    // last scaling of a single-pass transform, in [0, p)
+    __device__ __forceinline__ T scale_out(T x, T w, T wq) const { return red1(shoup(x, w, wq)); }
     // Shoup companion floor(w 2^32 / p) of w < p: a double-precision estimate
     // w (2^32 / p) is within 2^-20 of the quotient (below 2^32, relative error
     // under 2^-51), so its floor is exact or one off, and the exact remainder
@@ -120,6 +126,7 @@ struct Ar32 {
 struct Ar64 {
     using T = uint64_t;
     static constexpr int BITS = 64;
+    static constexpr bool kF64 = false;
     uint64_t p;
     uint64_t p2;    // 2p
     uint64_t pinv;  // -p^-1 mod 2^64
@@ -254,6 +261,10 @@ struct Ar64 {
     __device__ __forceinline__ T inv_out(T a) const { return red1(min(a, a - p2)); }
     // x * w for a twiddle applied between transform passes, in [0, 3p)
     __device__ __forceinline__ T mulc(T x, T w, T wq) const { return shoup3(x, w, wq); }
+    // a 16- or 32-bit coefficient as a residue
+    static __device__ __forceinline__ T from_u32(uint32_t x) { return (T)x; }
+    // last scaling of a single-pass transform, in [0, p)
+    __device__ __forceinline__ T scale_out(T x, T w, T wq) const { return red1(shoup(x, w, wq)); }
     // Shoup companion floor(w 2^64 / p) of w < p by a Barrett step with
     // mu = floor(2^128 / p): the estimate is at most 2 short.
     __device__ __forceinline__ T companion(T w) const {
@@ -268,6 +279,133 @@ struct Ar64 {
     }
 };
 
+// Exact modular arithmetic in double precision, for the 64-bit path's 64-bit
+// coefficients.  A residue is a double holding an integer of either sign below
+// 2^53 in magnitude, so sums and differences are exact, and a product by a
+// constant w (|w| <= p/2, companion wq = w / p) takes six operations:
+//
+//   h = x w (rounded), l = x w - h (exact, one FMA), q = round(x wq),
+//   r = (h - q p) + l = x w - q p.
+//
+// q comes from adding and subtracting 1.5 2^52, which rounds to an integer
+// while |q| <= 2^51.  q is within 1/2 + |x w / p| 2^-53 of x w / p, so
+// |r| <= p (1/2 + X p 2^-54) for |x| = X p; h - q p is an integer below 2^53,
+// so the FMA and the last addition are exact.  The FP64 pipe of an SM takes 64
+// such operations per cycle, beside the integer pipe's addressing: a butterfly
+// is 8 of them against about 40 integer instructions for a 58-bit prime
+// (measured 6.7 against 2.83 butterflies per SM-cycle).
+//
+// POL 0: primes just above 2^50 (X <= 4 keeps q below 2^51).  Forward: a round
+//   reduces the half it does not multiply in its first stage and then adds four
+//   stages: from X <= 4 at most 1.25, 1.83, 2.44, 3.10.  Inverse: the sums of
+//   every second stage, and of a round's last, are reduced (X <= 0.7 between
+//   rounds, differences at most 2.8).
+// POL 1: primes just above 2^51.66 (X <= 1.26 for q, 2.5 for exact sums), for
+//   transforms whose coefficients need three such primes: a forward round
+//   reduces all its values before its first and third stage (X <= 1.85 at its
+//   end), an inverse stage reduces both outputs.
+template <int POL>
+struct ArD {
+    using T = double;
+    static constexpr int BITS = 0;  // products carry no power of two to cancel
+    static constexpr bool kF64 = true;
+    double p;
+    double pinv;  // 1 / p
+
+    static __device__ __forceinline__ double rnd(double t) {
+        return __dadd_rn(t, -6755399441055744.0);
+    }
+    static constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52
+    // x - p round(x / p): at most p/2 (1 + 2^-49) in magnitude
+    __device__ __forceinline__ T red(T x) const {
+        const double q = rnd(__fma_rn(x, pinv, kMagic));
+        return __fma_rn(-q, p, x);
+    }
+    __device__ __forceinline__ T mul(T x, T w, T wq) const {
+        const double q = rnd(__fma_rn(x, wq, kMagic));
+        const double h = __dmul_rn(x, w);
+        const double l = __fma_rn(x, w, -h);
+        return __dadd_rn(__fma_rn(-q, p, h), l);
+    }
+    // product of two residues reduced by red
+    __device__ __forceinline__ T mont(T a, T b) const {
+        const double h = __dmul_rn(a, b);
+        const double q = rnd(__fma_rn(h, pinv, kMagic));
+        const double l = __fma_rn(a, b, -h);
+        const double r = __dadd_rn(__fma_rn(-q, p, h), l);
+        return POL ? red(r) : r;
+    }
+    // before the stage l of a forward round (h: the stage's half width)
+    template <int RL>
+    __device__ __forceinline__ void ct_enter(T* x, int l, int s0) const {
+        if (POL == 0) {
+            if (l == 0 && s0 > 0) {
+#pragma unroll
+                for (int u = 0; u < (1 << (RL - 1)); ++u) x[u] = red(x[u]);
+            }
+        } else if ((l & 1) == 0) {
+#pragma unroll
+            for (int u = 0; u < (1 << RL); ++u) x[u] = red(x[u]);
+        }
+    }
+    __device__ __forceinline__ void ct(T& a, T& b, T w, T wq) const {
+        const T x = a;
+        const T t = mul(b, w, wq);
+        a = __dadd_rn(x, t);
+        b = __dsub_rn(x, t);
+    }
+    __device__ __forceinline__ void ct1(T& a, T& b) const {
+        const T x = a;
+        a = __dadd_rn(x, b);
+        b = __dsub_rn(x, b);
+    }
+    // RED: this stage's sums are reduced
+    template <bool RED>
+    __device__ __forceinline__ void gs(T& a, T& b, T w, T wq) const {
+        const T u = __dadd_rn(a, b);
+        const T v = __dsub_rn(a, b);
+        a = RED || POL ? red(u) : u;
+        const T r = mul(v, w, wq);
+        b = POL ? red(r) : r;
+    }
+    __device__ __forceinline__ void gs1(T& a, T& b) const {
+        const T u = __dadd_rn(a, b);
+        const T v = __dsub_rn(a, b);
+        a = red(u);
+        b = red(v);
+    }
+    __device__ __forceinline__ T fwd_to_2p(T a) const { return red(a); }
+    // twiddles between passes: any forward or inverse output in, at most
+    // 0.75 p out
+    __device__ __forceinline__ T mulc(T x, T w, T wq) const {
+        return POL ? red(mul(red(x), w, wq)) : mul(x, w, wq);
+    }
+    __device__ __forceinline__ T shoup(T x, T w, T wq) const { return mulc(x, w, wq); }
+    __device__ __forceinline__ T red1(T x) const { return red(x); }
+    __device__ __forceinline__ T companion(T w) const { return __dmul_rn(w, pinv); }
+    // an integer below 2^32 or 2^64 as a residue: its words land in the
+    // mantissas of 2^52 and 2^84; the high word's multiple of 2^32 is reduced
+    // (|hi - q p| < 2^51 is exact) before the low word is added
+    static __device__ __forceinline__ T from_u32(uint32_t x) {
+        return __dsub_rn(__hiloint2double(0x43300000, (int)x), 4503599627370496.0);
+    }
+    __device__ __forceinline__ T from_u64(uint64_t x) const {
+        const double lo = from_u32((uint32_t)x);
+        const double hi = __dsub_rn(__hiloint2double(0x45300000, (int)(x >> 32)),
+                                    19342813113834066795298816.0);
+        const double q = rnd(__fma_rn(hi, pinv, kMagic));
+        return __dadd_rn(__fma_rn(-q, p, hi), lo);
+    }
+    // an inverse output (|x| < p) as an integer in [0, p), in the bits of a
+    // double (the Garner kernels read integers)
+    __device__ __forceinline__ T inv_out(T x) const {
+        const double y = x < 0.0 ? __dadd_rn(x, p) : x;
+        const double z = __dadd_rn(y, 4503599627370496.0);
+        return __longlong_as_double(__double_as_longlong(z) & 0x000fffffffffffffll);
+    }
+    __device__ __forceinline__ T scale_out(T x, T w, T wq) const { return inv_out(mulc(x, w, wq)); }
+};
+
 // Twiddle load from shared memory (generic pointer into the CTA's tables).
 template <typename T>
 __device__ __forceinline__ Tw<T> ld_tw_s(const Tw<T>* p) {
@@ -277,7 +415,11 @@ __device__ __forceinline__ Tw<T> ld_tw_s(const Tw<T>* p) {
 template <typename T>
 __device__ __forceinline__ Tw<T> ld_tw(const Tw<T>* p) {
     Tw<T> r;
-    if constexpr (sizeof(T) == 8) {
+    if constexpr (std::is_same<T, double>::value) {
+        const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+        r.w = v.x;
+        r.wq = v.y;
+    } else if constexpr (sizeof(T) == 8) {
         const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p));
         r.w = v.x;
         r.wq = v.y;

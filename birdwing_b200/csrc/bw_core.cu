@@ -42,15 +42,6 @@ int bw_fail(int code, const char* fmt, ...) {
 }
 void bw_clear_error() { g_last_error.clear(); }
 
-#define BW_CUDA(call)                                                                   \
-    do {                                                                                \
-        cudaError_t e_ = (call);                                                        \
-        if (e_ != cudaSuccess) {                                                        \
-            return bw_fail(e_ == cudaErrorMemoryAllocation ? BW_ENOMEM : BW_ECUDA,      \
-                           "%s failed: %s", #call, cudaGetErrorString(e_));             \
-        }                                                                               \
-    } while (0)
-
 // ------------------------------------------------------------------ host math
 
 namespace {
@@ -109,6 +100,13 @@ const uint64_t kP32W[6] = {595591169ull, 645922817ull, 754974721ull,
                            880803841ull, 897581057ull, 998244353ull};
 const uint64_t kG32W[6] = {3, 3, 11, 26, 3, 3};
 
+// 64-bit path, 64-bit coefficients in double-precision arithmetic (ArD): the
+// smallest primes c 2^32 + 1 above 2^50, and the smallest whose product is
+// above 2^155.
+const uint64_t kPD[2][3] = {{0x4000e00000001ull, 0x4001100000001ull, 0x4002100000001ull},
+                            {0xcb30200000001ull, 0xcb30a00000001ull, 0xcb3a400000001ull}};
+const uint64_t kGD[2][3] = {{19, 7, 3}, {3, 5, 3}};
+
 int v2(uint64_t x) {
     int k = 0;
     while ((x & 1) == 0) {
@@ -134,16 +132,39 @@ const uint64_t* bw_path_primes(int path) { return path == BW_PATH_P64 ? kP64 : k
 
 // The prime set of a plan and its generators: the path's own, or the six
 // 32-bit primes when the 32-bit path carries 64-bit coefficients.
-static const uint64_t* plan_primes(int path, bool w64) {
+static const uint64_t* plan_primes(int path, bool w64, int f64) {
+    if (f64) return kPD[f64 - 1];
     return (w64 && path == BW_PATH_P32) ? kP32W : bw_path_primes(path);
 }
-static const uint64_t* plan_gens(int path, bool w64) {
+static const uint64_t* plan_gens(int path, bool w64, int f64) {
+    if (f64) return kGD[f64 - 1];
     return (w64 && path == BW_PATH_P32) ? kG32W : path == BW_PATH_P64 ? kG64 : kG32;
+}
+
+// Double-precision primes of a product with 64-bit coefficients on the 64-bit
+// path: the first set while min(na, nb) <= 2^22 (its product is above 2^150),
+// the second up to 2^27 (above 2^155); 0: the 58-bit integer primes.
+static int choose_f64(size_t nca, size_t ncb) {
+    const size_t m = std::min(nca, ncb);
+    return m <= ((size_t)1 << 22) ? 1 : m <= ((size_t)1 << 27) ? 2 : 0;
 }
 
 // ------------------------------------------------------------------ plan
 
 namespace {
+
+// A table entry: a constant and its companion.  Integers: floor(w 2^bits / p);
+// double precision: w taken to [-p/2, p/2] and w / p.
+template <class Ar>
+Tw<typename Ar::T> make_tw(uint64_t w, uint64_t p) {
+    using T = typename Ar::T;
+    if constexpr (Ar::kF64) {
+        const double b = w > p / 2 ? -(double)(p - w) : (double)w;
+        return Tw<T>{b, b / (double)p};
+    } else {
+        return Tw<T>{(T)w, (T)shoup_pre(w, p, Ar::BITS)};
+    }
+}
 
 template <class Ar>
 struct TableBuilder {
@@ -155,7 +176,7 @@ struct TableBuilder {
     void align_even() {
         if (host.size() & 1) host.push_back(Tw<T>{0, 0});
     }
-    size_t add_stage_table(uint64_t p, uint64_t root, int log_len, int bits) {
+    size_t add_stage_table(uint64_t p, uint64_t root, int log_len) {
         const size_t L = (size_t)1 << log_len;
         align_even();
         const size_t off = host.size();
@@ -169,18 +190,18 @@ struct TableBuilder {
             for (size_t i = 0; i < m; ++i) {
                 const size_t e = (L >> (s + 1)) * bitrev_h((uint32_t)i, s);
                 const uint64_t w = pw[e];
-                host[off + m + i] = Tw<T>{(T)w, (T)shoup_pre(w, p, bits)};
+                host[off + m + i] = make_tw<Ar>(w, p);
             }
         }
         return off;
     }
-    size_t add_power_table(uint64_t p, uint64_t base, size_t count, uint64_t scale, int bits) {
+    size_t add_power_table(uint64_t p, uint64_t base, size_t count, uint64_t scale) {
         align_even();
         const size_t off = host.size();
         host.resize(off + count);
         uint64_t w = scale % p;
         for (size_t j = 0; j < count; ++j) {
-            host[off + j] = Tw<T>{(T)w, (T)shoup_pre(w, p, bits)};
+            host[off + j] = make_tw<Ar>(w, p);
             w = mulmod(w, base, p);
         }
         return off;
@@ -204,90 +225,29 @@ inline void set_c(Ar64& a, uint64_t p) {
     a.oneq = (uint64_t)(((u128)1 << 64) / p);
 }
 
+// A plan's arithmetic and Garner constants and its geometry (everything but
+// the tables).
 template <class Ar>
-int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
+void fill_constants(const bw_plan* pl, PlanDev<Ar>& pd) {
     using T = typename Ar::T;
-    const int bits = Ar::BITS;
-    const uint64_t* P = plan_primes(pl->path, pl->w64 != 0);
-    const uint64_t* Gn = plan_gens(pl->path, pl->w64 != 0);
-    TableBuilder<Ar> tb;
-    size_t off[kMaxPrimes][12];
-    const size_t n = (size_t)1 << pl->log_n;
-    // row-level twiddle length: R * C (two passes) or R2 * C (three passes)
-    const int log_rr = pl->log_r2 ? pl->log_r2 : pl->log_r;
-    const size_t n_row = (size_t)1 << (log_rr + pl->log_c);
-    uint64_t scale_k[kMaxPrimes] = {};
-    for (int k = 0; k < pl->K; ++k) {
-        const uint64_t p = P[k];
-        scale_k[k] = mulmod(invmod(n % p, p), powmod(2, bits, p), p);
-        if (pl->small) {
-            // single pass: n-point stage tables only
-            const uint64_t wn = powmod(Gn[k], (p - 1) >> pl->log_n, p);
-            off[k][2] = tb.add_stage_table(p, wn, pl->log_n, bits);
-            off[k][3] = tb.add_stage_table(p, invmod(wn, p), pl->log_n, bits);
-            continue;
-        }
-        const uint64_t wn = powmod(Gn[k], (p - 1) >> pl->log_n, p);  // primitive n-th root
-        const uint64_t wrow = powmod(wn, n / n_row, p);               // n_row-th root
-        const uint64_t wrowi = invmod(wrow, p);
-        const uint64_t wr = powmod(wn, n >> pl->log_r, p);            // R-th root
-        const uint64_t wc = powmod(wn, n >> pl->log_c, p);            // C-th root
-        off[k][0] = tb.add_stage_table(p, wr, pl->log_r, bits);
-        off[k][1] = tb.add_stage_table(p, invmod(wr, p), pl->log_r, bits);
-        off[k][2] = tb.add_stage_table(p, wc, pl->log_c, bits);
-        off[k][3] = tb.add_stage_table(p, invmod(wc, p), pl->log_c, bits);
-        const size_t nlo = (size_t)1 << pl->lo, nhi = n_row >> pl->lo;
-        const uint64_t scale = mulmod(invmod(n % p, p), powmod(2, bits, p), p);
-        off[k][4] = tb.add_power_table(p, wrow, nlo, 1, bits);
-        off[k][5] = tb.add_power_table(p, powmod(wrow, nlo, p), nhi, 1, bits);
-        off[k][6] = tb.add_power_table(p, wrowi, nlo, 1, bits);
-        off[k][7] = tb.add_power_table(p, powmod(wrowi, nlo, p), nhi, scale, bits);
-        if (pl->log_r2) {
-            const uint64_t wm = powmod(wn, n >> pl->log_r2, p);  // R2-th root
-            off[k][8] = tb.add_stage_table(p, wm, pl->log_r2, bits);
-            off[k][9] = tb.add_stage_table(p, invmod(wm, p), pl->log_r2, bits);
-            const size_t olo = (size_t)1 << pl->lo_out, ohi = n >> pl->lo_out;
-            off[k][10] = tb.add_power_table(p, wn, olo, 1, bits);
-            off[k][11] = tb.add_power_table(p, powmod(wn, olo, p), ohi, 1, bits);
-        }
-    }
-    pl->table_bytes = tb.host.size() * sizeof(Tw<T>);
-    BW_CUDA(cudaMalloc(&pl->d_tables, pl->table_bytes));
-    BW_CUDA(cudaMemcpy(pl->d_tables, tb.host.data(), pl->table_bytes, cudaMemcpyHostToDevice));
-    const Tw<T>* base = reinterpret_cast<const Tw<T>*>(pl->d_tables);
+    constexpr int bits = Ar::BITS;
+    const uint64_t* P = plan_primes(pl->path, pl->w64 != 0, pl->f64);
     for (int k = 0; k < pl->K; ++k) {
         auto& pr = pd.pr[k];
-        pr.scale = Tw<T>{(T)scale_k[k], (T)shoup_pre(scale_k[k], P[k], bits)};
-        if (pl->small) {
-            pr.WCf = base + off[k][2];
-            pr.WCi = base + off[k][3];
+        if constexpr (Ar::kF64) {
+            pr.ar.p = (double)P[k];
+            pr.ar.pinv = 1.0 / (double)P[k];
+        } else {
             pr.ar.p = (T)P[k];
             pr.ar.p2 = (T)(2 * P[k]);
             pr.ar.pinv = (T)neg_inv_pow2(P[k], bits);
             set_c(pr.ar, P[k]);
             pr.one_q = (T)shoup_pre(1, P[k], bits);
-            continue;
         }
-        pr.WRf = base + off[k][0];
-        pr.WRi = base + off[k][1];
-        pr.WCf = base + off[k][2];
-        pr.WCi = base + off[k][3];
-        pr.TLf = base + off[k][4];
-        pr.THf = base + off[k][5];
-        pr.TLi = base + off[k][6];
-        pr.THi = base + off[k][7];
-        pr.WMf = pl->log_r2 ? base + off[k][8] : nullptr;
-        pr.WMi = pl->log_r2 ? base + off[k][9] : nullptr;
-        pr.OLf = pl->log_r2 ? base + off[k][10] : nullptr;
-        pr.OHf = pl->log_r2 ? base + off[k][11] : nullptr;
-        pr.ar.p = (T)P[k];
-        pr.ar.p2 = (T)(2 * P[k]);
-        pr.ar.pinv = (T)neg_inv_pow2(P[k], bits);
-        set_c(pr.ar, P[k]);
-        pr.one_q = (T)shoup_pre(1, P[k], bits);
     }
     // unused prime slots get harmless arithmetic constants
     for (int k = pl->K; k < kMaxPrimes; ++k) pd.pr[k] = pd.pr[0];
+    if constexpr (!Ar::kF64) {
     auto& g = pd.gar;
     const uint64_t p0 = P[0], p1 = P[1], p2 = P[2];
     g.p0 = p0;
@@ -306,6 +266,8 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
                 g.inv6[i * (i - 1) / 2 + j] = Tw<T>{(T)v, (T)shoup_pre(v, P[i], bits)};
             }
     }
+    g.top_bound = std::min(pl->nca, pl->ncb);
+    }
     pd.K = pl->K;
     pd.log_n = pl->log_n;
     pd.log_r = pl->log_r;
@@ -318,6 +280,81 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
     pd.log_r2 = pl->log_r2;
     pd.log_cb2 = pl->log_cb2;
     pd.lo_out = pl->lo_out;
+}
+
+template <class Ar>
+int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
+    using T = typename Ar::T;
+    const int bits = Ar::BITS;
+    const uint64_t* P = plan_primes(pl->path, pl->w64 != 0, pl->f64);
+    const uint64_t* Gn = plan_gens(pl->path, pl->w64 != 0, pl->f64);
+    TableBuilder<Ar> tb;
+    size_t off[kMaxPrimes][12];
+    const size_t n = (size_t)1 << pl->log_n;
+    // row-level twiddle length: R * C (two passes) or R2 * C (three passes)
+    const int log_rr = pl->log_r2 ? pl->log_r2 : pl->log_r;
+    const size_t n_row = (size_t)1 << (log_rr + pl->log_c);
+    uint64_t scale_k[kMaxPrimes] = {};
+    for (int k = 0; k < pl->K; ++k) {
+        const uint64_t p = P[k];
+        scale_k[k] = mulmod(invmod(n % p, p), powmod(2, bits, p), p);
+        if (pl->small) {
+            // single pass: n-point stage tables only
+            const uint64_t wn = powmod(Gn[k], (p - 1) >> pl->log_n, p);
+            off[k][2] = tb.add_stage_table(p, wn, pl->log_n);
+            off[k][3] = tb.add_stage_table(p, invmod(wn, p), pl->log_n);
+            continue;
+        }
+        const uint64_t wn = powmod(Gn[k], (p - 1) >> pl->log_n, p);  // primitive n-th root
+        const uint64_t wrow = powmod(wn, n / n_row, p);               // n_row-th root
+        const uint64_t wrowi = invmod(wrow, p);
+        const uint64_t wr = powmod(wn, n >> pl->log_r, p);            // R-th root
+        const uint64_t wc = powmod(wn, n >> pl->log_c, p);            // C-th root
+        off[k][0] = tb.add_stage_table(p, wr, pl->log_r);
+        off[k][1] = tb.add_stage_table(p, invmod(wr, p), pl->log_r);
+        off[k][2] = tb.add_stage_table(p, wc, pl->log_c);
+        off[k][3] = tb.add_stage_table(p, invmod(wc, p), pl->log_c);
+        const size_t nlo = (size_t)1 << pl->lo, nhi = n_row >> pl->lo;
+        const uint64_t scale = mulmod(invmod(n % p, p), powmod(2, bits, p), p);
+        off[k][4] = tb.add_power_table(p, wrow, nlo, 1);
+        off[k][5] = tb.add_power_table(p, powmod(wrow, nlo, p), nhi, 1);
+        off[k][6] = tb.add_power_table(p, wrowi, nlo, 1);
+        off[k][7] = tb.add_power_table(p, powmod(wrowi, nlo, p), nhi, scale);
+        if (pl->log_r2) {
+            const uint64_t wm = powmod(wn, n >> pl->log_r2, p);  // R2-th root
+            off[k][8] = tb.add_stage_table(p, wm, pl->log_r2);
+            off[k][9] = tb.add_stage_table(p, invmod(wm, p), pl->log_r2);
+            const size_t olo = (size_t)1 << pl->lo_out, ohi = n >> pl->lo_out;
+            off[k][10] = tb.add_power_table(p, wn, olo, 1);
+            off[k][11] = tb.add_power_table(p, powmod(wn, olo, p), ohi, 1);
+        }
+    }
+    pl->table_bytes = tb.host.size() * sizeof(Tw<T>);
+    BW_CUDA(cudaMalloc(&pl->d_tables, pl->table_bytes));
+    BW_CUDA(cudaMemcpy(pl->d_tables, tb.host.data(), pl->table_bytes, cudaMemcpyHostToDevice));
+    const Tw<T>* base = reinterpret_cast<const Tw<T>*>(pl->d_tables);
+    for (int k = 0; k < pl->K; ++k) {
+        auto& pr = pd.pr[k];
+        pr.scale = make_tw<Ar>(scale_k[k], P[k]);
+        if (pl->small) {
+            pr.WCf = base + off[k][2];
+            pr.WCi = base + off[k][3];
+            continue;
+        }
+        pr.WRf = base + off[k][0];
+        pr.WRi = base + off[k][1];
+        pr.WCf = base + off[k][2];
+        pr.WCi = base + off[k][3];
+        pr.TLf = base + off[k][4];
+        pr.THf = base + off[k][5];
+        pr.TLi = base + off[k][6];
+        pr.THi = base + off[k][7];
+        pr.WMf = pl->log_r2 ? base + off[k][8] : nullptr;
+        pr.WMi = pl->log_r2 ? base + off[k][9] : nullptr;
+        pr.OLf = pl->log_r2 ? base + off[k][10] : nullptr;
+        pr.OHf = pl->log_r2 ? base + off[k][11] : nullptr;
+    }
+    fill_constants(pl, pd);
     return BW_OK;
 }
 
@@ -621,10 +658,13 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
         pl->lo = ((pl->log_r2 ? pl->log_r2 : pl->log_r) + pl->log_c + 1) / 2;
         pl->lo_out = (log_n + 1) / 2;
     }
-    for (int k = 0; k < K; ++k) pl->primes[k] = plan_primes(path, pl->w64 != 0)[k];
+    for (int k = 0; k < K; ++k) pl->primes[k] = plan_primes(path, pl->w64 != 0, pl->f64)[k];
     cudaGetDevice(&pl->device);
-    const int rc =
-        path == BW_PATH_P64 ? build_tables<Ar64>(pl, pl->pd64) : build_tables<Ar32>(pl, pl->pd32);
+    const int rc = pl->f64 == 1            ? build_tables<ArD<0>>(pl, pl->pdd0)
+                   : pl->f64 == 2          ? build_tables<ArD<1>>(pl, pl->pdd1)
+                   : path == BW_PATH_P64 ? build_tables<Ar64>(pl, pl->pd64)
+                                           : build_tables<Ar32>(pl, pl->pd32);
+    if (pl->f64) fill_constants<Ar64>(pl, pl->pd64);  // Garner reads integers
     if (rc && pl->d_tables) {
         cudaFree(pl->d_tables);
         pl->d_tables = nullptr;
@@ -651,6 +691,7 @@ extern "C" int bw_plan_create(bw_plan** out, int path, size_t la, size_t lb, int
     const int cpw = path == BW_PATH_P32 ? 2 : 1;
     pl->nca = w64 ? (la + 1) / 2 : la * cpw;
     pl->ncb = w64 ? (lb + 1) / 2 : lb * cpw;
+    if (w64 && path == BW_PATH_P64) pl->f64 = choose_f64(pl->nca, pl->ncb);
     const size_t half = ((size_t)1 << log_n) / 2;
     pl->zt_a = pl->nca <= half;
     pl->zt_b = pl->ncb <= half;
@@ -706,50 +747,6 @@ extern "C" int bw_plan_get_info(const bw_plan* pl, bw_plan_info* o) {
 }
 
 // ------------------------------------------------------------------ context
-
-// Most chunks a host copy is split into (see bw_ctx::copy_chunks).
-constexpr int kMaxCopyChunks = 16;
-
-struct bw_ctx {
-    const bw_plan* plan = nullptr;
-    cudaStream_t stream = nullptr;
-    bool own_stream = false;
-    void* d_res_a = nullptr;
-    void* d_res_b = nullptr;
-    uint32_t* d_in = nullptr;   // staging: a then b
-    uint32_t* d_out = nullptr;  // staging: product
-    unsigned char* d_state = nullptr;
-    size_t state_bytes = 0;
-    CarryState* cst = nullptr;
-    uint32_t* err = nullptr;
-    uint4* rec_x = nullptr;
-    uint32_t* rec_s = nullptr;
-    size_t ntiles = 0;
-    // look-back record tag of the last product.  Direct launches use 2, 3, ..;
-    // the replayable graph clears the records and always uses 1.
-    uint32_t epoch = 1;
-    bool capturing = false;
-    cudaGraphExec_t gexec = nullptr;  // device-pointer product, replayed while
-    const void* g_a = nullptr;        // the pointers stay the same
-    const void* g_b = nullptr;
-    const void* g_out = nullptr;
-    bool g_sq = false;
-    uint32_t* h_err = nullptr;  // pinned
-    cudaEvent_t ev[8] = {};
-    cudaEvent_t stage_ev[3] = {};  // ends of copy-in, kernels, copy-out (stage order)
-    bool counted = false;          // included in the plan's live contexts
-    // host copies split into chunks that overlap the first and last kernels
-    // (created on first use): copy-in on in_stream, copy-out on out_stream
-    int copy_chunks = 0;           // 0: automatic, 1: whole copies on the stream
-    cudaStream_t in_stream = nullptr, out_stream = nullptr;
-    cudaEvent_t in_ev[kMaxCopyChunks] = {}, out_ev[kMaxCopyChunks] = {};
-    cudaEvent_t ready_ev = nullptr, out_done_ev = nullptr;
-    int out_pieces = 0;            // K4 launches of the last chunked product
-    size_t out_tiles_per = 0;      // carry tiles per K4 launch
-    int spin_limit = 1 << 22;
-    bool inject_wait_fault = false;
-    CUtensorMap tmap_res;          // residues of A as [prime][row][column] (tma_cols)
-};
 
 // Tensor map of a context's A residues for the TMA form of the inverse column
 // pass: dims (columns, rows, primes), boxes of CB columns x min(R, 256) rows.
@@ -938,155 +935,16 @@ extern "C" int bw_ctx_sync(bw_ctx* c) {
 
 // ------------------------------------------------------------------ launch
 
-namespace {
-
-template <class Ar>
-const PlanDev<Ar>& plan_dev(const bw_plan* pl);
-template <>
-const PlanDev<Ar32>& plan_dev<Ar32>(const bw_plan* pl) {
-    return pl->pd32;
-}
-template <>
-const PlanDev<Ar64>& plan_dev<Ar64>(const bw_plan* pl) {
-    return pl->pd64;
-}
-
-constexpr int kMaxDynSmem = 200 * 1024;
-
-template <class Ar, bool SPLIT16>
-int set_smem_attrs() {
-    static std::once_flag once;
-    static cudaError_t st = cudaSuccess;
-    std::call_once(once, [] {
-        auto set = [](const void* f) {
-            cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 kMaxDynSmem);
-            if (e != cudaSuccess) st = e;
-        };
-        set((const void*)k_fwd_col<Ar, SPLIT16, 4, true>);
-        set((const void*)k_fwd_col<Ar, SPLIT16, 4, false>);
-        set((const void*)k_inv_col<Ar, 4, true>);
-        set((const void*)k_inv_col<Ar, 4, false>);
-        set((const void*)k_row<Ar, 64, 4>);
-        set((const void*)k_row<Ar, 128, 4>);
-        set((const void*)k_row<Ar, 256, 4>);
-        set((const void*)k_row<Ar, 512, 4>);
-        set((const void*)k_row<Ar, 64, 3>);
-        set((const void*)k_row<Ar, 128, 3>);
-        set((const void*)k_row<Ar, 256, 3>);
-        set((const void*)k_row<Ar, 512, 3>);
-        if constexpr (sizeof(typename Ar::T) == 4) set((const void*)k_row<Ar, 256, 4, true>);
-        if constexpr (sizeof(typename Ar::T) == 4 && !SPLIT16) {
-            // 64-bit coefficients on the 32-bit path
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, false>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, false>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, true>);
-        }
-        set((const void*)k_mid_col<Ar, false>);
-        set((const void*)k_mid_col<Ar, true>);
-        set((const void*)k_inv_col_tma<Ar, 4>);
-        if constexpr (sizeof(typename Ar::T) == 8) {
-            set((const void*)k_fwd_col<Ar, SPLIT16, 3, true, false, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 3, false, false, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 3, true, true, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 3, false, true, true>);
-            set((const void*)k_inv_col<Ar, 3, true>);
-            set((const void*)k_inv_col<Ar, 3, false>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, false, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, false, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, true>);
-        }
-    });
-    if (st != cudaSuccess) return bw_fail(BW_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(st));
-    return BW_OK;
-}
-
-}  // namespace
-
 int bw_set_kernel_attrs() {
-    int rc = set_smem_attrs<Ar64, false>();
-    if (!rc) rc = set_smem_attrs<Ar32, true>();
+    int rc = bw_set_transform_attrs<Ar64, false>();
+    if (!rc) rc = bw_set_transform_attrs<Ar32, true>();
+    if (!rc) rc = bw_set_transform_attrs<Ar32, false>();
+    if (!rc) rc = bw_set_transform_attrs<ArD<0>, false>();
+    if (!rc) rc = bw_set_transform_attrs<ArD<1>, false>();
     return rc;
 }
 
 namespace {
-
-template <class Ar, int RLOG>
-void launch_row(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
-                const typename Ar::T* rb, int sq, size_t smem, cudaStream_t s) {
-    dim3 g(1u << (pl->log_r + pl->log_r2), pl->K);
-    // one thread per sub-problem of a round, 64..512 threads (radix-8 rounds,
-    // and radix-16 rounds on the 32-bit path: at most 256, each thread taking
-    // several sub-problems, so that the CTA's registers leave room for more
-    // than one CTA per SM; 2^13-point rows on the 32-bit path ran one 512-thread
-    // CTA per SM at 70 registers)
-    const int cap = (RLOG == 3 || sizeof(typename Ar::T) == 4) ? 256 : 512;
-    const int want = std::min(cap, std::max(64, 1 << (pl->log_c - RLOG)));
-    if constexpr (sizeof(typename Ar::T) == 4 && RLOG == 4) {
-        if (pl->shfl_rows && want == 256) {
-            k_row<Ar, 256, 4, true><<<g, 256, smem, s>>>(pd, ra, rb, sq);
-            return;
-        }
-    }
-    switch (want) {
-        case 512: k_row<Ar, 512, RLOG><<<g, 512, smem, s>>>(pd, ra, rb, sq); break;
-        case 256: k_row<Ar, 256, RLOG><<<g, 256, smem, s>>>(pd, ra, rb, sq); break;
-        case 128: k_row<Ar, 128, RLOG><<<g, 128, smem, s>>>(pd, ra, rb, sq); break;
-        default: k_row<Ar, 64, RLOG><<<g, 64, smem, s>>>(pd, ra, rb, sq); break;
-    }
-}
-
-// Stage order of one host-pointer product (bw_stage_order): begin(i, s)
-// makes stream s wait for stage i of the plan's previous product; end(i, s)
-// records this product's stage i on s.  Off with one live context.  A
-// previous product of the same context needs no wait: every stream of a
-// product starts behind the context stream, which ends behind all of the
-// previous product's work.
-struct StageOrder {
-    bw_stage_order* so = nullptr;
-    const bw_ctx* c = nullptr;
-    bool on = false;
-    cudaError_t begin(int i, cudaStream_t s) const {
-        if (!on || !so->last[i] || so->owner[i] == c) return cudaSuccess;
-        return cudaStreamWaitEvent(s, so->last[i], 0);
-    }
-    cudaError_t end(int i, cudaStream_t s) const {
-        if (!on) return cudaSuccess;
-        const cudaError_t e = cudaEventRecord(c->stage_ev[i], s);
-        so->last[i] = c->stage_ev[i];
-        so->owner[i] = c;
-        return e;
-    }
-};
-
-// Host operands of a product whose copy-in is split into `chunks` column
-// blocks: block k holds the words of forward-column tiles
-// [k T/chunks, (k+1) T/chunks) of every row, and K1 runs over those tiles
-// as soon as the block has landed.
-struct HostIO {
-    const uint32_t* ha = nullptr;
-    const uint32_t* hb = nullptr;  // nullptr when squaring
-    int chunks = 1;
-    const StageOrder* order = nullptr;
-};
-
-// Copy words [w0, w1) of every row (row length wc words) of an operand of lx
-// words: one 2D copy over the full rows, one plain copy of the partial last
-// row's part.  Nothing at or beyond lx is read or written.
-cudaError_t copy_cols(cudaStream_t s, uint32_t* dst, const uint32_t* src, size_t lx, size_t wc,
-                      size_t w0, size_t w1) {
-    const size_t full = lx / wc;
-    cudaError_t e = cudaSuccess;
-    if (full)
-        e = cudaMemcpy2DAsync(dst + w0, wc * 4, src + w0, wc * 4, (w1 - w0) * 4, full,
-                              cudaMemcpyHostToDevice, s);
-    const size_t lo = full * wc + w0, hi = std::min(lx, full * wc + w1);
-    if (e == cudaSuccess && hi > lo)
-        e = cudaMemcpyAsync(dst + lo, src + lo, (hi - lo) * 4, cudaMemcpyHostToDevice, s);
-    return e;
-}
 
 int ensure_copy_streams(bw_ctx* c) {
     if (c->in_stream) return BW_OK;
@@ -1120,161 +978,6 @@ int copy_chunks_for(const bw_ctx* c, bool ordered) {
     const int cpw = (pl->path == BW_PATH_P32 && !pl->w64) ? 2 : 1;
     if (S > 1 && ((tiles1 / S) << pl->log_cb1) % cpw) S = 1;
     return S;
-}
-
-// Enqueue K1..K3 (the transform part) for one product.  With io (chunks > 1)
-// the operands' copy-in runs on the context's copy stream in column blocks
-// and K1 runs block by block behind it.
-template <class Ar, bool SPLIT16, bool W64 = false>
-int enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool square,
-                      bool timing, const HostIO* io = nullptr) {
-    using T = typename Ar::T;
-    const bw_plan* pl = c->plan;
-    const PlanDev<Ar>& pd = plan_dev<Ar>(pl);
-    int rc = set_smem_attrs<Ar, SPLIT16>();
-    if (rc) return rc;
-    const int R = 1 << pl->log_r, C = 1 << pl->log_c, CB = 1 << pl->log_cb;
-    T* ra = reinterpret_cast<T*>(c->d_res_a);
-    T* rb = reinterpret_cast<T*>(c->d_res_b);
-    const bool ts = pl->tw_smem_r != 0;
-    const size_t tw_bytes = ts ? (size_t)R * sizeof(Tw<T>) : 0;
-
-    const int CB1 = 1 << pl->log_cb1;
-    // the 64-bit path stages the coefficients inside the residue tile and
-    // runs one prime per CTA (grid.x = tile * K + prime); so does the 32-bit
-    // path with 64-bit coefficients when asked (BW_PLAN_K1_ONE_PRIME); the
-    // 32-bit path keeps a u16 (16-bit) or u64 (64-bit coefficients) copy
-    constexpr bool PP = sizeof(T) == 8;
-    const bool pp32 = W64 && sizeof(T) == 4 && pl->k1_pp;
-    // (64-bit coefficients on the 32-bit path: the u64 copy holds the loaded
-    // rows only, half the tile when both operands fill at most half of it)
-    const size_t coef_rows = (W64 && sizeof(T) == 4 && pl->coef_half) ? (size_t)R / 2 : R;
-    const size_t smem1 = tw_bytes + tile_elems((size_t)R * CB1) * sizeof(T) +
-                         coef_rows * CB1 * ((PP || pp32) ? 0 : SPLIT16 ? 2 : W64 ? 8 : 4) +
-                         (W64 && sizeof(T) == 4 && !pp32 ? 16 : 0);
-    // K1 takes coefficient counts, or word counts for 64-bit coefficients
-    const size_t in_a = W64 ? pl->la : pl->nca, in_b = W64 ? pl->lb : pl->ncb;
-    const int cols_outer = 1 << (pl->log_c + pl->log_r2);
-    const int tiles1 = cols_outer / CB1;
-    const unsigned zt = (pl->zt_a ? 1u : 0u) | (pl->zt_b ? 2u : 0u);
-    auto k1 = [&](int tile0, int ntiles) {
-        dim3 g1(ntiles * ((PP || pp32) ? pl->K : 1), 1, square ? 1 : 2);
-        if constexpr (W64 && sizeof(T) == 4) {
-            if (pp32) {
-                if (ts) {
-                    k_fwd_col<Ar, SPLIT16, 4, true, true, true>
-                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
-                                                                tile0);
-                } else {
-                    k_fwd_col<Ar, SPLIT16, 4, false, true, true>
-                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
-                                                                tile0);
-                }
-                return;
-            }
-        }
-        if constexpr (PP) {
-            if (pl->rlog_col == 3) {
-                if (ts) {
-                    k_fwd_col<Ar, SPLIT16, 3, true, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
-                        pd, a, in_a, b, in_b, ra, rb, zt, tile0);
-                } else {
-                    k_fwd_col<Ar, SPLIT16, 3, false, W64, PP>
-                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
-                                                                tile0);
-                }
-                return;
-            }
-        }
-        if (ts) {
-            k_fwd_col<Ar, SPLIT16, 4, true, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
-                pd, a, in_a, b, in_b, ra, rb, zt, tile0);
-        } else {
-            k_fwd_col<Ar, SPLIT16, 4, false, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
-                pd, a, in_a, b, in_b, ra, rb, zt, tile0);
-        }
-    };
-    if (!io || io->chunks <= 1) {
-        k1(0, tiles1);
-    } else {
-        // the copy stream starts where the context stream is (the previous
-        // product has read the staging buffer); block k: copy, event, K1
-        // words per row of coefficients: cols / 2 (16-bit), cols (32-bit),
-        // 2 cols (64-bit coefficients)
-        const int S = io->chunks, per = tiles1 / S, cpw = SPLIT16 ? 2 : 1;
-        const size_t wpc = W64 ? 2 : 1;
-        const size_t wc = (size_t)cols_outer * wpc / cpw;
-        uint32_t* da = const_cast<uint32_t*>(a);
-        uint32_t* db = const_cast<uint32_t*>(b);
-        BW_CUDA(cudaEventRecord(c->ready_ev, c->stream));
-        BW_CUDA(cudaStreamWaitEvent(c->in_stream, c->ready_ev, 0));
-        BW_CUDA(io->order->begin(0, c->in_stream));
-        BW_CUDA(io->order->begin(1, c->stream));
-        for (int k = 0; k < S; ++k) {
-            const size_t w0 = ((size_t)k * per << pl->log_cb1) * wpc / cpw;
-            const size_t w1 = ((size_t)(k + 1) * per << pl->log_cb1) * wpc / cpw;
-            BW_CUDA(copy_cols(c->in_stream, da, io->ha, pl->la, wc, w0, w1));
-            if (!square) BW_CUDA(copy_cols(c->in_stream, db, io->hb, pl->lb, wc, w0, w1));
-            BW_CUDA(cudaEventRecord(c->in_ev[k], c->in_stream));
-            if (k == S - 1) BW_CUDA(io->order->end(0, c->in_stream));
-            BW_CUDA(cudaStreamWaitEvent(c->stream, c->in_ev[k], 0));
-            k1(k * per, per);
-        }
-    }
-    // three passes: middle column pass with the outer twiddle
-    const int CB2 = 1 << pl->log_cb2;
-    const size_t smem_mid = (((size_t)1 << pl->log_r2) + CB2) * sizeof(Tw<T>) +
-                            tile_elems((size_t)CB2 << pl->log_r2) * sizeof(T);
-    if (pl->log_r2) {
-        dim3 gm(C / CB2, R, pl->K * (square ? 1 : 2));
-        k_mid_col<Ar, false><<<gm, kColThreads, smem_mid, c->stream>>>(pd, ra, rb);
-    }
-    if (timing) cudaEventRecord(c->ev[2], c->stream);
-
-    const int la = pl->log_c / 2;
-    const size_t ntab = 2 * (((size_t)1 << la) + ((size_t)C >> la));
-    const size_t smem2 = ntab * sizeof(Tw<T>) + tile_elems(C) * sizeof(T) * (square ? 1 : 2);
-    const T* rbs = square ? ra : rb;
-    const int sq = square ? 1 : 0;
-    if (pl->rlog_row == 3) {
-        launch_row<Ar, 3>(pl, pd, ra, rbs, sq, smem2, c->stream);
-    } else {
-        launch_row<Ar, 4>(pl, pd, ra, rbs, sq, smem2, c->stream);
-    }
-    if (timing) cudaEventRecord(c->ev[3], c->stream);
-
-    if (pl->log_r2) {
-        dim3 gm(C / CB2, R, pl->K);
-        k_mid_col<Ar, true><<<gm, kColThreads, smem_mid, c->stream>>>(pd, ra, ra);
-    }
-    const size_t smem3 = tw_bytes + tile_elems((size_t)R * CB) * sizeof(T);
-    dim3 g3(cols_outer / CB, pl->K);
-    bool inv_done = false;
-    if (pl->tma_cols) {
-        k_inv_col_tma<Ar, 4><<<g3, kColThreads, (size_t)R * CB * sizeof(T) + 128, c->stream>>>(
-            pd, ra, c->cst, c->tmap_res, c->err, c->spin_limit);
-        inv_done = true;
-    }
-    if constexpr (PP) {
-        if (!inv_done && pl->rlog_col == 3) {
-            if (ts) {
-                k_inv_col<Ar, 3, true><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
-            } else {
-                k_inv_col<Ar, 3, false><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
-            }
-            inv_done = true;
-        }
-    }
-    if (!inv_done) {
-        if (ts) {
-            k_inv_col<Ar, 4, true><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
-        } else {
-            k_inv_col<Ar, 4, false><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
-        }
-    }
-    if (timing) cudaEventRecord(c->ev[4], c->stream);
-    BW_CUDA(cudaGetLastError());
-    return BW_OK;
 }
 
 template <class Ar, bool SPLIT16, bool W64 = false>
@@ -1336,16 +1039,19 @@ int enqueue_product(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_t* o
     const int pieces = io ? io->chunks : 1;
     int rc;
     if (pl->w64 && pl->path == BW_PATH_P32) {
-        rc = enqueue_transform<Ar32, false, true>(c, a, b, square, timing, io);
+        rc = bw_enqueue_transform<Ar32, false, true>(c, a, b, square, timing, io);
         if (!rc) rc = enqueue_carry<Ar32, false, true>(c, out, pieces);
     } else if (pl->w64) {
-        rc = enqueue_transform<Ar64, false, true>(c, a, b, square, timing, io);
+        rc = pl->f64 == 1 ? bw_enqueue_transform<ArD<0>, false, true>(c, a, b, square, timing, io)
+             : pl->f64 == 2
+                 ? bw_enqueue_transform<ArD<1>, false, true>(c, a, b, square, timing, io)
+                 : bw_enqueue_transform<Ar64, false, true>(c, a, b, square, timing, io);
         if (!rc) rc = enqueue_carry<Ar64, false, true>(c, out, pieces);
     } else if (pl->path == BW_PATH_P64) {
-        rc = enqueue_transform<Ar64, false>(c, a, b, square, timing, io);
+        rc = bw_enqueue_transform<Ar64, false>(c, a, b, square, timing, io);
         if (!rc) rc = enqueue_carry<Ar64, false>(c, out, pieces);
     } else {
-        rc = enqueue_transform<Ar32, true>(c, a, b, square, timing, io);
+        rc = bw_enqueue_transform<Ar32, true>(c, a, b, square, timing, io);
         if (!rc) rc = enqueue_carry<Ar32, true>(c, out, pieces);
     }
     return rc;
@@ -1561,12 +1267,12 @@ extern "C" int bw_multiply_coeffs(bw_ctx* c, const uint32_t* a, size_t la, const
     if (!sq) cudaMemcpyAsync(c->d_in + la, b, lb * 4, cudaMemcpyHostToDevice, c->stream);
     const uint32_t* db = sq ? c->d_in : c->d_in + la;
     if (pl->path == BW_PATH_P64) {
-        rc = enqueue_transform<Ar64, false>(c, c->d_in, db, sq, false);
+        rc = bw_enqueue_transform<Ar64, false>(c, c->d_in, db, sq, false);
         if (!rc)
             k_garner_dump<Ar64, false><<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
                 pl->pd64, reinterpret_cast<const uint64_t*>(c->d_res_a), d_words, n);
     } else {
-        rc = enqueue_transform<Ar32, true>(c, c->d_in, db, sq, false);
+        rc = bw_enqueue_transform<Ar32, true>(c, c->d_in, db, sq, false);
         if (!rc)
             k_garner_dump<Ar32, true><<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
                 pl->pd32, reinterpret_cast<const uint32_t*>(c->d_res_a), d_words, n);

@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <mutex>
 
+#include "bw_host.h"
+
 #include "bw_kernels.cuh"
 
 // Stage order of the host-pointer products of one plan.  Contexts of one
@@ -43,6 +45,12 @@ struct bw_plan {
     size_t table_bytes = 0;
     bw::PlanDev<bw::Ar32> pd32{};
     bw::PlanDev<bw::Ar64> pd64{};
+    // double-precision transforms (64-bit path, 64-bit coefficients): 0 off,
+    // 1 primes just above 2^50, 2 primes just above 2^51.66 (pd64 then holds
+    // the Garner constants of the same primes)
+    int f64 = 0;
+    bw::PlanDev<bw::ArD<0>> pdd0{};
+    bw::PlanDev<bw::ArD<1>> pdd1{};
     uint64_t primes[bw::kMaxPrimes] = {};
     bw_stage_order* order = nullptr;  // plans of bw_plan_create only
 };
@@ -88,3 +96,125 @@ size_t bw_group_state_stride(size_t ntiles);
 void bw_tune_lookup(int path, int K, int log_n, int* small, int* log_cols);
 // Point a descriptor's look-back fields into its state block.
 void bw_group_fill_state(bw::BatchProd& d, unsigned char* state, size_t ntiles);
+
+// Most chunks a host copy is split into (see bw_ctx::copy_chunks).
+constexpr int kMaxCopyChunks = 16;
+
+struct bw_ctx {
+    const bw_plan* plan = nullptr;
+    cudaStream_t stream = nullptr;
+    bool own_stream = false;
+    void* d_res_a = nullptr;
+    void* d_res_b = nullptr;
+    uint32_t* d_in = nullptr;   // staging: a then b
+    uint32_t* d_out = nullptr;  // staging: product
+    unsigned char* d_state = nullptr;
+    size_t state_bytes = 0;
+    bw::CarryState* cst = nullptr;
+    uint32_t* err = nullptr;
+    uint4* rec_x = nullptr;
+    uint32_t* rec_s = nullptr;
+    size_t ntiles = 0;
+    // look-back record tag of the last product.  Direct launches use 2, 3, ..;
+    // the replayable graph clears the records and always uses 1.
+    uint32_t epoch = 1;
+    bool capturing = false;
+    cudaGraphExec_t gexec = nullptr;  // device-pointer product, replayed while
+    const void* g_a = nullptr;        // the pointers stay the same
+    const void* g_b = nullptr;
+    const void* g_out = nullptr;
+    bool g_sq = false;
+    uint32_t* h_err = nullptr;  // pinned
+    cudaEvent_t ev[8] = {};
+    cudaEvent_t stage_ev[3] = {};  // ends of copy-in, kernels, copy-out (stage order)
+    bool counted = false;          // included in the plan's live contexts
+    // host copies split into chunks that overlap the first and last kernels
+    // (created on first use): copy-in on in_stream, copy-out on out_stream
+    int copy_chunks = 0;           // 0: automatic, 1: whole copies on the stream
+    cudaStream_t in_stream = nullptr, out_stream = nullptr;
+    cudaEvent_t in_ev[kMaxCopyChunks] = {}, out_ev[kMaxCopyChunks] = {};
+    cudaEvent_t ready_ev = nullptr, out_done_ev = nullptr;
+    int out_pieces = 0;            // K4 launches of the last chunked product
+    size_t out_tiles_per = 0;      // carry tiles per K4 launch
+    int spin_limit = 1 << 22;
+    bool inject_wait_fault = false;
+    CUtensorMap tmap_res;          // residues of A as [prime][row][column] (tma_cols)
+};
+
+// Stage order of one host-pointer product (bw_stage_order): begin(i, s)
+// makes stream s wait for stage i of the plan's previous product; end(i, s)
+// records this product's stage i on s.  Off with one live context.  A
+// previous product of the same context needs no wait: every stream of a
+// product starts behind the context stream, which ends behind all of the
+// previous product's work.
+struct StageOrder {
+    bw_stage_order* so = nullptr;
+    const bw_ctx* c = nullptr;
+    bool on = false;
+    cudaError_t begin(int i, cudaStream_t s) const {
+        if (!on || !so->last[i] || so->owner[i] == c) return cudaSuccess;
+        return cudaStreamWaitEvent(s, so->last[i], 0);
+    }
+    cudaError_t end(int i, cudaStream_t s) const {
+        if (!on) return cudaSuccess;
+        const cudaError_t e = cudaEventRecord(c->stage_ev[i], s);
+        so->last[i] = c->stage_ev[i];
+        so->owner[i] = c;
+        return e;
+    }
+};
+
+// Host operands of a product whose copy-in is split into `chunks` column
+// blocks: block k holds the words of forward-column tiles
+// [k T/chunks, (k+1) T/chunks) of every row, and K1 runs over those tiles
+// as soon as the block has landed.
+struct HostIO {
+    const uint32_t* ha = nullptr;
+    const uint32_t* hb = nullptr;  // nullptr when squaring
+    int chunks = 1;
+    const StageOrder* order = nullptr;
+};
+
+// Return a failed CUDA call's status from a function that returns one.
+#define BW_CUDA(call)                                                                   \
+    do {                                                                                \
+        cudaError_t e_ = (call);                                                        \
+        if (e_ != cudaSuccess) {                                                        \
+            return bw_fail(e_ == cudaErrorMemoryAllocation ? BW_ENOMEM : BW_ECUDA,      \
+                           "%s failed: %s", #call, cudaGetErrorString(e_));             \
+        }                                                                               \
+    } while (0)
+
+namespace bw {
+
+// A plan's device view in one arithmetic.
+template <class Ar>
+const PlanDev<Ar>& plan_dev(const bw_plan* pl);
+template <>
+inline const PlanDev<Ar32>& plan_dev<Ar32>(const bw_plan* pl) {
+    return pl->pd32;
+}
+template <>
+inline const PlanDev<Ar64>& plan_dev<Ar64>(const bw_plan* pl) {
+    return pl->pd64;
+}
+template <>
+inline const PlanDev<ArD<0>>& plan_dev<ArD<0>>(const bw_plan* pl) {
+    return pl->pdd0;
+}
+template <>
+inline const PlanDev<ArD<1>>& plan_dev<ArD<1>>(const bw_plan* pl) {
+    return pl->pdd1;
+}
+
+// Enqueue K1..K3 (the transform part) for one product.  With io (chunks > 1)
+// the operands' copy-in runs on the context's copy stream in column blocks
+// and K1 runs block by block behind it.
+template <class Ar, bool SPLIT16, bool W64 = false>
+int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool square,
+                         bool timing, const HostIO* io = nullptr);
+// Set the dynamic shared-memory limit of one arithmetic's kernels (once).
+template <class Ar, bool SPLIT16>
+int bw_set_transform_attrs();
+
+}  // namespace bw

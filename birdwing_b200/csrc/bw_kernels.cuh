@@ -82,6 +82,9 @@ struct GarnerDev {
     T inv2, inv2q;      // (p0 p1)^-1 mod p2
     uint64_t p0;        // p0 as an integer
     uint64_t p01_lo, p01_hi;  // p0 p1 as a 128-bit integer (64-bit coefficients)
+    // 64-bit coefficients: a product's coefficients stay below this times
+    // 2^128 (min(na, nb)); one that reaches it flags an error
+    uint64_t top_bound;
     // six primes (32-bit path, 64-bit coefficients): p_j^-1 mod p_i with
     // Shoup companions, pair (i, j < i) at index i (i - 1) / 2 + j
     Tw<T> inv6[15];
@@ -249,6 +252,7 @@ __device__ __forceinline__ void ct_stages(typename Ar::T* x, int s0, int g,
 #pragma unroll
     for (int l = 0; l < RL; ++l) {
         const int h = 1 << (RL - l - 1);
+        if constexpr (Ar::kF64) ar.template ct_enter<RL>(x, l, s0);
         if (l == 0 && s0 == 0) {
             if (zt) {
 #pragma unroll
@@ -329,7 +333,15 @@ __device__ __forceinline__ void gs_stages(typename Ar::T* x, int s0, int g,
 #pragma unroll
             for (int u = 0; u < h; ++u) {
                 const int k = (q << (RL - l)) + u;
-                ar.gs(x[k], x[k + h], w.w, w.wq);
+                if constexpr (Ar::kF64) {
+                    if (l == 0 || ((RL - 1 - l) & 1)) {
+                        ar.template gs<true>(x[k], x[k + h], w.w, w.wq);
+                    } else {
+                        ar.template gs<false>(x[k], x[k + h], w.w, w.wq);
+                    }
+                } else {
+                    ar.gs(x[k], x[k + h], w.w, w.wq);
+                }
             }
         }
     }
@@ -622,8 +634,16 @@ __device__ __forceinline__ void fwd_col_body(const PlanDev<Ar>& P,
                             return ar.reduce64(coef[(idx << log_cb) + v]);
                         }
                     } else {
+                        if constexpr (Ar::kF64) {
+                            // the staged coefficient's bits as a residue
+                            if constexpr (PP && W64) {
+                                return ar.from_u64((uint64_t)__double_as_longlong(buf[p]));
+                            } else {
+                                return ar.from_u32((uint32_t)coef[(idx << log_cb) + v]);
+                            }
+                        }
                         T x = PP ? buf[p] : (T)coef[(idx << log_cb) + v];
-                        if constexpr (W64) {
+                        if constexpr (W64 && !Ar::kF64) {
                             // a 64-bit coefficient (up to 64p) enters reduced
                             // to [0, 2p), leaving the transform its headroom
                             x = ar.reduce_in(x);
@@ -1294,8 +1314,8 @@ __device__ __forceinline__ void garner_digits(const PlanDev<Ar>& P,
 // 64-bit coefficients (three primes): the E output words from word j0 (j0
 // even, E/2 coefficients from coefficient j0/2) and the carry-out X.  Each
 // coefficient is the full mixed-radix value c = r0 + p0 k1 + p0 p1 k2
-// (< p0 p1 p2 < 2^186; the coefficients of a product stay below
-// min(na, nb) 2^128 < 2^160, so c2 >= 2^32 flags an error).  The words are
+// (< p0 p1 p2; the coefficients of a product stay below min(na, nb) 2^128, so a
+// c2 at or above G.top_bound = min(na, nb) flags an error).  The words are
 // the low 32 E bits of V = sum_q c_q 2^(64 q), X = V >> 32 E (< 2^96).
 // Coefficients at or beyond NL / 2 read nothing and are zero.
 template <class Ar, int E, bool NC>
@@ -1344,7 +1364,7 @@ __device__ __forceinline__ void garner3_words_at(const PlanDev<Ar>& P,
             (unsigned __int128)G.p0 * k1 + r0 + (unsigned __int128)G.p01_lo * k2;  // < 2^127
         const unsigned __int128 hi = (lo >> 64) + (unsigned __int128)G.p01_hi * k2;
         const uint64_t c0 = (uint64_t)lo, c1 = (uint64_t)hi, c2 = (uint64_t)(hi >> 64);
-        bad |= (uint32_t)((c2 >> 32) != 0);
+        bad |= (uint32_t)(c2 >= G.top_bound);
         // add c to the running carry; emit 64 bits; shift
         const unsigned __int128 s0 = (unsigned __int128)acc0 + c0;
         l[2 * q] = (uint32_t)s0;
@@ -1366,8 +1386,8 @@ __device__ __forceinline__ void garner3_words_at(const PlanDev<Ar>& P,
 // k_i = (...((r_i - k_0) p_0^-1 - k_1) p_1^-1 ... - k_(i-1)) p_(i-1)^-1 mod p_i;
 // c = k_0 + p_0 (k_1 + p_1 (k_2 + p_2 (k_3 + p_3 (k_4 + p_4 k_5)))) < P < 2^178.
 // A product's coefficients stay below min(na, nb) 2^128 <= 2^150, so a top
-// word c2 >= 2^32 flags an error (residues that disagree give a c spread over
-// [0, P)).
+// word c2 at or above G.top_bound = min(na, nb) flags an error (residues that
+// disagree give a c spread over [0, P)).
 template <class Ar, int E, bool NC>
 __device__ __forceinline__ void garner6_words_at(const PlanDev<Ar>& P,
                                                  const uint32_t* __restrict__ base,
@@ -1438,7 +1458,7 @@ __device__ __forceinline__ void garner6_words_at(const PlanDev<Ar>& P,
         const uint64_t c0 = ((uint64_t)w[1] << 32) | w[0];
         const uint64_t c1 = ((uint64_t)w[3] << 32) | w[2];
         const uint64_t c2 = ((uint64_t)w[5] << 32) | w[4];
-        bad |= (uint32_t)((c2 >> 32) != 0);
+        bad |= (uint32_t)(c2 >= G.top_bound);
         const unsigned __int128 s0 = (unsigned __int128)acc0 + c0;
         l[2 * q] = (uint32_t)s0;
         l[2 * q + 1] = (uint32_t)((uint64_t)s0 >> 32);
@@ -1977,7 +1997,7 @@ __device__ __forceinline__ void ks_product_body(const PlanDev<Ar>& P, const Batc
         if constexpr (SPLIT16) {
             return (T)((__ldg(src + (i >> 1)) >> ((i & 1) * 16)) & 0xFFFFu);
         } else {
-            return (T)__ldg(src + i);
+            return Ar::from_u32(__ldg(src + i));
         }
     };
     auto ldA = [&](int, int, int p) -> T { return bufA[p]; };
@@ -1987,7 +2007,7 @@ __device__ __forceinline__ void ks_product_body(const PlanDev<Ar>& P, const Batc
         const Ar ar = pr.ar;
         const Tw<T> sc = pr.scale;
         auto st_res = [&](int idx, T v) {
-            res[(size_t)kp * n + idx] = ar.red1(ar.shoup(v, sc.w, sc.wq));
+            res[(size_t)kp * n + idx] = ar.scale_out(v, sc.w, sc.wq);
         };
         for (int i = threadIdx.x; i < n; i += NT) {
             bufA[LayRow::p(i)] = coef(d.a, nca, i);

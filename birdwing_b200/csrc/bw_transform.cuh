@@ -1,0 +1,270 @@
+// bw_transform.cuh -- launches of the transform kernels (K1..K3) of one
+// arithmetic, instantiated by one translation unit each (bw_tr_*.cu) so that
+// they compile side by side.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "../../include/birdwing.h"
+#include "bw_host.h"
+#include "bw_internal.h"
+#include "bw_kernels.cuh"
+
+namespace bw {
+
+constexpr int kMaxDynSmem = 200 * 1024;
+
+template <class Ar, bool SPLIT16>
+int bw_set_transform_attrs() {
+    static std::once_flag once;
+    static cudaError_t st = cudaSuccess;
+    std::call_once(once, [] {
+        auto set = [](const void* f) {
+            cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 kMaxDynSmem);
+            if (e != cudaSuccess) st = e;
+        };
+        if constexpr (!Ar::kF64) {
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false>);
+        }
+        set((const void*)k_inv_col<Ar, 4, true>);
+        set((const void*)k_inv_col<Ar, 4, false>);
+        set((const void*)k_row<Ar, 64, 4>);
+        set((const void*)k_row<Ar, 128, 4>);
+        set((const void*)k_row<Ar, 256, 4>);
+        set((const void*)k_row<Ar, 512, 4>);
+        set((const void*)k_row<Ar, 64, 3>);
+        set((const void*)k_row<Ar, 128, 3>);
+        set((const void*)k_row<Ar, 256, 3>);
+        set((const void*)k_row<Ar, 512, 3>);
+        if constexpr (sizeof(typename Ar::T) == 4) set((const void*)k_row<Ar, 256, 4, true>);
+        if constexpr (sizeof(typename Ar::T) == 4 && !SPLIT16) {
+            // 64-bit coefficients on the 32-bit path
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, false>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, false>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, true>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, true>);
+        }
+        set((const void*)k_mid_col<Ar, false>);
+        set((const void*)k_mid_col<Ar, true>);
+        set((const void*)k_inv_col_tma<Ar, 4>);
+        if constexpr (sizeof(typename Ar::T) == 8) {
+            if constexpr (!Ar::kF64) {
+                set((const void*)k_fwd_col<Ar, SPLIT16, 3, true, false, true>);
+                set((const void*)k_fwd_col<Ar, SPLIT16, 3, false, false, true>);
+                set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, false, true>);
+                set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, false, true>);
+            }
+            set((const void*)k_fwd_col<Ar, SPLIT16, 3, true, true, true>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 3, false, true, true>);
+            set((const void*)k_inv_col<Ar, 3, true>);
+            set((const void*)k_inv_col<Ar, 3, false>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, true>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, true>);
+        }
+    });
+    if (st != cudaSuccess) return bw_fail(BW_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(st));
+    return BW_OK;
+}
+
+
+template <class Ar, int RLOG>
+void launch_row(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
+                const typename Ar::T* rb, int sq, size_t smem, cudaStream_t s) {
+    dim3 g(1u << (pl->log_r + pl->log_r2), pl->K);
+    // one thread per sub-problem of a round, 64..512 threads (radix-8 rounds,
+    // and radix-16 rounds on the 32-bit path: at most 256, each thread taking
+    // several sub-problems, so that the CTA's registers leave room for more
+    // than one CTA per SM; 2^13-point rows on the 32-bit path ran one 512-thread
+    // CTA per SM at 70 registers)
+    const int cap = (RLOG == 3 || sizeof(typename Ar::T) == 4) ? 256 : 512;
+    const int want = std::min(cap, std::max(64, 1 << (pl->log_c - RLOG)));
+    if constexpr (sizeof(typename Ar::T) == 4 && RLOG == 4) {
+        if (pl->shfl_rows && want == 256) {
+            k_row<Ar, 256, 4, true><<<g, 256, smem, s>>>(pd, ra, rb, sq);
+            return;
+        }
+    }
+    switch (want) {
+        case 512: k_row<Ar, 512, RLOG><<<g, 512, smem, s>>>(pd, ra, rb, sq); break;
+        case 256: k_row<Ar, 256, RLOG><<<g, 256, smem, s>>>(pd, ra, rb, sq); break;
+        case 128: k_row<Ar, 128, RLOG><<<g, 128, smem, s>>>(pd, ra, rb, sq); break;
+        default: k_row<Ar, 64, RLOG><<<g, 64, smem, s>>>(pd, ra, rb, sq); break;
+    }
+}
+
+// Copy words [w0, w1) of every row (row length wc words) of an operand of lx
+// words: one 2D copy over the full rows, one plain copy of the partial last
+// row's part.  Nothing at or beyond lx is read or written.
+inline cudaError_t copy_cols(cudaStream_t s, uint32_t* dst, const uint32_t* src, size_t lx, size_t wc,
+                      size_t w0, size_t w1) {
+    const size_t full = lx / wc;
+    cudaError_t e = cudaSuccess;
+    if (full)
+        e = cudaMemcpy2DAsync(dst + w0, wc * 4, src + w0, wc * 4, (w1 - w0) * 4, full,
+                              cudaMemcpyHostToDevice, s);
+    const size_t lo = full * wc + w0, hi = std::min(lx, full * wc + w1);
+    if (e == cudaSuccess && hi > lo)
+        e = cudaMemcpyAsync(dst + lo, src + lo, (hi - lo) * 4, cudaMemcpyHostToDevice, s);
+    return e;
+}
+
+// Enqueue K1..K3 (the transform part) for one product.  With io (chunks > 1)
+// the operands' copy-in runs on the context's copy stream in column blocks
+// and K1 runs block by block behind it.
+template <class Ar, bool SPLIT16, bool W64>
+int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool square,
+                      bool timing, const HostIO* io) {
+    using T = typename Ar::T;
+    const bw_plan* pl = c->plan;
+    const PlanDev<Ar>& pd = plan_dev<Ar>(pl);
+    int rc = bw_set_transform_attrs<Ar, SPLIT16>();
+    if (rc) return rc;
+    const int R = 1 << pl->log_r, C = 1 << pl->log_c, CB = 1 << pl->log_cb;
+    T* ra = reinterpret_cast<T*>(c->d_res_a);
+    T* rb = reinterpret_cast<T*>(c->d_res_b);
+    const bool ts = pl->tw_smem_r != 0;
+    const size_t tw_bytes = ts ? (size_t)R * sizeof(Tw<T>) : 0;
+
+    const int CB1 = 1 << pl->log_cb1;
+    // the 64-bit path stages the coefficients inside the residue tile and
+    // runs one prime per CTA (grid.x = tile * K + prime); so does the 32-bit
+    // path with 64-bit coefficients when asked (BW_PLAN_K1_ONE_PRIME); the
+    // 32-bit path keeps a u16 (16-bit) or u64 (64-bit coefficients) copy
+    constexpr bool PP = sizeof(T) == 8;
+    const bool pp32 = W64 && sizeof(T) == 4 && pl->k1_pp;
+    // (64-bit coefficients on the 32-bit path: the u64 copy holds the loaded
+    // rows only, half the tile when both operands fill at most half of it)
+    const size_t coef_rows = (W64 && sizeof(T) == 4 && pl->coef_half) ? (size_t)R / 2 : R;
+    const size_t smem1 = tw_bytes + tile_elems((size_t)R * CB1) * sizeof(T) +
+                         coef_rows * CB1 * ((PP || pp32) ? 0 : SPLIT16 ? 2 : W64 ? 8 : 4) +
+                         (W64 && sizeof(T) == 4 && !pp32 ? 16 : 0);
+    // K1 takes coefficient counts, or word counts for 64-bit coefficients
+    const size_t in_a = W64 ? pl->la : pl->nca, in_b = W64 ? pl->lb : pl->ncb;
+    const int cols_outer = 1 << (pl->log_c + pl->log_r2);
+    const int tiles1 = cols_outer / CB1;
+    const unsigned zt = (pl->zt_a ? 1u : 0u) | (pl->zt_b ? 2u : 0u);
+    auto k1 = [&](int tile0, int ntiles) {
+        dim3 g1(ntiles * ((PP || pp32) ? pl->K : 1), 1, square ? 1 : 2);
+        if constexpr (W64 && sizeof(T) == 4) {
+            if (pp32) {
+                if (ts) {
+                    k_fwd_col<Ar, SPLIT16, 4, true, true, true>
+                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
+                                                                tile0);
+                } else {
+                    k_fwd_col<Ar, SPLIT16, 4, false, true, true>
+                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
+                                                                tile0);
+                }
+                return;
+            }
+        }
+        if constexpr (PP) {
+            if (pl->rlog_col == 3) {
+                if (ts) {
+                    k_fwd_col<Ar, SPLIT16, 3, true, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
+                        pd, a, in_a, b, in_b, ra, rb, zt, tile0);
+                } else {
+                    k_fwd_col<Ar, SPLIT16, 3, false, W64, PP>
+                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
+                                                                tile0);
+                }
+                return;
+            }
+        }
+        if (ts) {
+            k_fwd_col<Ar, SPLIT16, 4, true, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
+                pd, a, in_a, b, in_b, ra, rb, zt, tile0);
+        } else {
+            k_fwd_col<Ar, SPLIT16, 4, false, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
+                pd, a, in_a, b, in_b, ra, rb, zt, tile0);
+        }
+    };
+    if (!io || io->chunks <= 1) {
+        k1(0, tiles1);
+    } else {
+        // the copy stream starts where the context stream is (the previous
+        // product has read the staging buffer); block k: copy, event, K1
+        // words per row of coefficients: cols / 2 (16-bit), cols (32-bit),
+        // 2 cols (64-bit coefficients)
+        const int S = io->chunks, per = tiles1 / S, cpw = SPLIT16 ? 2 : 1;
+        const size_t wpc = W64 ? 2 : 1;
+        const size_t wc = (size_t)cols_outer * wpc / cpw;
+        uint32_t* da = const_cast<uint32_t*>(a);
+        uint32_t* db = const_cast<uint32_t*>(b);
+        BW_CUDA(cudaEventRecord(c->ready_ev, c->stream));
+        BW_CUDA(cudaStreamWaitEvent(c->in_stream, c->ready_ev, 0));
+        BW_CUDA(io->order->begin(0, c->in_stream));
+        BW_CUDA(io->order->begin(1, c->stream));
+        for (int k = 0; k < S; ++k) {
+            const size_t w0 = ((size_t)k * per << pl->log_cb1) * wpc / cpw;
+            const size_t w1 = ((size_t)(k + 1) * per << pl->log_cb1) * wpc / cpw;
+            BW_CUDA(copy_cols(c->in_stream, da, io->ha, pl->la, wc, w0, w1));
+            if (!square) BW_CUDA(copy_cols(c->in_stream, db, io->hb, pl->lb, wc, w0, w1));
+            BW_CUDA(cudaEventRecord(c->in_ev[k], c->in_stream));
+            if (k == S - 1) BW_CUDA(io->order->end(0, c->in_stream));
+            BW_CUDA(cudaStreamWaitEvent(c->stream, c->in_ev[k], 0));
+            k1(k * per, per);
+        }
+    }
+    // three passes: middle column pass with the outer twiddle
+    const int CB2 = 1 << pl->log_cb2;
+    const size_t smem_mid = (((size_t)1 << pl->log_r2) + CB2) * sizeof(Tw<T>) +
+                            tile_elems((size_t)CB2 << pl->log_r2) * sizeof(T);
+    if (pl->log_r2) {
+        dim3 gm(C / CB2, R, pl->K * (square ? 1 : 2));
+        k_mid_col<Ar, false><<<gm, kColThreads, smem_mid, c->stream>>>(pd, ra, rb);
+    }
+    if (timing) cudaEventRecord(c->ev[2], c->stream);
+
+    const int la = pl->log_c / 2;
+    const size_t ntab = 2 * (((size_t)1 << la) + ((size_t)C >> la));
+    const size_t smem2 = ntab * sizeof(Tw<T>) + tile_elems(C) * sizeof(T) * (square ? 1 : 2);
+    const T* rbs = square ? ra : rb;
+    const int sq = square ? 1 : 0;
+    if (pl->rlog_row == 3) {
+        launch_row<Ar, 3>(pl, pd, ra, rbs, sq, smem2, c->stream);
+    } else {
+        launch_row<Ar, 4>(pl, pd, ra, rbs, sq, smem2, c->stream);
+    }
+    if (timing) cudaEventRecord(c->ev[3], c->stream);
+
+    if (pl->log_r2) {
+        dim3 gm(C / CB2, R, pl->K);
+        k_mid_col<Ar, true><<<gm, kColThreads, smem_mid, c->stream>>>(pd, ra, ra);
+    }
+    const size_t smem3 = tw_bytes + tile_elems((size_t)R * CB) * sizeof(T);
+    dim3 g3(cols_outer / CB, pl->K);
+    bool inv_done = false;
+    if (pl->tma_cols) {
+        k_inv_col_tma<Ar, 4><<<g3, kColThreads, (size_t)R * CB * sizeof(T) + 128, c->stream>>>(
+            pd, ra, c->cst, c->tmap_res, c->err, c->spin_limit);
+        inv_done = true;
+    }
+    if constexpr (PP) {
+        if (!inv_done && pl->rlog_col == 3) {
+            if (ts) {
+                k_inv_col<Ar, 3, true><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
+            } else {
+                k_inv_col<Ar, 3, false><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
+            }
+            inv_done = true;
+        }
+    }
+    if (!inv_done) {
+        if (ts) {
+            k_inv_col<Ar, 4, true><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
+        } else {
+            k_inv_col<Ar, 4, false><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
+        }
+    }
+    if (timing) cudaEventRecord(c->ev[4], c->stream);
+    BW_CUDA(cudaGetLastError());
+    return BW_OK;
+}
+
+}  // namespace bw

@@ -15,7 +15,10 @@
  *                 arithmetic (the reference's LIMB_BITS=32 pipeline, whose
  *                 transform length is twice the limb count).
  *   BW_PATH_P64 : 32-bit coefficients, 58-bit primes of the form c*2^32+1,
- *                 64-bit modular arithmetic (the reference's LIMB_BITS=64
+ *                 64-bit modular arithmetic; with 64-bit coefficients
+ *                 (BW_PLAN_COEF64) primes of 50 to 52 bits in exact
+ *                 double-precision modular arithmetic (58-bit ones when the
+ *                 shorter operand has more than 2^28 words) (the reference's LIMB_BITS=64
  *                 "hybrid" and NATIVE_HOST_LIMBS pipelines; a u64 limb array
  *                 is passed as twice as many u32 words).
  *
