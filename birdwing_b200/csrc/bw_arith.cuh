@@ -26,6 +26,12 @@ struct alignas(2 * sizeof(T)) Tw {
     T w;
     T wq;
 };
+// double precision: the quotient comes from the rounded product (ArD), so an
+// entry is the constant alone and two fit in a 16-byte load
+template <>
+struct Tw<double> {
+    double w;
+};
 
 struct Ar32 {
     using T = uint32_t;
@@ -53,18 +59,18 @@ struct Ar32 {
         return (uint32_t)((t + (uint64_t)m * p) >> 32);
     }
     // forward CT butterfly, inputs/outputs in [0, 4p)
-    __device__ __forceinline__ void ct(T& a, T& b, T w, T wq) const {
+    __device__ __forceinline__ void ct(T& a, T& b, const Tw<T>& w) const {
         const T x = red2(a);
-        const T t = shoup(b, w, wq);
+        const T t = shoup(b, w.w, w.wq);
         a = x + t;
         b = x - t + p2;
     }
     // inverse GS butterfly, inputs/outputs in [0, 2p)
-    __device__ __forceinline__ void gs(T& a, T& b, T w, T wq) const {
+    __device__ __forceinline__ void gs(T& a, T& b, const Tw<T>& w) const {
         const T u = a + b;
         const T v = a - b + p2;
         a = red2(u);
-        b = shoup(v, w, wq);
+        b = shoup(v, w.w, w.wq);
     }
     // twiddle-1 butterflies of stage 0 (inputs known to be in [0, 2p))
     __device__ __forceinline__ void ct1(T& a, T& b) const {
@@ -82,11 +88,18 @@ struct Ar32 {
     // inverse-transform output range [0, 2p) -> [0, p)
     __device__ __forceinline__ T inv_out(T a) const { return red1(a); }
     // x * w for a twiddle applied between transform passes, in [0, 2p)
-    __device__ __forceinline__ T mulc(T x, T w, T wq) const { return shoup(x, w, wq); }
+    __device__ __forceinline__ T mulc(T x, const Tw<T>& w) const { return shoup(x, w.w, w.wq); }
     // a 16- or 32-bit coefficient as a residue
     static __device__ __forceinline__ T from_u32(uint32_t x) { return (T)x; }
     // last scaling of a single-pass transform, in [0, p)
-    __device__ __forceinline__ T scale_out(T x, T w, T wq) const { return red1(shoup(x, w, wq)); }
+    __device__ __forceinline__ T scale_out(T x, const Tw<T>& w) const {
+        return red1(shoup(x, w.w, w.wq));
+    }
+    // the product of two table constants, with its companion
+    __device__ __forceinline__ Tw<T> mul_tw(const Tw<T>& a, const Tw<T>& b) const {
+        const T w = red1(shoup(a.w, b.w, b.wq));
+        return Tw<T>{w, companion(w)};
+    }
     // Shoup companion floor(w 2^32 / p) of w < p: a double-precision estimate
     // w (2^32 / p) is within 2^-20 of the quotient (below 2^32, relative error
     // under 2^-51), so its floor is exact or one off, and the exact remainder
@@ -224,18 +237,18 @@ struct Ar64 {
     }
     // forward CT butterfly: a + t and a - t + 3p with t = b w in [0, 3p), no
     // reduction (each stage grows the bound by less than 3p)
-    __device__ __forceinline__ void ct(T& a, T& b, T w, T wq) const {
+    __device__ __forceinline__ void ct(T& a, T& b, const Tw<T>& w) const {
         const T x = a;
-        const T t = shoup3(b, w, wq);  // [0, 3p)
+        const T t = shoup3(b, w.w, w.wq);  // [0, 3p)
         a = x + t;
         b = x - t + p3;
     }
     // inverse GS butterfly, inputs/outputs in [0, 3p)
-    __device__ __forceinline__ void gs(T& a, T& b, T w, T wq) const {
+    __device__ __forceinline__ void gs(T& a, T& b, const Tw<T>& w) const {
         const T u = a + b;       // [0, 6p)
         const T v = a - b + p3;  // (0, 6p)
         a = min(u, u - p3);
-        b = shoup3(v, w, wq);
+        b = shoup3(v, w.w, w.wq);
     }
     // twiddle-1 butterflies of stage 0 (inputs in [0, 3p))
     __device__ __forceinline__ void ct1(T& a, T& b) const {
@@ -260,11 +273,18 @@ struct Ar64 {
     // inverse-transform output range [0, 3p) -> [0, p)
     __device__ __forceinline__ T inv_out(T a) const { return red1(min(a, a - p2)); }
     // x * w for a twiddle applied between transform passes, in [0, 3p)
-    __device__ __forceinline__ T mulc(T x, T w, T wq) const { return shoup3(x, w, wq); }
+    __device__ __forceinline__ T mulc(T x, const Tw<T>& w) const { return shoup3(x, w.w, w.wq); }
     // a 16- or 32-bit coefficient as a residue
     static __device__ __forceinline__ T from_u32(uint32_t x) { return (T)x; }
     // last scaling of a single-pass transform, in [0, p)
-    __device__ __forceinline__ T scale_out(T x, T w, T wq) const { return red1(shoup(x, w, wq)); }
+    __device__ __forceinline__ T scale_out(T x, const Tw<T>& w) const {
+        return red1(shoup(x, w.w, w.wq));
+    }
+    // the product of two table constants, with its companion
+    __device__ __forceinline__ Tw<T> mul_tw(const Tw<T>& a, const Tw<T>& b) const {
+        const T w = red1(shoup(a.w, b.w, b.wq));
+        return Tw<T>{w, companion(w)};
+    }
     // Shoup companion floor(w 2^64 / p) of w < p by a Barrett step with
     // mu = floor(2^128 / p): the estimate is at most 2 short.
     __device__ __forceinline__ T companion(T w) const {
@@ -282,28 +302,32 @@ struct Ar64 {
 // Exact modular arithmetic in double precision, for the 64-bit path's 64-bit
 // coefficients.  A residue is a double holding an integer of either sign below
 // 2^53 in magnitude, so sums and differences are exact, and a product by a
-// constant w (|w| <= p/2, companion wq = w / p) takes six operations:
+// constant w (|w| <= p/2) takes six operations:
 //
-//   h = x w (rounded), l = x w - h (exact, one FMA), q = round(x wq),
+//   h = x w (rounded), l = x w - h (exact, one FMA), q = round(h / p),
 //   r = (h - q p) + l = x w - q p.
 //
 // q comes from adding and subtracting 1.5 2^52, which rounds to an integer
-// while |q| <= 2^51.  q is within 1/2 + |x w / p| 2^-53 of x w / p, so
-// |r| <= p (1/2 + X p 2^-54) for |x| = X p; h - q p is an integer below 2^53,
+// while |q| <= 2^51.  q is within 1/2 + |x w / p| 2^-52 of x w / p, so
+// |r| <= p (1/2 + X p 2^-53) for |x| = X p; h - q p is an integer below 2^53,
 // so the FMA and the last addition are exact.  The FP64 pipe of an SM takes 64
 // such operations per cycle, beside the integer pipe's addressing: a butterfly
 // is 8 of them against about 40 integer instructions for a 58-bit prime
-// (measured 6.7 against 2.83 butterflies per SM-cycle).
+// (measured 6.5 against 2.83 butterflies per SM-cycle).  A companion w / p per
+// constant would shorten the chain by one operation and measured 6.7, but
+// doubles the twiddle loads, and those bound the last round of a row.
 //
-// POL 0: primes just above 2^50 (X <= 4 keeps q below 2^51).  Forward: a round
-//   reduces the half it does not multiply in its first stage and then adds four
-//   stages: from X <= 4 at most 1.25, 1.83, 2.44, 3.10.  Inverse: the sums of
-//   every second stage, and of a round's last, are reduced (X <= 0.7 between
-//   rounds, differences at most 2.8).
-// POL 1: primes just above 2^51.66 (X <= 1.26 for q, 2.5 for exact sums), for
-//   transforms whose coefficients need three such primes: a forward round
-//   reduces all its values before its first and third stage (X <= 1.85 at its
-//   end), an inverse stage reduces both outputs.
+// POL 0: primes just above 2^50 (X < 4 keeps q below 2^51; |r| <= p (1/2 +
+//   X/8)).  Forward: a round reduces the half it does not multiply in its
+//   first stage and then adds four stages: from X = 3.9 at most 1.49, 2.18,
+//   2.95, 3.82.  Inverse: the sums of every second stage, and of a round's
+//   last, are reduced: from E at most 4E in a difference and 1/2 + E/2 at the
+//   round's end, E = 0.62, 0.81, 0.91, 0.96 over four rounds.
+// POL 1: primes just above 2^51.66 (X <= 1.26 for q, 2.5 for exact sums,
+//   |r| <= p (1/2 + 0.4 X)), for transforms whose coefficients need three such
+//   primes: a forward round reduces all its values before its first and third
+//   stage (at most 0.7 + 0.5 = 1.2, then 2.2), an inverse stage reduces both
+//   outputs.
 template <int POL>
 struct ArD {
     using T = double;
@@ -321,36 +345,23 @@ struct ArD {
         const double q = rnd(__fma_rn(x, pinv, kMagic));
         return __fma_rn(-q, p, x);
     }
-    __device__ __forceinline__ T mul(T x, T w, T wq) const {
-        const double q = rnd(__fma_rn(x, wq, kMagic));
+    __device__ __forceinline__ T mul(T x, T w) const {
         const double h = __dmul_rn(x, w);
+        const double q = rnd(__fma_rn(h, pinv, kMagic));
         const double l = __fma_rn(x, w, -h);
         return __dadd_rn(__fma_rn(-q, p, h), l);
     }
     // product of two residues reduced by red
-    __device__ __forceinline__ T mont(T a, T b) const {
-        const double h = __dmul_rn(a, b);
-        const double q = rnd(__fma_rn(h, pinv, kMagic));
-        const double l = __fma_rn(a, b, -h);
-        const double r = __dadd_rn(__fma_rn(-q, p, h), l);
-        return POL ? red(r) : r;
+    __device__ __forceinline__ T mont(T a, T b) const { return POL ? red(mul(a, b)) : mul(a, b); }
+    // value u of a round of half width h before its stage l; ent: the round's
+    // inputs may be any forward output (else they are reduced)
+    __device__ __forceinline__ T ct_enter(T x, int u, int h, int l, bool ent) const {
+        if (l == 0 && !ent) return x;
+        return (POL == 0 ? l == 0 && u < h : (l & 1) == 0) ? red(x) : x;
     }
-    // before the stage l of a forward round (h: the stage's half width)
-    template <int RL>
-    __device__ __forceinline__ void ct_enter(T* x, int l, int s0) const {
-        if (POL == 0) {
-            if (l == 0 && s0 > 0) {
-#pragma unroll
-                for (int u = 0; u < (1 << (RL - 1)); ++u) x[u] = red(x[u]);
-            }
-        } else if ((l & 1) == 0) {
-#pragma unroll
-            for (int u = 0; u < (1 << RL); ++u) x[u] = red(x[u]);
-        }
-    }
-    __device__ __forceinline__ void ct(T& a, T& b, T w, T wq) const {
+    __device__ __forceinline__ void ct(T& a, T& b, const Tw<T>& w) const {
         const T x = a;
-        const T t = mul(b, w, wq);
+        const T t = mul(b, w.w);
         a = __dadd_rn(x, t);
         b = __dsub_rn(x, t);
     }
@@ -361,11 +372,11 @@ struct ArD {
     }
     // RED: this stage's sums are reduced
     template <bool RED>
-    __device__ __forceinline__ void gs(T& a, T& b, T w, T wq) const {
+    __device__ __forceinline__ void gs(T& a, T& b, const Tw<T>& w) const {
         const T u = __dadd_rn(a, b);
         const T v = __dsub_rn(a, b);
         a = RED || POL ? red(u) : u;
-        const T r = mul(v, w, wq);
+        const T r = mul(v, w.w);
         b = POL ? red(r) : r;
     }
     __device__ __forceinline__ void gs1(T& a, T& b) const {
@@ -375,14 +386,15 @@ struct ArD {
         b = red(v);
     }
     __device__ __forceinline__ T fwd_to_2p(T a) const { return red(a); }
-    // twiddles between passes: any forward or inverse output in, at most
-    // 0.75 p out
-    __device__ __forceinline__ T mulc(T x, T w, T wq) const {
-        return POL ? red(mul(red(x), w, wq)) : mul(x, w, wq);
+    // twiddles between passes: any forward or inverse output in, below p out
+    // (POL 1: reduced)
+    __device__ __forceinline__ T mulc(T x, const Tw<T>& w) const {
+        return POL ? red(mul(red(x), w.w)) : mul(x, w.w);
     }
-    __device__ __forceinline__ T shoup(T x, T w, T wq) const { return mulc(x, w, wq); }
-    __device__ __forceinline__ T red1(T x) const { return red(x); }
-    __device__ __forceinline__ T companion(T w) const { return __dmul_rn(w, pinv); }
+    // the product of two table constants
+    __device__ __forceinline__ Tw<T> mul_tw(const Tw<T>& a, const Tw<T>& b) const {
+        return Tw<T>{red(mul(a.w, b.w))};
+    }
     // an integer below 2^32 or 2^64 as a residue: its words land in the
     // mantissas of 2^52 and 2^84; the high word's multiple of 2^32 is reduced
     // (|hi - q p| < 2^51 is exact) before the low word is added
@@ -403,7 +415,7 @@ struct ArD {
         const double z = __dadd_rn(y, 4503599627370496.0);
         return __longlong_as_double(__double_as_longlong(z) & 0x000fffffffffffffll);
     }
-    __device__ __forceinline__ T scale_out(T x, T w, T wq) const { return inv_out(mulc(x, w, wq)); }
+    __device__ __forceinline__ T scale_out(T x, const Tw<T>& w) const { return inv_out(mulc(x, w)); }
 };
 
 // Twiddle load from shared memory (generic pointer into the CTA's tables).
@@ -416,9 +428,7 @@ template <typename T>
 __device__ __forceinline__ Tw<T> ld_tw(const Tw<T>* p) {
     Tw<T> r;
     if constexpr (std::is_same<T, double>::value) {
-        const double2 v = __ldg(reinterpret_cast<const double2*>(p));
-        r.w = v.x;
-        r.wq = v.y;
+        r.w = __ldg(reinterpret_cast<const double*>(p));
     } else if constexpr (sizeof(T) == 8) {
         const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p));
         r.w = v.x;

@@ -23,7 +23,7 @@
 #include "../../include/birdwing.h"
 #include "bw_host.h"
 #include "bw_internal.h"
-#include "bw_kernels.cuh"
+#include "bw_ntt.cuh"
 
 using namespace bw;
 
@@ -154,13 +154,13 @@ static int choose_f64(size_t nca, size_t ncb) {
 namespace {
 
 // A table entry: a constant and its companion.  Integers: floor(w 2^bits / p);
-// double precision: w taken to [-p/2, p/2] and w / p.
+// double precision: w taken to [-p/2, p/2].
 template <class Ar>
 Tw<typename Ar::T> make_tw(uint64_t w, uint64_t p) {
     using T = typename Ar::T;
     if constexpr (Ar::kF64) {
         const double b = w > p / 2 ? -(double)(p - w) : (double)w;
-        return Tw<T>{b, b / (double)p};
+        return Tw<T>{b};
     } else {
         return Tw<T>{(T)w, (T)shoup_pre(w, p, Ar::BITS)};
     }
@@ -174,9 +174,10 @@ struct TableBuilder {
     // every table starts at an even entry (16 bytes for 4-byte residues), so
     // that the transforms can load its entries in pairs
     void align_even() {
-        if (host.size() & 1) host.push_back(Tw<T>{0, 0});
+        if (host.size() & 1) host.push_back(Tw<T>{});
     }
-    size_t add_stage_table(uint64_t p, uint64_t root, int log_len) {
+    // round_order: entries placed as the fixed-length passes read them (tw_perm)
+    size_t add_stage_table(uint64_t p, uint64_t root, int log_len, bool round_order = false) {
         const size_t L = (size_t)1 << log_len;
         align_even();
         const size_t off = host.size();
@@ -184,13 +185,14 @@ struct TableBuilder {
         std::vector<uint64_t> pw(std::max<size_t>(L / 2, 1));
         pw[0] = 1;
         for (size_t j = 1; j < pw.size(); ++j) pw[j] = mulmod(pw[j - 1], root, p);
-        host[off] = Tw<T>{0, 0};
+        host[off] = Tw<T>{};
         for (int s = 0; s < log_len; ++s) {
             const size_t m = (size_t)1 << s;
             for (size_t i = 0; i < m; ++i) {
                 const size_t e = (L >> (s + 1)) * bitrev_h((uint32_t)i, s);
                 const uint64_t w = pw[e];
-                host[off + m + i] = make_tw<Ar>(w, p);
+                const uint32_t t = (uint32_t)(m + i);
+                host[off + (round_order ? tw_perm(t, log_len) : t)] = make_tw<Ar>(w, p);
             }
         }
         return off;
@@ -310,10 +312,11 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
         const uint64_t wrowi = invmod(wrow, p);
         const uint64_t wr = powmod(wn, n >> pl->log_r, p);            // R-th root
         const uint64_t wc = powmod(wn, n >> pl->log_c, p);            // C-th root
-        off[k][0] = tb.add_stage_table(p, wr, pl->log_r);
-        off[k][1] = tb.add_stage_table(p, invmod(wr, p), pl->log_r);
-        off[k][2] = tb.add_stage_table(p, wc, pl->log_c);
-        off[k][3] = tb.add_stage_table(p, invmod(wc, p), pl->log_c);
+        const bool vr = pl->v2_rows != 0, vc = pl->v2_cols != 0;
+        off[k][0] = tb.add_stage_table(p, wr, pl->log_r, vc);
+        off[k][1] = tb.add_stage_table(p, invmod(wr, p), pl->log_r, vc);
+        off[k][2] = tb.add_stage_table(p, wc, pl->log_c, vr);
+        off[k][3] = tb.add_stage_table(p, invmod(wc, p), pl->log_c, vr);
         const size_t nlo = (size_t)1 << pl->lo, nhi = n_row >> pl->lo;
         const uint64_t scale = mulmod(invmod(n % p, p), powmod(2, bits, p), p);
         off[k][4] = tb.add_power_table(p, wrow, nlo, 1);
@@ -655,6 +658,25 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
                          pl->log_c == 12 && pl->rlog_row == 4)
                             ? 1
                             : 0;
+        // passes with compile-time lengths: single products of the 32-bit and
+        // double-precision arithmetics
+        if (mode == 2 && (path == BW_PATH_P32 || pl->f64)) {
+            pl->v2_rows = pl->log_c >= kRow2MinLog && pl->log_c <= kRow2MaxLog;
+            const int top = w == 8 ? kCol2MaxLog64 : kCol2MaxLog32;
+            if (pl->log_r >= kCol2MinLog && pl->log_r <= top && !pl->tw_smem_r) {
+                pl->v2_cols = 1;
+                pl->tma_cols = 0;
+                // tiles of 64 KiB (8-byte residues: 32 KiB to 64 KiB in 2-8 columns;
+                // 4-byte: 4-16 columns); one prime per CTA, so that the narrower
+                // ones are taken only until every SM has two CTAs
+                const int lo_cb = w == 8 ? 1 : 2, hi_cb = w == 8 ? 3 : 4;
+                int cb = std::max(lo_cb, std::min(hi_cb, (w == 8 ? 13 : 14) - pl->log_r));
+                cb = std::min(cb, log_cols_outer);
+                while (cb > lo_cb && ((size_t)K << (log_cols_outer - cb)) < 2u * sms) --cb;
+                pl->log_cb = pl->log_cb1 = cb;
+                if (cb < lo_cb) pl->v2_cols = 0;
+            }
+        }
         pl->lo = ((pl->log_r2 ? pl->log_r2 : pl->log_r) + pl->log_c + 1) / 2;
         pl->lo_out = (log_n + 1) / 2;
     }

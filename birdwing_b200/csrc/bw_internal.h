@@ -49,6 +49,9 @@ struct bw_plan {
     // 1 primes just above 2^50, 2 primes just above 2^51.66 (pd64 then holds
     // the Garner constants of the same primes)
     int f64 = 0;
+    // passes with compile-time lengths (bw_ntt.cuh); their tables are stored in
+    // round order
+    int v2_rows = 0, v2_cols = 0;
     bw::PlanDev<bw::ArD<0>> pdd0{};
     bw::PlanDev<bw::ArD<1>> pdd1{};
     uint64_t primes[bw::kMaxPrimes] = {};

@@ -228,15 +228,22 @@ __device__ __forceinline__ Tw<T> ld_w(const Tw<T>* p) {
     }
 }
 
-// Two consecutive twiddles (4-byte residues: one 16-byte load; the pair's
+// Two consecutive twiddles of 8 bytes each in one 16-byte load (the pair's
 // first entry has an even index in a 16-byte-aligned table).
 template <bool TS, typename T>
 __device__ __forceinline__ void ld_w2(const Tw<T>* p, Tw<T>& a, Tw<T>& b) {
-    static_assert(sizeof(T) == 4, "4-byte residues");
-    const uint4 v = TS ? *reinterpret_cast<const uint4*>(p)
-                       : __ldg(reinterpret_cast<const uint4*>(p));
-    a = Tw<T>{v.x, v.y};
-    b = Tw<T>{v.z, v.w};
+    static_assert(sizeof(Tw<T>) == 8, "8-byte entries");
+    if constexpr (sizeof(T) == 8) {
+        const double2 v = TS ? *reinterpret_cast<const double2*>(p)
+                             : __ldg(reinterpret_cast<const double2*>(p));
+        a.w = v.x;
+        b.w = v.y;
+    } else {
+        const uint4 v = TS ? *reinterpret_cast<const uint4*>(p)
+                           : __ldg(reinterpret_cast<const uint4*>(p));
+        a = Tw<T>{v.x, v.y};
+        b = Tw<T>{v.z, v.w};
+    }
 }
 
 // Forward CT stages s0 .. s0+RL-1 on one sub-problem of 2^RL elements that
@@ -252,7 +259,10 @@ __device__ __forceinline__ void ct_stages(typename Ar::T* x, int s0, int g,
 #pragma unroll
     for (int l = 0; l < RL; ++l) {
         const int h = 1 << (RL - l - 1);
-        if constexpr (Ar::kF64) ar.template ct_enter<RL>(x, l, s0);
+        if constexpr (Ar::kF64) {
+#pragma unroll
+            for (int u = 0; u < (1 << RL); ++u) x[u] = ar.ct_enter(x[u], u, 1 << (RL - 1), l, s0 > 0);
+        }
         if (l == 0 && s0 == 0) {
             if (zt) {
 #pragma unroll
@@ -264,7 +274,7 @@ __device__ __forceinline__ void ct_stages(typename Ar::T* x, int s0, int g,
             continue;
         }
         const Tw<T>* Ws = W + (1 << (s0 + l)) + (g << l);
-        if constexpr (sizeof(T) == 4) {
+        if constexpr (sizeof(Tw<T>) == 8) {
             if (l > 0) {
                 // the level's 2^l twiddles in pairs
 #pragma unroll
@@ -276,7 +286,7 @@ __device__ __forceinline__ void ct_stages(typename Ar::T* x, int s0, int g,
 #pragma unroll
                         for (int u = 0; u < h; ++u) {
                             const int k = ((q + e) << (RL - l)) + u;
-                            ar.ct(x[k], x[k + h], w[e].w, w[e].wq);
+                            ar.ct(x[k], x[k + h], w[e]);
                         }
                 }
                 continue;
@@ -288,7 +298,7 @@ __device__ __forceinline__ void ct_stages(typename Ar::T* x, int s0, int g,
 #pragma unroll
             for (int u = 0; u < h; ++u) {
                 const int k = (q << (RL - l)) + u;
-                ar.ct(x[k], x[k + h], w.w, w.wq);
+                ar.ct(x[k], x[k + h], w);
             }
         }
     }
@@ -310,7 +320,7 @@ __device__ __forceinline__ void gs_stages(typename Ar::T* x, int s0, int g,
             continue;
         }
         const Tw<T>* Ws = W + (1 << (s0 + l)) + (g << l);
-        if constexpr (sizeof(T) == 4) {
+        if constexpr (sizeof(Tw<T>) == 8) {
             if (l > 0) {
 #pragma unroll
                 for (int q = 0; q < (1 << l); q += 2) {
@@ -321,7 +331,15 @@ __device__ __forceinline__ void gs_stages(typename Ar::T* x, int s0, int g,
 #pragma unroll
                         for (int u = 0; u < h; ++u) {
                             const int k = ((q + e) << (RL - l)) + u;
-                            ar.gs(x[k], x[k + h], w[e].w, w[e].wq);
+                            if constexpr (Ar::kF64) {
+                                if (l == 0 || ((RL - 1 - l) & 1)) {
+                                    ar.template gs<true>(x[k], x[k + h], w[e]);
+                                } else {
+                                    ar.template gs<false>(x[k], x[k + h], w[e]);
+                                }
+                            } else {
+                                ar.gs(x[k], x[k + h], w[e]);
+                            }
                         }
                 }
                 continue;
@@ -335,12 +353,12 @@ __device__ __forceinline__ void gs_stages(typename Ar::T* x, int s0, int g,
                 const int k = (q << (RL - l)) + u;
                 if constexpr (Ar::kF64) {
                     if (l == 0 || ((RL - 1 - l) & 1)) {
-                        ar.template gs<true>(x[k], x[k + h], w.w, w.wq);
+                        ar.template gs<true>(x[k], x[k + h], w);
                     } else {
-                        ar.template gs<false>(x[k], x[k + h], w.w, w.wq);
+                        ar.template gs<false>(x[k], x[k + h], w);
                     }
                 } else {
-                    ar.gs(x[k], x[k + h], w.w, w.wq);
+                    ar.gs(x[k], x[k + h], w);
                 }
             }
         }
@@ -734,8 +752,7 @@ __device__ __forceinline__ Tw<typename Ar::T> pow_entry(const Ar& ar, uint64_t e
     using T = typename Ar::T;
     const auto a = ld_tw(TL + (e & ((1ull << lo) - 1)));
     const auto b = ld_tw(TH + (e >> lo));
-    const T w = ar.red1(ar.shoup(a.w, b.w, b.wq));
-    return Tw<T>{w, ar.companion(w)};
+    return ar.mul_tw(a, b);
 }
 
 // Fused row pass for row blockIdx.x and prime blockIdx.y: inter-pass twiddle
@@ -787,8 +804,8 @@ __device__ __forceinline__ void row_body(const PlanDev<Ar>& P, typename Ar::T* r
     // the in-place twiddle then costs one more shared-memory pass)
     for (int i = threadIdx.x; i < C; i += NT) {
         const Tw<T> f = F[i & (nf - 1)], g = G[i >> la];
-        bufA[LayRow::p(i)] = ar.mulc(ar.mulc(ga[i], f.w, f.wq), g.w, g.wq);
-        if (!square) bufB[LayRow::p(i)] = ar.mulc(ar.mulc(gb[i], f.w, f.wq), g.w, g.wq);
+        bufA[LayRow::p(i)] = ar.mulc(ar.mulc(ga[i], f), g);
+        if (!square) bufB[LayRow::p(i)] = ar.mulc(ar.mulc(gb[i], f), g);
     }
     __syncthreads();
 
@@ -796,7 +813,7 @@ __device__ __forceinline__ void row_body(const PlanDev<Ar>& P, typename Ar::T* r
     auto ldA = [&](int, int, int p) -> T { return bufA[p]; };
     auto st_glob = [&](int idx, T v) {
         const Tw<T> f = Fi[idx & (nf - 1)], g = Gi[idx >> la];
-        ga[idx] = ar.mulc(ar.mulc(v, f.w, f.wq), g.w, g.wq);
+        ga[idx] = ar.mulc(ar.mulc(v, f), g);
     };
 
     // the warp-shuffle exchange (BW_PLAN_SHFL_ROWS): 2^12-point rows of the
@@ -985,7 +1002,7 @@ k_mid_col(const PlanDev<Ar> P, typename Ar::T* res_a, typename Ar::T* res_b) {
         for (int e = threadIdx.x; e < (R2 << log_cb); e += blockDim.x) {
             const int i2 = e >> log_cb, v = e & (CB - 1);
             const Tw<T> a = Tcol[v], b = Trow[i2];
-            buf[LayCol<T>::p(e)] = ar.mulc(ar.mulc(buf[LayCol<T>::p(e)], a.w, a.wq), b.w, b.wq);
+            buf[LayCol<T>::p(e)] = ar.mulc(ar.mulc(buf[LayCol<T>::p(e)], a), b);
         }
         __syncthreads();
         for (int r = 0; r < nr; ++r) {
@@ -1011,7 +1028,7 @@ k_mid_col(const PlanDev<Ar> P, typename Ar::T* res_a, typename Ar::T* res_b) {
                 if (last) {
                     const Tw<T> a = Tcol[v], b = Trow[idx];
                     g[((size_t)idx << log_c) + c0 + v] =
-                        ar.mulc(ar.mulc(val, a.w, a.wq), b.w, b.wq);
+                        ar.mulc(ar.mulc(val, a), b);
                 } else {
                     buf[p] = val;
                 }
@@ -2007,7 +2024,7 @@ __device__ __forceinline__ void ks_product_body(const PlanDev<Ar>& P, const Batc
         const Ar ar = pr.ar;
         const Tw<T> sc = pr.scale;
         auto st_res = [&](int idx, T v) {
-            res[(size_t)kp * n + idx] = ar.scale_out(v, sc.w, sc.wq);
+            res[(size_t)kp * n + idx] = ar.scale_out(v, sc);
         };
         for (int i = threadIdx.x; i < n; i += NT) {
             bufA[LayRow::p(i)] = coef(d.a, nca, i);

@@ -1,0 +1,589 @@
+// bw_ntt.cuh -- the transform passes with lengths known at compile time.
+//
+// The passes of bw_kernels.cuh take any length at run time.  The common
+// lengths run these instead: every stride, slot offset and trip count is an
+// immediate, the first round of a pass loads global memory straight into
+// registers and the last one stores from them (nothing is staged through
+// shared memory only to be moved), and the twiddles of a round come in an
+// order in which a warp's loads are consecutive.
+//
+// Twiddle order.  A transform of length 2^L runs rounds of 4 stages, a
+// remainder round of L mod 4 stages first.  The round that starts at stage
+// S0 uses the table range [2^S0, 2^(S0+RL)); inside it the entries are stored
+// by (position in the sub-problem, group) rather than by (stage, group,
+// position), the positions in pairs:
+//   stage S0:      entry of group g at 2^S0 + g
+//   stage S0 + l:  positions q, q + 1 (q even) of group g at
+//                  2^(S0+1) + 2 (P 2^S0 + g), P = 2^(l-1) - 1 + q / 2
+// In a row's last round every thread has a group of its own: its 15 twiddles,
+// contiguous in the (stage, group, position) order, put the lanes of a warp 8
+// to 64 bytes apart, 86 wavefronts per sub-problem against the 32 (4-byte
+// residues) of its data; in this order they are 30.  tw_perm maps an index to
+// its place.
+#pragma once
+#include "bw_kernels.cuh"
+
+namespace bw {
+
+// Lengths the passes are instantiated for (log2): rows, and columns of 4- and
+// 8-byte residues.
+constexpr int kRow2MinLog = 5, kRow2MaxLog = 13;
+constexpr int kCol2MinLog = 5, kCol2MaxLog32 = 12, kCol2MaxLog64 = 13;
+
+// Rounds of a 2^L-point transform: the remainder round first.
+__host__ __device__ constexpr int first_rl(int L) { return L % 4 == 0 ? (L < 4 ? L : 4) : L % 4; }
+
+// Place of the stage table's entry t (t in [1, 2^L)) in the round order.
+__host__ __device__ inline uint32_t tw_perm(uint32_t t, int L) {
+    int s = 0;  // stage of entry t
+    while ((2u << s) <= t) ++s;
+    const int rl0 = first_rl(L);
+    const int s0 = s < rl0 ? 0 : rl0 + (s - rl0) / 4 * 4;
+    const int l = s - s0;
+    const uint32_t i = t - (1u << s), g = i >> l, q = i & ((1u << l) - 1), G = 1u << s0;
+    if (l == 0) return G + g;
+    return 2 * G + 2 * (((1u << (l - 1)) - 1 + (q >> 1)) * G + g) + (q & 1);
+}
+
+// One round's twiddles of a thread's sub-problem in group g (G = 2^S0 groups).
+template <typename T, int G, bool SM>
+struct RoundTw {
+    const Tw<T>* p1;
+    const Tw<T>* p2;
+    __device__ __forceinline__ RoundTw(const Tw<T>* W, int g) : p1(W + G + g), p2(W + 2 * G + 2 * g) {}
+    __device__ __forceinline__ Tw<T> one() const { return ld_w<SM>(p1); }
+    // positions 2 j, 2 j + 1 of stage l: P = 2^(l-1) - 1 + j
+    __device__ __forceinline__ void pair(int P, Tw<T>& a, Tw<T>& b) const {
+        ld_w2<SM>(p2 + (size_t)P * 2 * G, a, b);
+    }
+};
+
+// Forward (CT) round on a sub-problem in registers.  ONE: the first stage's
+// twiddle is 1 (stage 0 of a column); ZT: the upper half is zero and the first
+// stage (twiddle 1) copies the lower one; ENT: the inputs may be any forward
+// output (ArD reduces some of them; the integer arithmetics ignore it).
+template <class Ar, int RL, bool ONE, bool ZT, bool ENT, class TW>
+__device__ __forceinline__ void ct_round(typename Ar::T* x, const Ar& ar, const TW& tw) {
+    using T = typename Ar::T;
+#pragma unroll
+    for (int l = 0; l < RL; ++l) {
+        const int h = 1 << (RL - l - 1);
+        if constexpr (Ar::kF64) {
+#pragma unroll
+            for (int u = 0; u < (1 << RL); ++u) x[u] = ar.ct_enter(x[u], u, 1 << (RL - 1), l, ENT);
+        }
+        if (l == 0) {
+            if constexpr (ZT) {
+#pragma unroll
+                for (int u = 0; u < h; ++u) x[u + h] = x[u];
+            } else if constexpr (ONE) {
+#pragma unroll
+                for (int u = 0; u < h; ++u) ar.ct1(x[u], x[u + h]);
+            } else {
+                const Tw<T> w = tw.one();
+#pragma unroll
+                for (int u = 0; u < h; ++u) ar.ct(x[u], x[u + h], w);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int q = 0; q < (1 << l); q += 2) {
+            Tw<T> w[2];
+            tw.pair((1 << (l - 1)) - 1 + q / 2, w[0], w[1]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int u = 0; u < h; ++u) {
+                    const int k = ((q + e) << (RL - l)) + u;
+                    ar.ct(x[k], x[k + h], w[e]);
+                }
+        }
+    }
+}
+
+// Inverse (GS) round, the mirror of ct_round.  LAST: ArD reduces the sums of
+// the round's last stage (not needed before a multiplication).
+template <class Ar, int RL, bool ONE, bool LAST, class TW>
+__device__ __forceinline__ void gs_round(typename Ar::T* x, const Ar& ar, const TW& tw) {
+    using T = typename Ar::T;
+    auto gs = [&](T& a, T& b, const Tw<T>& w, bool red) {
+        if constexpr (Ar::kF64) {
+            if (red) {
+                ar.template gs<true>(a, b, w);
+            } else {
+                ar.template gs<false>(a, b, w);
+            }
+        } else {
+            ar.gs(a, b, w);
+        }
+    };
+#pragma unroll
+    for (int l = RL - 1; l >= 0; --l) {
+        const int h = 1 << (RL - l - 1);
+        const bool red = l == 0 ? LAST : ((RL - 1 - l) & 1) != 0;
+        if (l == 0) {
+            if constexpr (ONE) {
+#pragma unroll
+                for (int u = 0; u < h; ++u) ar.gs1(x[u], x[u + h]);
+            } else {
+                const Tw<T> w = tw.one();
+#pragma unroll
+                for (int u = 0; u < h; ++u) gs(x[u], x[u + h], w, red);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int q = 0; q < (1 << l); q += 2) {
+            Tw<T> w[2];
+            tw.pair((1 << (l - 1)) - 1 + q / 2, w[0], w[1]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int u = 0; u < h; ++u) {
+                    const int k = ((q + e) << (RL - l)) + u;
+                    gs(x[k], x[k + h], w[e], red);
+                }
+        }
+    }
+}
+
+// Row layout: 8-byte residues e + e/16, conflict-free for every round (a
+// 64-bit access is served 16 lanes at a time).  4-byte residues e + e/32:
+// conflict-free for unit-stride lanes and for the stride-16 lanes of a last
+// round; the 16 x 16 middle round takes groups two apart in one warp
+// (row_group), which puts its two runs of 16 lanes on different banks.
+template <typename T>
+using LayRow2 = typename std::conditional<sizeof(T) == 4, Lay<5, 1>, Lay<4, 1>>::type;
+
+// Sub-problem sp of a round with 2^D sub-problems per group -> (group, j).
+template <typename T, int D, int NSUB>
+__device__ __forceinline__ void row_group(int sp, int& g, int& j) {
+    j = sp & ((1 << D) - 1);
+    g = sp >> D;
+    if constexpr (sizeof(T) == 4 && D == 4 && NSUB >= 64) {
+        // swap the group's two low bits: lanes 0-15 and 16-31 of a warp take
+        // groups two apart
+        g = (g & ~3) | ((g & 1) << 1) | ((g >> 1) & 1);
+    }
+}
+
+// ------------------------------------------------------------------ rows
+// Fused row pass for one row and prime: forward transforms of both operands'
+// rows, pointwise product, inverse transform, with the twiddles between the
+// passes, w^(c k1) on element c, mostly folded into the stage twiddles.  The
+// row's transform evaluates sum_c x_c y^c at y = zeta w_C^j with zeta = w^k1:
+// CT stages on y^C - zeta^C split it by (y^(C/2m) - r)(y^(C/2m) + r) with
+// r = zeta^(C/2m) W[m + i], so a table R[m + i] = zeta^(C/2m) W[m + i] of
+// C / 16 entries per row, built in shared memory, takes the first stages
+// through the whole twist; before the last round, whose sub-problems are 16
+// consecutive elements, substituting y = zeta z leaves zeta^j on element j and
+// the plain twiddles after it.  One multiplication per element and transform
+// instead of two, and the inverse mirrors it (zeta^-j n^-1 2^bits after its
+// first round).
+template <class Ar, int LOGC>
+struct RowCfg {
+    static constexpr int C = 1 << LOGC;
+    static constexpr int RLAST = LOGC < 4 ? LOGC : 4;
+    static constexpr int S1 = LOGC - RLAST;  // stages with row twiddles
+    static constexpr int NSUB = C >> RLAST;
+    static constexpr int NT = NSUB < 32 ? 32 : NSUB > 256 ? 256 : NSUB;
+    // shared memory: row twiddles, their inverses, zeta powers, two row buffers
+    static constexpr size_t smem(bool sq) {
+        return ((size_t)2 * (1 << S1) + 32 + 32) * sizeof(Tw<typename Ar::T>) +
+               tile_elems(C) * sizeof(typename Ar::T) * (sq ? 1 : 2);
+    }
+    // resident CTAs the register bound aims at: 768 threads of 80 registers
+    // (double precision), 1024 of 64
+    static constexpr int kMinCtas = (sizeof(typename Ar::T) == 8 ? 768 : 1024) / NT;
+};
+
+// One CT round (starting at stage S0) of a row in shared memory, from global
+// memory when FROM_G.
+template <class Ar, int LOGC, int S0, int RL, bool FROM_G, class TWB>
+__device__ __forceinline__ void row_ct(const typename Ar::T* __restrict__ gsrc,
+                                       typename Ar::T* buf, const Ar& ar, const TWB* W) {
+    using T = typename Ar::T;
+    using L = LayRow2<T>;
+    constexpr int D = LOGC - S0 - RL, NSUB = 1 << (LOGC - RL), NT = RowCfg<Ar, LOGC>::NT;
+#pragma unroll 1
+    for (int sp = threadIdx.x; sp < NSUB; sp += NT) {
+        int g, j;
+        row_group<T, D, NSUB>(sp, g, j);
+        const int base = (g << (D + RL)) + j;
+        const int p0 = L::p(base);
+        T x[1 << RL];
+#pragma unroll
+        for (int k = 0; k < (1 << RL); ++k) {
+            if constexpr (FROM_G) {
+                x[k] = gsrc[base + (k << D)];
+            } else {
+                x[k] = buf[p0 + L::template off<false>(k, D, 0)];
+            }
+        }
+        ct_round<Ar, RL, false, false, true>(x, ar, RoundTw<T, (1 << S0), true>(W, g));
+#pragma unroll
+        for (int k = 0; k < (1 << RL); ++k) buf[p0 + L::template off<false>(k, D, 0)] = x[k];
+    }
+}
+
+// One GS round of a row in shared memory, to global memory when TO_G.
+template <class Ar, int LOGC, int S0, int RL, bool TO_G, class TWB>
+__device__ __forceinline__ void row_gs(typename Ar::T* __restrict__ gdst, typename Ar::T* buf,
+                                       const Ar& ar, const TWB* W) {
+    using T = typename Ar::T;
+    using L = LayRow2<T>;
+    constexpr int D = LOGC - S0 - RL, NSUB = 1 << (LOGC - RL), NT = RowCfg<Ar, LOGC>::NT;
+#pragma unroll 1
+    for (int sp = threadIdx.x; sp < NSUB; sp += NT) {
+        int g, j;
+        row_group<T, D, NSUB>(sp, g, j);
+        const int base = (g << (D + RL)) + j;
+        const int p0 = L::p(base);
+        T x[1 << RL];
+#pragma unroll
+        for (int k = 0; k < (1 << RL); ++k) x[k] = buf[p0 + L::template off<false>(k, D, 0)];
+        gs_round<Ar, RL, false, true>(x, ar, RoundTw<T, (1 << S0), true>(W, g));
+#pragma unroll
+        for (int k = 0; k < (1 << RL); ++k) {
+            if constexpr (TO_G) {
+                gdst[base + (k << D)] = x[k];
+            } else {
+                buf[p0 + L::template off<false>(k, D, 0)] = x[k];
+            }
+        }
+    }
+}
+
+template <class Ar, int LOGC>
+__device__ __forceinline__ void row2_body(const PlanDev<Ar>& P, typename Ar::T* res_a,
+                                          const typename Ar::T* res_b, bool square, int prow,
+                                          int kp, unsigned char* smem_raw) {
+    using T = typename Ar::T;
+    using Cfg = RowCfg<Ar, LOGC>;
+    using L = LayRow2<T>;
+    constexpr int C = Cfg::C, S1 = Cfg::S1, RLAST = Cfg::RLAST, NT = Cfg::NT, NSUB = Cfg::NSUB;
+    constexpr int RL0 = first_rl(LOGC), NE = 1 << RLAST;
+    static_assert(LOGC > 4 && LOGC <= 13, "two to four rounds");
+    const size_t n = (size_t)1 << P.log_n;
+    const int log_rr = P.log_r2 ? P.log_r2 : P.log_r;
+    const PrimeDev<Ar>& pr = P.pr[kp];
+    const Ar ar = pr.ar;
+    T* ga = res_a + (size_t)kp * n + (size_t)prow * C;
+    const T* gb = res_b + (size_t)kp * n + (size_t)prow * C;
+    Tw<T>* R = reinterpret_cast<Tw<T>*>(smem_raw);   // row twiddles
+    Tw<T>* Ri = R + (1 << S1);                       // inverse
+    Tw<T>* Z = Ri + (1 << S1);                       // zeta^j, then zeta^-j n^-1 2^bits
+    Tw<T>* ZL = Z + 32;                              // zeta^(C/2m) and inverse, by stage
+    T* bufA = reinterpret_cast<T*>(ZL + 32);
+    T* bufB = bufA + tile_elems(C);
+
+    // ---- the row's powers of zeta, then its twiddles
+    {
+        const size_t n_row = (size_t)C << log_rr;
+        const uint64_t nmask = n_row - 1;
+        const uint64_t k1 = bitrev((uint32_t)prow & ((1u << log_rr) - 1), log_rr);
+        for (int i = threadIdx.x; i < 2 * NE + 2 * S1; i += NT) {
+            if (i < NE) {
+                Z[i] = pow_entry(ar, ((uint64_t)i * k1) & nmask, P.lo, pr.TLf, pr.THf);
+            } else if (i < 2 * NE) {
+                Z[i] = pow_entry(ar, ((uint64_t)(i - NE) * k1) & nmask, P.lo, pr.TLi, pr.THi);
+            } else {
+                const int s = (i - 2 * NE) >> 1;
+                uint64_t e = (((uint64_t)C >> (s + 1)) * k1) & nmask;
+                if (i & 1) e = (n_row - e) & nmask;
+                ZL[i - 2 * NE] = pow_entry(ar, e, P.lo, pr.TLf, pr.THf);
+            }
+        }
+        __syncthreads();
+        for (int i = 1 + threadIdx.x; i < (1 << S1); i += NT) {
+            // the stage of place i in the round order
+            int s0 = RL0;
+            while (i >= (16 << s0)) s0 += 4;
+            if (i < (1 << RL0)) s0 = 0;
+            const int u = (i - (1 << s0)) >> s0;  // 0: first stage; else 2 P + 1, 2 P + 2
+            const int s = s0 + (u == 0 ? 0 : 32 - __clz((u + 1) >> 1));
+            R[i] = ar.mul_tw(ZL[2 * s], ld_tw(pr.WCf + i));
+            Ri[i] = ar.mul_tw(ZL[2 * s + 1], ld_tw(pr.WCi + i));
+        }
+        __syncthreads();
+    }
+
+    // ---- forward rounds with row twiddles, global memory -> shared memory
+    row_ct<Ar, LOGC, 0, RL0, true>(ga, bufA, ar, R);
+    if (!square) row_ct<Ar, LOGC, 0, RL0, true>(gb, bufB, ar, R);
+    __syncthreads();
+    if constexpr (S1 > RL0) {
+        row_ct<Ar, LOGC, RL0, 4, false>(nullptr, bufA, ar, R);
+        if (!square) row_ct<Ar, LOGC, RL0, 4, false>(nullptr, bufB, ar, R);
+        __syncthreads();
+    }
+    if constexpr (S1 > RL0 + 4) {
+        row_ct<Ar, LOGC, RL0 + 4, 4, false>(nullptr, bufA, ar, R);
+        if (!square) row_ct<Ar, LOGC, RL0 + 4, 4, false>(nullptr, bufB, ar, R);
+        __syncthreads();
+    }
+
+    // ---- last forward round of both, product, first inverse round: 16
+    // consecutive elements per thread, no exchange in between
+#pragma unroll 1
+    for (int g = threadIdx.x; g < NSUB; g += NT) {
+        const int p0 = L::p(g << RLAST);
+        const RoundTw<T, (1 << S1), false> tf(pr.WCf, g), ti(pr.WCi, g);
+        T x[NE];
+        auto fwd = [&](const T* buf) {
+#pragma unroll
+            for (int k = 0; k < NE; ++k) x[k] = ar.mulc(buf[p0 + k], ld_w<true>(Z + k));
+            ct_round<Ar, RLAST, false, false, false>(x, ar, tf);
+        };
+        fwd(bufA);
+        if (square) {
+#pragma unroll
+            for (int k = 0; k < NE; ++k) {
+                const T v = ar.fwd_to_2p(x[k]);
+                x[k] = ar.mont(v, v);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < NE; ++k) bufA[p0 + k] = ar.fwd_to_2p(x[k]);
+            fwd(bufB);
+#pragma unroll
+            for (int k = 0; k < NE; ++k) x[k] = ar.mont(ar.fwd_to_2p(x[k]), bufA[p0 + k]);
+        }
+        gs_round<Ar, RLAST, false, false>(x, ar, ti);
+#pragma unroll
+        for (int k = 0; k < NE; ++k) bufA[p0 + k] = ar.mulc(x[k], ld_w<true>(Z + NE + k));
+    }
+    __syncthreads();
+
+    // ---- remaining inverse rounds, the last one to global memory
+    if constexpr (S1 > RL0 + 4) {
+        row_gs<Ar, LOGC, RL0 + 4, 4, false>(nullptr, bufA, ar, Ri);
+        __syncthreads();
+    }
+    if constexpr (S1 > RL0) {
+        row_gs<Ar, LOGC, RL0, 4, false>(nullptr, bufA, ar, Ri);
+        __syncthreads();
+    }
+    row_gs<Ar, LOGC, 0, RL0, true>(ga, bufA, ar, Ri);
+}
+
+template <class Ar, int LOGC>
+__global__ void __launch_bounds__(RowCfg<Ar, LOGC>::NT, RowCfg<Ar, LOGC>::kMinCtas)
+k_row2(const PlanDev<Ar> P, typename Ar::T* res_a, const typename Ar::T* res_b, int square) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    row2_body<Ar, LOGC>(P, res_a, res_b, square != 0, blockIdx.x, blockIdx.y, smem_raw);
+}
+
+// ------------------------------------------------------------------ columns
+// A tile is 2^LCB columns of a 2^LOGR-point transform, element (idx, v) at
+// layout slot p((idx << LCB) + v).  Threads take sub-problems with v fastest,
+// so a warp's global accesses cover 2^LCB consecutive elements of several rows.
+template <class Ar, int LOGR, int LCB>
+struct ColCfg {
+    static constexpr int RLAST = LOGR < 4 ? LOGR : 4;
+    static constexpr int NSUB = 1 << (LOGR + LCB - RLAST);
+    static constexpr int NT = NSUB < 32 ? 32 : NSUB > 256 ? 256 : NSUB;
+    static constexpr size_t smem = tile_elems((size_t)1 << (LOGR + LCB)) * sizeof(typename Ar::T);
+    static constexpr int kMinCtas = (sizeof(typename Ar::T) == 8 ? 768 : 1024) / NT;
+};
+
+// The tile's coefficients, as the first forward round reads them.
+// CW: coefficient width in bits (16, 32 or 64); ncoef: 16- or 32-bit
+// coefficients, or words (64-bit, an odd count's last high word is zero).
+template <class Ar, int CW>
+struct CoefLoad {
+    using T = typename Ar::T;
+    const uint32_t* __restrict__ limbs;
+    uint32_t ncoef;  // whole coefficients
+    uint32_t lone;   // 64-bit: 1 if a single low word follows them
+    bool al8;
+    __device__ __forceinline__ CoefLoad(const uint32_t* l, size_t nc) : limbs(l) {
+        ncoef = CW == 64 ? (uint32_t)(nc >> 1) : (uint32_t)nc;
+        lone = CW == 64 ? (uint32_t)(nc & 1) : 0u;
+        al8 = (reinterpret_cast<uintptr_t>(l) & 7u) == 0;
+    }
+    // coefficient ci, zero beyond the operand, as a residue
+    __device__ __forceinline__ T operator()(const Ar& ar, uint32_t ci) const {
+        if constexpr (CW == 16) {
+            const uint16_t* h = reinterpret_cast<const uint16_t*>(limbs);
+            return Ar::from_u32(ci < ncoef ? (uint32_t)__ldg(h + ci) : 0u);
+        } else if constexpr (CW == 32) {
+            return Ar::from_u32(ci < ncoef ? __ldg(limbs + ci) : 0u);
+        } else {
+            uint64_t v = 0;
+            const uint32_t* w = limbs + 2 * (size_t)ci;
+            if (ci < ncoef) {
+                if (al8) {
+                    v = __ldg(reinterpret_cast<const unsigned long long*>(w));
+                } else {
+                    v = ((uint64_t)__ldg(w + 1) << 32) | __ldg(w);
+                }
+            } else if (ci == ncoef && lone) {
+                v = __ldg(w);
+            }
+            if constexpr (Ar::kF64) {
+                return ar.from_u64(v);
+            } else {
+                return ar.reduce64(v);
+            }
+        }
+    }
+};
+
+// Forward column pass of one tile, operand and prime.  zt: the upper half of
+// the rows is zero pad.
+template <class Ar, int LOGR, int LCB, int CW>
+__device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
+                                              const uint32_t* __restrict__ limbs, size_t ncoef,
+                                              typename Ar::T* res, bool zt, int tile, int kp,
+                                              unsigned char* smem_raw) {
+    using T = typename Ar::T;
+    using L = LayCol<T>;
+    using Cfg = ColCfg<Ar, LOGR, LCB>;
+    constexpr int RL0 = first_rl(LOGR), NT = Cfg::NT, CB = 1 << LCB;
+    const int log_c = P.log_c + P.log_r2;
+    const PrimeDev<Ar>& pr = P.pr[kp];
+    const Ar ar = pr.ar;
+    const uint32_t c0 = (uint32_t)tile << LCB;
+    T* gout = res + ((size_t)kp << P.log_n) + c0;
+    T* buf = reinterpret_cast<T*>(smem_raw);
+    const CoefLoad<Ar, CW> coef(limbs, ncoef);
+
+    auto round = [&](auto s0_, auto rl_, auto zt_) {
+        constexpr int S0 = decltype(s0_)::value, RL = decltype(rl_)::value;
+        constexpr bool ZT = decltype(zt_)::value;
+        constexpr bool FIRST = S0 == 0, LAST = S0 + RL == LOGR;
+        constexpr int D = LOGR - S0 - RL, DS = D + LCB, N = 1 << (LOGR + LCB - RL);
+#pragma unroll 1
+        for (int sp = threadIdx.x; sp < N; sp += NT) {
+            const int v = sp & (CB - 1), rest = sp >> LCB;
+            const int j = rest & ((1 << D) - 1), g = rest >> D;
+            const int base = (g << (D + RL)) + j;
+            const int p0 = L::p((base << LCB) + v);
+            T x[1 << RL];
+#pragma unroll
+            for (int k = 0; k < (1 << RL); ++k) {
+                if constexpr (FIRST) {
+                    if (ZT && k >= (1 << (RL - 1))) continue;
+                    x[k] = coef(ar, ((uint32_t)(base + (k << D)) << log_c) + c0 + v);
+                } else {
+                    x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
+                }
+            }
+            ct_round<Ar, RL, FIRST, ZT, !FIRST>(x, ar, RoundTw<T, (1 << S0), false>(pr.WRf, g));
+#pragma unroll
+            for (int k = 0; k < (1 << RL); ++k) {
+                if constexpr (LAST) {
+                    gout[((size_t)(base + (k << D)) << log_c) + v] = x[k];
+                } else {
+                    buf[p0 + L::template off<false>(k, DS, 0)] = x[k];
+                }
+            }
+        }
+    };
+    using std::false_type;
+    using std::true_type;
+    if (zt) {
+        round(std::integral_constant<int, 0>{}, std::integral_constant<int, RL0>{}, true_type{});
+    } else {
+        round(std::integral_constant<int, 0>{}, std::integral_constant<int, RL0>{}, false_type{});
+    }
+    if constexpr (LOGR > RL0) {
+        __syncthreads();
+        round(std::integral_constant<int, RL0>{}, std::integral_constant<int, 4>{}, false_type{});
+    }
+    if constexpr (LOGR > RL0 + 4) {
+        __syncthreads();
+        round(std::integral_constant<int, RL0 + 4>{}, std::integral_constant<int, 4>{},
+              false_type{});
+    }
+    if constexpr (LOGR > RL0 + 8) {
+        __syncthreads();
+        round(std::integral_constant<int, RL0 + 8>{}, std::integral_constant<int, 4>{},
+              false_type{});
+    }
+}
+
+// blockIdx.x = tile * K + prime: the K CTAs of a tile run side by side, so the
+// operand words come from L2 after the first of them.
+template <class Ar, int LOGR, int LCB, int CW>
+__global__ void __launch_bounds__(ColCfg<Ar, LOGR, LCB>::NT, ColCfg<Ar, LOGR, LCB>::kMinCtas)
+k_fwd_col2(const PlanDev<Ar> P, const uint32_t* __restrict__ limbs_a, size_t ncoef_a,
+           const uint32_t* __restrict__ limbs_b, size_t ncoef_b, typename Ar::T* res_a,
+           typename Ar::T* res_b, unsigned zt_mask, int tile0) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int op = blockIdx.z;
+    fwd_col2_body<Ar, LOGR, LCB, CW>(P, op ? limbs_b : limbs_a, op ? ncoef_b : ncoef_a,
+                                     op ? res_b : res_a, (zt_mask >> op) & 1u,
+                                     tile0 + (int)(blockIdx.x / P.K), blockIdx.x % P.K, smem_raw);
+}
+
+// Inverse column pass of one tile and prime, in place, residues fully reduced.
+template <class Ar, int LOGR, int LCB>
+__device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar::T* res,
+                                              CarryState* cst, int tile, int kp,
+                                              unsigned char* smem_raw) {
+    using T = typename Ar::T;
+    using L = LayCol<T>;
+    using Cfg = ColCfg<Ar, LOGR, LCB>;
+    constexpr int RL0 = first_rl(LOGR), NT = Cfg::NT, CB = 1 << LCB;
+    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = 0;
+    const int log_c = P.log_c + P.log_r2;
+    const PrimeDev<Ar>& pr = P.pr[kp];
+    const Ar ar = pr.ar;
+    T* g0 = res + ((size_t)kp << P.log_n) + ((size_t)tile << LCB);
+    T* buf = reinterpret_cast<T*>(smem_raw);
+
+    auto round = [&](auto s0_, auto rl_) {
+        constexpr int S0 = decltype(s0_)::value, RL = decltype(rl_)::value;
+        constexpr bool FIRST = S0 + RL == LOGR, LAST = S0 == 0;
+        constexpr int D = LOGR - S0 - RL, DS = D + LCB, N = 1 << (LOGR + LCB - RL);
+#pragma unroll 1
+        for (int sp = threadIdx.x; sp < N; sp += NT) {
+            const int v = sp & (CB - 1), rest = sp >> LCB;
+            const int j = rest & ((1 << D) - 1), g = rest >> D;
+            const int base = (g << (D + RL)) + j;
+            const int p0 = L::p((base << LCB) + v);
+            T x[1 << RL];
+#pragma unroll
+            for (int k = 0; k < (1 << RL); ++k) {
+                if constexpr (FIRST) {
+                    x[k] = g0[((size_t)(base + (k << D)) << log_c) + v];
+                } else {
+                    x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
+                }
+            }
+            gs_round<Ar, RL, LAST, true>(x, ar, RoundTw<T, (1 << S0), false>(pr.WRi, g));
+#pragma unroll
+            for (int k = 0; k < (1 << RL); ++k) {
+                if constexpr (LAST) {
+                    g0[((size_t)(base + (k << D)) << log_c) + v] = ar.inv_out(x[k]);
+                } else {
+                    buf[p0 + L::template off<false>(k, DS, 0)] = x[k];
+                }
+            }
+        }
+    };
+    if constexpr (LOGR > RL0 + 8) {
+        round(std::integral_constant<int, RL0 + 8>{}, std::integral_constant<int, 4>{});
+        __syncthreads();
+    }
+    if constexpr (LOGR > RL0 + 4) {
+        round(std::integral_constant<int, RL0 + 4>{}, std::integral_constant<int, 4>{});
+        __syncthreads();
+    }
+    if constexpr (LOGR > RL0) {
+        round(std::integral_constant<int, RL0>{}, std::integral_constant<int, 4>{});
+        __syncthreads();
+    }
+    round(std::integral_constant<int, 0>{}, std::integral_constant<int, RL0>{});
+}
+
+template <class Ar, int LOGR, int LCB>
+__global__ void __launch_bounds__(ColCfg<Ar, LOGR, LCB>::NT, ColCfg<Ar, LOGR, LCB>::kMinCtas)
+k_inv_col2(const PlanDev<Ar> P, typename Ar::T* res, CarryState* cst) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    inv_col2_body<Ar, LOGR, LCB>(P, res, cst, blockIdx.x, blockIdx.y, smem_raw);
+}
+
+}  // namespace bw

@@ -47,7 +47,7 @@ k_bfly_rate(const ProbeArgs<Ar> P, int iters, typename Ar::T* out) {
 #pragma unroll
                 for (int q = 0; q < (1 << l); ++q)
 #pragma unroll
-                    for (int u = 0; u < h; ++u) ar.ct(x[(q << (4 - l)) + u], x[(q << (4 - l)) + u + h], w.w, w.wq);
+                    for (int u = 0; u < h; ++u) ar.ct(x[(q << (4 - l)) + u], x[(q << (4 - l)) + u + h], w);
             }
 #pragma unroll
             for (int k = 0; k < 16; ++k) x[k] = ar.fwd_to_2p(x[k]);
@@ -59,7 +59,7 @@ k_bfly_rate(const ProbeArgs<Ar> P, int iters, typename Ar::T* out) {
 #pragma unroll
             for (int q = 0; q < (1 << l); ++q)
 #pragma unroll
-                for (int u = 0; u < h; ++u) ar.gs(x[(q << (4 - l)) + u], x[(q << (4 - l)) + u + h], w.w, w.wq);
+                for (int u = 0; u < h; ++u) ar.gs(x[(q << (4 - l)) + u], x[(q << (4 - l)) + u + h], w);
         }
     }
     T acc = 0;

@@ -10,7 +10,7 @@
 #include "../../include/birdwing.h"
 #include "bw_host.h"
 #include "bw_internal.h"
-#include "bw_kernels.cuh"
+#include "bw_ntt.cuh"
 
 namespace bw {
 
@@ -70,6 +70,86 @@ int bw_set_transform_attrs() {
     return BW_OK;
 }
 
+
+// Whether an arithmetic has the fixed-length passes.
+template <class Ar>
+constexpr bool kHasV2 = Ar::kF64 || sizeof(typename Ar::T) == 4;
+
+// Raise a kernel's dynamic shared-memory limit once.
+template <auto KERN>
+cudaError_t allow_smem() {
+    static const cudaError_t st = cudaFuncSetAttribute(
+        (const void*)KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+    return st;
+}
+
+// Calls f(integral_constant<L>) for the runtime length l in [LO, HI].
+template <int LO, int HI, class F>
+cudaError_t with_length(int l, F f) {
+    if constexpr (LO > HI) {
+        return cudaErrorInvalidValue;
+    } else {
+        if (l == LO) return f(std::integral_constant<int, LO>{});
+        return with_length<LO + 1, HI>(l, f);
+    }
+}
+
+template <class Ar>
+cudaError_t launch_row2(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
+                        const typename Ar::T* rb, int sq, cudaStream_t s) {
+    return with_length<kRow2MinLog, kRow2MaxLog>(pl->log_c, [&](auto lc) {
+        constexpr int LC = decltype(lc)::value;
+        using Cfg = RowCfg<Ar, LC>;
+        const cudaError_t e = allow_smem<&k_row2<Ar, LC>>();
+        if (e != cudaSuccess) return e;
+        const dim3 g(1u << (pl->log_r + pl->log_r2), pl->K);
+        k_row2<Ar, LC><<<g, Cfg::NT, Cfg::smem(sq != 0), s>>>(pd, ra, rb, sq);
+        return cudaSuccess;
+    });
+}
+
+// f(integral_constant<log_r>, integral_constant<log_cb>) for a plan's column
+// tile.
+template <class Ar, class F>
+cudaError_t with_tile(int log_r, int log_cb, F f) {
+    constexpr bool W8 = sizeof(typename Ar::T) == 8;
+    return with_length<kCol2MinLog, W8 ? kCol2MaxLog64 : kCol2MaxLog32>(log_r, [&](auto lr) {
+        constexpr int LR = decltype(lr)::value;
+        constexpr int LO = W8 ? 1 : 2, TOP = (W8 ? 13 : 14) - LR;
+        constexpr int HI = TOP < LO ? LO : TOP > LO + 2 ? LO + 2 : TOP;
+        return with_length<LO, HI>(log_cb, [&](auto cb) { return f(lr, cb); });
+    });
+}
+
+template <class Ar, int CW>
+cudaError_t launch_fwd_col2(const bw_plan* pl, const PlanDev<Ar>& pd, const uint32_t* a,
+                            size_t na, const uint32_t* b, size_t nb, typename Ar::T* ra,
+                            typename Ar::T* rb, unsigned zt, int tile0, int ntiles, bool square,
+                            cudaStream_t s) {
+    return with_tile<Ar>(pl->log_r, pl->log_cb1, [&](auto lr, auto cb) {
+        constexpr int LR = decltype(lr)::value, CB = decltype(cb)::value;
+        using Cfg = ColCfg<Ar, LR, CB>;
+        const cudaError_t e = allow_smem<&k_fwd_col2<Ar, LR, CB, CW>>();
+        if (e != cudaSuccess) return e;
+        const dim3 g((unsigned)ntiles * pl->K, 1, square ? 1 : 2);
+        k_fwd_col2<Ar, LR, CB, CW><<<g, Cfg::NT, Cfg::smem, s>>>(pd, a, na, b, nb, ra, rb, zt,
+                                                                 tile0);
+        return cudaSuccess;
+    });
+}
+
+template <class Ar>
+cudaError_t launch_inv_col2(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
+                            CarryState* cst, int tiles, cudaStream_t s) {
+    return with_tile<Ar>(pl->log_r, pl->log_cb, [&](auto lr, auto cb) {
+        constexpr int LR = decltype(lr)::value, CB = decltype(cb)::value;
+        using Cfg = ColCfg<Ar, LR, CB>;
+        const cudaError_t e = allow_smem<&k_inv_col2<Ar, LR, CB>>();
+        if (e != cudaSuccess) return e;
+        k_inv_col2<Ar, LR, CB><<<dim3(tiles, pl->K), Cfg::NT, Cfg::smem, s>>>(pd, ra, cst);
+        return cudaSuccess;
+    });
+}
 
 template <class Ar, int RLOG>
 void launch_row(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
@@ -147,7 +227,15 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const int cols_outer = 1 << (pl->log_c + pl->log_r2);
     const int tiles1 = cols_outer / CB1;
     const unsigned zt = (pl->zt_a ? 1u : 0u) | (pl->zt_b ? 2u : 0u);
+    cudaError_t ke = cudaSuccess;  // a fixed-length launch's status
     auto k1 = [&](int tile0, int ntiles) {
+        if constexpr (kHasV2<Ar>) {
+            if (pl->v2_cols) {
+                ke = launch_fwd_col2<Ar, W64 ? 64 : SPLIT16 ? 16 : 32>(
+                    pl, pd, a, in_a, b, in_b, ra, rb, zt, tile0, ntiles, square, c->stream);
+                return;
+            }
+        }
         dim3 g1(ntiles * ((PP || pp32) ? pl->K : 1), 1, square ? 1 : 2);
         if constexpr (W64 && sizeof(T) == 4) {
             if (pp32) {
@@ -226,7 +314,16 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const size_t smem2 = ntab * sizeof(Tw<T>) + tile_elems(C) * sizeof(T) * (square ? 1 : 2);
     const T* rbs = square ? ra : rb;
     const int sq = square ? 1 : 0;
-    if (pl->rlog_row == 3) {
+    bool row_done = false;
+    BW_CUDA(ke);
+    if constexpr (kHasV2<Ar>) {
+        if (pl->v2_rows) {
+            BW_CUDA(launch_row2<Ar>(pl, pd, ra, rbs, sq, c->stream));
+            row_done = true;
+        }
+    }
+    if (row_done) {
+    } else if (pl->rlog_row == 3) {
         launch_row<Ar, 3>(pl, pd, ra, rbs, sq, smem2, c->stream);
     } else {
         launch_row<Ar, 4>(pl, pd, ra, rbs, sq, smem2, c->stream);
@@ -240,6 +337,12 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const size_t smem3 = tw_bytes + tile_elems((size_t)R * CB) * sizeof(T);
     dim3 g3(cols_outer / CB, pl->K);
     bool inv_done = false;
+    if constexpr (kHasV2<Ar>) {
+        if (pl->v2_cols) {
+            BW_CUDA(launch_inv_col2<Ar>(pl, pd, ra, c->cst, cols_outer / CB, c->stream));
+            inv_done = true;
+        }
+    }
     if (pl->tma_cols) {
         k_inv_col_tma<Ar, 4><<<g3, kColThreads, (size_t)R * CB * sizeof(T) + 128, c->stream>>>(
             pd, ra, c->cst, c->tmap_res, c->err, c->spin_limit);
