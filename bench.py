@@ -426,12 +426,12 @@ def batch_items(cfg, rank):
 
 def plain_launches(path, la, lb):
     """Kernels one plain product launches: the three transform passes, then
-    the boundary pre-pass, the words pass and the carry fix when the output
-    spans more than one 2048-word tile (the words pass alone otherwise)."""
+    the words pass and the carry fix when the output spans more than one
+    2048-word tile (the words pass alone otherwise)."""
     cpw = 2 if path == 32 else 1
     log_n = max(4, ((la + lb) * cpw - 2).bit_length())
     words = max((1 << log_n) // cpw, la + lb)
-    return 3 + (3 if words > 2048 else 1)
+    return 3 + (2 if words > 2048 else 1)
 
 
 def batch_model_bytes(items, K, small_max=None):
@@ -1029,11 +1029,10 @@ def fixed_model(cfg):
 def plain_launches_of(info, la, lb):
     """Kernels one plain product launches: the forward column, row and inverse
     column passes (two middle-column passes more in the three-pass
-    schedule), and Garner + carry: the boundary pre-pass, the words pass and
-    the carry fix when the output spans more than one 2048-word tile, else
-    the words pass alone."""
+    schedule), and Garner + carry: the words pass and the carry fix when the
+    output spans more than one 2048-word tile, else the words pass alone."""
     log_r2 = info["log_n"] - info["log_rows"] - info["log_cols"]
-    return 3 + (2 if log_r2 > 0 else 0) + (3 if la + lb > 2048 else 1)
+    return 3 + (2 if log_r2 > 0 else 0) + (2 if la + lb > 2048 else 1)
 
 
 def plan_butterflies(info, square):

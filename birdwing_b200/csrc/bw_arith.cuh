@@ -408,13 +408,8 @@ struct ArD {
         const double q = rnd(__fma_rn(hi, pinv, kMagic));
         return __dadd_rn(__fma_rn(-q, p, hi), lo);
     }
-    // an inverse output (|x| < p) as an integer in [0, p), in the bits of a
-    // double (the Garner kernels read integers)
-    __device__ __forceinline__ T inv_out(T x) const {
-        const double y = x < 0.0 ? __dadd_rn(x, p) : x;
-        const double z = __dadd_rn(y, 4503599627370496.0);
-        return __longlong_as_double(__double_as_longlong(z) & 0x000fffffffffffffll);
-    }
+    // an inverse output (|x| < p) in [0, p)
+    __device__ __forceinline__ T inv_out(T x) const { return x < 0.0 ? __dadd_rn(x, p) : x; }
     __device__ __forceinline__ T scale_out(T x, const Tw<T>& w) const { return inv_out(mulc(x, w)); }
 };
 

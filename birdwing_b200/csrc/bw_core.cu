@@ -227,6 +227,47 @@ inline void set_c(Ar64& a, uint64_t p) {
     a.oneq = (uint64_t)(((u128)1 << 64) / p);
 }
 
+// Constants of the 64-bit coefficients' reconstruction.
+template <class Ar>
+void crt_constants(const bw_plan* pl, const uint64_t* P, GarnerDev<Ar>& g) {
+    // product of the primes but one (skip), modulo 2^160
+    auto product = [&](int skip, uint32_t* v) {
+        for (int i = 0; i < 5; ++i) v[i] = i == 0;
+        for (int k = 0; k < pl->K; ++k) {
+            if (k == skip) continue;
+            u128 c = 0;
+            for (int i = 0; i < 5; ++i) {
+                c += (u128)v[i] * P[k];
+                v[i] = (uint32_t)c;
+                c >>= 32;
+            }
+        }
+    };
+    for (int k = 0; k < pl->K; ++k) {
+        product(k, g.m[k]);
+        if (pl->K == 6) g.v[k] = (uint32_t)((1ull << 61) / P[k]);
+        if (k < kDigitPrimes) g.vi[k] = 1.0 / (double)P[k];
+    }
+    uint32_t p[5];
+    product(-1, p);
+    uint64_t borrow = 0;  // 0 - P
+    for (int i = 0; i < 5; ++i) {
+        const uint64_t d = 0 - (uint64_t)p[i] - borrow;
+        g.np[i] = (uint32_t)d;
+        borrow = (d >> 32) & 1;
+    }
+    g.top_bound = std::min(pl->nca, pl->ncb);
+}
+
+// (P / p_k)^-1 mod p_k, the factor the inverse transform's scale carries for
+// 64-bit coefficients.
+uint64_t crt_factor(const uint64_t* P, int K, int k) {
+    uint64_t m = 1;
+    for (int j = 0; j < K; ++j)
+        if (j != k) m = mulmod(m, P[j] % P[k], P[k]);
+    return invmod(m, P[k]);
+}
+
 // A plan's arithmetic and Garner constants and its geometry (everything but
 // the tables).
 template <class Ar>
@@ -249,8 +290,9 @@ void fill_constants(const bw_plan* pl, PlanDev<Ar>& pd) {
     }
     // unused prime slots get harmless arithmetic constants
     for (int k = pl->K; k < kMaxPrimes; ++k) pd.pr[k] = pd.pr[0];
-    if constexpr (!Ar::kF64) {
     auto& g = pd.gar;
+    if (pl->w64) crt_constants<Ar>(pl, P, g);
+    if constexpr (!Ar::kF64) {
     const uint64_t p0 = P[0], p1 = P[1], p2 = P[2];
     g.p0 = p0;
     g.inv1 = (T)invmod(p0 % p1, p1);
@@ -259,16 +301,6 @@ void fill_constants(const bw_plan* pl, PlanDev<Ar>& pd) {
     g.p0m2q = (T)shoup_pre(g.p0m2, p2, bits);
     g.inv2 = (T)invmod(mulmod(p0 % p2, p1 % p2, p2), p2);
     g.inv2q = (T)shoup_pre(g.inv2, p2, bits);
-    g.p01_lo = (uint64_t)((u128)p0 * p1);
-    g.p01_hi = (uint64_t)(((u128)p0 * p1) >> 64);
-    if (pl->K == 6) {
-        for (int i = 1; i < 6; ++i)
-            for (int j = 0; j < i; ++j) {
-                const uint64_t v = invmod(P[j] % P[i], P[i]);
-                g.inv6[i * (i - 1) / 2 + j] = Tw<T>{(T)v, (T)shoup_pre(v, P[i], bits)};
-            }
-    }
-    g.top_bound = std::min(pl->nca, pl->ncb);
     }
     pd.K = pl->K;
     pd.log_n = pl->log_n;
@@ -300,6 +332,7 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
     for (int k = 0; k < pl->K; ++k) {
         const uint64_t p = P[k];
         scale_k[k] = mulmod(invmod(n % p, p), powmod(2, bits, p), p);
+        if (pl->w64) scale_k[k] = mulmod(scale_k[k], crt_factor(P, pl->K, k), p);
         if (pl->small) {
             // single pass: n-point stage tables only
             const uint64_t wn = powmod(Gn[k], (p - 1) >> pl->log_n, p);
@@ -318,11 +351,10 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
         off[k][2] = tb.add_stage_table(p, wc, pl->log_c, vr);
         off[k][3] = tb.add_stage_table(p, invmod(wc, p), pl->log_c, vr);
         const size_t nlo = (size_t)1 << pl->lo, nhi = n_row >> pl->lo;
-        const uint64_t scale = mulmod(invmod(n % p, p), powmod(2, bits, p), p);
         off[k][4] = tb.add_power_table(p, wrow, nlo, 1);
         off[k][5] = tb.add_power_table(p, powmod(wrow, nlo, p), nhi, 1);
         off[k][6] = tb.add_power_table(p, wrowi, nlo, 1);
-        off[k][7] = tb.add_power_table(p, powmod(wrowi, nlo, p), nhi, scale);
+        off[k][7] = tb.add_power_table(p, powmod(wrowi, nlo, p), nhi, scale_k[k]);
         if (pl->log_r2) {
             const uint64_t wm = powmod(wn, n >> pl->log_r2, p);  // R2-th root
             off[k][8] = tb.add_stage_table(p, wm, pl->log_r2);
@@ -686,7 +718,6 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
                    : pl->f64 == 2          ? build_tables<ArD<1>>(pl, pl->pdd1)
                    : path == BW_PATH_P64 ? build_tables<Ar64>(pl, pl->pd64)
                                            : build_tables<Ar32>(pl, pl->pd32);
-    if (pl->f64) fill_constants<Ar64>(pl, pl->pd64);  // Garner reads integers
     if (rc && pl->d_tables) {
         cudaFree(pl->d_tables);
         pl->d_tables = nullptr;
@@ -1010,14 +1041,26 @@ int enqueue_carry(bw_ctx* c, uint32_t* out, int pieces = 1) {
     const size_t n = (size_t)1 << pl->log_n;
     const size_t NL = W64 ? 2 * n : n / (SPLIT16 ? 2 : 1);
     const size_t M = pl->la + pl->lb;
-    uint32_t epoch = 1;
-    if (!c->capturing) {
-        if (++c->epoch >= (1u << 28)) {
-            c->epoch = 2;
-            BW_CUDA(cudaMemsetAsync(c->d_state + 32, 0, c->state_bytes - 32, c->stream));
-        }
-        epoch = c->epoch;
+    if (pieces == 1 && !c->inject_wait_fault) {
+        // one piece: no waits between tiles; the look-back form below stays
+        // for pieces that are copied out one by one and for the
+        // fault-injection hook, whose waits it tests
+        c->out_tiles_per = c->ntiles;
+        k_carry_words<Ar, SPLIT16, W64><<<(unsigned)c->ntiles, kWordsThreads, 0, c->stream>>>(
+            pd, reinterpret_cast<const T*>(c->d_res_a), out, M, NL, c->rec_s, &c->cst->any,
+            c->err);
+        if (c->ntiles > 1)
+            k_carry_fix<<<1, kFixThreads, 0, c->stream>>>(c->rec_s, (uint32_t)c->ntiles, out, M,
+                                                          &c->cst->any);
+        c->out_pieces = 1;
+        BW_CUDA(cudaGetLastError());
+        return BW_OK;
     }
+    if (++c->epoch >= (1u << 28)) {
+        c->epoch = 2;
+        BW_CUDA(cudaMemsetAsync(c->d_state + 32, 0, c->state_bytes - 32, c->stream));
+    }
+    const uint32_t epoch = c->epoch;
     if (c->ntiles > 1) {
         const unsigned nb = (unsigned)((c->ntiles - 1 + 255) / 256);
         k_carry_bounds<Ar, SPLIT16, W64><<<nb, 256, 0, c->stream>>>(
@@ -1030,18 +1073,6 @@ int enqueue_carry(bw_ctx* c, uint32_t* out, int pieces = 1) {
     const size_t per = (c->ntiles + pieces - 1) / pieces;
     c->out_pieces = 0;
     c->out_tiles_per = per;
-    if (pieces == 1 && !c->inject_wait_fault) {
-        // one piece: the words pass (no waits between tiles) and the carry
-        // fix; the look-back form below stays for pieces that are copied out
-        // one by one and for the fault-injection hook, whose waits it tests
-        k_garner_words<Ar, SPLIT16, W64><<<(unsigned)c->ntiles, kCarryThreads, 0, c->stream>>>(
-            pd, reinterpret_cast<const T*>(c->d_res_a), out, M, NL, c->rec_x, c->rec_s, c->err);
-        if (c->ntiles > 1)
-            k_carry_fix<<<1, kFixThreads, 0, c->stream>>>(c->rec_s, (uint32_t)c->ntiles, out, M);
-        c->out_pieces = 1;
-        BW_CUDA(cudaGetLastError());
-        return BW_OK;
-    }
     for (size_t t0 = 0; t0 < c->ntiles; t0 += per) {
         const unsigned nb = (unsigned)std::min(per, c->ntiles - t0);
         k_garner_carry<Ar, SPLIT16, W64><<<nb, kCarryThreads, 0, c->stream>>>(
@@ -1068,7 +1099,10 @@ int enqueue_product(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_t* o
              : pl->f64 == 2
                  ? bw_enqueue_transform<ArD<1>, false, true>(c, a, b, square, timing, io)
                  : bw_enqueue_transform<Ar64, false, true>(c, a, b, square, timing, io);
-        if (!rc) rc = enqueue_carry<Ar64, false, true>(c, out, pieces);
+        if (!rc)
+            rc = pl->f64 == 1   ? enqueue_carry<ArD<0>, false, true>(c, out, pieces)
+                 : pl->f64 == 2 ? enqueue_carry<ArD<1>, false, true>(c, out, pieces)
+                                : enqueue_carry<Ar64, false, true>(c, out, pieces);
     } else if (pl->path == BW_PATH_P64) {
         rc = bw_enqueue_transform<Ar64, false>(c, a, b, square, timing, io);
         if (!rc) rc = enqueue_carry<Ar64, false>(c, out, pieces);
@@ -1103,10 +1137,8 @@ static int launch_graph(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_
         int rc = bw_set_kernel_attrs();
         if (rc) return rc;
         BW_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        c->capturing = true;
-        cudaError_t e = cudaMemsetAsync(c->d_state + 32, 0, c->state_bytes - 32, c->stream);
-        rc = e == cudaSuccess ? enqueue_product(c, a, b, out, sq, false) : BW_OK;
-        c->capturing = false;
+        cudaError_t e = cudaSuccess;
+        rc = enqueue_product(c, a, b, out, sq, false);
         cudaGraph_t g = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
         if (rc || e != cudaSuccess || e2 != cudaSuccess) {

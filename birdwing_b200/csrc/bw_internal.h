@@ -121,7 +121,6 @@ struct bw_ctx {
     // look-back record tag of the last product.  Direct launches use 2, 3, ..;
     // the replayable graph clears the records and always uses 1.
     uint32_t epoch = 1;
-    bool capturing = false;
     cudaGraphExec_t gexec = nullptr;  // device-pointer product, replayed while
     const void* g_a = nullptr;        // the pointers stay the same
     const void* g_b = nullptr;

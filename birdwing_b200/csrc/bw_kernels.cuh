@@ -81,13 +81,14 @@ struct GarnerDev {
     T p0m2, p0m2q;      // p0 mod p2
     T inv2, inv2q;      // (p0 p1)^-1 mod p2
     uint64_t p0;        // p0 as an integer
-    uint64_t p01_lo, p01_hi;  // p0 p1 as a 128-bit integer (64-bit coefficients)
-    // 64-bit coefficients: a product's coefficients stay below this times
-    // 2^128 (min(na, nb)); one that reaches it flags an error
+    // 64-bit coefficients (garner_words_w64_at), 32-bit limbs:
+    uint32_t m[kMaxPrimes][5];  // M_k = P / p_k, P the product of the primes
+    uint32_t np[5];             // 2^160 - P mod 2^160
+    uint32_t v[kMaxPrimes];     // six primes: floor(2^61 / p_k)
+    double vi[kDigitPrimes];    // three primes: 1 / p_k
+    // a product's coefficients stay below this times 2^128 (min(na, nb)); one
+    // that reaches it flags an error
     uint64_t top_bound;
-    // six primes (32-bit path, 64-bit coefficients): p_j^-1 mod p_i with
-    // Shoup companions, pair (i, j < i) at index i (i - 1) / 2 + j
-    Tw<T> inv6[15];
 };
 
 template <class Ar>
@@ -107,7 +108,8 @@ struct PlanDev {
 // Carry look-back state of one context.
 struct CarryState {
     uint32_t counter;   // dynamic tile ticket (reset by K3 before every K4)
-    uint32_t pad[3];
+    uint32_t any;       // some tile's kind is not kill (k_carry_words, cleared by k_carry_fix)
+    uint32_t pad[2];
 };
 
 // One product of a batch (device memory).  Residues of product i live at
@@ -1328,181 +1330,151 @@ __device__ __forceinline__ void garner_digits(const PlanDev<Ar>& P,
                                          bad_out);
 }
 
-// 64-bit coefficients (three primes): the E output words from word j0 (j0
-// even, E/2 coefficients from coefficient j0/2) and the carry-out X.  Each
-// coefficient is the full mixed-radix value c = r0 + p0 k1 + p0 p1 k2
-// (< p0 p1 p2; the coefficients of a product stay below min(na, nb) 2^128, so a
-// c2 at or above G.top_bound = min(na, nb) flags an error).  The words are
-// the low 32 E bits of V = sum_q c_q 2^(64 q), X = V >> 32 E (< 2^96).
-// Coefficients at or beyond NL / 2 read nothing and are zero.
-template <class Ar, int E, bool NC>
-__device__ __forceinline__ void garner3_words_at(const PlanDev<Ar>& P,
-                                                 const typename Ar::T* __restrict__ base,
-                                                 size_t pstride, bool valid,
-                                                 uint32_t (&l)[E], uint32_t (&X)[3],
-                                                 uint32_t* bad_out) {
-    using T = typename Ar::T;
-    static_assert(sizeof(T) == 8 && E % 4 == 0, "64-bit residues, whole 16-byte loads");
-    constexpr int Q = E / 2;
-    T r[3][Q];
+// Multi-word additions by carry chains.
+// w[0..N] = sum_i col[i] 2^(32 i), col[i] 64 bits
+template <int N>
+__device__ __forceinline__ void columns_to_words(const uint64_t (&col)[N], uint32_t (&w)[N + 1]) {
+    uint32_t h = (uint32_t)(col[0] >> 32);
+    w[0] = (uint32_t)col[0];
 #pragma unroll
-    for (int kp = 0; kp < 3; ++kp)
-#pragma unroll
-        for (int q = 0; q < Q; ++q) r[kp][q] = 0;
-    if (valid) {
-#pragma unroll
-        for (int kp = 0; kp < 3; ++kp) {
-            const uint4* src = reinterpret_cast<const uint4*>(base + (size_t)kp * pstride);
-#pragma unroll
-            for (int h = 0; h < Q / 2; ++h) {
-                const uint4 v = NC ? __ldg(src + h) : src[h];
-                r[kp][2 * h] = ((uint64_t)v.y << 32) | v.x;
-                r[kp][2 * h + 1] = ((uint64_t)v.w << 32) | v.z;
-            }
-        }
+    for (int i = 1; i < N; ++i) {
+        const uint32_t lo = (uint32_t)col[i], hi = (uint32_t)(col[i] >> 32);
+        asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, 0;"
+            : "=&r"(w[i]), "=r"(h)
+            : "r"(lo), "r"(h), "r"(hi));
     }
-    const Ar a1 = P.pr[1].ar, a2 = P.pr[2].ar;
-    const GarnerDev<Ar>& G = P.gar;
-    uint32_t bad = 0;
-    uint64_t acc0 = 0, acc1 = 0;  // running carry (< 2^96)
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        const T r0 = r[0][q];
-        const T r0m1 = a1.red1(a1.shoup(r0, 1, P.pr[1].one_q));
-        const T t1 = r[1][q] >= r0m1 ? r[1][q] - r0m1 : r[1][q] + a1.p - r0m1;
-        const T k1 = a1.red1(a1.shoup(t1, G.inv1, G.inv1q));
-        const T r0m2 = a2.red1(a2.shoup(r0, 1, P.pr[2].one_q));
-        const T y = a2.red1(r0m2 + a2.red1(a2.shoup(k1, G.p0m2, G.p0m2q)));
-        const T r2 = r[2][q];
-        const T t2 = r2 >= y ? r2 - y : r2 + a2.p - y;
-        const T k2 = a2.red1(a2.shoup(t2, G.inv2, G.inv2q));
-        // c = (r0 + p0 k1) + p01_lo k2 + (p01_hi k2) 2^64
-        const unsigned __int128 lo =
-            (unsigned __int128)G.p0 * k1 + r0 + (unsigned __int128)G.p01_lo * k2;  // < 2^127
-        const unsigned __int128 hi = (lo >> 64) + (unsigned __int128)G.p01_hi * k2;
-        const uint64_t c0 = (uint64_t)lo, c1 = (uint64_t)hi, c2 = (uint64_t)(hi >> 64);
-        bad |= (uint32_t)(c2 >= G.top_bound);
-        // add c to the running carry; emit 64 bits; shift
-        const unsigned __int128 s0 = (unsigned __int128)acc0 + c0;
-        l[2 * q] = (uint32_t)s0;
-        l[2 * q + 1] = (uint32_t)((uint64_t)s0 >> 32);
-        const unsigned __int128 s1 = (unsigned __int128)acc1 + c1 + (uint64_t)(s0 >> 64);
-        acc0 = (uint64_t)s1;
-        acc1 = c2 + (uint64_t)(s1 >> 64);
-    }
-    X[0] = (uint32_t)acc0;
-    X[1] = (uint32_t)(acc0 >> 32);
-    X[2] = (uint32_t)acc1;
-    bad |= (uint32_t)((acc1 >> 32) != 0);
-    *bad_out |= bad;
+    w[N] = h;
+}
+// a += b (5 words; the carry out of the last is dropped)
+__device__ __forceinline__ void add5(uint32_t (&a)[5], const uint32_t (&b)[5]) {
+    asm("add.cc.u32 %0, %0, %5;\n\taddc.cc.u32 %1, %1, %6;\n\taddc.cc.u32 %2, %2, %7;\n\t"
+        "addc.cc.u32 %3, %3, %8;\n\taddc.u32 %4, %4, %9;"
+        : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4])
+        : "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]));
 }
 
-// Six primes below 2^30 (32-bit path, 64-bit coefficients): the same words
-// and carry-out as garner3_words_at.  The primes ascend, so a digit k_j
-// (< p_j) is already below every later prime.  Mixed radix: k_0 = r_0 and
-// k_i = (...((r_i - k_0) p_0^-1 - k_1) p_1^-1 ... - k_(i-1)) p_(i-1)^-1 mod p_i;
-// c = k_0 + p_0 (k_1 + p_1 (k_2 + p_2 (k_3 + p_3 (k_4 + p_4 k_5)))) < P < 2^178.
-// A product's coefficients stay below min(na, nb) 2^128 <= 2^150, so a top
-// word c2 at or above G.top_bound = min(na, nb) flags an error (residues that
-// disagree give a c spread over [0, P)).
-template <class Ar, int E, bool NC>
-__device__ __forceinline__ void garner6_words_at(const PlanDev<Ar>& P,
-                                                 const uint32_t* __restrict__ base,
-                                                 size_t pstride, bool valid, uint32_t (&l)[E],
-                                                 uint32_t (&X)[3], uint32_t* bad_out) {
-    constexpr int Q = E / 2;
-    static_assert(Q % 4 == 0, "whole 16-byte loads");
-    uint32_t r[6][Q];
-#pragma unroll
-    for (int kp = 0; kp < 6; ++kp)
-#pragma unroll
-        for (int q = 0; q < Q; ++q) r[kp][q] = 0;
-    if (valid) {
-#pragma unroll
-        for (int kp = 0; kp < 6; ++kp) {
-            const uint4* src = reinterpret_cast<const uint4*>(base + (size_t)kp * pstride);
-#pragma unroll
-            for (int h = 0; h < Q / 4; ++h) {
-                const uint4 v = NC ? __ldg(src + h) : src[h];
-                r[kp][4 * h] = v.x;
-                r[kp][4 * h + 1] = v.y;
-                r[kp][4 * h + 2] = v.z;
-                r[kp][4 * h + 3] = v.w;
-            }
-        }
-    }
-    const GarnerDev<Ar>& G = P.gar;
-    uint32_t bad = 0;
-    uint64_t acc0 = 0, acc1 = 0;  // running carry (< 2^96)
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        uint32_t k[6];
-        k[0] = r[0][q];
-#pragma unroll
-        for (int i = 1; i < 6; ++i) {
-            const Ar ai = P.pr[i].ar;
-            // t stays in [0, 2p_i): t - k_j + p_i < 3p_i < 2^32 is a valid
-            // Shoup input, and only the digit itself is reduced to [0, p_i)
-            uint32_t t = r[i][q];
-#pragma unroll
-            for (int j = 0; j < i; ++j) {
-                const Tw<uint32_t> iv = G.inv6[i * (i - 1) / 2 + j];
-                t = ai.shoup(t - k[j] + ai.p, iv.w, iv.wq);  // k_j < p_j < p_i
-            }
-            k[i] = ai.red1(t);
-        }
-        // Horner in 32-bit limbs, each step a chain of 32 x 32 + 64-bit
-        // multiply-adds: (k5 p4 + k4) (2 limbs), times p3 plus k3 (3), ...,
-        // times p0 plus k0 (6 limbs, < 2^178)
-        uint32_t w[6];
-        {
-            const uint64_t t = (uint64_t)k[5] * P.pr[4].ar.p + k[4];
-            w[0] = (uint32_t)t;
-            w[1] = (uint32_t)(t >> 32);
-        }
-#pragma unroll
-        for (int st = 0; st < 4; ++st) {
-            const uint32_t pm = P.pr[3 - st].ar.p;
-            uint64_t t = k[3 - st];
-#pragma unroll
-            for (int i = 0; i < 2 + st; ++i) {
-                t = (uint64_t)w[i] * pm + t;
-                w[i] = (uint32_t)t;
-                t >>= 32;
-            }
-            w[2 + st] = (uint32_t)t;
-        }
-        const uint64_t c0 = ((uint64_t)w[1] << 32) | w[0];
-        const uint64_t c1 = ((uint64_t)w[3] << 32) | w[2];
-        const uint64_t c2 = ((uint64_t)w[5] << 32) | w[4];
-        bad |= (uint32_t)(c2 >= G.top_bound);
-        const unsigned __int128 s0 = (unsigned __int128)acc0 + c0;
-        l[2 * q] = (uint32_t)s0;
-        l[2 * q + 1] = (uint32_t)((uint64_t)s0 >> 32);
-        const unsigned __int128 s1 = (unsigned __int128)acc1 + c1 + (uint64_t)(s0 >> 64);
-        acc0 = (uint64_t)s1;
-        acc1 = c2 + (uint64_t)(s1 >> 64);
-    }
-    X[0] = (uint32_t)acc0;
-    X[1] = (uint32_t)(acc0 >> 32);
-    X[2] = (uint32_t)acc1;
-    bad |= (uint32_t)((acc1 >> 32) != 0);
-    *bad_out |= bad;
-}
-
-// 64-bit coefficients: three 58-bit primes (64-bit path) or six 30-bit
-// primes (32-bit path).
+// 64-bit coefficients: the E output words from word j0 (j0 even, E/2
+// coefficients from coefficient j0/2) and the carry-out X.  The inverse
+// transform's scale carries the factor (P / p_k)^-1 mod p_k besides n^-1, so
+// the residues are y_k with
+//
+//   c = sum_k y_k M_k - q P,   M_k = P / p_k,   q = floor(sum_k y_k / p_k)
+//
+// -- no modular arithmetic is left here (mixed-radix digits took 6 to 15
+// modular products in a chain per coefficient: 177 (six primes) to 235 (three)
+// instructions, bound by the multiply pipe at 70-83%).  All of it runs modulo
+// 2^160, above every coefficient: y_k M_k as columns of 32 x 32-bit products,
+// y_k whole (six primes, two sets of columns so that none overflows) or in two
+// parts of B bits (two sets, the second shifted by B), and -q P as q (2^160 - P).
+// q: c / P stays below 1 - 2^-13 (three primes; 2^-27 for six), so the estimate
+// of the sum plus 2^-20 (2^-28) has the right floor.  Coefficients of a product
+// stay below min(na, nb) 2^128: a c at or above it flags an error.
+// The words are the low 32 E bits of V = sum_q c_q 2^(64 q), X = V >> 32 E
+// (< 2^96).  Coefficients at or beyond NL / 2 read nothing and are zero.
 template <class Ar, int E, bool NC = true>
 __device__ __forceinline__ void garner_words_w64_at(const PlanDev<Ar>& P,
                                                     const typename Ar::T* __restrict__ base,
                                                     size_t pstride, bool valid,
                                                     uint32_t (&l)[E], uint32_t (&X)[3],
                                                     uint32_t* bad_out) {
-    if constexpr (sizeof(typename Ar::T) == 4) {
-        garner6_words_at<Ar, E, NC>(P, base, pstride, valid, l, X, bad_out);
-    } else {
-        garner3_words_at<Ar, E, NC>(P, base, pstride, valid, l, X, bad_out);
+    using T = typename Ar::T;
+    constexpr bool SIX = sizeof(T) == 4;
+    constexpr int Q = E / 2, K = SIX ? 6 : 3, ML = SIX ? 5 : 4;
+    constexpr int B = Ar::kF64 ? 26 : 29;  // the lower part of a residue
+    constexpr int PER = 16 / (int)sizeof(T);
+    static_assert(Q % PER == 0, "whole 16-byte loads");
+    uint4 raw[K][Q / PER];
+#pragma unroll
+    for (int kp = 0; kp < K; ++kp) {
+        const uint4* src = reinterpret_cast<const uint4*>(base + (size_t)kp * pstride);
+#pragma unroll
+        for (int h = 0; h < Q / PER; ++h)
+            raw[kp][h] = valid ? (NC ? __ldg(src + h) : src[h]) : make_uint4(0, 0, 0, 0);
     }
+    const GarnerDev<Ar>& G = P.gar;
+    uint32_t bad = 0;
+    uint32_t acc[5] = {0, 0, 0, 0, 0};  // running carry (< 2^96)
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        // c0, c1: the two sets' columns
+        uint64_t c0[ML] = {}, c1[ML] = {};
+        uint32_t quo;
+        if constexpr (SIX) {
+            uint64_t s61 = 1ull << 33;
+#pragma unroll
+            for (int kp = 0; kp < K; ++kp) {
+                const uint4 v = raw[kp][q / 4];
+                const uint32_t y = q % 4 == 0 ? v.x : q % 4 == 1 ? v.y : q % 4 == 2 ? v.z : v.w;
+                s61 += (uint64_t)y * G.v[kp];
+#pragma unroll
+                for (int i = 0; i < ML; ++i) (kp < 4 ? c0 : c1)[i] += (uint64_t)y * G.m[kp][i];
+            }
+            quo = (uint32_t)(s61 >> 61);
+#pragma unroll
+            for (int i = 0; i < ML; ++i) c1[i] += (uint64_t)quo * G.np[i];
+        } else {
+            double sd = 1.0 / (1 << 20) - 0.5;
+#pragma unroll
+            for (int kp = 0; kp < K; ++kp) {
+                const uint4 v = raw[kp][q / 2];
+                uint32_t lo = q % 2 == 0 ? v.x : v.z, hi = q % 2 == 0 ? v.y : v.w;
+                if constexpr (Ar::kF64) {
+                    const double d = __hiloint2double((int)hi, (int)lo);
+                    sd = __fma_rn(d, G.vi[kp], sd);
+                    // the integer is the low 52 bits of d + 2^52
+                    const double z = __dadd_rn(d, 4503599627370496.0);
+                    lo = (uint32_t)__double2loint(z);
+                    hi = (uint32_t)__double2hiint(z) & 0xfffffu;
+                } else {
+                    sd = __fma_rn((double)(((uint64_t)hi << 32) | lo), G.vi[kp], sd);
+                }
+                const uint32_t y0 = lo & ((1u << B) - 1), y1 = __funnelshift_r(lo, hi, B);
+#pragma unroll
+                for (int i = 0; i < ML; ++i) {
+                    c0[i] += (uint64_t)y0 * G.m[kp][i];
+                    c1[i] += (uint64_t)y1 * G.m[kp][i];
+                }
+            }
+            // the floor: (sum + 2^-20) - 1/2 rounded to an integer
+            quo = (uint32_t)__double2loint(__dadd_rn(sd, 6755399441055744.0));
+        }
+        uint32_t c[5], d[5];
+        if constexpr (SIX) {
+            uint32_t w0[6], w1[6];
+            columns_to_words<5>(c0, w0);
+            columns_to_words<5>(c1, w1);
+#pragma unroll
+            for (int i = 0; i < 5; ++i) {
+                c[i] = w0[i];
+                d[i] = w1[i];
+            }
+        } else {
+            uint64_t c0p[5] = {c0[0], c0[1], c0[2], c0[3], 0};
+#pragma unroll
+            for (int i = 0; i < 5; ++i) c0p[i] += (uint64_t)quo * G.np[i];
+            uint32_t w0[6], w1[5];
+            columns_to_words<5>(c0p, w0);
+            columns_to_words<4>(c1, w1);
+            d[0] = w1[0] << B;
+#pragma unroll
+            for (int i = 1; i < 5; ++i) d[i] = __funnelshift_l(w1[i - 1], w1[i], B);
+#pragma unroll
+            for (int i = 0; i < 5; ++i) c[i] = w0[i];
+        }
+        add5(c, d);
+        bad |= (uint32_t)(c[4] >= (uint32_t)G.top_bound);
+        // add c to the running carry; emit 64 bits; shift
+        add5(c, acc);
+        l[2 * q] = c[0];
+        l[2 * q + 1] = c[1];
+        acc[0] = c[2];
+        acc[1] = c[3];
+        acc[2] = c[4];
+    }
+    X[0] = acc[0];
+    X[1] = acc[1];
+    X[2] = acc[2];
+    *bad_out |= bad;
 }
 
 template <class Ar, int E, bool NC = true>
@@ -1536,9 +1508,8 @@ __device__ __forceinline__ ChainMasks chain_prepare(int st, uint32_t* s_w) {
     }
     return m;
 }
-__device__ __forceinline__ uint32_t chain_out(const uint32_t* s_w, uint32_t cin) {
+__device__ __forceinline__ uint32_t chain_out(const uint32_t* s_w, uint32_t cin, int nw) {
     uint32_t c = cin;
-    const int nw = blockDim.x >> 5;
     for (int w = 0; w < nw; ++w) c = (s_w[w] >> c) & 1u;
     return c;
 }
@@ -1642,7 +1613,8 @@ __device__ __forceinline__ void carry_finish_tile(
 
     // ---- tile status, publish, look back (thread 0)
     if (tid == 0) {
-        const uint32_t c0 = chain_out(sh.w, 0u), c1 = chain_out(sh.w, 1u);
+        const uint32_t c0 = chain_out(sh.w, 0u, kCarryThreads / 32),
+                       c1 = chain_out(sh.w, 1u, kCarryThreads / 32);
         const uint32_t kind = c0 ? 2u : (c1 ? 1u : 0u);
         const uint32_t tag = epoch << 4;
         uint32_t eps_in = 0;
@@ -1767,108 +1739,29 @@ __device__ __forceinline__ void garner_carry_body(
 
 // K4 without waits (single products).  The look-back form above keeps every
 // CTA of a tile waiting on its predecessor's records: two or three dependent
-// L2 round trips per tile with the whole CTA at a barrier.  Here the 1-bit
-// tile carry is left out of the first pass instead: k_carry_bounds has
-// already published every tile boundary's carry words X, so tile t writes its
-// words as if the carry bit eps into it were 0 and records its kind -- the
-// carry bit it passes on for eps = 0 and for eps = 1 (kill: 0/0, propagate:
-// 0/1, generate: 1/1).  k_carry_fix then scans the kinds (eps into tile 0 is
-// 0) and adds 1 at the first word of each tile whose eps is 1, rippling
-// inside the tile (a tile that propagates passes the carry on through the
-// next tile's own eps).  For operands of random words no tile but an
-// all-ones span generates or propagates, so the fix pass writes nothing.
-template <class Ar, bool SPLIT16, bool W64 = false>
-__global__ void __launch_bounds__(kCarryThreads, 4)
-k_garner_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
-               uint32_t* __restrict__ out, size_t M, size_t NL,
-               const uint4* __restrict__ rec_x, uint32_t* __restrict__ kinds,
-               uint32_t* __restrict__ err) {
-    constexpr int E = kCarryWordsPerThread;
-    constexpr int TL = kCarryTileWords;
-    __shared__ CarryShared sh;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t t = blockIdx.x;
-    const size_t j0 = (size_t)t * TL + (size_t)tid * E;
-    const size_t n = (size_t)1 << P.log_n;
-    if (tid == 0) {
-        // the previous tile's boundary carry words, from the pre-pass
-        uint4 px = make_uint4(0, 0, 0, 0);
-        if (t > 0) px = __ldcg(rec_x + (t - 1));
-        sh.cin[0] = px.x;
-        sh.cin[1] = px.y;
-        sh.cin[2] = px.z;
-    }
-    uint32_t l[E];
-    uint32_t X[3];
-    uint32_t bad = 0;
-    garner_local<Ar, SPLIT16, W64, true>(P, res + j0 * elems_per_word2<SPLIT16, W64>() / 2, n,
-                                         j0 < NL, l, X, &bad);
-    if (bad) atomicOr(err, 2u);
-    uint32_t PX[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) PX[q] = __shfl_up_sync(0xffffffffu, X[q], 1);
-    if (lane == 31) {
-        sh.lastx[warp][0] = X[0];
-        sh.lastx[warp][1] = X[1];
-        sh.lastx[warp][2] = X[2];
-    }
-    __syncthreads();
-    if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) PX[q] = warp > 0 ? sh.lastx[warp - 1][q] : sh.cin[q];
-    }
-    uint32_t S[E];
-    int st;
-    {
-        uint64_t c = 0;
-        uint32_t all = 0xffffffffu;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const uint64_t sum = (uint64_t)l[e] + (e < 3 ? PX[e] : 0u) + c;
-            S[e] = (uint32_t)sum;
-            c = sum >> 32;
-            all &= S[e];
-        }
-        st = c ? 2 : (all == 0xffffffffu ? 1 : 0);
-    }
-    const ChainMasks cm = chain_prepare(st, sh.w);
-    __syncthreads();
-    if (tid == 0) {
-        const uint32_t c0 = chain_out(sh.w, 0u), c1 = chain_out(sh.w, 1u);
-        kinds[t] = c0 | (c1 << 1);
-    }
-    const uint32_t mc = chain_mine(cm, sh.w, 0u);
-    uint32_t w[E];
-    {
-        uint64_t c = mc;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const uint64_t sum = (uint64_t)S[e] + c;
-            w[e] = (uint32_t)sum;
-            c = sum >> 32;
-        }
-    }
-    if (j0 + E <= M && ((reinterpret_cast<uintptr_t>(out + j0) & 15u) == 0)) {
-        uint4* o = reinterpret_cast<uint4*>(out + j0);
-        o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        o[1] = make_uint4(w[4], w[5], w[6], w[7]);
-    } else {
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-            if (j0 + e < M) out[j0 + e] = w[e];
-    }
-}
+// L2 round trips per tile with the whole CTA at a barrier.  Here a ninth warp
+// computes the carry words X into the tile itself, from the eight words before
+// it (a pre-pass kernel for them took 4 us); the 1-bit tile carry is left out
+// of the words pass: tile t writes its words as if the carry bit eps into it
+// were 0 and records its kind -- the carry bit it passes on for eps = 0 and for
+// eps = 1 (kill: 0/0, propagate: 0/1, generate: 1/1).  Where any tile is not
+// kill, k_carry_fix scans the kinds (eps into tile 0 is 0) and adds 1 at the
+// first word of each tile whose eps is 1, rippling inside the tile (a tile that
+// propagates passes the carry on through the next tile's own eps).  For
+// operands of random words every tile but an all-ones span kills, and it
+// returns at once.  (Letting the tile that finishes last do the fix saves the
+// launch, but every tile's arrival then waits for its words to be visible:
+// 72 -> 92 us at 2^24 words, and no gain in a graph at 2^16.)
+constexpr int kWordsThreads = kCarryThreads + 32;
 
-// One CTA: the carry bit into every tile from the kinds k_garner_words left
-// (bit 0: carry out for carry-in 0, bit 1: for carry-in 1), then +1 at the
-// first word of every tile whose carry-in is 1, rippling inside the tile.
-// Each thread takes a contiguous run of tiles; a run passes on a constant
-// (its last non-propagating tile's carry) or its own carry-in, and a scan over
-// the runs in shared memory gives each run its carry-in.
+// One CTA: each thread takes a contiguous run of tiles; a run passes on a
+// constant (its last non-propagating tile's carry) or its own carry-in, and a
+// scan over the runs in shared memory gives each run its carry-in.
 constexpr int kFixThreads = 1024;
 static __global__ void __launch_bounds__(kFixThreads)
 k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __restrict__ out,
-            size_t M) {
+            size_t M, uint32_t* __restrict__ any) {
+    if (__ldcg(any) == 0u) return;  // every tile kills
     __shared__ uint32_t s_f[kFixThreads];  // 0, 1: constant carry out; 2: passes carry-in
     const int tid = threadIdx.x;
     const uint32_t per = (ntiles + kFixThreads - 1) / kFixThreads;
@@ -1880,6 +1773,7 @@ k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __res
     }
     s_f[tid] = f;
     __syncthreads();
+    if (tid == 0) *any = 0u;  // for the next product (every thread has read it)
     // inclusive scan of "the latest constant": combine(a, b) = b unless b
     // passes its carry-in
     for (int d = 1; d < kFixThreads; d <<= 1) {
@@ -1908,6 +1802,88 @@ k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __res
             }
         }
         eps = (k >> eps) & 1u;
+    }
+}
+
+// any: set when a tile's kind is not kill (zero between products).
+template <class Ar, bool SPLIT16, bool W64 = false>
+__global__ void __launch_bounds__(kWordsThreads, 3)
+k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
+              uint32_t* __restrict__ out, size_t M, size_t NL, uint32_t* __restrict__ kinds,
+              uint32_t* __restrict__ any, uint32_t* __restrict__ err) {
+    constexpr int E = kCarryWordsPerThread;
+    constexpr int TL = kCarryTileWords;
+    __shared__ CarryShared sh;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool own = tid < kCarryThreads;
+    const uint32_t t = blockIdx.x;
+    // this thread's words; the first thread of the ninth warp takes the eight
+    // words before the tile
+    const size_t j0 = own ? (size_t)t * TL + (size_t)tid * E : (size_t)t * TL - E;
+    const bool valid = (own || (tid == kCarryThreads && t > 0)) && j0 < NL;
+    const size_t n = (size_t)1 << P.log_n;
+    uint32_t l[E];
+    uint32_t X[3];
+    uint32_t bad = 0;
+    garner_local<Ar, SPLIT16, W64, true>(
+        P, res + (valid ? j0 : 0) * elems_per_word2<SPLIT16, W64>() / 2, n, valid, l, X, &bad);
+    if (bad && own) atomicOr(err, 2u);
+    uint32_t PX[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) PX[q] = __shfl_up_sync(0xffffffffu, X[q], 1);
+    if (own ? lane == 31 : lane == 0) {
+        uint32_t* d = own ? sh.lastx[warp] : sh.cin;
+        d[0] = X[0];
+        d[1] = X[1];
+        d[2] = X[2];
+    }
+    __syncthreads();
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) PX[q] = warp > 0 ? sh.lastx[own ? warp - 1 : 0][q] : sh.cin[q];
+    }
+    uint32_t S[E];
+    int st;
+    {
+        uint64_t c = 0;
+        uint32_t all = 0xffffffffu;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const uint64_t sum = (uint64_t)l[e] + (e < 3 ? PX[e] : 0u) + c;
+            S[e] = (uint32_t)sum;
+            c = sum >> 32;
+            all &= S[e];
+        }
+        st = c ? 2 : (all == 0xffffffffu ? 1 : 0);
+    }
+    ChainMasks cm{0, 0};
+    if (own) cm = chain_prepare(st, sh.w);
+    __syncthreads();
+    if (own) {
+        const uint32_t mc = chain_mine(cm, sh.w, 0u);
+        uint32_t w[E];
+        uint64_t c = mc;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const uint64_t sum = (uint64_t)S[e] + c;
+            w[e] = (uint32_t)sum;
+            c = sum >> 32;
+        }
+        if (j0 + E <= M && ((reinterpret_cast<uintptr_t>(out + j0) & 15u) == 0)) {
+            uint4* o = reinterpret_cast<uint4*>(out + j0);
+            o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if (j0 + e < M) out[j0 + e] = w[e];
+        }
+    }
+    if (tid == 0 && gridDim.x > 1) {
+        const uint32_t kind = chain_out(sh.w, 0u, kCarryThreads / 32) |
+                              (chain_out(sh.w, 1u, kCarryThreads / 32) << 1);
+        kinds[t] = kind;
+        if (kind) atomicOr(any, 1u);
     }
 }
 
@@ -2159,7 +2135,7 @@ __device__ __forceinline__ void ks_product_body(const PlanDev<Ar>& P, const Batc
         __syncthreads();
         const uint32_t eps_in = s_eps;
         const uint32_t mc = chain_mine(cm, s_w, eps_in);
-        const uint32_t cout = chain_out(s_w, eps_in);
+        const uint32_t cout = chain_out(s_w, eps_in, NT / 32);
         {
             uint64_t c = mc;
 #pragma unroll
