@@ -402,13 +402,14 @@ struct CoefLoad {
         lone = CW == 64 ? (uint32_t)(nc & 1) : 0u;
         al8 = (reinterpret_cast<uintptr_t>(l) & 7u) == 0;
     }
-    // coefficient ci, zero beyond the operand, as a residue
-    __device__ __forceinline__ T operator()(const Ar& ar, uint32_t ci) const {
+    using Raw = typename std::conditional<
+        CW == 64, uint64_t, typename std::conditional<CW == 32, uint32_t, uint16_t>::type>::type;
+    // coefficient ci, zero beyond the operand
+    __device__ __forceinline__ Raw load(uint32_t ci) const {
         if constexpr (CW == 16) {
-            const uint16_t* h = reinterpret_cast<const uint16_t*>(limbs);
-            return Ar::from_u32(ci < ncoef ? (uint32_t)__ldg(h + ci) : 0u);
+            return ci < ncoef ? __ldg(reinterpret_cast<const uint16_t*>(limbs) + ci) : (uint16_t)0;
         } else if constexpr (CW == 32) {
-            return Ar::from_u32(ci < ncoef ? __ldg(limbs + ci) : 0u);
+            return ci < ncoef ? __ldg(limbs + ci) : 0u;
         } else {
             uint64_t v = 0;
             const uint32_t* w = limbs + 2 * (size_t)ci;
@@ -421,11 +422,16 @@ struct CoefLoad {
             } else if (ci == ncoef && lone) {
                 v = __ldg(w);
             }
-            if constexpr (Ar::kF64) {
-                return ar.from_u64(v);
-            } else {
-                return ar.reduce64(v);
-            }
+            return v;
+        }
+    }
+    static __device__ __forceinline__ T residue(const Ar& ar, Raw v) {
+        if constexpr (CW != 64) {
+            return Ar::from_u32(v);
+        } else if constexpr (Ar::kF64) {
+            return ar.from_u64(v);
+        } else {
+            return ar.reduce64(v);
         }
     }
 };
@@ -454,6 +460,23 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
         constexpr bool ZT = decltype(zt_)::value;
         constexpr bool FIRST = S0 == 0, LAST = S0 + RL == LOGR;
         constexpr int D = LOGR - S0 - RL, DS = D + LCB, N = 1 << (LOGR + LCB - RL);
+        // the first round's loads run one sub-problem ahead of the arithmetic:
+        // every thread takes several sub-problems, each a DRAM or L2 latency
+        // (six primes at 2^23 words 0.408 -> 0.285 ms; long scoreboard stalls
+        // 7.3 per issue before).  Not in double precision, whose 80 registers
+        // have no room for it (0.225 -> 0.232 ms).
+        constexpr int NL = 1 << (ZT ? RL - 1 : RL);  // coefficients loaded
+        using Raw = typename CoefLoad<Ar, CW>::Raw;
+        constexpr bool AHEAD =
+            FIRST && N > NT && sizeof(T) == 4 && NL * sizeof(Raw) <= 64;
+        Raw raw[FIRST ? NL : 1];
+        auto load = [&](int sp) {
+            const int v = sp & (CB - 1), j = sp >> LCB;  // g = 0
+#pragma unroll
+            for (int k = 0; k < NL; ++k)
+                raw[k] = coef.load(((uint32_t)(j + (k << D)) << log_c) + c0 + v);
+        };
+        if constexpr (AHEAD) load(threadIdx.x);
 #pragma unroll 1
         for (int sp = threadIdx.x; sp < N; sp += NT) {
             const int v = sp & (CB - 1), rest = sp >> LCB;
@@ -461,14 +484,17 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
             const int base = (g << (D + RL)) + j;
             const int p0 = L::p((base << LCB) + v);
             T x[1 << RL];
+            if constexpr (FIRST) {
+                if constexpr (!AHEAD) load(sp);
 #pragma unroll
-            for (int k = 0; k < (1 << RL); ++k) {
-                if constexpr (FIRST) {
-                    if (ZT && k >= (1 << (RL - 1))) continue;
-                    x[k] = coef(ar, ((uint32_t)(base + (k << D)) << log_c) + c0 + v);
-                } else {
-                    x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
+                for (int k = 0; k < NL; ++k) x[k] = CoefLoad<Ar, CW>::residue(ar, raw[k]);
+                if constexpr (AHEAD) {
+                    if (sp + NT < N) load(sp + NT);
                 }
+            } else {
+#pragma unroll
+                for (int k = 0; k < (1 << RL); ++k)
+                    x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
             }
             ct_round<Ar, RL, FIRST, ZT, !FIRST>(x, ar, RoundTw<T, (1 << S0), false>(pr.WRf, g));
 #pragma unroll
