@@ -698,13 +698,16 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
             if (pl->log_r >= kCol2MinLog && pl->log_r <= top && !pl->tw_smem_r) {
                 pl->v2_cols = 1;
                 pl->tma_cols = 0;
-                // tiles of 64 KiB (8-byte residues: 32 KiB to 64 KiB in 2-8 columns;
-                // 4-byte: 4-16 columns); one prime per CTA, so that the narrower
-                // ones are taken only until every SM has two CTAs
-                const int lo_cb = w == 8 ? 1 : 2, hi_cb = w == 8 ? 3 : 4;
-                int cb = std::max(lo_cb, std::min(hi_cb, (w == 8 ? 13 : 14) - pl->log_r));
-                cb = std::min(cb, log_cols_outer);
-                while (cb > lo_cb && ((size_t)K << (log_cols_outer - cb)) < 2u * sms) --cb;
+                // tiles 32 bytes wide (4-byte residues) or up to 64, whole
+                // sectors, down to half of that for the longest columns.
+                // Narrower tiles to have more CTAs lose at every size: 4-byte
+                // residues in 16, 32 or 64 bytes measured, K1 + K3, 33 / 27 /
+                // 31 us (2^21 points of 16-bit coefficients), 0.146 / 0.121 /
+                // 0.131 ms (six primes, 2^21); 8-byte residues in 16, 32 or 64
+                // bytes 0.134 / 0.106 / 0.104 ms (2^21 points)
+                const int lo_cb = w == 8 ? 1 : 2;
+                const int cb = std::min(
+                    std::max(lo_cb, std::min(3, (w == 8 ? 13 : 14) - pl->log_r)), log_cols_outer);
                 pl->log_cb = pl->log_cb1 = cb;
                 if (cb < lo_cb) pl->v2_cols = 0;
             }
@@ -1034,7 +1037,7 @@ int copy_chunks_for(const bw_ctx* c, bool ordered) {
 }
 
 template <class Ar, bool SPLIT16, bool W64 = false>
-int enqueue_carry(bw_ctx* c, uint32_t* out, int pieces = 1) {
+int enqueue_carry(bw_ctx* c, uint32_t* out, bool timing, int pieces = 1) {
     using T = typename Ar::T;
     const bw_plan* pl = c->plan;
     const PlanDev<Ar>& pd = plan_dev<Ar>(pl);
@@ -1046,14 +1049,14 @@ int enqueue_carry(bw_ctx* c, uint32_t* out, int pieces = 1) {
         // for pieces that are copied out one by one and for the
         // fault-injection hook, whose waits it tests
         c->out_tiles_per = c->ntiles;
-        k_carry_words<Ar, SPLIT16, W64><<<(unsigned)c->ntiles, kWordsThreads, 0, c->stream>>>(
-            pd, reinterpret_cast<const T*>(c->d_res_a), out, M, NL, c->rec_s, &c->cst->any,
-            c->err);
+        BW_CUDA(launch_after(!timing, k_carry_words<Ar, SPLIT16, W64>,
+                             dim3((unsigned)c->ntiles), kWordsThreads, 0, c->stream, pd,
+                             reinterpret_cast<const T*>(c->d_res_a), out, M, NL, c->rec_s,
+                             &c->cst->any, c->err));
         if (c->ntiles > 1)
-            k_carry_fix<<<1, kFixThreads, 0, c->stream>>>(c->rec_s, (uint32_t)c->ntiles, out, M,
-                                                          &c->cst->any);
+            BW_CUDA(launch_after(!timing, k_carry_fix, dim3(1), kFixThreads, 0, c->stream,
+                                 c->rec_s, (uint32_t)c->ntiles, out, M, &c->cst->any));
         c->out_pieces = 1;
-        BW_CUDA(cudaGetLastError());
         return BW_OK;
     }
     if (++c->epoch >= (1u << 28)) {
@@ -1093,22 +1096,22 @@ int enqueue_product(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_t* o
     int rc;
     if (pl->w64 && pl->path == BW_PATH_P32) {
         rc = bw_enqueue_transform<Ar32, false, true>(c, a, b, square, timing, io);
-        if (!rc) rc = enqueue_carry<Ar32, false, true>(c, out, pieces);
+        if (!rc) rc = enqueue_carry<Ar32, false, true>(c, out, timing, pieces);
     } else if (pl->w64) {
         rc = pl->f64 == 1 ? bw_enqueue_transform<ArD<0>, false, true>(c, a, b, square, timing, io)
              : pl->f64 == 2
                  ? bw_enqueue_transform<ArD<1>, false, true>(c, a, b, square, timing, io)
                  : bw_enqueue_transform<Ar64, false, true>(c, a, b, square, timing, io);
         if (!rc)
-            rc = pl->f64 == 1   ? enqueue_carry<ArD<0>, false, true>(c, out, pieces)
-                 : pl->f64 == 2 ? enqueue_carry<ArD<1>, false, true>(c, out, pieces)
-                                : enqueue_carry<Ar64, false, true>(c, out, pieces);
+            rc = pl->f64 == 1   ? enqueue_carry<ArD<0>, false, true>(c, out, timing, pieces)
+                 : pl->f64 == 2 ? enqueue_carry<ArD<1>, false, true>(c, out, timing, pieces)
+                                : enqueue_carry<Ar64, false, true>(c, out, timing, pieces);
     } else if (pl->path == BW_PATH_P64) {
         rc = bw_enqueue_transform<Ar64, false>(c, a, b, square, timing, io);
-        if (!rc) rc = enqueue_carry<Ar64, false>(c, out, pieces);
+        if (!rc) rc = enqueue_carry<Ar64, false>(c, out, timing, pieces);
     } else {
         rc = bw_enqueue_transform<Ar32, true>(c, a, b, square, timing, io);
-        if (!rc) rc = enqueue_carry<Ar32, true>(c, out, pieces);
+        if (!rc) rc = enqueue_carry<Ar32, true>(c, out, timing, pieces);
     }
     return rc;
 }

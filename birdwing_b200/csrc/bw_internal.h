@@ -209,6 +209,26 @@ inline const PlanDev<ArD<1>>& plan_dev<ArD<1>>(const bw_plan* pl) {
     return pl->pdd1;
 }
 
+// Launch a kernel behind the previous one in the stream.  early: it may start
+// while that one's last CTAs run (programmatic dependent launch); the kernel
+// must then run grid_wait() before it reads what that one writes.  Not for a
+// product's first kernel, which reads operands of the caller's.
+template <class... P, class... A>
+cudaError_t launch_after(bool early, void (*kern)(P...), dim3 grid, unsigned block, size_t smem,
+                         cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // Enqueue K1..K3 (the transform part) for one product.  With io (chunks > 1)
 // the operands' copy-in runs on the context's copy stream in column blocks
 // and K1 runs block by block behind it.

@@ -184,6 +184,15 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Programmatic dependent launch: grid_wait returns once the previous kernel of
+// the stream has finished and its writes are visible (at once when this kernel
+// was launched without the attribute); grid_release lets the next one start
+// when every CTA of this one has called it or exited.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Asynchronous global -> shared copy of one element (cp.async): a tile's
 // loads are all issued at once and land while the CTA builds its twiddle
 // tables; the issuing thread waits for its own copies with cp_async_wait.
@@ -1273,8 +1282,9 @@ __device__ __forceinline__ void garner_digits_at(const PlanDev<Ar>& P,
 #pragma unroll
                 for (int q = 0; q < (E * CPW * (int)sizeof(T)) / 16; ++q) {
                     // NC: read-only path (residues from an earlier kernel);
-                    // plain loads when this kernel wrote them
-                    const uint4 v = NC ? __ldg(src + q) : src[q];
+                    // L2 loads when this kernel wrote them or started before
+                    // that one had finished
+                    const uint4 v = NC ? __ldg(src + q) : __ldcg(src + q);
                     if constexpr (sizeof(T) == 8) {
                         r[kp][2 * q] = ((uint64_t)v.y << 32) | v.x;
                         r[kp][2 * q + 1] = ((uint64_t)v.w << 32) | v.z;
@@ -1389,7 +1399,7 @@ __device__ __forceinline__ void garner_words_w64_at(const PlanDev<Ar>& P,
         const uint4* src = reinterpret_cast<const uint4*>(base + (size_t)kp * pstride);
 #pragma unroll
         for (int h = 0; h < Q / PER; ++h)
-            raw[kp][h] = valid ? (NC ? __ldg(src + h) : src[h]) : make_uint4(0, 0, 0, 0);
+            raw[kp][h] = valid ? (NC ? __ldg(src + h) : __ldcg(src + h)) : make_uint4(0, 0, 0, 0);
     }
     const GarnerDev<Ar>& G = P.gar;
     uint32_t bad = 0;
@@ -1761,6 +1771,8 @@ constexpr int kFixThreads = 1024;
 static __global__ void __launch_bounds__(kFixThreads)
 k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __restrict__ out,
             size_t M, uint32_t* __restrict__ any) {
+    grid_release();
+    grid_wait();
     if (__ldcg(any) == 0u) return;  // every tile kills
     __shared__ uint32_t s_f[kFixThreads];  // 0, 1: constant carry out; 2: passes carry-in
     const int tid = threadIdx.x;
@@ -1825,7 +1837,9 @@ k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
     uint32_t l[E];
     uint32_t X[3];
     uint32_t bad = 0;
-    garner_local<Ar, SPLIT16, W64, true>(
+    grid_release();
+    grid_wait();
+    garner_local<Ar, SPLIT16, W64, false>(
         P, res + (valid ? j0 : 0) * elems_per_word2<SPLIT16, W64>() / 2, n, valid, l, X, &bad);
     if (bad && own) atomicOr(err, 2u);
     uint32_t PX[3];

@@ -197,11 +197,43 @@ struct RowCfg {
     static constexpr int kMinCtas = (sizeof(typename Ar::T) == 8 ? 768 : 1024) / NT;
 };
 
+// A thread's elements of a row's first round, all loaded at once (rows of one
+// sub-problem of 16 per thread): they arrive while the twiddles are built, or
+// while the other operand's round runs.  L2 loads: the previous kernel wrote
+// them, and each is read once.
+template <class Ar, int LOGC>
+struct RowPre {
+    static constexpr int RL = first_rl(LOGC), D = LOGC - RL;
+    static constexpr int NT = RowCfg<Ar, LOGC>::NT, IT = (1 << D) < NT ? 1 : (1 << D) / NT;
+    typename Ar::T x[IT << RL];
+    __device__ __forceinline__ void load(const typename Ar::T* g) {
+#pragma unroll
+        for (int i = 0; i < IT; ++i)
+#pragma unroll
+            for (int k = 0; k < (1 << RL); ++k)
+                x[(i << RL) + k] = __ldcg(g + threadIdx.x + i * NT + (k << D));
+    }
+    // the round itself, into shared memory
+    __device__ __forceinline__ void round(typename Ar::T* buf, const Ar& ar,
+                                          const Tw<typename Ar::T>* W) {
+        using T = typename Ar::T;
+        using L = LayRow2<T>;
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int p0 = L::p(threadIdx.x + i * NT);
+            ct_round<Ar, RL, false, false, true>(x + (i << RL), ar, RoundTw<T, 1, true>(W, 0));
+#pragma unroll
+            for (int k = 0; k < (1 << RL); ++k)
+                buf[p0 + L::template off<false>(k, D, 0)] = x[(i << RL) + k];
+        }
+    }
+};
+
 // One CT round (starting at stage S0) of a row in shared memory, from global
 // memory when FROM_G.
 template <class Ar, int LOGC, int S0, int RL, bool FROM_G, class TWB>
-__device__ __forceinline__ void row_ct(const typename Ar::T* __restrict__ gsrc,
-                                       typename Ar::T* buf, const Ar& ar, const TWB* W) {
+__device__ __forceinline__ void row_ct(const typename Ar::T* gsrc, typename Ar::T* buf,
+                                       const Ar& ar, const TWB* W) {
     using T = typename Ar::T;
     using L = LayRow2<T>;
     constexpr int D = LOGC - S0 - RL, NSUB = 1 << (LOGC - RL), NT = RowCfg<Ar, LOGC>::NT;
@@ -215,7 +247,7 @@ __device__ __forceinline__ void row_ct(const typename Ar::T* __restrict__ gsrc,
 #pragma unroll
         for (int k = 0; k < (1 << RL); ++k) {
             if constexpr (FROM_G) {
-                x[k] = gsrc[base + (k << D)];
+                x[k] = __ldcg(gsrc + base + (k << D));
             } else {
                 x[k] = buf[p0 + L::template off<false>(k, D, 0)];
             }
@@ -228,7 +260,7 @@ __device__ __forceinline__ void row_ct(const typename Ar::T* __restrict__ gsrc,
 
 // One GS round of a row in shared memory, to global memory when TO_G.
 template <class Ar, int LOGC, int S0, int RL, bool TO_G, class TWB>
-__device__ __forceinline__ void row_gs(typename Ar::T* __restrict__ gdst, typename Ar::T* buf,
+__device__ __forceinline__ void row_gs(typename Ar::T* gdst, typename Ar::T* buf,
                                        const Ar& ar, const TWB* W) {
     using T = typename Ar::T;
     using L = LayRow2<T>;
@@ -254,7 +286,9 @@ __device__ __forceinline__ void row_gs(typename Ar::T* __restrict__ gdst, typena
     }
 }
 
-template <class Ar, int LOGC>
+// WAIT: the rows come from a kernel that may still be running (grid_wait before
+// they are read; the twiddles do not depend on it).
+template <class Ar, int LOGC, bool WAIT>
 __device__ __forceinline__ void row2_body(const PlanDev<Ar>& P, typename Ar::T* res_a,
                                           const typename Ar::T* res_b, bool square, int prow,
                                           int kp, unsigned char* smem_raw) {
@@ -277,6 +311,11 @@ __device__ __forceinline__ void row2_body(const PlanDev<Ar>& P, typename Ar::T* 
     T* bufA = reinterpret_cast<T*>(ZL + 32);
     T* bufB = bufA + tile_elems(C);
 
+    // ---- the rows' elements, where every thread takes 16: A's (4-byte
+    // residues: B's too) before the tables, which need neither
+    constexpr bool PRE = NSUB == NT && sizeof(T) == 4;
+    RowPre<Ar, PRE ? LOGC : 8> xa, xb;
+
     // ---- the row's powers of zeta, then its twiddles
     {
         const size_t n_row = (size_t)C << log_rr;
@@ -295,6 +334,11 @@ __device__ __forceinline__ void row2_body(const PlanDev<Ar>& P, typename Ar::T* 
             }
         }
         __syncthreads();
+        if (WAIT) grid_wait();
+        if constexpr (PRE) {
+            xa.load(ga);
+            if (!square) xb.load(gb);
+        }
         for (int i = 1 + threadIdx.x; i < (1 << S1); i += NT) {
             // the stage of place i in the round order
             int s0 = RL0;
@@ -309,8 +353,13 @@ __device__ __forceinline__ void row2_body(const PlanDev<Ar>& P, typename Ar::T* 
     }
 
     // ---- forward rounds with row twiddles, global memory -> shared memory
-    row_ct<Ar, LOGC, 0, RL0, true>(ga, bufA, ar, R);
-    if (!square) row_ct<Ar, LOGC, 0, RL0, true>(gb, bufB, ar, R);
+    if constexpr (PRE) {
+        xa.round(bufA, ar, R);
+        if (!square) xb.round(bufB, ar, R);
+    } else {
+        row_ct<Ar, LOGC, 0, RL0, true>(ga, bufA, ar, R);
+        if (!square) row_ct<Ar, LOGC, 0, RL0, true>(gb, bufB, ar, R);
+    }
     __syncthreads();
     if constexpr (S1 > RL0) {
         row_ct<Ar, LOGC, RL0, 4, false>(nullptr, bufA, ar, R);
@@ -371,7 +420,8 @@ template <class Ar, int LOGC>
 __global__ void __launch_bounds__(RowCfg<Ar, LOGC>::NT, RowCfg<Ar, LOGC>::kMinCtas)
 k_row2(const PlanDev<Ar> P, typename Ar::T* res_a, const typename Ar::T* res_b, int square) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    row2_body<Ar, LOGC>(P, res_a, res_b, square != 0, blockIdx.x, blockIdx.y, smem_raw);
+    grid_release();
+    row2_body<Ar, LOGC, true>(P, res_a, res_b, square != 0, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 // ------------------------------------------------------------------ columns
@@ -538,6 +588,7 @@ k_fwd_col2(const PlanDev<Ar> P, const uint32_t* __restrict__ limbs_a, size_t nco
            const uint32_t* __restrict__ limbs_b, size_t ncoef_b, typename Ar::T* res_a,
            typename Ar::T* res_b, unsigned zt_mask, int tile0) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    grid_release();
     const int op = blockIdx.z;
     fwd_col2_body<Ar, LOGR, LCB, CW>(P, op ? limbs_b : limbs_a, op ? ncoef_b : ncoef_a,
                                      op ? res_b : res_a, (zt_mask >> op) & 1u,
@@ -574,7 +625,7 @@ __device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar:
 #pragma unroll
             for (int k = 0; k < (1 << RL); ++k) {
                 if constexpr (FIRST) {
-                    x[k] = g0[((size_t)(base + (k << D)) << log_c) + v];
+                    x[k] = __ldcg(g0 + ((size_t)(base + (k << D)) << log_c) + v);
                 } else {
                     x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
                 }
@@ -609,6 +660,8 @@ template <class Ar, int LOGR, int LCB>
 __global__ void __launch_bounds__(ColCfg<Ar, LOGR, LCB>::NT, ColCfg<Ar, LOGR, LCB>::kMinCtas)
 k_inv_col2(const PlanDev<Ar> P, typename Ar::T* res, CarryState* cst) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    grid_release();
+    grid_wait();
     inv_col2_body<Ar, LOGR, LCB>(P, res, cst, blockIdx.x, blockIdx.y, smem_raw);
 }
 

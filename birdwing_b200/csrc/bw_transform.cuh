@@ -94,17 +94,25 @@ cudaError_t with_length(int l, F f) {
     }
 }
 
+// Whether a pass of `ctas` CTAs starts early (launch_after): only with at least
+// four waves of them.  A grid that fits the SMs at once is placed on the SMs
+// the previous pass leaves first, many CTAs on some and few on others: rows and
+// inverse columns started early took a 2^20-point product from 48 to 53 us and
+// a 2^17-point one from 23 to 31; with five waves or more it gained 1.5%.
+inline bool start_early(size_t ctas, int per_sm) { return ctas >= (size_t)4 * 148 * per_sm; }
+
 template <class Ar>
 cudaError_t launch_row2(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
-                        const typename Ar::T* rb, int sq, cudaStream_t s) {
+                        const typename Ar::T* rb, int sq, bool early, cudaStream_t s) {
     return with_length<kRow2MinLog, kRow2MaxLog>(pl->log_c, [&](auto lc) {
         constexpr int LC = decltype(lc)::value;
         using Cfg = RowCfg<Ar, LC>;
         const cudaError_t e = allow_smem<&k_row2<Ar, LC>>();
         if (e != cudaSuccess) return e;
         const dim3 g(1u << (pl->log_r + pl->log_r2), pl->K);
-        k_row2<Ar, LC><<<g, Cfg::NT, Cfg::smem(sq != 0), s>>>(pd, ra, rb, sq);
-        return cudaSuccess;
+        early = early && start_early((size_t)g.x * g.y, Cfg::kMinCtas);
+        return launch_after(early, k_row2<Ar, LC>, g, Cfg::NT, Cfg::smem(sq != 0), s, pd, ra, rb,
+                            sq);
     });
 }
 
@@ -116,7 +124,7 @@ cudaError_t with_tile(int log_r, int log_cb, F f) {
     return with_length<kCol2MinLog, W8 ? kCol2MaxLog64 : kCol2MaxLog32>(log_r, [&](auto lr) {
         constexpr int LR = decltype(lr)::value;
         constexpr int LO = W8 ? 1 : 2, TOP = (W8 ? 13 : 14) - LR;
-        constexpr int HI = TOP < LO ? LO : TOP > LO + 2 ? LO + 2 : TOP;
+        constexpr int HI = TOP < LO ? LO : TOP > 3 ? 3 : TOP;
         return with_length<LO, HI>(log_cb, [&](auto cb) { return f(lr, cb); });
     });
 }
@@ -140,14 +148,15 @@ cudaError_t launch_fwd_col2(const bw_plan* pl, const PlanDev<Ar>& pd, const uint
 
 template <class Ar>
 cudaError_t launch_inv_col2(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
-                            CarryState* cst, int tiles, cudaStream_t s) {
+                            CarryState* cst, int tiles, bool early, cudaStream_t s) {
     return with_tile<Ar>(pl->log_r, pl->log_cb, [&](auto lr, auto cb) {
         constexpr int LR = decltype(lr)::value, CB = decltype(cb)::value;
         using Cfg = ColCfg<Ar, LR, CB>;
         const cudaError_t e = allow_smem<&k_inv_col2<Ar, LR, CB>>();
         if (e != cudaSuccess) return e;
-        k_inv_col2<Ar, LR, CB><<<dim3(tiles, pl->K), Cfg::NT, Cfg::smem, s>>>(pd, ra, cst);
-        return cudaSuccess;
+        early = early && start_early((size_t)tiles * pl->K, Cfg::kMinCtas);
+        return launch_after(early, k_inv_col2<Ar, LR, CB>, dim3(tiles, pl->K), Cfg::NT, Cfg::smem,
+                            s, pd, ra, cst);
     });
 }
 
@@ -318,7 +327,7 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     BW_CUDA(ke);
     if constexpr (kHasV2<Ar>) {
         if (pl->v2_rows) {
-            BW_CUDA(launch_row2<Ar>(pl, pd, ra, rbs, sq, c->stream));
+            BW_CUDA(launch_row2<Ar>(pl, pd, ra, rbs, sq, !timing, c->stream));
             row_done = true;
         }
     }
@@ -339,7 +348,8 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     bool inv_done = false;
     if constexpr (kHasV2<Ar>) {
         if (pl->v2_cols) {
-            BW_CUDA(launch_inv_col2<Ar>(pl, pd, ra, c->cst, cols_outer / CB, c->stream));
+            BW_CUDA(launch_inv_col2<Ar>(pl, pd, ra, c->cst, cols_outer / CB, !timing,
+                                        c->stream));
             inv_done = true;
         }
     }
