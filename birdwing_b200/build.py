@@ -13,8 +13,10 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libbirdwing.so")
 SOURCES = ["bw_core.cu", "bw_tr_p32.cu", "bw_tr_p32w.cu", "bw_tr_p64.cu", "bw_tr_f64_0.cu", "bw_tr_f64_1.cu",
            "bw_noalloc.cu", "bw_batch.cu",
+           "bw_group_p32.cu", "bw_group_f64.cu", "bw_one.cu",
            "bw_server.cu", "bw_probe.cu"]
-HEADERS = ["bw_arith.cuh", "bw_kernels.cuh", "bw_ntt.cuh", "bw_host.h", "bw_internal.h", "bw_transform.cuh"]
+HEADERS = ["bw_arith.cuh", "bw_kernels.cuh", "bw_ntt.cuh", "bw_host.h", "bw_internal.h", "bw_transform.cuh",
+           "bw_group.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -206,117 +206,16 @@ void drop_layout(bw_batch* bt) {
 namespace {
 
 template <class Ar>
-const PlanDev<Ar>& pdev(const bw_plan& p);
-template <>
-const PlanDev<Ar32>& pdev<Ar32>(const bw_plan& p) {
-    return p.pd32;
-}
-template <>
-const PlanDev<Ar64>& pdev<Ar64>(const bw_plan& p) {
-    return p.pd64;
-}
-
-template <class Ar, bool SPLIT16>
-void enqueue_group_t(const bw_group_launch& g, cudaStream_t s) {
-    using T = typename Ar::T;
-    const bw_plan& pl = *g.plan;
-    const PlanDev<Ar>& P = pdev<Ar>(pl);
-    const unsigned np = g.np;
-    T* ra = static_cast<T*>(g.res_a);
-    T* rb = static_cast<T*>(g.res_b);
-    if (pl.small) {
-        const int n = 1 << pl.log_n;
-        const size_t smem = 2 * tile_elems(n) * sizeof(T);
-        const int want = std::min(256, std::max(64, n >> 4));
-        if (want >= 256) {
-            ks_product<Ar, SPLIT16, 256><<<np, 256, smem, s>>>(P, g.d_desc, ra, g.d_err);
-        } else if (want >= 128) {
-            ks_product<Ar, SPLIT16, 128><<<np, 128, smem, s>>>(P, g.d_desc, ra, g.d_err);
-        } else {
-            ks_product<Ar, SPLIT16, 64><<<np, 64, smem, s>>>(P, g.d_desc, ra, g.d_err);
-        }
-        return;
-    }
-    const int R = 1 << pl.log_r, C = 1 << pl.log_c, CB = 1 << pl.log_cb;
-    const int CB1 = 1 << pl.log_cb1;
-    const size_t smem1 = tile_elems((size_t)R * CB1) * sizeof(T) + (size_t)R * CB1 * (SPLIT16 ? 2 : 4);
-    kb_fwd_col<Ar, SPLIT16, 4><<<dim3(C / CB1, 1, 2 * np), kColThreads, smem1, s>>>(
-        P, g.d_desc, ra, rb);
-    const int la = pl.log_c / 2;
-    const size_t ntab = 2 * (((size_t)1 << la) + ((size_t)C >> la));
-    const size_t smem2 = ntab * sizeof(Tw<T>) + tile_elems(C) * sizeof(T) * 2;
-    const dim3 g2(R, pl.K, np);
-    // row rounds: radix 8 on the 64-bit path (at most 256 threads, 64
-    // registers, as its single-product row pass), radix 16 on the 32-bit
-    // path, unless the tune table chose the other radix for the bucket
-    const int rl = g.rlog ? g.rlog : (sizeof(T) == 8 ? 3 : 4);
-    if (rl == 3) {
-        switch (std::min(sizeof(T) == 8 ? 256 : 512, std::max(64, C >> 3))) {
-            case 512: kb_row<Ar, 512, 3><<<g2, 512, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            case 256: kb_row<Ar, 256, 3><<<g2, 256, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            case 128: kb_row<Ar, 128, 3><<<g2, 128, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            default: kb_row<Ar, 64, 3><<<g2, 64, smem2, s>>>(P, g.d_desc, ra, rb); break;
-        }
-    } else {
-        switch (std::min(512, std::max(64, C >> 4))) {
-            case 512: kb_row<Ar, 512, 4><<<g2, 512, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            case 256: kb_row<Ar, 256, 4><<<g2, 256, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            case 128: kb_row<Ar, 128, 4><<<g2, 128, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            default: kb_row<Ar, 64, 4><<<g2, 64, smem2, s>>>(P, g.d_desc, ra, rb); break;
-        }
-    }
-    const size_t smem3 = tile_elems((size_t)R * CB) * sizeof(T);
-    kb_inv_col<Ar, 4><<<dim3(C / CB, pl.K, np), kColThreads, smem3, s>>>(P, g.d_desc, ra);
-    kb_garner_carry<Ar, SPLIT16><<<dim3((unsigned)g.ntiles, np), kCarryThreads, 0, s>>>(
-        P, g.d_desc, ra, 1u, g.inject_wait_fault ? 1u + (1u << 27) : 1u, g.d_err, g.spin_limit);
-}
-
-int set_group_attrs() {
-    static std::once_flag once;
-    static cudaError_t st = cudaSuccess;
-    std::call_once(once, [] {
-        auto set = [](const void* f) {
-            cudaError_t e =
-                cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            if (e != cudaSuccess) st = e;
-        };
-        set((const void*)ks_product<Ar64, false, 64>);
-        set((const void*)ks_product<Ar64, false, 128>);
-        set((const void*)ks_product<Ar64, false, 256>);
-        set((const void*)ks_product<Ar32, true, 64>);
-        set((const void*)ks_product<Ar32, true, 128>);
-        set((const void*)ks_product<Ar32, true, 256>);
-        set((const void*)kq_small<Ar64, false, kQueueThreads>);
-        set((const void*)kq_small<Ar32, true, kQueueThreads>);
-        set((const void*)kb_fwd_col<Ar64, false, 4>);
-        set((const void*)kb_fwd_col<Ar32, true, 4>);
-        set((const void*)kb_inv_col<Ar64, 4>);
-        set((const void*)kb_inv_col<Ar32, 4>);
-        for (auto f : {(const void*)kb_row<Ar64, 64, 3>, (const void*)kb_row<Ar64, 128, 3>,
-                       (const void*)kb_row<Ar64, 256, 3>, (const void*)kb_row<Ar64, 512, 3>,
-                       (const void*)kb_row<Ar64, 64, 4>, (const void*)kb_row<Ar64, 128, 4>,
-                       (const void*)kb_row<Ar64, 256, 4>, (const void*)kb_row<Ar64, 512, 4>,
-                       (const void*)kb_row<Ar32, 64, 3>, (const void*)kb_row<Ar32, 128, 3>,
-                       (const void*)kb_row<Ar32, 256, 3>, (const void*)kb_row<Ar32, 512, 3>,
-                       (const void*)kb_row<Ar32, 64, 4>, (const void*)kb_row<Ar32, 128, 4>,
-                       (const void*)kb_row<Ar32, 256, 4>, (const void*)kb_row<Ar32, 512, 4>})
-            set(f);
-    });
-    if (st != cudaSuccess)
-        return bw_fail(BW_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(st));
-    return BW_OK;
+const PlanDev<Ar>& pdev(const bw_plan& p) {
+    return plan_dev<Ar>(&p);
 }
 
 }  // namespace
 
 int bw_enqueue_group(const bw_group_launch& g, cudaStream_t s) {
-    int rc = set_group_attrs();
-    if (rc) return rc;
-    if (g.plan->path == BW_PATH_P64) {
-        enqueue_group_t<Ar64, false>(g, s);
-    } else {
-        enqueue_group_t<Ar32, true>(g, s);
-    }
+    const cudaError_t e = g.plan->path == BW_PATH_P64 ? bw_enqueue_group_of<ArD<0>, false>(g, s)
+                                                      : bw_enqueue_group_of<Ar32, true>(g, s);
+    if (e != cudaSuccess) return bw_fail(BW_ECUDA, "group launch: %s", cudaGetErrorString(e));
     return BW_OK;
 }
 
@@ -380,7 +279,9 @@ cudaError_t launch_queue(bw_batch* bt, int slot, cudaStream_t s) {
     const size_t smem = 2 * tile_elems((size_t)1 << bt->qlog_max[slot]) * sizeof(T);
     auto kern = kq_small<Ar, SPLIT16, kQueueThreads>;
     int per_sm = 0, dev = 0, sms = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kQueueThreads, smem);
+    cudaError_t e = cudaFuncSetAttribute((const void*)kern,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kQueueThreads, smem);
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
@@ -458,6 +359,7 @@ int build_layout(bw_batch* bt) {
     // per bucket: plan, residues, carry state, descriptors
     for (Bucket& bk : bt->buckets) {
         const unsigned flags = BW_PLAN_LOG_COLS(bk.log_cols);
+        bk.plan.no_v2_one = bt->persistent;
         rc = bw_plan_setup(&bk.plan, bk.path, bk.K, bk.log_n, flags, bk.small ? 1 : 0);
         if (rc) return rc;
         const size_t n = (size_t)1 << bk.log_n;
@@ -504,7 +406,7 @@ int build_layout(bw_batch* bt) {
             for (size_t i = 0; i < bt->buckets.size(); ++i)
                 if (bt->buckets[i].small && bt->buckets[i].path == path) sb.push_back(i);
             if (sb.empty()) continue;
-            rc = slot == 0 ? upload_queue<Ar64>(bt, slot, sb) : upload_queue<Ar32>(bt, slot, sb);
+            rc = slot == 0 ? upload_queue<ArD<0>>(bt, slot, sb) : upload_queue<Ar32>(bt, slot, sb);
             if (rc) return rc;
         }
     }
@@ -538,10 +440,9 @@ int build_layout(bw_batch* bt) {
     // buckets round-robin after them
     size_t branch = 0;
     if (bt->persistent) {
-        rc = set_group_attrs();
         for (int slot = 0; slot < 2 && rc == BW_OK; ++slot) {
             if (!bt->qcount[slot]) continue;
-            chk(slot == 0 ? launch_queue<Ar64, false>(bt, slot, bt->side[branch % nside])
+            chk(slot == 0 ? launch_queue<ArD<0>, false>(bt, slot, bt->side[branch % nside])
                           : launch_queue<Ar32, true>(bt, slot, bt->side[branch % nside]));
             ++branch;
         }

@@ -48,7 +48,10 @@ namespace {
 
 using u128 = unsigned __int128;
 
-uint64_t mulmod(uint64_t a, uint64_t b, uint64_t p) { return (uint64_t)((u128)a * b % p); }
+uint64_t mulmod(uint64_t a, uint64_t b, uint64_t p) {
+    if (p >> 32 == 0 && (a | b) >> 32 == 0) return a * b % p;
+    return (uint64_t)((u128)a * b % p);
+}
 uint64_t powmod(uint64_t a, uint64_t e, uint64_t p) {
     uint64_t r = 1 % p;
     a %= p;
@@ -191,8 +194,8 @@ struct TableBuilder {
             for (size_t i = 0; i < m; ++i) {
                 const size_t e = (L >> (s + 1)) * bitrev_h((uint32_t)i, s);
                 const uint64_t w = pw[e];
-                const uint32_t t = (uint32_t)(m + i);
-                host[off + (round_order ? tw_perm(t, log_len) : t)] = make_tw<Ar>(w, p);
+                host[off + (round_order ? tw_place(s, (uint32_t)i, log_len) : m + i)] =
+                    make_tw<Ar>(w, p);
             }
         }
         return off;
@@ -292,15 +295,19 @@ void fill_constants(const bw_plan* pl, PlanDev<Ar>& pd) {
     for (int k = pl->K; k < kMaxPrimes; ++k) pd.pr[k] = pd.pr[0];
     auto& g = pd.gar;
     if (pl->w64) crt_constants<Ar>(pl, P, g);
-    if constexpr (!Ar::kF64) {
     const uint64_t p0 = P[0], p1 = P[1], p2 = P[2];
     g.p0 = p0;
-    g.inv1 = (T)invmod(p0 % p1, p1);
-    g.inv1q = (T)shoup_pre(g.inv1, p1, bits);
-    g.p0m2 = (T)(p0 % p2);
-    g.p0m2q = (T)shoup_pre(g.p0m2, p2, bits);
-    g.inv2 = (T)invmod(mulmod(p0 % p2, p1 % p2, p2), p2);
-    g.inv2q = (T)shoup_pre(g.inv2, p2, bits);
+    if constexpr (Ar::kF64) {
+        g.inv1 = make_tw<Ar>(invmod(p0 % p1, p1), p1).w;
+        g.p0m2 = make_tw<Ar>(invmod(p0 % p2, p2), p2).w;
+        g.inv2 = make_tw<Ar>(invmod(p1 % p2, p2), p2).w;
+    } else {
+        g.inv1 = (T)invmod(p0 % p1, p1);
+        g.inv1q = (T)shoup_pre(g.inv1, p1, bits);
+        g.p0m2 = (T)(p0 % p2);
+        g.p0m2q = (T)shoup_pre(g.p0m2, p2, bits);
+        g.inv2 = (T)invmod(mulmod(p0 % p2, p1 % p2, p2), p2);
+        g.inv2q = (T)shoup_pre(g.inv2, p2, bits);
     }
     pd.K = pl->K;
     pd.log_n = pl->log_n;
@@ -323,7 +330,7 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
     const uint64_t* P = plan_primes(pl->path, pl->w64 != 0, pl->f64);
     const uint64_t* Gn = plan_gens(pl->path, pl->w64 != 0, pl->f64);
     TableBuilder<Ar> tb;
-    size_t off[kMaxPrimes][12];
+    size_t off[kMaxPrimes][14];
     const size_t n = (size_t)1 << pl->log_n;
     // row-level twiddle length: R * C (two passes) or R2 * C (three passes)
     const int log_rr = pl->log_r2 ? pl->log_r2 : pl->log_r;
@@ -336,8 +343,8 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
         if (pl->small) {
             // single pass: n-point stage tables only
             const uint64_t wn = powmod(Gn[k], (p - 1) >> pl->log_n, p);
-            off[k][2] = tb.add_stage_table(p, wn, pl->log_n);
-            off[k][3] = tb.add_stage_table(p, invmod(wn, p), pl->log_n);
+            off[k][2] = tb.add_stage_table(p, wn, pl->log_n, pl->v2_one != 0);
+            off[k][3] = tb.add_stage_table(p, invmod(wn, p), pl->log_n, pl->v2_one != 0);
             continue;
         }
         const uint64_t wn = powmod(Gn[k], (p - 1) >> pl->log_n, p);  // primitive n-th root
@@ -345,6 +352,10 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
         const uint64_t wrowi = invmod(wrow, p);
         const uint64_t wr = powmod(wn, n >> pl->log_r, p);            // R-th root
         const uint64_t wc = powmod(wn, n >> pl->log_c, p);            // C-th root
+        if (pl->one) {
+            off[k][12] = tb.add_stage_table(p, wn, pl->log_n, true);
+            off[k][13] = tb.add_stage_table(p, invmod(wn, p), pl->log_n, true);
+        }
         const bool vr = pl->v2_rows != 0, vc = pl->v2_cols != 0;
         off[k][0] = tb.add_stage_table(p, wr, pl->log_r, vc);
         off[k][1] = tb.add_stage_table(p, invmod(wr, p), pl->log_r, vc);
@@ -390,6 +401,15 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
         pr.OHf = pl->log_r2 ? base + off[k][11] : nullptr;
     }
     fill_constants(pl, pd);
+    if constexpr (std::is_same<Ar, Ar32>::value) {
+        if (pl->one) {
+            pl->pd_one = pd;
+            for (int k = 0; k < pl->K; ++k) {
+                pl->pd_one.pr[k].WCf = base + off[k][12];
+                pl->pd_one.pr[k].WCi = base + off[k][13];
+            }
+        }
+    }
     return BW_OK;
 }
 
@@ -559,10 +579,15 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
     pl->path = path;
     pl->K = K;
     pl->log_n = log_n;
+    // groups on the 64-bit path: 32-bit coefficients in double precision (two
+    // 50-bit primes carry min(na, nb) 2^64 for every length; a group does not
+    // show its residues)
+    if (mode != 2 && path == BW_PATH_P64) pl->f64 = 1;
     const int w = path == BW_PATH_P64 ? 8 : 4;
     const int max_c = path == BW_PATH_P64 ? 13 : 14;
     if (mode == 1) {
         pl->small = 1;
+        pl->v2_one = log_n <= kOneMaxLog && !pl->no_v2_one;
         pl->log_c = log_n;
         pl->log_r = 0;
     } else {
@@ -572,11 +597,17 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
         const int want_c = (int)((flags >> 8) & 0x1f);
         if (!three) {
             // one product: a square split; a batch group (mode 0): long rows
-            // (C = 2^min(12, log n - 3) on the 64-bit path) and short columns:
-            // the rows keep every thread of the row pass busy even for small
-            // n, and the group's grid has a product dimension to fill the SMs
-            pl->log_c = mode == 0 ? std::max(std::min(max_c - 1, log_n - 3), (log_n + 1) / 2)
-                                  : std::min(max_c, (log_n + 1) / 2);
+            // and columns of 8 or 16 points (a radix-8 or -16 pass straight
+            // through registers), whose grid has a product dimension to fill
+            // the SMs: 2^13 points R x C = 8 x 1024 54 us, 32 x 256 78 us (207
+            // products, 32-bit path), 2^14 points 8 x 2048 107, 32 x 512 128;
+            // 2^16 points 16 x 4096 436, 128 x 512 465; 2^17 points 128 x 1024
+            // 469, 32 x 4096 516
+            const int square = (log_n + 1) / 2;
+            const int group_c = log_n <= 14   ? std::max(log_n - 3, square)
+                                : log_n <= 16 ? log_n - 4
+                                              : std::max(10, square);
+            pl->log_c = std::min(max_c, mode == 0 ? group_c : square);
             if (want_c) {
                 if (want_c > max_c || want_c >= log_n || log_n - want_c > 13)
                     return bw_fail(BW_EINVAL, "BW_PLAN_LOG_COLS(%d) invalid for n = 2^%d",
@@ -690,26 +721,20 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
                          pl->log_c == 12 && pl->rlog_row == 4)
                             ? 1
                             : 0;
-        // passes with compile-time lengths: single products of the 32-bit and
-        // double-precision arithmetics
-        if (mode == 2 && (path == BW_PATH_P32 || pl->f64)) {
+        // passes with compile-time lengths: the 32-bit and double-precision
+        // arithmetics
+        if (path == BW_PATH_P32 || pl->f64) {
             pl->v2_rows = pl->log_c >= kRow2MinLog && pl->log_c <= kRow2MaxLog;
             const int top = w == 8 ? kCol2MaxLog64 : kCol2MaxLog32;
             if (pl->log_r >= kCol2MinLog && pl->log_r <= top && !pl->tw_smem_r) {
                 pl->v2_cols = 1;
-                pl->tma_cols = 0;
-                // tiles 32 bytes wide (4-byte residues) or up to 64, whole
-                // sectors, down to half of that for the longest columns.
-                // Narrower tiles to have more CTAs lose at every size: 4-byte
-                // residues in 16, 32 or 64 bytes measured, K1 + K3, 33 / 27 /
-                // 31 us (2^21 points of 16-bit coefficients), 0.146 / 0.121 /
-                // 0.131 ms (six primes, 2^21); 8-byte residues in 16, 32 or 64
-                // bytes 0.134 / 0.106 / 0.104 ms (2^21 points)
-                const int lo_cb = w == 8 ? 1 : 2;
-                const int cb = std::min(
-                    std::max(lo_cb, std::min(3, (w == 8 ? 13 : 14) - pl->log_r)), log_cols_outer);
-                pl->log_cb = pl->log_cb1 = cb;
-                if (cb < lo_cb) pl->v2_cols = 0;
+                const int cb = w == 8 ? col_log_cb<8>(pl->log_r) : col_log_cb<4>(pl->log_r);
+                if (cb > log_cols_outer) {
+                    pl->v2_cols = 0;
+                } else {
+                    pl->log_cb = pl->log_cb1 = cb;
+                    pl->tma_cols = 0;
+                }
             }
         }
         pl->lo = ((pl->log_r2 ? pl->log_r2 : pl->log_r) + pl->log_c + 1) / 2;
@@ -751,6 +776,7 @@ extern "C" int bw_plan_create(bw_plan** out, int path, size_t la, size_t lb, int
     const size_t half = ((size_t)1 << log_n) / 2;
     pl->zt_a = pl->nca <= half;
     pl->zt_b = pl->ncb <= half;
+    pl->one = path == BW_PATH_P32 && !w64 && log_n <= kOneMaxLogSingle && flags == 0;
     rc = bw_plan_setup(pl, path, K, log_n, flags, 2);
     if (rc) {
         delete pl;
@@ -991,15 +1017,6 @@ extern "C" int bw_ctx_sync(bw_ctx* c) {
 
 // ------------------------------------------------------------------ launch
 
-int bw_set_kernel_attrs() {
-    int rc = bw_set_transform_attrs<Ar64, false>();
-    if (!rc) rc = bw_set_transform_attrs<Ar32, true>();
-    if (!rc) rc = bw_set_transform_attrs<Ar32, false>();
-    if (!rc) rc = bw_set_transform_attrs<ArD<0>, false>();
-    if (!rc) rc = bw_set_transform_attrs<ArD<1>, false>();
-    return rc;
-}
-
 namespace {
 
 int ensure_copy_streams(bw_ctx* c) {
@@ -1094,6 +1111,11 @@ int enqueue_product(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_t* o
     const bw_plan* pl = c->plan;
     const int pieces = io ? io->chunks : 1;
     int rc;
+    if (pl->one && !timing && pieces == 1 && !c->inject_wait_fault) {
+        BW_CUDA(bw_launch_one(pl, a, square ? a : b, out, square, c->err, c->stream));
+        c->out_pieces = 1;
+        return BW_OK;
+    }
     if (pl->w64 && pl->path == BW_PATH_P32) {
         rc = bw_enqueue_transform<Ar32, false, true>(c, a, b, square, timing, io);
         if (!rc) rc = enqueue_carry<Ar32, false, true>(c, out, timing, pieces);
@@ -1137,11 +1159,9 @@ static int launch_graph(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_
             cudaGraphExecDestroy(c->gexec);
             c->gexec = nullptr;
         }
-        int rc = bw_set_kernel_attrs();
-        if (rc) return rc;
         BW_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaSuccess;
-        rc = enqueue_product(c, a, b, out, sq, false);
+        const int rc = enqueue_product(c, a, b, out, sq, false);
         cudaGraph_t g = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
         if (rc || e != cudaSuccess || e2 != cudaSuccess) {
@@ -1187,7 +1207,7 @@ static int do_multiply(bw_ctx* c, const uint32_t* a, size_t la, const uint32_t* 
     if (timing) cudaEventRecord(c->ev[0], c->stream);
     int rc;
     if (flags & BW_PTR_DEVICE) {
-        if (!timing && !c->inject_wait_fault) {
+        if (!timing && !c->inject_wait_fault && !pl->one) {
             rc = launch_graph(c, a, b, out, sq);
             if (rc <= 0) return rc;  // 1: fall back to direct launches
         }

@@ -51,7 +51,12 @@ struct bw_plan {
     int f64 = 0;
     // passes with compile-time lengths (bw_ntt.cuh); their tables are stored in
     // round order
-    int v2_rows = 0, v2_cols = 0;
+    int v2_rows = 0, v2_cols = 0, v2_one = 0;
+    bool no_v2_one = false;  // set before bw_plan_setup: tables in stage order (kq_small)
+    // a single product of at most 2^12 points with 16-bit coefficients and no
+    // tuning flags: one CTA (k_one), with its own n-point tables
+    bool one = false;
+    bw::PlanDev<bw::Ar32> pd_one{};
     bw::PlanDev<bw::ArD<0>> pdd0{};
     bw::PlanDev<bw::ArD<1>> pdd1{};
     uint64_t primes[bw::kMaxPrimes] = {};
@@ -64,9 +69,6 @@ struct bw_plan {
 // n^-1 scale); mode 2: the 4-step pipeline for one product at a time, with
 // column tiles narrowed for small n so that the column passes fill the SMs.
 int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int mode);
-
-// Set the dynamic shared-memory limit of every kernel instantiation once.
-int bw_set_kernel_attrs();
 
 // Largest transform of a launch group: the two-pass schedule.
 constexpr int kMaxGroupLogN = 26;
@@ -90,6 +92,12 @@ struct bw_group_launch {
     int rlog = 0;       // row-pass radix log2 (0: radix 8 on the 64-bit path, 16 on the 32-bit)
 };
 int bw_enqueue_group(const bw_group_launch& g, cudaStream_t s);
+// ... of one arithmetic (bw_group_*.cu).
+template <class Ar, bool SPLIT16>
+cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s);
+// One product in one CTA (plans with `one`).
+cudaError_t bw_launch_one(const bw_plan* pl, const uint32_t* a, const uint32_t* b, uint32_t* out,
+                          bool square, uint32_t* err, cudaStream_t s);
 // Carry tiles of a group whose longest product has max_words output words.
 size_t bw_group_ntiles(int path, int log_n, size_t max_words);
 // Bytes of one product's look-back state (16-byte multiple).

@@ -78,8 +78,8 @@ template <class Ar>
 struct GarnerDev {
     using T = typename Ar::T;
     T inv1, inv1q;      // p0^-1 mod p1
-    T p0m2, p0m2q;      // p0 mod p2
-    T inv2, inv2q;      // (p0 p1)^-1 mod p2
+    T p0m2, p0m2q;      // p0 mod p2 (double precision: p0^-1 mod p2)
+    T inv2, inv2q;      // (p0 p1)^-1 mod p2 (double precision: p1^-1 mod p2)
     uint64_t p0;        // p0 as an integer
     // 64-bit coefficients (garner_words_w64_at), 32-bit limbs:
     uint32_t m[kMaxPrimes][5];  // M_k = P / p_k, P the product of the primes
@@ -1250,13 +1250,75 @@ kb_inv_col(const PlanDev<Ar> P, const BatchProd* __restrict__ D, typename Ar::T*
 // three-pass carry (src/carry_prop.cu:8-80) with its host-polled fixup loop
 // (src/gpu_ntt.cu:908-924).
 
-// Garner reconstruction of the E output words starting at word j0: digit
-// sums D[e] < 2^96 (one coefficient per word, or two 16-bit ones).  Words at
-// or beyond NL read nothing and are zero.  Sets *bad when the redundant
-// third prime disagrees or a value reaches 2^96.
-// base: this thread's first residue of prime 0 (global memory, or a tile
-// staged in shared memory); prime k's residues start pstride elements later.
-// valid: the words exist (false: they read as zero).
+// One coefficient below p0 p1 (16- or 32-bit coefficients) from its residues.
+// Sets *bad when the redundant third prime disagrees.
+template <class Ar>
+__device__ __forceinline__ unsigned __int128 garner_one(const PlanDev<Ar>& P, typename Ar::T r0,
+                                                        typename Ar::T r1, typename Ar::T r2,
+                                                        uint32_t& bad) {
+    using T = typename Ar::T;
+    const Ar a1 = P.pr[1].ar;
+    const GarnerDev<Ar>& G = P.gar;
+    if constexpr (Ar::kF64) {
+        // k1 = (r1 - r0) p0^-1 mod p1; the residues are integers in doubles
+        auto whole = [](double d) {
+            return (uint64_t)__double_as_longlong(__dadd_rn(d, 4503599627370496.0)) &
+                   0x000fffffffffffffull;
+        };
+        const double k1 = a1.inv_out(a1.mul(__dsub_rn(r1, r0), G.inv1));
+        if (P.K == 3) {
+            // the third prime is redundant for every supported size: the
+            // mixed-radix digit ((r2 - r0) p0^-1 - k1) p1^-1 mod p2 must be 0,
+            // otherwise flag an error
+            const Ar a2 = P.pr[2].ar;
+            const double t = __dsub_rn(a2.mul(__dsub_rn(r2, r0), G.p0m2), k1);
+            bad |= (uint32_t)(a2.mul(t, G.inv2) != 0.0);
+        }
+        return (unsigned __int128)G.p0 * whole(k1) + whole(r0);
+    } else {
+        // k1 = (r1 - r0) * p0^-1 mod p1
+        const T r0m1 = a1.red1(a1.shoup(r0, 1, P.pr[1].one_q));
+        const T t1 = r1 >= r0m1 ? r1 - r0m1 : r1 + a1.p - r0m1;
+        const T k1 = a1.red1(a1.shoup(t1, G.inv1, G.inv1q));
+        if (P.K == 3) {
+            // (as above)
+            const Ar a2 = P.pr[2].ar;
+            const T r0m2 = a2.red1(a2.shoup(r0, 1, P.pr[2].one_q));
+            const T y = a2.red1(r0m2 + a2.red1(a2.shoup(k1, G.p0m2, G.p0m2q)));
+            const T t2 = r2 >= y ? r2 - y : r2 + a2.p - y;
+            const T k2 = a2.red1(a2.shoup(t2, G.inv2, G.inv2q));
+            bad |= (uint32_t)(k2 != 0);
+        }
+        return (unsigned __int128)G.p0 * k1 + r0;
+    }
+}
+
+// Digit sums D[e] < 2^96 of E output words from their coefficients' residues
+// r[k] (one coefficient per word, or two 16-bit ones).  Sets *bad when the
+// redundant third prime disagrees or a value reaches 2^96.
+template <class Ar, bool SPLIT16, int E>
+__device__ __forceinline__ void garner_combine(
+    const PlanDev<Ar>& P, const typename Ar::T (&r)[kDigitPrimes][E * (SPLIT16 ? 2 : 1)],
+    unsigned __int128 (&D)[E], uint32_t* bad_out) {
+    uint32_t bad = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        if constexpr (SPLIT16) {
+            const unsigned __int128 lo = garner_one(P, r[0][2 * e], r[1][2 * e], r[2][2 * e], bad);
+            D[e] = lo + (garner_one(P, r[0][2 * e + 1], r[1][2 * e + 1], r[2][2 * e + 1], bad)
+                         << 16);
+        } else {
+            D[e] = garner_one(P, r[0][e], r[1][e], r[2][e], bad);
+        }
+        bad |= (uint32_t)((D[e] >> 96) != 0);
+    }
+    *bad_out |= bad;
+}
+
+// Garner reconstruction of the E output words starting at word j0.  Words at
+// or beyond NL read nothing and are zero.
+// base: this thread's first residue of prime 0; prime k's residues start
+// pstride elements later.  valid: the words exist (false: they read as zero).
 template <class Ar, bool SPLIT16, int E, bool NC = true>
 __device__ __forceinline__ void garner_digits_at(const PlanDev<Ar>& P,
                                                  const typename Ar::T* __restrict__ base,
@@ -1264,71 +1326,39 @@ __device__ __forceinline__ void garner_digits_at(const PlanDev<Ar>& P,
                                                  unsigned __int128 (&D)[E], uint32_t* bad_out) {
     using T = typename Ar::T;
     constexpr int CPW = SPLIT16 ? 2 : 1;
-    uint32_t bad = 0;
-    {
-        const Ar a1 = P.pr[1].ar;
-        const GarnerDev<Ar>& G = P.gar;
-        T r[kDigitPrimes][E * CPW];
+    T r[kDigitPrimes][E * CPW];
 #pragma unroll
-        for (int kp = 0; kp < kDigitPrimes; ++kp)
+    for (int kp = 0; kp < kDigitPrimes; ++kp)
 #pragma unroll
-            for (int q = 0; q < E * CPW; ++q) r[kp][q] = 0;
-        if (valid) {
-            // 128-bit vector loads of E*CPW consecutive residues per prime
+        for (int q = 0; q < E * CPW; ++q) r[kp][q] = 0;
+    if (valid) {
+        // 128-bit vector loads of E*CPW consecutive residues per prime
 #pragma unroll
-            for (int kp = 0; kp < kDigitPrimes; ++kp) {
-                if (kp >= P.K) break;
-                const uint4* src = reinterpret_cast<const uint4*>(base + (size_t)kp * pstride);
+        for (int kp = 0; kp < kDigitPrimes; ++kp) {
+            if (kp >= P.K) break;
+            const uint4* src = reinterpret_cast<const uint4*>(base + (size_t)kp * pstride);
 #pragma unroll
-                for (int q = 0; q < (E * CPW * (int)sizeof(T)) / 16; ++q) {
-                    // NC: read-only path (residues from an earlier kernel);
-                    // L2 loads when this kernel wrote them or started before
-                    // that one had finished
-                    const uint4 v = NC ? __ldg(src + q) : __ldcg(src + q);
-                    if constexpr (sizeof(T) == 8) {
-                        r[kp][2 * q] = ((uint64_t)v.y << 32) | v.x;
-                        r[kp][2 * q + 1] = ((uint64_t)v.w << 32) | v.z;
-                    } else {
-                        r[kp][4 * q] = v.x;
-                        r[kp][4 * q + 1] = v.y;
-                        r[kp][4 * q + 2] = v.z;
-                        r[kp][4 * q + 3] = v.w;
-                    }
+            for (int q = 0; q < (E * CPW * (int)sizeof(T)) / 16; ++q) {
+                // NC: read-only path (residues from an earlier kernel);
+                // L2 loads when this kernel wrote them or started before
+                // that one had finished
+                const uint4 v = NC ? __ldg(src + q) : __ldcg(src + q);
+                if constexpr (Ar::kF64) {
+                    r[kp][2 * q] = __hiloint2double((int)v.y, (int)v.x);
+                    r[kp][2 * q + 1] = __hiloint2double((int)v.w, (int)v.z);
+                } else if constexpr (sizeof(T) == 8) {
+                    r[kp][2 * q] = ((uint64_t)v.y << 32) | v.x;
+                    r[kp][2 * q + 1] = ((uint64_t)v.w << 32) | v.z;
+                } else {
+                    r[kp][4 * q] = v.x;
+                    r[kp][4 * q + 1] = v.y;
+                    r[kp][4 * q + 2] = v.z;
+                    r[kp][4 * q + 3] = v.w;
                 }
             }
         }
-        unsigned __int128 x[E * CPW];
-#pragma unroll
-        for (int q = 0; q < E * CPW; ++q) {
-            const T r0 = r[0][q];
-            // k1 = (r1 - r0) * p0^-1 mod p1
-            const T r0m1 = a1.red1(a1.shoup(r0, 1, P.pr[1].one_q));
-            const T t1 = r[1][q] >= r0m1 ? r[1][q] - r0m1 : r[1][q] + a1.p - r0m1;
-            const T k1 = a1.red1(a1.shoup(t1, G.inv1, G.inv1q));
-            x[q] = (unsigned __int128)G.p0 * k1 + r0;
-            if (P.K == 3) {
-                // the third prime is redundant for every supported size: the
-                // mixed-radix digit k2 must be 0, otherwise flag an error
-                const Ar a2 = P.pr[2].ar;
-                const T r0m2 = a2.red1(a2.shoup(r0, 1, P.pr[2].one_q));
-                const T y = a2.red1(r0m2 + a2.red1(a2.shoup(k1, G.p0m2, G.p0m2q)));
-                const T r2 = r[2][q];
-                const T t2 = r2 >= y ? r2 - y : r2 + a2.p - y;
-                const T k2 = a2.red1(a2.shoup(t2, G.inv2, G.inv2q));
-                bad |= (k2 != 0);
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            if constexpr (SPLIT16) {
-                D[e] = x[2 * e] + (x[2 * e + 1] << 16);
-            } else {
-                D[e] = x[e];
-            }
-            bad |= (uint32_t)((D[e] >> 96) != 0);
-        }
     }
-    *bad_out |= bad;
+    garner_combine<Ar, SPLIT16, E>(P, r, D, bad_out);
 }
 
 template <class Ar, bool SPLIT16, int E, bool NC = true>

@@ -18,7 +18,7 @@
 // In a row's last round every thread has a group of its own: its 15 twiddles,
 // contiguous in the (stage, group, position) order, put the lanes of a warp 8
 // to 64 bytes apart, 86 wavefronts per sub-problem against the 32 (4-byte
-// residues) of its data; in this order they are 30.  tw_perm maps an index to
+// residues) of its data; in this order they are 30.  tw_place maps an entry to
 // its place.
 #pragma once
 #include "bw_kernels.cuh"
@@ -28,19 +28,17 @@ namespace bw {
 // Lengths the passes are instantiated for (log2): rows, and columns of 4- and
 // 8-byte residues.
 constexpr int kRow2MinLog = 5, kRow2MaxLog = 13;
-constexpr int kCol2MinLog = 5, kCol2MaxLog32 = 12, kCol2MaxLog64 = 13;
+constexpr int kCol2MinLog = 3, kCol2MaxLog32 = 12, kCol2MaxLog64 = 13;
 
 // Rounds of a 2^L-point transform: the remainder round first.
 __host__ __device__ constexpr int first_rl(int L) { return L % 4 == 0 ? (L < 4 ? L : 4) : L % 4; }
 
-// Place of the stage table's entry t (t in [1, 2^L)) in the round order.
-__host__ __device__ inline uint32_t tw_perm(uint32_t t, int L) {
-    int s = 0;  // stage of entry t
-    while ((2u << s) <= t) ++s;
+// Place of the stage table's entry 2^s + i in the round order.
+__host__ __device__ inline uint32_t tw_place(int s, uint32_t i, int L) {
     const int rl0 = first_rl(L);
     const int s0 = s < rl0 ? 0 : rl0 + (s - rl0) / 4 * 4;
     const int l = s - s0;
-    const uint32_t i = t - (1u << s), g = i >> l, q = i & ((1u << l) - 1), G = 1u << s0;
+    const uint32_t g = i >> l, q = i & ((1u << l) - 1), G = 1u << s0;
     if (l == 0) return G + g;
     return 2 * G + 2 * (((1u << (l - 1)) - 1 + (q >> 1)) * G + g) + (q & 1);
 }
@@ -425,11 +423,26 @@ k_row2(const PlanDev<Ar> P, typename Ar::T* res_a, const typename Ar::T* res_b, 
 }
 
 // ------------------------------------------------------------------ columns
-// A tile is 2^LCB columns of a 2^LOGR-point transform, element (idx, v) at
+// Columns of a tile (log2): 32 bytes (4-byte residues) to 64 wide, whole
+// sectors, half of that for the longest columns, and more for short ones, so
+// that a tile holds 1024 elements.  Narrower tiles to have more CTAs lose at
+// every size: 4-byte residues in 16, 32 or 64 bytes measured, K1 + K3, 33 / 27
+// / 31 us (2^21 points of 16-bit coefficients), 0.146 / 0.121 / 0.131 ms (six
+// primes, 2^21); 8-byte residues in 16, 32 or 64 bytes 0.134 / 0.106 / 0.104 ms
+// (2^21 points).
+template <int BYTES>
+__host__ __device__ constexpr int col_log_cb(int log_r) {
+    const int top = (BYTES == 8 ? 13 : 14) - log_r, lo = BYTES == 8 ? 1 : 2;
+    const int cb = log_r <= 7 ? 10 - log_r : 3;
+    return cb < top ? cb : top < lo ? lo : top;
+}
+
+// A tile is 2^LCB columns (col_log_cb) of a 2^LOGR-point transform, element (idx, v) at
 // layout slot p((idx << LCB) + v).  Threads take sub-problems with v fastest,
 // so a warp's global accesses cover 2^LCB consecutive elements of several rows.
-template <class Ar, int LOGR, int LCB>
+template <class Ar, int LOGR>
 struct ColCfg {
+    static constexpr int LCB = col_log_cb<sizeof(typename Ar::T)>(LOGR);
     static constexpr int RLAST = LOGR < 4 ? LOGR : 4;
     static constexpr int NSUB = 1 << (LOGR + LCB - RLAST);
     static constexpr int NT = NSUB < 32 ? 32 : NSUB > 256 ? 256 : NSUB;
@@ -488,14 +501,15 @@ struct CoefLoad {
 
 // Forward column pass of one tile, operand and prime.  zt: the upper half of
 // the rows is zero pad.
-template <class Ar, int LOGR, int LCB, int CW>
+template <class Ar, int LOGR, int CW>
 __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
                                               const uint32_t* __restrict__ limbs, size_t ncoef,
                                               typename Ar::T* res, bool zt, int tile, int kp,
                                               unsigned char* smem_raw) {
     using T = typename Ar::T;
     using L = LayCol<T>;
-    using Cfg = ColCfg<Ar, LOGR, LCB>;
+    using Cfg = ColCfg<Ar, LOGR>;
+    constexpr int LCB = Cfg::LCB;
     constexpr int RL0 = first_rl(LOGR), NT = Cfg::NT, CB = 1 << LCB;
     const int log_c = P.log_c + P.log_r2;
     const PrimeDev<Ar>& pr = P.pr[kp];
@@ -582,27 +596,28 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
 
 // blockIdx.x = tile * K + prime: the K CTAs of a tile run side by side, so the
 // operand words come from L2 after the first of them.
-template <class Ar, int LOGR, int LCB, int CW>
-__global__ void __launch_bounds__(ColCfg<Ar, LOGR, LCB>::NT, ColCfg<Ar, LOGR, LCB>::kMinCtas)
+template <class Ar, int LOGR, int CW>
+__global__ void __launch_bounds__(ColCfg<Ar, LOGR>::NT, ColCfg<Ar, LOGR>::kMinCtas)
 k_fwd_col2(const PlanDev<Ar> P, const uint32_t* __restrict__ limbs_a, size_t ncoef_a,
            const uint32_t* __restrict__ limbs_b, size_t ncoef_b, typename Ar::T* res_a,
            typename Ar::T* res_b, unsigned zt_mask, int tile0) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     grid_release();
     const int op = blockIdx.z;
-    fwd_col2_body<Ar, LOGR, LCB, CW>(P, op ? limbs_b : limbs_a, op ? ncoef_b : ncoef_a,
+    fwd_col2_body<Ar, LOGR, CW>(P, op ? limbs_b : limbs_a, op ? ncoef_b : ncoef_a,
                                      op ? res_b : res_a, (zt_mask >> op) & 1u,
                                      tile0 + (int)(blockIdx.x / P.K), blockIdx.x % P.K, smem_raw);
 }
 
 // Inverse column pass of one tile and prime, in place, residues fully reduced.
-template <class Ar, int LOGR, int LCB>
+template <class Ar, int LOGR>
 __device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar::T* res,
                                               CarryState* cst, int tile, int kp,
                                               unsigned char* smem_raw) {
     using T = typename Ar::T;
     using L = LayCol<T>;
-    using Cfg = ColCfg<Ar, LOGR, LCB>;
+    using Cfg = ColCfg<Ar, LOGR>;
+    constexpr int LCB = Cfg::LCB;
     constexpr int RL0 = first_rl(LOGR), NT = Cfg::NT, CB = 1 << LCB;
     if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = 0;
     const int log_c = P.log_c + P.log_r2;
@@ -656,13 +671,331 @@ __device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar:
     round(std::integral_constant<int, 0>{}, std::integral_constant<int, RL0>{});
 }
 
-template <class Ar, int LOGR, int LCB>
-__global__ void __launch_bounds__(ColCfg<Ar, LOGR, LCB>::NT, ColCfg<Ar, LOGR, LCB>::kMinCtas)
+template <class Ar, int LOGR>
+__global__ void __launch_bounds__(ColCfg<Ar, LOGR>::NT, ColCfg<Ar, LOGR>::kMinCtas)
 k_inv_col2(const PlanDev<Ar> P, typename Ar::T* res, CarryState* cst) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     grid_release();
     grid_wait();
-    inv_col2_body<Ar, LOGR, LCB>(P, res, cst, blockIdx.x, blockIdx.y, smem_raw);
+    inv_col2_body<Ar, LOGR>(P, res, cst, blockIdx.x, blockIdx.y, smem_raw);
+}
+
+// ------------------------------------------------------------------ batched
+// The same passes with a product grid dimension.
+// blockIdx.x = tile * K + prime, blockIdx.z = 2 * product + operand
+template <class Ar, int LOGR, int CW>
+__global__ void __launch_bounds__(ColCfg<Ar, LOGR>::NT, ColCfg<Ar, LOGR>::kMinCtas)
+kb_fwd_col2(const PlanDev<Ar> P, const BatchProd* __restrict__ D, typename Ar::T* res_a,
+            typename Ar::T* res_b) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const BatchProd d = D[blockIdx.z >> 1];
+    const int op = blockIdx.z & 1;
+    if (op && d.square) return;
+    const size_t ncoef = (size_t)(op ? d.lb : d.la) * (CW == 16 ? 2 : 1);
+    const size_t n = (size_t)1 << P.log_n;
+    fwd_col2_body<Ar, LOGR, CW>(P, op ? d.b : d.a, ncoef, (op ? res_b : res_a) + d.res_off,
+                                ncoef <= n / 2, blockIdx.x / P.K, blockIdx.x % P.K, smem_raw);
+}
+
+// blockIdx.x = row, .y = prime, .z = product
+template <class Ar, int LOGC>
+__global__ void __launch_bounds__(RowCfg<Ar, LOGC>::NT, RowCfg<Ar, LOGC>::kMinCtas)
+kb_row2(const PlanDev<Ar> P, const BatchProd* __restrict__ D, typename Ar::T* res_a,
+        const typename Ar::T* res_b) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const BatchProd d = D[blockIdx.z];
+    row2_body<Ar, LOGC, false>(P, res_a + d.res_off, (d.square ? res_a : res_b) + d.res_off,
+                               d.square != 0, blockIdx.x, blockIdx.y, smem_raw);
+}
+
+template <class Ar, int LOGR>
+__global__ void __launch_bounds__(ColCfg<Ar, LOGR>::NT, ColCfg<Ar, LOGR>::kMinCtas)
+kb_inv_col2(const PlanDev<Ar> P, const BatchProd* __restrict__ D, typename Ar::T* res_a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const BatchProd d = D[blockIdx.z];
+    inv_col2_body<Ar, LOGR>(P, res_a + d.res_off, d.cst, blockIdx.x, blockIdx.y, smem_raw);
+}
+
+// ------------------------------------------------------------------ one CTA
+// A whole product of up to 2^12 points in one CTA and one launch: transforms,
+// pointwise product and inverse in shared memory, PG primes side by side (all
+// of them for a single product, whose latency counts; one at a time in a
+// batch, where the other CTAs fill the SM and shared memory is what limits
+// them), then Garner and carry from the residues where they lie.  Against the
+// 4-step kernels, five or six dependent launches of 2 to 10 us each with most
+// of the chip idle.
+// TH: threads; an item is one sub-problem of 16 elements of one operand and
+// prime, and threads take items in turn.
+// A single product takes it up to 2^11 points (measured alone, one CTA against
+// 4-step: 9.1 / 14.8 us at 2^8, 10.6 / 14.7 at 2^11, 16.9 / 14.7 at 2^12), a
+// batch up to 2^12 (267 products of 2^12 points on the 32-bit path 31 / 71 us,
+// 265 on the 64-bit path 47 / 101).
+constexpr int kOneMinLog = 4, kOneMaxLog = 12, kOneMaxLogSingle = 11;
+
+template <class Ar, int LOGN>
+struct OneCfg {
+    static constexpr int G = 1 << (LOGN - 4);  // sub-problems per transform
+    // shared memory with K primes, PG at a time: residues of every prime, and
+    // the other operand of PG of them
+    static size_t smem(int K, int PG) {
+        return (size_t)(K + PG) * tile_elems(1 << LOGN) * sizeof(typename Ar::T);
+    }
+};
+
+template <class Ar, int LOGN, int CW, int TH>
+__device__ __forceinline__ void one_body(const PlanDev<Ar>& P, const uint32_t* a, uint32_t la,
+                                         const uint32_t* b, uint32_t lb, uint32_t* out, bool sq,
+                                         int pg, uint32_t* err, unsigned char* smem_raw) {
+    using T = typename Ar::T;
+    using L = LayRow2<T>;
+    constexpr int N = 1 << LOGN, RL0 = first_rl(LOGN), G = OneCfg<Ar, LOGN>::G;
+    constexpr int CPW = CW == 16 ? 2 : 1;
+    constexpr int E = CW == 16 ? 4 : 8;  // words per thread in the carry pass
+    const int tid = threadIdx.x, K = P.K;
+    T* buf = reinterpret_cast<T*>(smem_raw);
+    constexpr size_t TE = N + (N >> 4);
+    auto bufA = [&](int k) { return buf + (size_t)k * TE; };
+    auto bufB = [&](int s) { return buf + (size_t)(K + s) * TE; };  // s: slot of the group
+
+    for (int k0 = 0; k0 < K; k0 += pg) {
+        const int kn = min(pg, K - k0), ops = sq ? 1 : 2;
+        // one round of every transform of the group: f(item's operand buffer,
+        // prime, sub-problem)
+        auto each = [&](int transforms, int nsub, auto f) {
+#pragma unroll 1
+            for (int it = tid; it < transforms * nsub; it += TH) {
+                const int t = it / nsub, sp = it - t * nsub;
+                f(t, sp);
+            }
+        };
+        // ... with four items in flight: a short first round's operand loads
+        auto each4 = [&](int transforms, int nsub, auto f) {
+#pragma unroll 4
+            for (int it = tid; it < transforms * nsub; it += TH) {
+                const int t = it / nsub, sp = it - t * nsub;
+                f(t, sp);
+            }
+        };
+        // forward rounds but the last; the first reads the operands
+        auto fwd = [&](auto s0_, auto rl_) {
+            constexpr int S0 = decltype(s0_)::value, RL = decltype(rl_)::value;
+            constexpr int D = LOGN - S0 - RL, NSUB = 1 << (LOGN - RL);
+            auto body = [&](int t, int sp) {
+                const int op = t >= kn ? 1 : 0, k = k0 + t - op * kn;
+                T* dst = op ? bufB(k - k0) : bufA(k);
+                const PrimeDev<Ar>& pr = P.pr[k];
+                const Ar ar = pr.ar;
+                int g, j;
+                row_group<T, D, NSUB>(sp, g, j);
+                const int base = (g << (D + RL)) + j;
+                const int p0 = L::p(base);
+                T x[1 << RL];
+                if constexpr (S0 == 0) {
+                    const CoefLoad<Ar, CW> coef(op ? b : a, (size_t)(op ? lb : la) * CPW);
+#pragma unroll
+                    for (int i = 0; i < (1 << RL); ++i)
+                        x[i] = CoefLoad<Ar, CW>::residue(ar, coef.load(base + (i << D)));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < (1 << RL); ++i)
+                        x[i] = dst[p0 + L::template off<false>(i, D, 0)];
+                }
+                ct_round<Ar, RL, S0 == 0, false, S0 != 0>(
+                    x, ar, RoundTw<T, (1 << S0), false>(pr.WCf, g));
+#pragma unroll
+                for (int i = 0; i < (1 << RL); ++i)
+                    dst[p0 + L::template off<false>(i, D, 0)] = x[i];
+            };
+            if constexpr (S0 == 0 && RL <= 2) {
+                each4(kn * ops, NSUB, body);
+            } else {
+                each(kn * ops, NSUB, body);
+            }
+            __syncthreads();
+        };
+        using std::integral_constant;
+        if constexpr (LOGN > 4) fwd(integral_constant<int, 0>{}, integral_constant<int, RL0>{});
+        if constexpr (LOGN > 4 && RL0 + 4 < LOGN)
+            fwd(integral_constant<int, RL0>{}, integral_constant<int, 4>{});
+        // last forward round of both operands, product, first inverse round
+        constexpr int SL = LOGN - 4;
+        each(kn, G, [&](int t, int g) {
+            const int k = k0 + t;
+            const PrimeDev<Ar>& pr = P.pr[k];
+            const Ar ar = pr.ar;
+            T* A = bufA(k);
+            T* B = bufB(t);
+            const int p0 = L::p(g << 4);
+            const RoundTw<T, (1 << SL), false> tf(pr.WCf, g), ti(pr.WCi, g);
+            T x[16];
+            auto last = [&](const T* src, const uint32_t* limbs, uint32_t len) {
+                if constexpr (SL == 0) {
+                    const CoefLoad<Ar, CW> coef(limbs, (size_t)len * CPW);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        x[i] = CoefLoad<Ar, CW>::residue(ar, coef.load(i));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) x[i] = src[p0 + L::template off<false>(i, 0, 0)];
+                }
+                ct_round<Ar, 4, SL == 0, false, SL != 0>(x, ar, tf);
+            };
+            last(A, a, la);
+            if (sq) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const T v = ar.fwd_to_2p(x[i]);
+                    x[i] = ar.mont(v, v);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) A[p0 + i] = ar.fwd_to_2p(x[i]);
+                last(B, b, lb);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] = ar.mont(ar.fwd_to_2p(x[i]), A[p0 + i]);
+            }
+            gs_round<Ar, 4, SL == 0, true>(x, ar, ti);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) A[p0 + i] = SL == 0 ? ar.scale_out(x[i], pr.scale) : x[i];
+        });
+        __syncthreads();
+        // remaining inverse rounds; the last one scales and reduces
+        auto inv = [&](auto s0_, auto rl_) {
+            constexpr int S0 = decltype(s0_)::value, RL = decltype(rl_)::value;
+            constexpr int D = LOGN - S0 - RL, NSUB = 1 << (LOGN - RL);
+            each(kn, NSUB, [&](int t, int sp) {
+                const PrimeDev<Ar>& pr = P.pr[k0 + t];
+                const Ar ar = pr.ar;
+                T* A = bufA(k0 + t);
+                int g, j;
+                row_group<T, D, NSUB>(sp, g, j);
+                const int p0 = L::p((g << (D + RL)) + j);
+                T x[1 << RL];
+#pragma unroll
+                for (int i = 0; i < (1 << RL); ++i) x[i] = A[p0 + L::template off<false>(i, D, 0)];
+                gs_round<Ar, RL, S0 == 0, true>(x, ar, RoundTw<T, (1 << S0), false>(pr.WCi, g));
+#pragma unroll
+                for (int i = 0; i < (1 << RL); ++i)
+                    A[p0 + L::template off<false>(i, D, 0)] =
+                        S0 == 0 ? ar.scale_out(x[i], pr.scale) : x[i];
+            });
+            __syncthreads();
+        };
+        if constexpr (LOGN > 4 && RL0 + 4 < LOGN)
+            inv(integral_constant<int, RL0>{}, integral_constant<int, 4>{});
+        if constexpr (LOGN > 4) inv(integral_constant<int, 0>{}, integral_constant<int, RL0>{});
+    }
+
+    // ---- Garner + carry, tile by tile; the carry into a tile is the previous
+    // tile's last carry words (s_cin) plus its chain carry-out bit (s_eps)
+    __shared__ uint32_t s_w[TH / 32];
+    __shared__ uint32_t s_lastx[TH / 32][3];
+    __shared__ uint32_t s_cin[3];
+    __shared__ uint32_t s_eps;
+    const int lane = tid & 31, warp = tid >> 5;
+    const uint32_t NLW = N / CPW, M = la + lb;
+    const uint32_t words = NLW > M ? NLW : M;
+    if (tid == 0) {
+        s_cin[0] = s_cin[1] = s_cin[2] = 0;
+        s_eps = 0;
+    }
+    __syncthreads();
+    uint32_t bad = 0;
+    for (uint32_t t0 = 0; t0 < words; t0 += TH * E) {
+        const uint32_t j0 = t0 + tid * E;
+        T r[kDigitPrimes][E * CPW];
+#pragma unroll
+        for (int k = 0; k < kDigitPrimes; ++k)
+#pragma unroll
+            for (int q = 0; q < E * CPW; ++q)
+                r[k][q] = k < K && j0 < NLW ? bufA(k)[L::p(j0 * CPW) + L::p(q)] : T(0);
+        unsigned __int128 Dg[E];
+        garner_combine<Ar, CW == 16, E>(P, r, Dg, &bad);
+        uint32_t l[E], X[3];
+        {
+            unsigned __int128 acc = 0;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                acc += Dg[e];
+                l[e] = (uint32_t)acc;
+                acc >>= 32;
+            }
+            X[0] = (uint32_t)acc;
+            X[1] = (uint32_t)(acc >> 32);
+            X[2] = (uint32_t)(acc >> 64);
+        }
+        uint32_t PX[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) PX[q] = __shfl_up_sync(0xffffffffu, X[q], 1);
+        if (lane == 31) {
+            s_lastx[warp][0] = X[0];
+            s_lastx[warp][1] = X[1];
+            s_lastx[warp][2] = X[2];
+        }
+        __syncthreads();
+        if (lane == 0) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) PX[q] = warp > 0 ? s_lastx[warp - 1][q] : s_cin[q];
+        }
+        uint32_t S[E];
+        int st;
+        {
+            uint64_t c = 0;
+            uint32_t all = 0xffffffffu;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const uint64_t v = (uint64_t)l[e] + (e < 3 ? PX[e] : 0u) + c;
+                S[e] = (uint32_t)v;
+                c = v >> 32;
+                all &= S[e];
+            }
+            st = c ? 2 : (all == 0xffffffffu ? 1 : 0);
+        }
+        const ChainMasks cm = chain_prepare(st, s_w);
+        __syncthreads();
+        const uint32_t eps_in = s_eps;
+        const uint32_t mc = chain_mine(cm, s_w, eps_in);
+        const uint32_t cout = chain_out(s_w, eps_in, TH / 32);
+        {
+            uint64_t c = mc;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const uint64_t v = (uint64_t)S[e] + c;
+                if (j0 + e < M) out[j0 + e] = (uint32_t)v;
+                c = v >> 32;
+            }
+        }
+        if (t0 + TH * E >= words) break;
+        __syncthreads();  // every thread has read s_cin, s_eps, s_lastx, s_w
+        if (tid == TH - 1) {
+            s_cin[0] = X[0];
+            s_cin[1] = X[1];
+            s_cin[2] = X[2];
+        }
+        if (tid == 0) s_eps = cout;
+        __syncthreads();
+    }
+    if (bad) atomicOr(err, 2u);
+}
+
+// A single product (all primes side by side).
+template <class Ar, int LOGN, int CW, int TH>
+__global__ void __launch_bounds__(TH)
+k_one(const PlanDev<Ar> P, const uint32_t* __restrict__ a, uint32_t la,
+      const uint32_t* __restrict__ b, uint32_t lb, uint32_t* __restrict__ out, int square,
+      uint32_t* __restrict__ err) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    one_body<Ar, LOGN, CW, TH>(P, a, la, b, lb, out, square != 0, P.K, err, smem_raw);
+}
+
+// Batched: blockIdx.x = product.
+template <class Ar, int LOGN, int CW, int TH>
+__global__ void __launch_bounds__(TH, (sizeof(typename Ar::T) == 8 ? 768 : 1024) / TH)
+kb_one(const PlanDev<Ar> P, const BatchProd* __restrict__ D, uint32_t* __restrict__ err) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const BatchProd d = D[blockIdx.x];
+    one_body<Ar, LOGN, CW, TH>(P, d.a, d.la, d.square ? d.a : d.b, d.lb, d.out, d.square != 0, 1,
+                               err, smem_raw);
 }
 
 }  // namespace bw

@@ -116,17 +116,11 @@ cudaError_t launch_row2(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T
     });
 }
 
-// f(integral_constant<log_r>, integral_constant<log_cb>) for a plan's column
-// tile.
+// f(integral_constant<log_r>) for a plan's columns.
 template <class Ar, class F>
-cudaError_t with_tile(int log_r, int log_cb, F f) {
-    constexpr bool W8 = sizeof(typename Ar::T) == 8;
-    return with_length<kCol2MinLog, W8 ? kCol2MaxLog64 : kCol2MaxLog32>(log_r, [&](auto lr) {
-        constexpr int LR = decltype(lr)::value;
-        constexpr int LO = W8 ? 1 : 2, TOP = (W8 ? 13 : 14) - LR;
-        constexpr int HI = TOP < LO ? LO : TOP > 3 ? 3 : TOP;
-        return with_length<LO, HI>(log_cb, [&](auto cb) { return f(lr, cb); });
-    });
+cudaError_t with_columns(int log_r, F f) {
+    return with_length<kCol2MinLog, sizeof(typename Ar::T) == 8 ? kCol2MaxLog64 : kCol2MaxLog32>(
+        log_r, f);
 }
 
 template <class Ar, int CW>
@@ -134,14 +128,13 @@ cudaError_t launch_fwd_col2(const bw_plan* pl, const PlanDev<Ar>& pd, const uint
                             size_t na, const uint32_t* b, size_t nb, typename Ar::T* ra,
                             typename Ar::T* rb, unsigned zt, int tile0, int ntiles, bool square,
                             cudaStream_t s) {
-    return with_tile<Ar>(pl->log_r, pl->log_cb1, [&](auto lr, auto cb) {
-        constexpr int LR = decltype(lr)::value, CB = decltype(cb)::value;
-        using Cfg = ColCfg<Ar, LR, CB>;
-        const cudaError_t e = allow_smem<&k_fwd_col2<Ar, LR, CB, CW>>();
+    return with_columns<Ar>(pl->log_r, [&](auto lr) {
+        constexpr int LR = decltype(lr)::value;
+        using Cfg = ColCfg<Ar, LR>;
+        const cudaError_t e = allow_smem<&k_fwd_col2<Ar, LR, CW>>();
         if (e != cudaSuccess) return e;
         const dim3 g((unsigned)ntiles * pl->K, 1, square ? 1 : 2);
-        k_fwd_col2<Ar, LR, CB, CW><<<g, Cfg::NT, Cfg::smem, s>>>(pd, a, na, b, nb, ra, rb, zt,
-                                                                 tile0);
+        k_fwd_col2<Ar, LR, CW><<<g, Cfg::NT, Cfg::smem, s>>>(pd, a, na, b, nb, ra, rb, zt, tile0);
         return cudaSuccess;
     });
 }
@@ -149,14 +142,14 @@ cudaError_t launch_fwd_col2(const bw_plan* pl, const PlanDev<Ar>& pd, const uint
 template <class Ar>
 cudaError_t launch_inv_col2(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
                             CarryState* cst, int tiles, bool early, cudaStream_t s) {
-    return with_tile<Ar>(pl->log_r, pl->log_cb, [&](auto lr, auto cb) {
-        constexpr int LR = decltype(lr)::value, CB = decltype(cb)::value;
-        using Cfg = ColCfg<Ar, LR, CB>;
-        const cudaError_t e = allow_smem<&k_inv_col2<Ar, LR, CB>>();
+    return with_columns<Ar>(pl->log_r, [&](auto lr) {
+        constexpr int LR = decltype(lr)::value;
+        using Cfg = ColCfg<Ar, LR>;
+        const cudaError_t e = allow_smem<&k_inv_col2<Ar, LR>>();
         if (e != cudaSuccess) return e;
         early = early && start_early((size_t)tiles * pl->K, Cfg::kMinCtas);
-        return launch_after(early, k_inv_col2<Ar, LR, CB>, dim3(tiles, pl->K), Cfg::NT, Cfg::smem,
-                            s, pd, ra, cst);
+        return launch_after(early, k_inv_col2<Ar, LR>, dim3(tiles, pl->K), Cfg::NT, Cfg::smem, s,
+                            pd, ra, cst);
     });
 }
 
@@ -210,8 +203,10 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     using T = typename Ar::T;
     const bw_plan* pl = c->plan;
     const PlanDev<Ar>& pd = plan_dev<Ar>(pl);
-    int rc = bw_set_transform_attrs<Ar, SPLIT16>();
-    if (rc) return rc;
+    if (!pl->v2_cols || !pl->v2_rows || pl->log_r2) {
+        const int rc = bw_set_transform_attrs<Ar, SPLIT16>();
+        if (rc) return rc;
+    }
     const int R = 1 << pl->log_r, C = 1 << pl->log_c, CB = 1 << pl->log_cb;
     T* ra = reinterpret_cast<T*>(c->d_res_a);
     T* rb = reinterpret_cast<T*>(c->d_res_b);

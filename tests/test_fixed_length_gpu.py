@@ -14,8 +14,8 @@ pytestmark = pytest.mark.gpu
 
 # (log2 rows, log2 columns): each row length, each column length with few and
 # with many columns, and lengths just outside the instantiated range
-SPLITS = ([(7, c) for c in range(4, 14)] + [(r, 6) for r in range(4, 14)] +
-          [(r, 12) for r in (5, 6, 8, 9, 10)] + [(5, 13), (6, 13), (3, 9), (12, 9)])
+SPLITS = ([(7, c) for c in range(4, 14)] + [(r, 6) for r in range(2, 14)] +
+          [(r, 12) for r in (5, 6, 8, 9, 10)] + [(5, 13), (6, 13), (3, 9), (12, 9), (3, 7), (4, 7), (3, 12)])
 # path, primes, plan flags, coefficients per 64-bit pair of words
 FORMS = [(32, 2, 0, 4), (32, 3, 0, 4), (32, 6, L.BW_PLAN_COEF64, 1),
          (64, 3, L.BW_PLAN_COEF64, 1)]
@@ -88,3 +88,68 @@ def test_carry_fix_between_products(path, K, flags):
             c.sync()
             assert (dc.cpu().numpy().view(np.uint32) == want).all()
             assert (c.multiply(a, b) == want).all()
+
+
+@pytest.mark.parametrize("K", [2, 3])
+@pytest.mark.parametrize("log_n", range(4, 14))
+def test_one_cta_products_exact(log_n, K):
+    # products of up to 2^11 points run in one CTA, 2^12 and more do not; every
+    # length filled exactly (the final carry lands past the last coefficient),
+    # one word short, and squared; alone, with stage times and in a batch
+    import torch
+    total = 1 << (log_n - 1)
+    cases = {(max(1, total // 2), max(1, total // 2)), (max(1, total - 2), 2), (total, 1),
+             (max(1, total // 2 + 1), max(1, total // 2 - 2))}
+    items = []
+    for la, lb in sorted(cases):
+        a = mt64.random_words_top_fast(la, 3 * la + log_n)
+        b = mt64.random_words_top_fast(lb, 5 * lb + log_n)
+        for x, y in ((a, b), (np.full(la, 0xFFFFFFFF, np.uint32), np.full(lb, 0xFFFFFFFF, np.uint32))):
+            items.append((x, y))
+            want = gmp_ref.mul(x, y)
+            with bw.Plan(la, lb, L.BW_PATH_P32, K) as p, bw.Context(p) as c:
+                assert (c.multiply(x, y) == want).all(), (la, lb)
+                assert (c.multiply(x, y, timing=True)[0] == want).all(), (la, lb)
+                da = torch.from_numpy(x.view(np.int32)).cuda()
+                db = torch.from_numpy(y.view(np.int32)).cuda()
+                dc = torch.full((la + lb + 1,), -1, dtype=torch.int32, device="cuda")
+                torch.cuda.synchronize()
+                c.multiply_device(da.data_ptr(), la, db.data_ptr(), lb, dc.data_ptr() + 4, la + lb)
+                c.sync()
+                got = dc.cpu().numpy().view(np.uint32)
+                assert got[0] == 0xFFFFFFFF and (got[1:] == want).all(), (la, lb)
+                if la == lb:
+                    assert (c.square(x) == gmp_ref.mul(x, x)).all()
+    with bw.Batch(num_primes=K) as bt:
+        outs = [(x, y, bt.add(x, y, path=path)) for x, y in items for path in (32, 64)]
+        outs += [(x, x, bt.add(x, x, path=path)) for x, _ in items for path in (32, 64)]
+        bt.run()
+        for x, y, got in outs:
+            assert (got == gmp_ref.mul(x, y)).all(), (x.size, y.size)
+
+
+@pytest.mark.parametrize("path", [32, 64])
+@pytest.mark.parametrize("log_n", range(10, 18))
+def test_group_splits_exact(log_n, path):
+    # batched 4-step products over the splits the group passes are
+    # instantiated for, with ragged sizes and squarings in one bucket
+    per = 2 if path == 32 else 1
+    total = (1 << log_n) // per
+    rng = np.random.default_rng(log_n)
+    shapes = [(total // 2, total // 2), (total // 2 + 7, total // 2 - 9), (total - 3, 3)]
+    ops = [tuple(rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32) for n in s)
+           for s in shapes]
+    ops.append((np.full(total // 2, 0xFFFFFFFF, np.uint32),) * 2)
+    want = [gmp_ref.mul(a, b) for a, b in ops]
+    for log_c in sorted({5, 7, 10, 13, log_n - 3, log_n - 4}):
+        if not 3 <= log_n - log_c <= 13 or log_c < 5 or log_c > 13:
+            continue
+        bw.set_tune_entry(path, 2, log_n, 0, log_c)
+        try:
+            with bw.Batch() as bt:
+                outs = [bt.add(a, b, path=path) for a, b in ops]
+                bt.run()
+        finally:
+            bw.set_tune_entry(path, 2, log_n, log_n <= 12, 0)
+        for w, got in zip(want, outs):
+            assert (w == got).all(), (log_n, log_c)
