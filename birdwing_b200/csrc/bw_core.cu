@@ -368,8 +368,8 @@ int build_tables(bw_plan* pl, PlanDev<Ar>& pd) {
         off[k][7] = tb.add_power_table(p, powmod(wrowi, nlo, p), nhi, scale_k[k]);
         if (pl->log_r2) {
             const uint64_t wm = powmod(wn, n >> pl->log_r2, p);  // R2-th root
-            off[k][8] = tb.add_stage_table(p, wm, pl->log_r2);
-            off[k][9] = tb.add_stage_table(p, invmod(wm, p), pl->log_r2);
+            off[k][8] = tb.add_stage_table(p, wm, pl->log_r2, pl->v2_mid != 0);
+            off[k][9] = tb.add_stage_table(p, invmod(wm, p), pl->log_r2, pl->v2_mid != 0);
             const size_t olo = (size_t)1 << pl->lo_out, ohi = n >> pl->lo_out;
             off[k][10] = tb.add_power_table(p, wn, olo, 1);
             off[k][11] = tb.add_power_table(p, powmod(wn, olo, p), ohi, 1);
@@ -593,7 +593,12 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
     } else {
         // two passes per transform while the column length fits a CTA
         // (R <= 2^13), three passes (n = R * R2 * C) beyond, or when asked for
-        const bool three = (flags & BW_PLAN_THREE_PASS) || log_n > 26;
+        // (R <= 2^13).  In double precision from 2^24 points unless a split is
+        // asked for: its rows are best at 2^12 points (2^13: one CTA per SM)
+        // and its columns at 2^11 or less; two passes against three measured
+        // 2.36 / 2.19 ms at 2^24, 6.59 / 4.33 at 2^25, 16.2 / 8.5 at 2^26
+        const bool three = (flags & BW_PLAN_THREE_PASS) || log_n > 26 ||
+                           (pl->f64 && mode == 2 && log_n >= 24 && ((flags >> 8) & 0x1f) == 0);
         const int want_c = (int)((flags >> 8) & 0x1f);
         if (!three) {
             // one product: a square split; a batch group (mode 0): long rows
@@ -725,6 +730,13 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
         // arithmetics
         if (path == BW_PATH_P32 || pl->f64) {
             pl->v2_rows = pl->log_c >= kRow2MinLog && pl->log_c <= kRow2MaxLog;
+            if (pl->log_r2 >= kMid2MinLog && pl->log_r2 <= kMid2MaxLog) {
+                const int cb2 = w == 8 ? col_log_cb<8>(pl->log_r2) : col_log_cb<4>(pl->log_r2);
+                if (cb2 <= pl->log_c) {
+                    pl->v2_mid = 1;
+                    pl->log_cb2 = cb2;
+                }
+            }
             const int top = w == 8 ? kCol2MaxLog64 : kCol2MaxLog32;
             if (pl->log_r >= kCol2MinLog && pl->log_r <= top && !pl->tw_smem_r) {
                 pl->v2_cols = 1;

@@ -51,7 +51,7 @@ struct bw_plan {
     int f64 = 0;
     // passes with compile-time lengths (bw_ntt.cuh); their tables are stored in
     // round order
-    int v2_rows = 0, v2_cols = 0, v2_one = 0;
+    int v2_rows = 0, v2_cols = 0, v2_mid = 0, v2_one = 0;
     bool no_v2_one = false;  // set before bw_plan_setup: tables in stage order (kq_small)
     // a single product of at most 2^12 points with 16-bit coefficients and no
     // tuning flags: one CTA (k_one), with its own n-point tables

@@ -29,6 +29,7 @@ namespace bw {
 // 8-byte residues.
 constexpr int kRow2MinLog = 5, kRow2MaxLog = 13;
 constexpr int kCol2MinLog = 3, kCol2MaxLog32 = 12, kCol2MaxLog64 = 13;
+constexpr int kMid2MinLog = 5, kMid2MaxLog = 11;
 
 // Rounds of a 2^L-point transform: the remainder round first.
 __host__ __device__ constexpr int first_rl(int L) { return L % 4 == 0 ? (L < 4 ? L : 4) : L % 4; }
@@ -41,6 +42,15 @@ __host__ __device__ inline uint32_t tw_place(int s, uint32_t i, int L) {
     const uint32_t g = i >> l, q = i & ((1u << l) - 1), G = 1u << s0;
     if (l == 0) return G + g;
     return 2 * G + 2 * (((1u << (l - 1)) - 1 + (q >> 1)) * G + g) + (q & 1);
+}
+
+// The stage of place i (i >= 1) when the first round has rl0 stages.
+__device__ __forceinline__ int stage_of_place(int i, int rl0) {
+    int s0 = rl0;
+    while (i >= (16 << s0)) s0 += 4;
+    if (i < (1 << rl0)) s0 = 0;
+    const int u = (i - (1 << s0)) >> s0;  // 0: first stage; else 2 P + 1, 2 P + 2
+    return s0 + (u == 0 ? 0 : 32 - __clz((u + 1) >> 1));
 }
 
 // One round's twiddles of a thread's sub-problem in group g (G = 2^S0 groups).
@@ -338,12 +348,7 @@ __device__ __forceinline__ void row2_body(const PlanDev<Ar>& P, typename Ar::T* 
             if (!square) xb.load(gb);
         }
         for (int i = 1 + threadIdx.x; i < (1 << S1); i += NT) {
-            // the stage of place i in the round order
-            int s0 = RL0;
-            while (i >= (16 << s0)) s0 += 4;
-            if (i < (1 << RL0)) s0 = 0;
-            const int u = (i - (1 << s0)) >> s0;  // 0: first stage; else 2 P + 1, 2 P + 2
-            const int s = s0 + (u == 0 ? 0 : 32 - __clz((u + 1) >> 1));
+            const int s = stage_of_place(i, RL0);
             R[i] = ar.mul_tw(ZL[2 * s], ld_tw(pr.WCf + i));
             Ri[i] = ar.mul_tw(ZL[2 * s + 1], ld_tw(pr.WCi + i));
         }
@@ -678,6 +683,138 @@ k_inv_col2(const PlanDev<Ar> P, typename Ar::T* res, CarryState* cst) {
     grid_release();
     grid_wait();
     inv_col2_body<Ar, LOGR>(P, res, cst, blockIdx.x, blockIdx.y, smem_raw);
+}
+
+// ------------------------------------------------------------------ middle
+// Middle column pass of the three-pass schedule (n = R * R2 * C), fixed length
+// R2 = 2^LOGR: sub-matrix s (blockIdx.y, k1 = bitrev(s) over R) is R2 rows of C
+// columns; a CTA takes a tile of columns for one prime and operand.  The outer
+// twiddle w_n^((i2 C + c) k1) is folded like a row's: zeta = w_n^(C k1) goes
+// into the stage twiddles of the first rounds, and one table of 16 x 2^LCB
+// factors zeta^j w_n^(c k1), applied before the last round, takes the rest --
+// one multiplication per element instead of two, and the tile goes from global
+// memory to registers and back without a staging pass.  The inverse mirrors it.
+template <class Ar, int LOGR>
+struct MidCfg : ColCfg<Ar, LOGR> {
+    using Base = ColCfg<Ar, LOGR>;
+    static constexpr int S1 = LOGR - 4, CB = 1 << Base::LCB;
+    static constexpr size_t tables = ((1 << S1) + 16 * CB + 16) * sizeof(Tw<typename Ar::T>);
+    static constexpr size_t smem = tables + Base::smem;
+};
+
+template <class Ar, int LOGR, bool INV>
+__global__ void __launch_bounds__(ColCfg<Ar, LOGR>::NT, ColCfg<Ar, LOGR>::kMinCtas)
+k_mid_col2(const PlanDev<Ar> P, typename Ar::T* res_a, typename Ar::T* res_b) {
+    using T = typename Ar::T;
+    using L = LayCol<T>;
+    using Cfg = MidCfg<Ar, LOGR>;
+    constexpr int LCB = ColCfg<Ar, LOGR>::LCB, CB = Cfg::CB, S1 = Cfg::S1;
+    constexpr int RL0 = first_rl(LOGR), NT = ColCfg<Ar, LOGR>::NT;
+    static_assert(LOGR > 4, "at least two rounds");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int log_c = P.log_c, s = blockIdx.y;
+    const int kp = blockIdx.z % P.K, op = blockIdx.z / P.K;
+    const PrimeDev<Ar>& pr = P.pr[kp];
+    const Ar ar = pr.ar;
+    const uint64_t c0 = (uint64_t)blockIdx.x << LCB;
+    T* g0 = (op ? res_b : res_a) + ((size_t)kp << P.log_n) + ((size_t)s << (LOGR + log_c)) + c0;
+    Tw<T>* R = reinterpret_cast<Tw<T>*>(smem_raw);  // stage twiddles of the first rounds
+    Tw<T>* Z = R + (1 << S1);                       // [j][v]: zeta^j w_n^(c k1)
+    Tw<T>* ZL = Z + 16 * CB;                        // zeta^(R2 / 2m) by stage
+    T* buf = reinterpret_cast<T*>(smem_raw + Cfg::tables);
+    const Tw<T>* W = INV ? pr.WMi : pr.WMf;
+    {
+        const uint64_t nmask = ((uint64_t)1 << P.log_n) - 1;
+        const uint64_t k1 = bitrev((uint32_t)s, P.log_r);
+        for (int i = threadIdx.x; i < 16 * CB + S1; i += NT) {
+            uint64_t e = i < 16 * CB
+                             ? (((uint64_t)(i >> LCB) << log_c) + c0 + (i & (CB - 1))) * k1
+                             : ((uint64_t)1 << (LOGR - 1 - (i - 16 * CB) + log_c)) * k1;
+            e &= nmask;
+            if (INV) e = (nmask + 1 - e) & nmask;
+            Z[i] = pow_entry(ar, e, P.lo_out, pr.OLf, pr.OHf);  // ZL follows Z
+        }
+        __syncthreads();
+        for (int i = 1 + threadIdx.x; i < (1 << S1); i += NT) {
+            const int st = stage_of_place(i, RL0);
+            R[i] = ar.mul_tw(ZL[st], ld_tw(W + i));
+        }
+        __syncthreads();
+    }
+    auto round = [&](auto s0_, auto rl_) {
+        constexpr int S0 = decltype(s0_)::value, RL = decltype(rl_)::value;
+        constexpr bool LOW = S0 == 0, HIGH = S0 + RL == LOGR;  // first / last stages
+        constexpr bool FROM_G = INV ? HIGH : LOW, TO_G = INV ? LOW : HIGH;
+        constexpr int D = LOGR - S0 - RL, DS = D + LCB, N = 1 << (LOGR + LCB - RL);
+#pragma unroll 1
+        for (int sp = threadIdx.x; sp < N; sp += NT) {
+            const int v = sp & (CB - 1), rest = sp >> LCB;
+            const int j = rest & ((1 << D) - 1), g = rest >> D;
+            const int base = (g << (D + RL)) + j;
+            const int p0 = L::p((base << LCB) + v);
+            T x[1 << RL];
+#pragma unroll
+            for (int k = 0; k < (1 << RL); ++k) {
+                if constexpr (FROM_G) {
+                    x[k] = __ldcg(g0 + ((size_t)(base + (k << D)) << log_c) + v);
+                } else {
+                    x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
+                }
+                if constexpr (HIGH && !INV) x[k] = ar.mulc(x[k], ld_w<true>(Z + (k << LCB) + v));
+            }
+            if constexpr (HIGH) {
+                const RoundTw<T, (1 << S0), false> tw(W, g);
+                if constexpr (INV) {
+                    gs_round<Ar, RL, false, false>(x, ar, tw);
+                } else {
+                    ct_round<Ar, RL, false, false, false>(x, ar, tw);
+                }
+            } else {
+                const RoundTw<T, (1 << S0), true> tw(R, g);
+                if constexpr (INV) {
+                    gs_round<Ar, RL, false, true>(x, ar, tw);
+                } else {
+                    ct_round<Ar, RL, false, false, true>(x, ar, tw);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < (1 << RL); ++k) {
+                if constexpr (HIGH && INV) x[k] = ar.mulc(x[k], ld_w<true>(Z + (k << LCB) + v));
+                if constexpr (TO_G) {
+                    g0[((size_t)(base + (k << D)) << log_c) + v] = x[k];
+                } else {
+                    buf[p0 + L::template off<false>(k, DS, 0)] = x[k];
+                }
+            }
+        }
+    };
+    using std::integral_constant;
+    constexpr bool MID1 = RL0 + 4 < LOGR, MID2 = RL0 + 8 < LOGR;  // rounds between
+    if constexpr (!INV) {
+        round(integral_constant<int, 0>{}, integral_constant<int, RL0>{});
+        __syncthreads();
+        if constexpr (MID1) {
+            round(integral_constant<int, RL0>{}, integral_constant<int, 4>{});
+            __syncthreads();
+        }
+        if constexpr (MID2) {
+            round(integral_constant<int, RL0 + 4>{}, integral_constant<int, 4>{});
+            __syncthreads();
+        }
+        round(integral_constant<int, S1>{}, integral_constant<int, 4>{});
+    } else {
+        round(integral_constant<int, S1>{}, integral_constant<int, 4>{});
+        __syncthreads();
+        if constexpr (MID2) {
+            round(integral_constant<int, RL0 + 4>{}, integral_constant<int, 4>{});
+            __syncthreads();
+        }
+        if constexpr (MID1) {
+            round(integral_constant<int, RL0>{}, integral_constant<int, 4>{});
+            __syncthreads();
+        }
+        round(integral_constant<int, 0>{}, integral_constant<int, RL0>{});
+    }
 }
 
 // ------------------------------------------------------------------ batched

@@ -153,6 +153,21 @@ cudaError_t launch_inv_col2(const bw_plan* pl, const PlanDev<Ar>& pd, typename A
     });
 }
 
+// Middle pass of `ops` operands (forward: one or two; inverse: one).
+template <class Ar, bool INV>
+cudaError_t launch_mid2(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
+                        typename Ar::T* rb, int ops, cudaStream_t s) {
+    return with_length<kMid2MinLog, kMid2MaxLog>(pl->log_r2, [&](auto lr) {
+        constexpr int LR = decltype(lr)::value;
+        using Cfg = MidCfg<Ar, LR>;
+        const cudaError_t e = allow_smem<&k_mid_col2<Ar, LR, INV>>();
+        if (e != cudaSuccess) return e;
+        const dim3 g(1u << (pl->log_c - pl->log_cb2), 1u << pl->log_r, pl->K * ops);
+        k_mid_col2<Ar, LR, INV><<<g, Cfg::NT, Cfg::smem, s>>>(pd, ra, rb);
+        return cudaSuccess;
+    });
+}
+
 template <class Ar, int RLOG>
 void launch_row(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
                 const typename Ar::T* rb, int sq, size_t smem, cudaStream_t s) {
@@ -203,7 +218,7 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     using T = typename Ar::T;
     const bw_plan* pl = c->plan;
     const PlanDev<Ar>& pd = plan_dev<Ar>(pl);
-    if (!pl->v2_cols || !pl->v2_rows || pl->log_r2) {
+    if (!pl->v2_cols || !pl->v2_rows || (pl->log_r2 && !pl->v2_mid)) {
         const int rc = bw_set_transform_attrs<Ar, SPLIT16>();
         if (rc) return rc;
     }
@@ -307,7 +322,15 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const int CB2 = 1 << pl->log_cb2;
     const size_t smem_mid = (((size_t)1 << pl->log_r2) + CB2) * sizeof(Tw<T>) +
                             tile_elems((size_t)CB2 << pl->log_r2) * sizeof(T);
-    if (pl->log_r2) {
+    bool mid2 = false;
+    if constexpr (kHasV2<Ar>) {
+        if (pl->v2_mid) {
+            mid2 = true;
+            BW_CUDA(ke);
+            BW_CUDA((launch_mid2<Ar, false>(pl, pd, ra, rb, square ? 1 : 2, c->stream)));
+        }
+    }
+    if (pl->log_r2 && !mid2) {
         dim3 gm(C / CB2, R, pl->K * (square ? 1 : 2));
         k_mid_col<Ar, false><<<gm, kColThreads, smem_mid, c->stream>>>(pd, ra, rb);
     }
@@ -334,7 +357,10 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     }
     if (timing) cudaEventRecord(c->ev[3], c->stream);
 
-    if (pl->log_r2) {
+    if constexpr (kHasV2<Ar>) {
+        if (pl->v2_mid) BW_CUDA((launch_mid2<Ar, true>(pl, pd, ra, ra, 1, c->stream)));
+    }
+    if (pl->log_r2 && !mid2) {
         dim3 gm(C / CB2, R, pl->K);
         k_mid_col<Ar, true><<<gm, kColThreads, smem_mid, c->stream>>>(pd, ra, ra);
     }

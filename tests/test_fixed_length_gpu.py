@@ -153,3 +153,28 @@ def test_group_splits_exact(log_n, path):
             bw.set_tune_entry(path, 2, log_n, log_n <= 12, 0)
         for w, got in zip(want, outs):
             assert (w == got).all(), (log_n, log_c)
+
+
+@pytest.mark.parametrize("log_r2", range(2, 12))
+@pytest.mark.parametrize("path,K,flags", [(32, 2, 0), (64, 3, L.BW_PLAN_COEF64)])
+def test_middle_lengths_exact(log_r2, path, K, flags):
+    # three passes at every middle length (below 2^5: the any-length pass), by
+    # way of the row length: n = R * R2 * C with R = R2 or 2 R2
+    for extra in (0, 1):
+        log_c = max(5, 12 - log_r2)
+        log_n = 2 * log_r2 + extra + log_c
+        if log_n > 25:
+            continue
+        total = (1 << log_n) // 2 if path == 32 else 2 << log_n
+        if total > 1 << 23:
+            continue
+        la, lb = total // 2 + 5, total // 2 - 9
+        a = mt64.random_words_top_fast(la, la)
+        b = mt64.random_words_top_fast(lb, lb)
+        a[: la // 2] = 0xFFFFFFFF
+        with bw.Plan(la, lb, path, K, log_cols=log_c, flags=flags | L.BW_PLAN_THREE_PASS) as p, \
+                bw.Context(p) as c:
+            assert p.info["log_n"] - p.info["log_rows"] - p.info["log_cols"] == log_r2
+            assert (c.multiply(a, b) == gmp_ref.mul(a, b)).all(), (la, lb)
+        with bw.Plan(la, la, path, K, flags=flags | L.BW_PLAN_THREE_PASS) as p, bw.Context(p) as c:
+            assert (c.square(a) == gmp_ref.mul(a, a)).all(), la
