@@ -738,7 +738,9 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
                 }
             }
             const int top = w == 8 ? kCol2MaxLog64 : kCol2MaxLog32;
-            if (pl->log_r >= kCol2MinLog && pl->log_r <= top && !pl->tw_smem_r) {
+            // (their addresses are 32-bit byte offsets into one prime's residues)
+            if (pl->log_r >= kCol2MinLog && pl->log_r <= top && !pl->tw_smem_r &&
+                ((size_t)w << log_n) < (size_t)1 << 32) {
                 pl->v2_cols = 1;
                 const int cb = w == 8 ? col_log_cb<8>(pl->log_r) : col_log_cb<4>(pl->log_r);
                 if (cb > log_cols_outer) {

@@ -461,33 +461,33 @@ struct ColCfg {
 template <class Ar, int CW>
 struct CoefLoad {
     using T = typename Ar::T;
-    const uint32_t* __restrict__ limbs;
-    uint32_t ncoef;  // whole coefficients
-    uint32_t lone;   // 64-bit: 1 if a single low word follows them
+    const char* __restrict__ limbs;
+    uint32_t end;   // bytes of whole coefficients
+    uint32_t lone;  // 64-bit: 1 if a single low word follows them
     bool al8;
-    __device__ __forceinline__ CoefLoad(const uint32_t* l, size_t nc) : limbs(l) {
-        ncoef = CW == 64 ? (uint32_t)(nc >> 1) : (uint32_t)nc;
+    static constexpr int kBytes = CW / 8;
+    __device__ __forceinline__ CoefLoad(const uint32_t* l, size_t nc)
+        : limbs(reinterpret_cast<const char*>(l)) {
+        end = (uint32_t)(CW == 64 ? nc >> 1 : nc) * kBytes;
         lone = CW == 64 ? (uint32_t)(nc & 1) : 0u;
         al8 = (reinterpret_cast<uintptr_t>(l) & 7u) == 0;
     }
     using Raw = typename std::conditional<
         CW == 64, uint64_t, typename std::conditional<CW == 32, uint32_t, uint16_t>::type>::type;
-    // coefficient ci, zero beyond the operand
-    __device__ __forceinline__ Raw load(uint32_t ci) const {
-        if constexpr (CW == 16) {
-            return ci < ncoef ? __ldg(reinterpret_cast<const uint16_t*>(limbs) + ci) : (uint16_t)0;
-        } else if constexpr (CW == 32) {
-            return ci < ncoef ? __ldg(limbs + ci) : 0u;
+    // the coefficient at byte offset o, zero beyond the operand
+    __device__ __forceinline__ Raw load(uint32_t o) const {
+        if constexpr (CW != 64) {
+            return o < end ? __ldg(reinterpret_cast<const Raw*>(limbs + o)) : (Raw)0;
         } else {
             uint64_t v = 0;
-            const uint32_t* w = limbs + 2 * (size_t)ci;
-            if (ci < ncoef) {
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(limbs + o);
+            if (o < end) {
                 if (al8) {
                     v = __ldg(reinterpret_cast<const unsigned long long*>(w));
                 } else {
                     v = ((uint64_t)__ldg(w + 1) << 32) | __ldg(w);
                 }
-            } else if (ci == ncoef && lone) {
+            } else if (o == end && lone) {
                 v = __ldg(w);
             }
             return v;
@@ -503,6 +503,17 @@ struct CoefLoad {
         }
     }
 };
+
+// Element at a byte offset of up to 2^32 from a CTA-uniform address: one add
+// per access instead of a 64-bit address each.
+template <typename T>
+__device__ __forceinline__ T ld_off(const T* base, uint32_t o) {
+    return __ldcg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + o));
+}
+template <typename T>
+__device__ __forceinline__ void st_off(T* base, uint32_t o, T v) {
+    *reinterpret_cast<T*>(reinterpret_cast<char*>(base) + o) = v;
+}
 
 // Forward column pass of one tile, operand and prime.  zt: the upper half of
 // the rows is zero pad.
@@ -540,10 +551,11 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
             FIRST && N > NT && sizeof(T) == 4 && NL * sizeof(Raw) <= 64;
         Raw raw[FIRST ? NL : 1];
         auto load = [&](int sp) {
-            const int v = sp & (CB - 1), j = sp >> LCB;  // g = 0
+            const uint32_t v = sp & (CB - 1), j = sp >> LCB;  // g = 0
+            const uint32_t o = ((j << log_c) + c0 + v) * coef.kBytes;
+            const uint32_t step = ((uint32_t)coef.kBytes << D) << log_c;
 #pragma unroll
-            for (int k = 0; k < NL; ++k)
-                raw[k] = coef.load(((uint32_t)(j + (k << D)) << log_c) + c0 + v);
+            for (int k = 0; k < NL; ++k) raw[k] = coef.load(o + k * step);
         };
         if constexpr (AHEAD) load(threadIdx.x);
 #pragma unroll 1
@@ -566,10 +578,12 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
                     x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
             }
             ct_round<Ar, RL, FIRST, ZT, !FIRST>(x, ar, RoundTw<T, (1 << S0), false>(pr.WRf, g));
+            const uint32_t o = (((uint32_t)base << log_c) + v) * (uint32_t)sizeof(T);
+            const uint32_t step = ((uint32_t)sizeof(T) << D) << log_c;
 #pragma unroll
             for (int k = 0; k < (1 << RL); ++k) {
                 if constexpr (LAST) {
-                    gout[((size_t)(base + (k << D)) << log_c) + v] = x[k];
+                    st_off(gout, o + k * step, x[k]);
                 } else {
                     buf[p0 + L::template off<false>(k, DS, 0)] = x[k];
                 }
@@ -641,11 +655,13 @@ __device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar:
             const int j = rest & ((1 << D) - 1), g = rest >> D;
             const int base = (g << (D + RL)) + j;
             const int p0 = L::p((base << LCB) + v);
+            const uint32_t o = (((uint32_t)base << log_c) + v) * (uint32_t)sizeof(T);
+            const uint32_t step = ((uint32_t)sizeof(T) << D) << log_c;
             T x[1 << RL];
 #pragma unroll
             for (int k = 0; k < (1 << RL); ++k) {
                 if constexpr (FIRST) {
-                    x[k] = __ldcg(g0 + ((size_t)(base + (k << D)) << log_c) + v);
+                    x[k] = ld_off(g0, o + k * step);
                 } else {
                     x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
                 }
@@ -654,7 +670,7 @@ __device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar:
 #pragma unroll
             for (int k = 0; k < (1 << RL); ++k) {
                 if constexpr (LAST) {
-                    g0[((size_t)(base + (k << D)) << log_c) + v] = ar.inv_out(x[k]);
+                    st_off(g0, o + k * step, ar.inv_out(x[k]));
                 } else {
                     buf[p0 + L::template off<false>(k, DS, 0)] = x[k];
                 }
@@ -752,11 +768,13 @@ k_mid_col2(const PlanDev<Ar> P, typename Ar::T* res_a, typename Ar::T* res_b) {
             const int j = rest & ((1 << D) - 1), g = rest >> D;
             const int base = (g << (D + RL)) + j;
             const int p0 = L::p((base << LCB) + v);
+            const uint32_t o = (((uint32_t)base << log_c) + v) * (uint32_t)sizeof(T);
+            const uint32_t step = ((uint32_t)sizeof(T) << D) << log_c;
             T x[1 << RL];
 #pragma unroll
             for (int k = 0; k < (1 << RL); ++k) {
                 if constexpr (FROM_G) {
-                    x[k] = __ldcg(g0 + ((size_t)(base + (k << D)) << log_c) + v);
+                    x[k] = ld_off(g0, o + k * step);
                 } else {
                     x[k] = buf[p0 + L::template off<false>(k, DS, 0)];
                 }
@@ -781,7 +799,7 @@ k_mid_col2(const PlanDev<Ar> P, typename Ar::T* res_a, typename Ar::T* res_b) {
             for (int k = 0; k < (1 << RL); ++k) {
                 if constexpr (HIGH && INV) x[k] = ar.mulc(x[k], ld_w<true>(Z + (k << LCB) + v));
                 if constexpr (TO_G) {
-                    g0[((size_t)(base + (k << D)) << log_c) + v] = x[k];
+                    st_off(g0, o + k * step, x[k]);
                 } else {
                     buf[p0 + L::template off<false>(k, DS, 0)] = x[k];
                 }
@@ -931,7 +949,7 @@ __device__ __forceinline__ void one_body(const PlanDev<Ar>& P, const uint32_t* a
                     const CoefLoad<Ar, CW> coef(op ? b : a, (size_t)(op ? lb : la) * CPW);
 #pragma unroll
                     for (int i = 0; i < (1 << RL); ++i)
-                        x[i] = CoefLoad<Ar, CW>::residue(ar, coef.load(base + (i << D)));
+                        x[i] = CoefLoad<Ar, CW>::residue(ar, coef.load((uint32_t)(base + (i << D)) * coef.kBytes));
                 } else {
 #pragma unroll
                     for (int i = 0; i < (1 << RL); ++i)
@@ -970,7 +988,7 @@ __device__ __forceinline__ void one_body(const PlanDev<Ar>& P, const uint32_t* a
                     const CoefLoad<Ar, CW> coef(limbs, (size_t)len * CPW);
 #pragma unroll
                     for (int i = 0; i < 16; ++i)
-                        x[i] = CoefLoad<Ar, CW>::residue(ar, coef.load(i));
+                        x[i] = CoefLoad<Ar, CW>::residue(ar, coef.load((uint32_t)i * coef.kBytes));
                 } else {
 #pragma unroll
                     for (int i = 0; i < 16; ++i) x[i] = src[p0 + L::template off<false>(i, 0, 0)];
