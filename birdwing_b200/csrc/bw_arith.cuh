@@ -58,6 +58,8 @@ struct Ar32 {
         const uint32_t m = (uint32_t)t * pinv;
         return (uint32_t)((t + (uint64_t)m * p) >> 32);
     }
+    // the pointwise product: a any forward output, b reduced to [0, 2p)
+    __device__ __forceinline__ T pointwise(T a, T b) const { return mont(fwd_to_2p(a), b); }
     // forward CT butterfly, inputs/outputs in [0, 4p)
     __device__ __forceinline__ void ct(T& a, T& b, const Tw<T>& w) const {
         const T x = red2(a);
@@ -201,6 +203,8 @@ struct Ar64 {
         const uint64_t mh = __umul64hi(m, p);
         return hi + mh + (lo != 0 ? 1ull : 0ull);
     }
+    // the pointwise product: a any forward output, b reduced to [0, 2p)
+    __device__ __forceinline__ T pointwise(T a, T b) const { return mont(fwd_to_2p(a), b); }
     // x < 2^64, w < p: x*w mod p in [0, 3p) from the truncated quotient
     // q' = x1 v1 + hi(x0 v1 + x1 v0) (the dropped x0 v0 term and the dropped
     // low bits make q' at most 2 below hi64(x * wq)).
@@ -308,26 +312,26 @@ struct Ar64 {
 //   r = (h - q p) + l = x w - q p.
 //
 // q comes from adding and subtracting 1.5 2^52, which rounds to an integer
-// while |q| <= 2^51.  q is within 1/2 + |x w / p| 2^-52 of x w / p, so
-// |r| <= p (1/2 + X p 2^-53) for |x| = X p; h - q p is an integer below 2^53,
-// so the FMA and the last addition are exact.  The FP64 pipe of an SM takes 64
-// such operations per cycle, beside the integer pipe's addressing: a butterfly
-// is 8 of them against about 40 integer instructions for a 58-bit prime
-// (measured 6.5 against 2.83 butterflies per SM-cycle).  A companion w / p per
-// constant would shorten the chain by one operation and measured 6.7, but
-// doubles the twiddle loads, and those bound the last round of a row.
+// while |q| <= 2^51.  The primes are chosen so that 1 / p is within 2^-58 of a
+// double, so q is within 1/2 + |x w / p| 2^-53 (1 + 2^-5) of x w / p, and with
+// |x| = X p, |r| <= p (1/2 + X p 2^-54 (1 + 2^-5)).  h - q p is an integer below
+// 2^53, so the FMA and the last addition are exact.  The FP64 pipe of an SM
+// takes 64 such operations per cycle, beside the integer pipe's addressing: a
+// butterfly is 8 of them against about 40 integer instructions for a 58-bit
+// prime (measured 6.5 against 2.83 butterflies per SM-cycle).  A companion
+// w / p per constant would shorten the chain by one operation and measured 6.7,
+// but doubles the twiddle loads, and those bound the last round of a row.
 //
-// POL 0: primes just above 2^50 (X < 4 keeps q below 2^51; |r| <= p (1/2 +
-//   X/8)).  Forward: a round reduces the half it does not multiply in its
-//   first stage and then adds four stages: from X = 3.9 at most 1.49, 2.18,
-//   2.95, 3.82.  Inverse: the sums of every second stage, and of a round's
-//   last, are reduced: from E at most 4E in a difference and 1/2 + E/2 at the
-//   round's end, E = 0.62, 0.81, 0.91, 0.96 over four rounds.
-// POL 1: primes just above 2^51.66 (X <= 1.26 for q, 2.5 for exact sums,
-//   |r| <= p (1/2 + 0.4 X)), for transforms whose coefficients need three such
+// POL 0: primes within 1% above 2^50: q needs X <= 3.96, |r| <= p (1/2 + 0.066
+//   X).  Forward: a round reduces the half it does not multiply in its first
+//   stage and then adds four stages: from X = 3.1 at most 1.21, 1.79, 2.41,
+//   3.07.  Inverse: the sums of every second stage, and of a round's last, are
+//   reduced: from E a difference of 4 E and an output of 1/2 + 0.27 E, so E
+//   stays below 0.69 and differences below 2.8.
+// POL 1: primes just above 2^51.67 (X <= 1.24 for q, 2.4 for exact sums, |r| <=
+//   p (1/2 + 0.21 X)), for transforms whose coefficients need three such
 //   primes: a forward round reduces all its values before its first and third
-//   stage (at most 0.7 + 0.5 = 1.2, then 2.2), an inverse stage reduces both
-//   outputs.
+//   stage (at most 1.11, then 1.85), an inverse stage reduces both outputs.
 template <int POL>
 struct ArD {
     using T = double;
@@ -351,8 +355,11 @@ struct ArD {
         const double l = __fma_rn(x, w, -h);
         return __dadd_rn(__fma_rn(-q, p, h), l);
     }
-    // product of two residues reduced by red
-    __device__ __forceinline__ T mont(T a, T b) const { return POL ? red(mul(a, b)) : mul(a, b); }
+    // the pointwise product: a any forward output, b reduced (POL 0: |a b| <=
+    // 3.1 p * p/2, so |q| < 2^51 and the result is below 0.61 p)
+    __device__ __forceinline__ T pointwise(T a, T b) const {
+        return POL ? red(mul(red(a), b)) : mul(a, b);
+    }
     // value u of a round of half width h before its stage l; ent: the round's
     // inputs may be any forward output (else they are reduced)
     __device__ __forceinline__ T ct_enter(T x, int u, int h, int l, bool ent) const {

@@ -103,12 +103,13 @@ const uint64_t kP32W[6] = {595591169ull, 645922817ull, 754974721ull,
                            880803841ull, 897581057ull, 998244353ull};
 const uint64_t kG32W[6] = {3, 3, 11, 26, 3, 3};
 
-// 64-bit path, 64-bit coefficients in double-precision arithmetic (ArD): the
-// smallest primes c 2^32 + 1 above 2^50, and the smallest whose product is
-// above 2^155.
-const uint64_t kPD[2][3] = {{0x4000e00000001ull, 0x4001100000001ull, 0x4002100000001ull},
-                            {0xcb30200000001ull, 0xcb30a00000001ull, 0xcb3a400000001ull}};
-const uint64_t kGD[2][3] = {{19, 7, 3}, {3, 5, 3}};
+// Double-precision arithmetic (ArD): primes c 2^32 + 1 above 2^50, at most 1%,
+// and above 2^(155/3) with a product above 2^155.  Among those the ones whose
+// reciprocal a double holds best: 1 / p rounds with a relative error below
+// 2^-58 (2^-61), so a quotient's error is the product's rounding alone.
+const uint64_t kPD[2][3] = {{0x40a1000000001ull, 0x408c100000001ull, 0x4044900000001ull},
+                            {0xcea1e00000001ull, 0xcc4c500000001ull, 0xce1a500000001ull}};
+const uint64_t kGD[2][3] = {{7, 3, 17}, {5, 13, 10}};
 
 int v2(uint64_t x) {
     int k = 0;

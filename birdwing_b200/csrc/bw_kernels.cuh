@@ -873,7 +873,7 @@ __device__ __forceinline__ void row_body(const PlanDev<Ar>& P, typename Ar::T* r
             ct_stages<Ar, 4, false>(x, s_last, tid, pr.WCf, ar, false);
 #pragma unroll
             for (int k = 0; k < 16; ++k)
-                x[k] = ar.mont(ar.fwd_to_2p(x[k]), ar.fwd_to_2p(bufA[pb + k]));
+                x[k] = ar.pointwise(bufA[pb + k], ar.fwd_to_2p(x[k]));
             gs_stages<Ar, 4, false>(x, s_last, tid, pr.WCi, ar);
 #pragma unroll
             for (int k = 0; k < 16; ++k) bufA[pb + k] = x[k];
@@ -904,8 +904,8 @@ __device__ __forceinline__ void row_body(const PlanDev<Ar>& P, typename Ar::T* r
         ct_stages<Ar, RL, false>(x, s0, g, pr.WCf, ar, false);                         \
         _Pragma("unroll") for (int k = 0; k < (1 << RL); ++k) {                        \
             const T xa = ar.fwd_to_2p(x[k]);                                           \
-            const T ya = square ? xa : ar.fwd_to_2p(bufA[p0 + k]);                     \
-            x[k] = ar.mont(xa, ya);                                                    \
+            const T ya = square ? xa : bufA[p0 + k];                                   \
+            x[k] = ar.pointwise(ya, xa);                                               \
         }                                                                              \
         gs_stages<Ar, RL, false>(x, s0, g, pr.WCi, ar);                                \
         _Pragma("unroll") for (int k = 0; k < (1 << RL); ++k) {                        \
@@ -1848,8 +1848,11 @@ k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __res
 }
 
 // any: set when a tile's kind is not kill (zero between products).
+// Four CTAs per SM with 64-bit coefficients (56 registers; 2^23 coefficients
+// 78 -> 71 us, double precision, 83 -> 77 six primes), three otherwise (at four
+// the digit sums spill: 2^20 points 47 -> 50 us for the product).
 template <class Ar, bool SPLIT16, bool W64 = false>
-__global__ void __launch_bounds__(kWordsThreads, 3)
+__global__ void __launch_bounds__(kWordsThreads, W64 ? 4 : 3)
 k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
               uint32_t* __restrict__ out, size_t M, size_t NL, uint32_t* __restrict__ kinds,
               uint32_t* __restrict__ any, uint32_t* __restrict__ err) {
@@ -2083,8 +2086,8 @@ __device__ __forceinline__ void ks_product_body(const PlanDev<Ar>& P, const Batc
         ct_stages<Ar, RL, false>(x, s0, g, pr.WCf, ar, false);                         \
         _Pragma("unroll") for (int k = 0; k < (1 << RL); ++k) {                        \
             const T xa = ar.fwd_to_2p(x[k]);                                           \
-            const T ya = sq ? xa : ar.fwd_to_2p(bufA[p0 + k]);                         \
-            x[k] = ar.mont(xa, ya);                                                    \
+            const T ya = sq ? xa : bufA[p0 + k];                                       \
+            x[k] = ar.pointwise(ya, xa);                                               \
         }                                                                              \
         gs_stages<Ar, RL, false>(x, s0, g, pr.WCi, ar);                                \
         _Pragma("unroll") for (int k = 0; k < (1 << RL); ++k) {                        \

@@ -392,14 +392,14 @@ __device__ __forceinline__ void row2_body(const PlanDev<Ar>& P, typename Ar::T* 
 #pragma unroll
             for (int k = 0; k < NE; ++k) {
                 const T v = ar.fwd_to_2p(x[k]);
-                x[k] = ar.mont(v, v);
+                x[k] = ar.pointwise(v, v);
             }
         } else {
 #pragma unroll
             for (int k = 0; k < NE; ++k) bufA[p0 + k] = ar.fwd_to_2p(x[k]);
             fwd(bufB);
 #pragma unroll
-            for (int k = 0; k < NE; ++k) x[k] = ar.mont(ar.fwd_to_2p(x[k]), bufA[p0 + k]);
+            for (int k = 0; k < NE; ++k) x[k] = ar.pointwise(x[k], bufA[p0 + k]);
         }
         gs_round<Ar, RLAST, false, false>(x, ar, ti);
 #pragma unroll
@@ -1000,14 +1000,14 @@ __device__ __forceinline__ void one_body(const PlanDev<Ar>& P, const uint32_t* a
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const T v = ar.fwd_to_2p(x[i]);
-                    x[i] = ar.mont(v, v);
+                    x[i] = ar.pointwise(v, v);
                 }
             } else {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) A[p0 + i] = ar.fwd_to_2p(x[i]);
                 last(B, b, lb);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) x[i] = ar.mont(ar.fwd_to_2p(x[i]), A[p0 + i]);
+                for (int i = 0; i < 16; ++i) x[i] = ar.pointwise(x[i], A[p0 + i]);
             }
             gs_round<Ar, 4, SL == 0, true>(x, ar, ti);
 #pragma unroll

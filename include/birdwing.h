@@ -16,7 +16,7 @@
  *                 transform length is twice the limb count).
  *   BW_PATH_P64 : 32-bit coefficients, 58-bit primes of the form c*2^32+1,
  *                 64-bit modular arithmetic; with 64-bit coefficients
- *                 (BW_PLAN_COEF64) primes of 50 to 52 bits in exact
+ *                 (BW_PLAN_COEF64) primes of 51 and 52 bits in exact
  *                 double-precision modular arithmetic (58-bit ones when the
  *                 shorter operand has more than 2^28 words) (the reference's LIMB_BITS=64
  *                 "hybrid" and NATIVE_HOST_LIMBS pipelines; a u64 limb array

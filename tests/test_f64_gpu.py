@@ -2,6 +2,8 @@
 arithmetic: two prime sets, chosen by the shorter operand's coefficients.
 Products are exact against GMP at the edges of the choice, of the transform
 lengths and of the coefficients' range (all words at their maximum)."""
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
@@ -43,5 +45,10 @@ def test_prime_sets_meet():
     assert first[0] * first[1] * first[2] > 1 << 150
     assert second[0] * second[1] * second[2] > 1 << 155
     assert check(ones, ones, L.BW_PLAN_THREE_PASS) == second
+    # the bounds on the quotients: 1 / p within 2^-58 of a double, 2 p < 2^53 / 1.2
+    for ps in (first, second):
+        for q in ps:
+            assert abs(Fraction(1.0 / q) * q - 1) < Fraction(1, 1 << 58)
+            assert (q - 1) % (1 << 32) == 0 and q.bit_length() in (51, 52)
     # unbalanced: a long transform with a short operand stays on the first set
     assert check(mt64.random_words_top_fast((1 << 24) + 3, 5), ones[:7]) == first
