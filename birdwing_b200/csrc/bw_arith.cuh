@@ -118,7 +118,7 @@ struct Ar32 {
     }
     // a 64-bit coefficient x = h 2^32 + l reduced to [0, 2p): h (2^32 mod p)
     // and l * 1 by Shoup, each in [0, 2p), their sum below 4p
-    __device__ __forceinline__ T reduce64(uint64_t x) const {
+    __device__ __forceinline__ T from_u64(uint64_t x) const {
         const T h = shoup((uint32_t)(x >> 32), r32, r32q);
         const T l = shoup((uint32_t)x, 1u, oneq);
         return red2(h + l);
@@ -270,7 +270,7 @@ struct Ar64 {
     // a 64-bit coefficient -> [0, 2p): the path's primes are c 2^32 + 1 with
     // 2^25 < c < 2^26, so q = x >> 58 is floor(x / p) or one less (x / p - q
     // < 1 + 2^-13), and x - q p = (x - q) - (q c) 2^32
-    __device__ __forceinline__ T reduce_in(T x) const {
+    __device__ __forceinline__ T from_u64(T x) const {
         const uint32_t q = (uint32_t)(x >> 58);
         return x - q - ((uint64_t)(q * c) << 32);
     }

@@ -727,10 +727,14 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
                          pl->log_c == 12 && pl->rlog_row == 4)
                             ? 1
                             : 0;
-        // passes with compile-time lengths: the 32-bit and double-precision
-        // arithmetics
-        if (path == BW_PATH_P32 || pl->f64) {
-            pl->v2_rows = pl->log_c >= kRow2MinLog && pl->log_c <= kRow2MaxLog;
+        // passes with compile-time lengths.  The row pass starts from the
+        // column pass's outputs without reducing them; 58-bit primes have room
+        // for 20 stages of 3p each before its first multiplication of every
+        // value (64p in a word)
+        {
+            const bool room = path == BW_PATH_P32 || pl->f64 ||
+                              (pl->log_r2 ? 4 + pl->log_c - 4 : pl->log_r + pl->log_c - 4) <= 20;
+            pl->v2_rows = pl->log_c >= kRow2MinLog && pl->log_c <= kRow2MaxLog && room;
             if (pl->log_r2 >= kMid2MinLog && pl->log_r2 <= kMid2MaxLog) {
                 const int cb2 = w == 8 ? col_log_cb<8>(pl->log_r2) : col_log_cb<4>(pl->log_r2);
                 if (cb2 <= pl->log_c) {

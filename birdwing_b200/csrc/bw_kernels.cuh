@@ -567,7 +567,7 @@ __device__ __forceinline__ void fwd_col_body(const PlanDev<Ar>& P,
             } else if (wi < ncoef) {
                 x = __ldg(limbs + wi);
             }
-            buf[LayCol<T>::p(e)] = ar0.reduce64(x);
+            buf[LayCol<T>::p(e)] = ar0.from_u64(x);
         }
     } else if (W64 && PP && (reinterpret_cast<uintptr_t>(limbs) & 7u) == 0) {
         // 64-bit coefficients of an 8-byte-aligned operand: one 8-byte copy
@@ -660,7 +660,7 @@ __device__ __forceinline__ void fwd_col_body(const PlanDev<Ar>& P,
                         if constexpr (PP) {
                             return buf[p];
                         } else {
-                            return ar.reduce64(coef[(idx << log_cb) + v]);
+                            return ar.from_u64(coef[(idx << log_cb) + v]);
                         }
                     } else {
                         if constexpr (Ar::kF64) {
@@ -675,7 +675,7 @@ __device__ __forceinline__ void fwd_col_body(const PlanDev<Ar>& P,
                         if constexpr (W64 && !Ar::kF64) {
                             // a 64-bit coefficient (up to 64p) enters reduced
                             // to [0, 2p), leaving the transform its headroom
-                            x = ar.reduce_in(x);
+                            x = ar.from_u64(x);
                         }
                         return x;
                     }

@@ -62,7 +62,13 @@ struct RoundTw {
     __device__ __forceinline__ Tw<T> one() const { return ld_w<SM>(p1); }
     // positions 2 j, 2 j + 1 of stage l: P = 2^(l-1) - 1 + j
     __device__ __forceinline__ void pair(int P, Tw<T>& a, Tw<T>& b) const {
-        ld_w2<SM>(p2 + (size_t)P * 2 * G, a, b);
+        const Tw<T>* p = p2 + (size_t)P * 2 * G;
+        if constexpr (sizeof(Tw<T>) == 8) {
+            ld_w2<SM>(p, a, b);
+        } else {
+            a = ld_w<SM>(p);
+            b = ld_w<SM>(p + 1);
+        }
     }
 };
 
@@ -155,6 +161,13 @@ __device__ __forceinline__ void gs_round(typename Ar::T* x, const Ar& ar, const 
     }
 }
 
+// Resident threads per SM the register bounds aim at: 1024 of 64 registers
+// (32-bit path), 768 of 80 (double precision), 512 of 128 (64-bit integers).
+template <class Ar>
+__host__ __device__ constexpr int resident_threads() {
+    return sizeof(typename Ar::T) == 4 ? 1024 : Ar::kF64 ? 768 : 512;
+}
+
 // Row layout: 8-byte residues e + e/16, conflict-free for every round (a
 // 64-bit access is served 16 lanes at a time).  4-byte residues e + e/32:
 // conflict-free for unit-stride lanes and for the stride-16 lanes of a last
@@ -200,9 +213,7 @@ struct RowCfg {
         return ((size_t)2 * (1 << S1) + 32 + 32) * sizeof(Tw<typename Ar::T>) +
                tile_elems(C) * sizeof(typename Ar::T) * (sq ? 1 : 2);
     }
-    // resident CTAs the register bound aims at: 768 threads of 80 registers
-    // (double precision), 1024 of 64
-    static constexpr int kMinCtas = (sizeof(typename Ar::T) == 8 ? 768 : 1024) / NT;
+    static constexpr int kMinCtas = resident_threads<Ar>() / NT;
 };
 
 // A thread's elements of a row's first round, all loaded at once (rows of one
@@ -452,7 +463,7 @@ struct ColCfg {
     static constexpr int NSUB = 1 << (LOGR + LCB - RLAST);
     static constexpr int NT = NSUB < 32 ? 32 : NSUB > 256 ? 256 : NSUB;
     static constexpr size_t smem = tile_elems((size_t)1 << (LOGR + LCB)) * sizeof(typename Ar::T);
-    static constexpr int kMinCtas = (sizeof(typename Ar::T) == 8 ? 768 : 1024) / NT;
+    static constexpr int kMinCtas = resident_threads<Ar>() / NT;
 };
 
 // The tile's coefficients, as the first forward round reads them.
@@ -496,10 +507,8 @@ struct CoefLoad {
     static __device__ __forceinline__ T residue(const Ar& ar, Raw v) {
         if constexpr (CW != 64) {
             return Ar::from_u32(v);
-        } else if constexpr (Ar::kF64) {
-            return ar.from_u64(v);
         } else {
-            return ar.reduce64(v);
+            return ar.from_u64(v);
         }
     }
 };

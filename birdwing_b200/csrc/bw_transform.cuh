@@ -71,10 +71,6 @@ int bw_set_transform_attrs() {
 }
 
 
-// Whether an arithmetic has the fixed-length passes.
-template <class Ar>
-constexpr bool kHasV2 = Ar::kF64 || sizeof(typename Ar::T) == 4;
-
 // Raise a kernel's dynamic shared-memory limit once.
 template <auto KERN>
 cudaError_t allow_smem() {
@@ -248,7 +244,7 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const unsigned zt = (pl->zt_a ? 1u : 0u) | (pl->zt_b ? 2u : 0u);
     cudaError_t ke = cudaSuccess;  // a fixed-length launch's status
     auto k1 = [&](int tile0, int ntiles) {
-        if constexpr (kHasV2<Ar>) {
+        {
             if (pl->v2_cols) {
                 ke = launch_fwd_col2<Ar, W64 ? 64 : SPLIT16 ? 16 : 32>(
                     pl, pd, a, in_a, b, in_b, ra, rb, zt, tile0, ntiles, square, c->stream);
@@ -323,7 +319,7 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const size_t smem_mid = (((size_t)1 << pl->log_r2) + CB2) * sizeof(Tw<T>) +
                             tile_elems((size_t)CB2 << pl->log_r2) * sizeof(T);
     bool mid2 = false;
-    if constexpr (kHasV2<Ar>) {
+    {
         if (pl->v2_mid) {
             mid2 = true;
             BW_CUDA(ke);
@@ -343,11 +339,9 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const int sq = square ? 1 : 0;
     bool row_done = false;
     BW_CUDA(ke);
-    if constexpr (kHasV2<Ar>) {
-        if (pl->v2_rows) {
-            BW_CUDA(launch_row2<Ar>(pl, pd, ra, rbs, sq, !timing, c->stream));
-            row_done = true;
-        }
+    if (pl->v2_rows) {
+        BW_CUDA(launch_row2<Ar>(pl, pd, ra, rbs, sq, !timing, c->stream));
+        row_done = true;
     }
     if (row_done) {
     } else if (pl->rlog_row == 3) {
@@ -357,7 +351,7 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     }
     if (timing) cudaEventRecord(c->ev[3], c->stream);
 
-    if constexpr (kHasV2<Ar>) {
+    {
         if (pl->v2_mid) BW_CUDA((launch_mid2<Ar, true>(pl, pd, ra, ra, 1, c->stream)));
     }
     if (pl->log_r2 && !mid2) {
@@ -367,7 +361,7 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const size_t smem3 = tw_bytes + tile_elems((size_t)R * CB) * sizeof(T);
     dim3 g3(cols_outer / CB, pl->K);
     bool inv_done = false;
-    if constexpr (kHasV2<Ar>) {
+    {
         if (pl->v2_cols) {
             BW_CUDA(launch_inv_col2<Ar>(pl, pd, ra, c->cst, cols_outer / CB, !timing,
                                         c->stream));

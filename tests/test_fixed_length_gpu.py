@@ -16,8 +16,8 @@ pytestmark = pytest.mark.gpu
 # with many columns, and lengths just outside the instantiated range
 SPLITS = ([(7, c) for c in range(4, 14)] + [(r, 6) for r in range(2, 14)] +
           [(r, 12) for r in (5, 6, 8, 9, 10)] + [(5, 13), (6, 13), (3, 9), (12, 9), (3, 7), (4, 7), (3, 12)])
-# path, primes, plan flags, coefficients per 64-bit pair of words
-FORMS = [(32, 2, 0, 4), (32, 3, 0, 4), (32, 6, L.BW_PLAN_COEF64, 1),
+# path, primes, plan flags, coefficients per pair of words
+FORMS = [(32, 2, 0, 4), (32, 3, 0, 4), (32, 6, L.BW_PLAN_COEF64, 1), (64, 2, 0, 2), (64, 3, 0, 2),
          (64, 3, L.BW_PLAN_COEF64, 1)]
 
 
@@ -26,7 +26,7 @@ FORMS = [(32, 2, 0, 4), (32, 3, 0, 4), (32, 6, L.BW_PLAN_COEF64, 1),
 def test_split_exact(log_r, log_c, path, K, flags, per):
     n = 1 << (log_r + log_c)
     # words of a product that fills the transform
-    total = n // 2 if per == 4 else 2 * n
+    total = 2 * n // per
     for la, lb in ((total // 2, total // 2), (total // 2 + 3, total // 2 - 7),
                    (total - 9, 5)):
         a = mt64.random_words_top_fast(la, 3 * la + log_r)
