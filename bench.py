@@ -427,9 +427,12 @@ def batch_items(cfg, rank):
 def plain_launches(path, la, lb):
     """Kernels one plain product launches: the three transform passes, then
     the words pass and the carry fix when the output spans more than one
-    2048-word tile (the words pass alone otherwise)."""
+    2048-word tile (the words pass alone otherwise); one kernel up to 2^11
+    points on the 32-bit path."""
     cpw = 2 if path == 32 else 1
     log_n = max(4, ((la + lb) * cpw - 2).bit_length())
+    if path == 32 and log_n <= 11:
+        return 1
     words = max((1 << log_n) // cpw, la + lb)
     return 3 + (2 if words > 2048 else 1)
 

@@ -609,11 +609,17 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
             // products, 32-bit path), 2^14 points 8 x 2048 107, 32 x 512 128;
             // 2^16 points 16 x 4096 436, 128 x 512 465; 2^17 points 128 x 1024
             // 469, 32 x 4096 516
+            // A single product from 2^17 to 2^20 points: columns of 2^7 or 2^8
+            // (two rounds) and longer rows, measured three products in flight,
+            // against the square split: 2^18 points 12.7 -> 10.7 us, 2^20 31.6
+            // -> 28.1 (two primes), 2^19 49 -> 40 and 2^20 94 -> 88 (six), 44
+            // -> 35 and 83 -> 77 (double precision); equal or slower elsewhere
             const int square = (log_n + 1) / 2;
+            const int single_c = log_n >= 17 && log_n <= 20 ? (log_n + 4) / 2 : square;
             const int group_c = log_n <= 14   ? std::max(log_n - 3, square)
                                 : log_n <= 16 ? log_n - 4
                                               : std::max(10, square);
-            pl->log_c = std::min(max_c, mode == 0 ? group_c : square);
+            pl->log_c = std::min(max_c, mode == 0 ? group_c : single_c);
             if (want_c) {
                 if (want_c > max_c || want_c >= log_n || log_n - want_c > 13)
                     return bw_fail(BW_EINVAL, "BW_PLAN_LOG_COLS(%d) invalid for n = 2^%d",

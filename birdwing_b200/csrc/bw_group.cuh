@@ -133,7 +133,16 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
     } else {
         kb_inv_col<Ar, 4><<<dim3(C / CB, pl.K, np), kColThreads, smem3, s>>>(P, g.d_desc, ra);
     }
-    kb_garner_carry<Ar, SPLIT16><<<dim3((unsigned)g.ntiles, np), kCarryThreads, 0, s>>>(
-        P, g.d_desc, ra, 1u, g.inject_wait_fault ? 1u + (1u << 27) : 1u, g.d_err, g.spin_limit);
+    if (g.inject_wait_fault) {
+        // the look-back form, whose waits the test hook makes run out
+        kb_garner_carry<Ar, SPLIT16><<<dim3((unsigned)g.ntiles, np), kCarryThreads, 0, s>>>(
+            P, g.d_desc, ra, 1u, 1u + (1u << 27), g.d_err, g.spin_limit);
+    } else {
+        kb_carry_words<Ar, SPLIT16><<<dim3((unsigned)g.ntiles, np), kWordsThreads, 0, s>>>(
+            P, g.d_desc, ra, g.d_err);
+        if (g.ntiles > 1)
+            kb_carry_fix<<<np, kBatchFixThreads, 0, s>>>(
+                g.d_desc, ((size_t)1 << pl.log_n) / (SPLIT16 ? 2 : 1));
+    }
     return cudaGetLastError();
 }

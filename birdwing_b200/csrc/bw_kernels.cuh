@@ -1794,19 +1794,19 @@ __device__ __forceinline__ void garner_carry_body(
 // 72 -> 92 us at 2^24 words, and no gain in a graph at 2^16.)
 constexpr int kWordsThreads = kCarryThreads + 32;
 
-// One CTA: each thread takes a contiguous run of tiles; a run passes on a
-// constant (its last non-propagating tile's carry) or its own carry-in, and a
-// scan over the runs in shared memory gives each run its carry-in.
+// One CTA of NT threads: each thread takes a contiguous run of tiles; a run
+// passes on a constant (its last non-propagating tile's carry) or its own
+// carry-in, and a scan over the runs in shared memory gives each run its
+// carry-in.
 constexpr int kFixThreads = 1024;
-static __global__ void __launch_bounds__(kFixThreads)
-k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __restrict__ out,
-            size_t M, uint32_t* __restrict__ any) {
-    grid_release();
-    grid_wait();
+template <int NT>
+__device__ __forceinline__ void carry_fix_body(const uint32_t* __restrict__ kinds,
+                                               uint32_t ntiles, uint32_t* __restrict__ out,
+                                               size_t M, uint32_t* __restrict__ any) {
     if (__ldcg(any) == 0u) return;  // every tile kills
-    __shared__ uint32_t s_f[kFixThreads];  // 0, 1: constant carry out; 2: passes carry-in
+    __shared__ uint32_t s_f[NT];    // 0, 1: constant carry out; 2: passes carry-in
     const int tid = threadIdx.x;
-    const uint32_t per = (ntiles + kFixThreads - 1) / kFixThreads;
+    const uint32_t per = (ntiles + NT - 1) / NT;
     const uint32_t t0 = min(ntiles, (uint32_t)tid * per), t1 = min(ntiles, t0 + per);
     uint32_t f = 2;
     for (uint32_t t = t0; t < t1; ++t) {
@@ -1818,7 +1818,7 @@ k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __res
     if (tid == 0) *any = 0u;  // for the next product (every thread has read it)
     // inclusive scan of "the latest constant": combine(a, b) = b unless b
     // passes its carry-in
-    for (int d = 1; d < kFixThreads; d <<= 1) {
+    for (int d = 1; d < NT; d <<= 1) {
         const uint32_t a = tid >= d ? s_f[tid - d] : 2u;
         __syncthreads();
         if (s_f[tid] == 2u) s_f[tid] = a;
@@ -1847,15 +1847,25 @@ k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __res
     }
 }
 
+static __global__ void __launch_bounds__(kFixThreads)
+k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __restrict__ out,
+            size_t M, uint32_t* __restrict__ any) {
+    grid_release();
+    grid_wait();
+    carry_fix_body<kFixThreads>(kinds, ntiles, out, M, any);
+}
+
 // any: set when a tile's kind is not kill (zero between products).
 // Four CTAs per SM with 64-bit coefficients (56 registers; 2^23 coefficients
 // 78 -> 71 us, double precision, 83 -> 77 six primes), three otherwise (at four
 // the digit sums spill: 2^20 points 47 -> 50 us for the product).
-template <class Ar, bool SPLIT16, bool W64 = false>
-__global__ void __launch_bounds__(kWordsThreads, W64 ? 4 : 3)
-k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
-              uint32_t* __restrict__ out, size_t M, size_t NL, uint32_t* __restrict__ kinds,
-              uint32_t* __restrict__ any, uint32_t* __restrict__ err) {
+template <class Ar, bool SPLIT16, bool W64>
+__device__ __forceinline__ void carry_words_body(const PlanDev<Ar>& P,
+                                                 const typename Ar::T* __restrict__ res,
+                                                 uint32_t* __restrict__ out, size_t M, size_t NL,
+                                                 uint32_t* __restrict__ kinds,
+                                                 uint32_t* __restrict__ any,
+                                                 uint32_t* __restrict__ err) {
     constexpr int E = kCarryWordsPerThread;
     constexpr int TL = kCarryTileWords;
     __shared__ CarryShared sh;
@@ -1870,8 +1880,6 @@ k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
     uint32_t l[E];
     uint32_t X[3];
     uint32_t bad = 0;
-    grid_release();
-    grid_wait();
     garner_local<Ar, SPLIT16, W64, false>(
         P, res + (valid ? j0 : 0) * elems_per_word2<SPLIT16, W64>() / 2, n, valid, l, X, &bad);
     if (bad && own) atomicOr(err, 2u);
@@ -1932,6 +1940,40 @@ k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
         kinds[t] = kind;
         if (kind) atomicOr(any, 1u);
     }
+}
+
+template <class Ar, bool SPLIT16, bool W64 = false>
+__global__ void __launch_bounds__(kWordsThreads, W64 ? 4 : 3)
+k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
+              uint32_t* __restrict__ out, size_t M, size_t NL, uint32_t* __restrict__ kinds,
+              uint32_t* __restrict__ any, uint32_t* __restrict__ err) {
+    grid_release();
+    grid_wait();
+    carry_words_body<Ar, SPLIT16, W64>(P, res, out, M, NL, kinds, any, err);
+}
+
+// batched: blockIdx.y = product; the look-back kernel's 22-34% of issue slots
+// were waits between a product's tiles (126 products of 2^17 points, 32-bit
+// path: 86 us of 470)
+template <class Ar, bool SPLIT16>
+__global__ void __launch_bounds__(kWordsThreads, 3)
+kb_carry_words(const PlanDev<Ar> P, const BatchProd* __restrict__ D,
+               const typename Ar::T* __restrict__ res_a, uint32_t* __restrict__ err) {
+    const BatchProd d = D[blockIdx.y];
+    const size_t NL = ((size_t)1 << P.log_n) / (SPLIT16 ? 2 : 1);
+    const size_t M = (size_t)d.la + d.lb;
+    if ((size_t)blockIdx.x * kCarryTileWords >= (NL > M ? NL : M)) return;
+    carry_words_body<Ar, SPLIT16, false>(P, res_a + d.res_off, d.out, M, NL, d.rec_s, &d.cst->any,
+                                         err);
+}
+constexpr int kBatchFixThreads = 64;
+static __global__ void __launch_bounds__(kBatchFixThreads)
+kb_carry_fix(const BatchProd* __restrict__ D, size_t NL) {
+    const BatchProd d = D[blockIdx.x];
+    const size_t M = (size_t)d.la + d.lb, words = NL > M ? NL : M;
+    carry_fix_body<kBatchFixThreads>(d.rec_s,
+                                     (uint32_t)((words + kCarryTileWords - 1) / kCarryTileWords),
+                                     d.out, M, &d.cst->any);
 }
 
 // Carry words of the last thread of every tile but the last (its 8 words'

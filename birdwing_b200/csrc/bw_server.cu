@@ -403,7 +403,7 @@ int launch_group(bw_server* s, Group* g) {
     if (e != cudaSuccess) return bw_fail(BW_ECUDA, "launch: %s", cudaGetErrorString(e));
     {
         std::lock_guard<std::mutex> lk(s->mu);
-        s->launches += small ? 1 : 4;
+        s->launches += small ? 1 : ntiles > 1 ? 5 : 4;
     }
     return BW_OK;
 }
