@@ -261,6 +261,9 @@ void finish_group_locked(bw_server* s, Group* g, int status, Clock::time_point t
     }
 }
 
+// Look-back states of a group up to this size ride in its H2D copy.
+constexpr size_t kStagedStates = 64 << 10;
+
 // Lay out, stage and issue one group on its lane.  Called without the lock.
 int launch_group(bw_server* s, Group* g) {
     const Req* r0 = g->reqs[0];
@@ -274,12 +277,14 @@ int launch_group(bw_server* s, Group* g) {
     size_t max_words = 0;
     for (const Req* r : g->reqs) max_words = std::max(max_words, r->la + r->lb);
     const size_t ntiles = bw_group_ntiles(path, log_n, max_words);
-    // Device block: [desc | staged inputs | direct inputs | err | staged
-    // outputs | direct outputs | states | res_a | res_b].  The pinned staging
-    // block holds [desc | staged inputs] and [err | staged outputs], so one
-    // H2D and one D2H copy move every staged operand and result; operands and
-    // results in the caller's own pinned memory (large ones) move by DMA
-    // straight from and to it.
+    // Device block: [desc | staged inputs | states | err | staged outputs |
+    // direct inputs | direct outputs | large states | res_a | res_b].  The
+    // pinned staging block holds the same up to the staged outputs: one H2D
+    // copy brings descriptors, operands and the cleared look-back states and
+    // error word, one D2H copy takes the error word and every staged result;
+    // operands and results in the caller's own pinned memory (large ones) move
+    // by DMA straight from and to it.  (Clearing by memset took one or two of
+    // the eight to eleven calls a group costs on the host.)
     auto direct = [](bool pinned, size_t words) { return pinned && words * 4 >= kDirectBytes; };
     size_t off = align_up(np * sizeof(BatchProd), 16);
     for (Req* r : g->reqs) {
@@ -292,7 +297,37 @@ int launch_group(bw_server* s, Group* g) {
             off += 4 * align_up(r->lb, 4);
         }
     }
+    const size_t st_stride = small ? 0 : bw_group_state_stride(ntiles);
+    const size_t st_bytes = np * st_stride;
+    size_t staged_out = 0;
+    for (const Req* r : g->reqs)
+        if (!direct(r->c_pin, r->la + r->lb)) staged_out += 4 * align_up(r->la + r->lb, 4);
+    // (only into the room a staging block's power-of-two size leaves: the
+    // requests' staging charge does not count the states)
+    auto block = [](size_t x) {
+        size_t b = 4096;
+        while (b < x) b <<= 1;
+        return b;
+    };
+    const bool st_staged = st_bytes <= kStagedStates &&
+                           block(off + 16 + staged_out + st_bytes) == block(off + 16 + staged_out);
+    const size_t in_end = off;
+    size_t st_off = off;
+    if (st_staged) off += st_bytes;  // (a 16-byte multiple)
+    g->err_off = off;
+    off += 16;
     const size_t staged_in_end = off;
+    size_t pin_off = off;  // the staging block has the same layout up to here
+    g->err_pin = g->err_off;
+    for (Req* r : g->reqs) {
+        if (!direct(r->c_pin, r->la + r->lb)) {
+            r->off_c = off / 4;
+            r->off_c_pin = pin_off / 4;
+            off += 4 * align_up(r->la + r->lb, 4);
+            pin_off += 4 * align_up(r->la + r->lb, 4);
+        }
+    }
+    g->out_bytes = off - g->err_off - 16;  // staged outputs only
     for (Req* r : g->reqs) {
         if (direct(r->a_pin, r->la)) {
             r->off_a = off / 4;
@@ -304,20 +339,6 @@ int launch_group(bw_server* s, Group* g) {
         }
         if (r->square) r->off_b = r->off_a;
     }
-    g->err_off = off;
-    off += 16;
-    size_t pin_off = staged_in_end;  // err + staged outputs follow the inputs
-    g->err_pin = pin_off;
-    pin_off += 16;
-    for (Req* r : g->reqs) {
-        if (!direct(r->c_pin, r->la + r->lb)) {
-            r->off_c = off / 4;
-            r->off_c_pin = pin_off / 4;
-            off += 4 * align_up(r->la + r->lb, 4);
-            pin_off += 4 * align_up(r->la + r->lb, 4);
-        }
-    }
-    g->out_bytes = off - g->err_off - 16;  // staged outputs only
     for (Req* r : g->reqs) {
         if (direct(r->c_pin, r->la + r->lb)) {
             r->off_c = off / 4;
@@ -325,9 +346,11 @@ int launch_group(bw_server* s, Group* g) {
             off += 4 * align_up(r->la + r->lb, 4);
         }
     }
-    const size_t st_stride = small ? 0 : bw_group_state_stride(ntiles);
-    const size_t st_off = align_up(off, 16);
-    off = align_up(st_off + np * st_stride, kAlign);
+    if (!st_staged) {
+        st_off = align_up(off, 16);
+        off = st_off + st_bytes;
+    }
+    off = align_up(off, kAlign);
     const size_t per = res_elems_bytes(path, s->K, log_n);
     const size_t ra_off = off;
     off += np * per;
@@ -363,6 +386,7 @@ int launch_group(bw_server* s, Group* g) {
         if (!small) bw_group_fill_state(d, g->dmem + st_off + q * st_stride, ntiles);
         desc[q] = d;
     }
+    memset(g->pin + in_end, 0, staged_in_end - in_end);  // staged states, error word
     const auto t_launch = Clock::now();
     for (Req* r : g->reqs) r->t_launch = t_launch;
     e = cudaMemcpyAsync(g->dmem, g->pin, staged_in_end, cudaMemcpyHostToDevice, st);
@@ -372,9 +396,7 @@ int launch_group(bw_server* s, Group* g) {
         if (e == cudaSuccess && !r->square && direct(r->b_pin, r->lb))
             e = cudaMemcpyAsync(dw + r->off_b, r->b, r->lb * 4, cudaMemcpyHostToDevice, st);
     }
-    if (e == cudaSuccess) e = cudaMemsetAsync(g->dmem + g->err_off, 0, 16, st);
-    if (e == cudaSuccess && !small)
-        e = cudaMemsetAsync(g->dmem + st_off, 0, np * st_stride, st);
+    if (e == cudaSuccess && !st_staged) e = cudaMemsetAsync(g->dmem + st_off, 0, st_bytes, st);
     if (e != cudaSuccess) return bw_fail(BW_ECUDA, "staging: %s", cudaGetErrorString(e));
     bw_group_launch gl{pl,
                        reinterpret_cast<const BatchProd*>(g->dmem),
