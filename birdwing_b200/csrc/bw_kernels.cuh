@@ -1289,6 +1289,8 @@ __device__ __forceinline__ unsigned __int128 garner_one(const PlanDev<Ar>& P, ty
             const T k2 = a2.red1(a2.shoup(t2, G.inv2, G.inv2q));
             bad |= (uint32_t)(k2 != 0);
         }
+        // (two 30-bit primes: the coefficient fits 64 bits)
+        if constexpr (sizeof(T) == 4) return (uint64_t)(uint32_t)G.p0 * k1 + r0;
         return (unsigned __int128)G.p0 * k1 + r0;
     }
 }
