@@ -3,7 +3,7 @@
 Default workload (configuration 2): one plain 2^28-bit x 2^28-bit product
 (2^23 u32 words each, uniform random with the top bit set, seeded), 32-bit
 coefficients, n = 2^24, two 58-bit primes (64-bit prime path); the library's
-plan for it runs 64-bit coefficients over three primes.  A "step" is
+plan for it runs 64-bit coefficients over three primes of 51 bits.  A "step" is
 one full product.  Metric: products/s (whole job), with the per-stage times,
 the HBM roofline of the dominant kernel and the product-level algorithmic
 byte model (12*K*n*w + in + out) beside it.
@@ -1034,6 +1034,8 @@ def plain_launches_of(info, la, lb):
     column passes (two middle-column passes more in the three-pass
     schedule), and Garner + carry: the words pass and the carry fix when the
     output spans more than one 2048-word tile, else the words pass alone."""
+    if info["path"] == 32 and info["coeff_bits"] == 16 and info["log_n"] <= 11:
+        return 1
     log_r2 = info["log_n"] - info["log_rows"] - info["log_cols"]
     return 3 + (2 if log_r2 > 0 else 0) + (2 if la + lb > 2048 else 1)
 
@@ -1404,16 +1406,23 @@ def bench_plain(args):
             other["int_floor_frac"] = ofloor / other["ms_per_step"]
             line["other_path"] = other
         if world == 1:
-            # integer-pipe floor: the plan's butterflies at the rate the
-            # path's butterflies reach with nothing else running
-            rate, _ = butterfly_rate(path)
+            # arithmetic floor: the plan's butterflies at the rate they reach
+            # with nothing else running -- integer butterflies as measured, or,
+            # in double precision (primes of at most 52 bits on the 64-bit
+            # path), 8 FP64 operations each at 64 per SM-cycle
             bfly = plan_butterflies(info, square)
+            if path == 64 and max(info["primes"]).bit_length() <= 52:
+                import torch
+                rate = (64 / 8 * torch.cuda.get_device_properties(0).multi_processor_count *
+                        1e6 * ((clocks or {}).get("sm_max_mhz") or 1965))
+                how = "8 FP64 operations per butterfly at 64 per SM-cycle, maximum SM clock"
+            else:
+                rate, _ = butterfly_rate(path)
+                how = ("bw_butterfly_rate: the path's own forward and inverse butterflies from "
+                       "registers, best over 2/4/8 CTAs per SM (bench.py --config intpeak)")
             floor_ms = bfly / rate * 1e3
             line["int_floor"] = {"butterflies": bfly, "butterflies_per_s": rate,
-                                 "floor_ms": floor_ms, "frac": floor_ms / ms,
-                                 "how": "bw_butterfly_rate: the path's own forward and inverse "
-                                        "butterflies from registers, best over 2/4/8 CTAs per SM "
-                                        "(bench.py --config intpeak)"}
+                                 "floor_ms": floor_ms, "frac": floor_ms / ms, "how": how}
             line["int_floor_frac"] = floor_ms / ms
         if not args.no_cpu_baseline and world == 1:   # the CPU baseline runs at N = 1 only
             line["cpu_baseline"] = cpu_baseline(cfg)

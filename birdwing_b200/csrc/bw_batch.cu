@@ -57,7 +57,7 @@ struct TuneKey {
 struct TuneVal {
     int small;     // 1: one CTA per product
     int log_cols;  // 4-step split (0 = automatic)
-    int rlog;      // row-pass radix log2, 3 or 4 (0 = the path's default)
+    int rlog;      // row-pass radix log2 asked for, 3 or 4 (kept; without effect)
     float ms;      // measured time of the bucket when tuned (0 = default)
 };
 std::mutex g_tune_mu;
@@ -96,7 +96,7 @@ struct Prod {
 
 struct Bucket {
     int path = 0, K = 2, log_n = 0;
-    int small = 0, log_cols = 0, rlog = 0;
+    int small = 0, log_cols = 0;
     bw_plan plan;
     std::vector<size_t> prods;
     BatchProd* d_desc = nullptr;
@@ -379,7 +379,6 @@ int build_layout(bw_batch* bt) {
             const TuneVal tv = tune_get(p.path, bt->K, p.log_n);
             b.small = tv.small && p.log_n <= small_max_log(p.path);
             b.log_cols = tv.log_cols;
-            b.rlog = tv.rlog;
             index[key] = bt->buckets.size();
             bt->buckets.push_back(std::move(b));
             it = index.find(key);
@@ -503,7 +502,7 @@ int build_layout(bw_batch* bt) {
         if (bt->persistent && bk.small) continue;
         bw_group_launch g{&bk.plan, bk.d_desc, (unsigned)bk.prods.size(), bk.d_res_a,
                           bk.d_res_b, bk.ntiles, bt->d_err, bt->spin_limit,
-                          bt->inject_wait_fault, bk.rlog};
+                          bt->inject_wait_fault};
         rc = bw_enqueue_group(g, bt->side[branch++ % nside]);
     }
     for (int s = 0; s < nside; ++s) {
@@ -765,12 +764,10 @@ extern "C" int bw_batch_autotune(bw_batch* bt, int reps) {
         if (cands.count(key)) continue;
         std::vector<TuneVal> v;
         if (p.log_n <= small_max_log(p.path)) v.push_back(TuneVal{1, 0, 0, 0.f});
-        // 4-step splits from square to long rows (columns of 2^2 at least),
-        // each with row rounds of radix 8 and of radix 16
+        // 4-step splits from square to long rows (columns of 2^2 at least)
         const int max_c = p.path == BW_PATH_P64 ? 13 : 14;
         for (int lc = (p.log_n + 1) / 2 - 1; lc <= std::min(max_c, p.log_n - 2); ++lc)
-            if (lc >= 2 && p.log_n - lc <= 13)
-                for (int rl = 3; rl <= 4; ++rl) v.push_back(TuneVal{0, lc, rl, 0.f});
+            if (lc >= 2 && p.log_n - lc <= 13) v.push_back(TuneVal{0, lc, 0, 0.f});
         cands[key] = v;
     }
     // one sub-batch per key with the batch's products of that key

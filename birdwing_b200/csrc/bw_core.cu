@@ -574,8 +574,6 @@ static unsigned sm_count() {
     return (unsigned)n;
 }
 
-constexpr int kTmaColsMinLogN = 20;
-
 int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int mode) {
     pl->path = path;
     pl->K = K;
@@ -669,23 +667,14 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
         // the residues count there.
         pl->tw_smem_r =
             ((flags & BW_PLAN_TW_SMEM) && ((size_t)2 * w << pl->log_r) <= 32768) ? 1 : 0;
-        // 64-bit coefficients on the 32-bit path: the forward column pass
-        // loops over the six primes with a u64 copy of the coefficients beside
-        // the residue tile, or (BW_PLAN_K1_ONE_PRIME) runs one prime per CTA
-        // and reduces the coefficients straight into its tile; the loop
-        // measured 0.3-4% faster from 2^20- to 2^23-word operands
-        pl->k1_pp = (path == BW_PATH_P32 && pl->w64 && mode == 2 &&
-                     (flags & BW_PLAN_K1_ONE_PRIME))
-                        ? 1
-                        : 0;
         // operands that both fill at most half the rows (the zero pad): only
         // those rows' coefficients are staged, so the u64 copy takes half
-        pl->coef_half = (path == BW_PATH_P32 && pl->w64 && mode == 2 && !pl->k1_pp &&
+        pl->coef_half = (path == BW_PATH_P32 && pl->w64 && mode == 2 &&
                          pl->zt_a && pl->zt_b)
                             ? 1
                             : 0;
         const size_t cbytes = path == BW_PATH_P32
-                                  ? (pl->w64 ? (pl->k1_pp ? 0 : pl->coef_half ? 4 : 8) : 2)
+                                  ? (pl->w64 ? (pl->coef_half ? 4 : 8) : 2)
                               : mode == 2         ? 0
                               : pl->w64           ? 8
                                                   : 4;
@@ -706,33 +695,6 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
         // column stage twiddles: read through L1 by default (measured faster
         // than staging them in shared memory, which costs occupancy); staged on
         // request when they take <= 32 KiB
-        // row pass rounds: radix 8 for single products on the 64-bit path with
-        // rows of at most 2^12 points (its 256-thread kernel takes 64
-        // registers, no spills, and fits three CTAs per SM; measured 3-8%
-        // faster per product from 2^20 to 2^23 words), radix 16 elsewhere
-        // (2^13-point rows take 128 KiB of shared memory: one CTA per SM)
-        const bool r8_default = mode == 2 && path == BW_PATH_P64 && pl->log_c <= 12;
-        // column passes: radix 8 on request (single products on the 64-bit path)
-        pl->rlog_col = ((flags & BW_PLAN_COL_RADIX8) && mode == 2 && path == BW_PATH_P64) ? 3 : 4;
-        pl->rlog_row = (flags & BW_PLAN_RADIX8)    ? 3
-                       : (flags & BW_PLAN_RADIX16) ? 4
-                       : r8_default                ? 3
-                                                   : 4;
-        // inverse column tiles by tensor copies: single products with two
-        // passes, from 2^20 points unless forced either way (a box is at most
-        // 256 columns wide and 16 bytes or more).  Measured at 2^23 words:
-        // the inverse pass 0.246 -> 0.231 ms (64-bit coefficients), 0.378 ->
-        // 0.348 ms (32-bit path); at 2^17 points 0.016 -> 0.018 ms.
-        const bool tma_want = (flags & BW_PLAN_TMA_COLS) ||
-                              (!(flags & BW_PLAN_NO_TMA_COLS) && log_n >= kTmaColsMinLogN);
-        pl->tma_cols = (tma_want && mode == 2 && pl->log_r2 == 0 && !pl->tw_smem_r &&
-                        pl->log_cb <= 8 && (w << pl->log_cb) >= 16)
-                           ? 1
-                           : 0;
-        pl->shfl_rows = ((flags & BW_PLAN_SHFL_ROWS) && mode == 2 && path == BW_PATH_P32 &&
-                         pl->log_c == 12 && pl->rlog_row == 4)
-                            ? 1
-                            : 0;
         // passes with compile-time lengths.  The row pass starts from the
         // column pass's outputs without reducing them; 58-bit primes have room
         // for 20 stages of 3p each before its first multiplication of every
@@ -758,7 +720,6 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
                     pl->v2_cols = 0;
                 } else {
                     pl->log_cb = pl->log_cb1 = cb;
-                    pl->tma_cols = 0;
                 }
             }
         }
@@ -855,44 +816,6 @@ extern "C" int bw_plan_get_info(const bw_plan* pl, bw_plan_info* o) {
 
 // ------------------------------------------------------------------ context
 
-// Tensor map of a context's A residues for the TMA form of the inverse column
-// pass: dims (columns, rows, primes), boxes of CB columns x min(R, 256) rows.
-// cuTensorMapEncodeTiled comes from the driver through the runtime's entry
-// point query, so the library needs no link to libcuda.
-static int encode_residue_map(bw_ctx* c) {
-    using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn encode = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            encode = reinterpret_cast<EncodeFn>(fn);
-    });
-    if (!encode) return bw_fail(BW_ECUDA, "cuTensorMapEncodeTiled is not available");
-    const bw_plan* pl = c->plan;
-    const int w = pl->path == BW_PATH_P64 ? 8 : 4;
-    const cuuint64_t C = (cuuint64_t)1 << pl->log_c, R = (cuuint64_t)1 << pl->log_r;
-    const cuuint64_t dims[3] = {C, R, (cuuint64_t)pl->K};
-    const cuuint64_t strides[2] = {C * w, C * R * w};
-    const cuuint32_t box[3] = {1u << pl->log_cb, (cuuint32_t)std::min<cuuint64_t>(R, 256), 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    if (((cuuint64_t)box[0] * w) % 16 != 0)
-        return bw_fail(BW_EINVAL, "column tile of %u x %d bytes is not a 16-byte multiple", box[0], w);
-    const CUresult r = encode(&c->tmap_res,
-                              w == 8 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32,
-                              3, c->d_res_a, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return bw_fail(BW_ECUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-    return BW_OK;
-}
-
 extern "C" int bw_ctx_create(bw_ctx** out, const bw_plan* pl, void* stream) {
     bw_clear_error();
     if (!out || !pl) return bw_fail(BW_EINVAL, "NULL argument");
@@ -942,10 +865,6 @@ extern "C" int bw_ctx_create(bw_ctx** out, const bw_plan* pl, void* stream) {
     for (auto& ev : c->stage_ev)
         if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
             return fail(bw_fail(BW_ECUDA, "event: %s", cudaGetErrorString(e)));
-    if (pl->tma_cols) {
-        const int rc = encode_residue_map(c);
-        if (rc) return fail(rc);
-    }
     if (pl->order) {
         std::lock_guard<std::mutex> lk(pl->order->mu);
         pl->order->contexts++;

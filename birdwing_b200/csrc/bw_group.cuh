@@ -14,10 +14,7 @@ cudaError_t group_attrs() {
                        (const void*)ks_product<Ar, SPLIT16, 128>,
                        (const void*)ks_product<Ar, SPLIT16, 256>,
                        (const void*)kb_fwd_col<Ar, SPLIT16, 4>, (const void*)kb_inv_col<Ar, 4>,
-                       (const void*)kb_row<Ar, 64, 3>, (const void*)kb_row<Ar, 128, 3>,
-                       (const void*)kb_row<Ar, 256, 3>, (const void*)kb_row<Ar, 512, 3>,
-                       (const void*)kb_row<Ar, 64, 4>, (const void*)kb_row<Ar, 128, 4>,
-                       (const void*)kb_row<Ar, 256, 4>, (const void*)kb_row<Ar, 512, 4>}) {
+                       (const void*)kb_row<Ar, 64, 4>, (const void*)kb_row<Ar, 512, 4>}) {
             const cudaError_t e =
                 cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
             if (e != cudaSuccess) r = e;
@@ -90,10 +87,6 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
     const size_t ntab = 2 * (((size_t)1 << la) + ((size_t)C >> la));
     const size_t smem2 = ntab * sizeof(Tw<T>) + tile_elems(C) * sizeof(T) * 2;
     const dim3 g2(R, pl.K, np);
-    // row rounds: radix 8 on the 64-bit path (at most 256 threads, 64
-    // registers, as its single-product row pass), radix 16 on the 32-bit
-    // path, unless the tune table chose the other radix for the bucket
-    const int rl = g.rlog ? g.rlog : (sizeof(T) == 8 ? 3 : 4);
     if (pl.v2_rows) {
         const cudaError_t e = with_length<kRow2MinLog, kRow2MaxLog>(pl.log_c, [&](auto lc) {
             constexpr int LC = decltype(lc)::value;
@@ -104,20 +97,10 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
             return cudaSuccess;
         });
         if (e != cudaSuccess) return e;
-    } else if (rl == 3) {
-        switch (std::min(sizeof(T) == 8 ? 256 : 512, std::max(64, C >> 3))) {
-            case 512: kb_row<Ar, 512, 3><<<g2, 512, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            case 256: kb_row<Ar, 256, 3><<<g2, 256, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            case 128: kb_row<Ar, 128, 3><<<g2, 128, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            default: kb_row<Ar, 64, 3><<<g2, 64, smem2, s>>>(P, g.d_desc, ra, rb); break;
-        }
+    } else if (C <= 1024) {
+        kb_row<Ar, 64, 4><<<g2, 64, smem2, s>>>(P, g.d_desc, ra, rb);
     } else {
-        switch (std::min(512, std::max(64, C >> 4))) {
-            case 512: kb_row<Ar, 512, 4><<<g2, 512, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            case 256: kb_row<Ar, 256, 4><<<g2, 256, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            case 128: kb_row<Ar, 128, 4><<<g2, 128, smem2, s>>>(P, g.d_desc, ra, rb); break;
-            default: kb_row<Ar, 64, 4><<<g2, 64, smem2, s>>>(P, g.d_desc, ra, rb); break;
-        }
+        kb_row<Ar, 512, 4><<<g2, 512, smem2, s>>>(P, g.d_desc, ra, rb);
     }
     const size_t smem3 = tile_elems((size_t)R * CB) * sizeof(T);
     if (pl.v2_cols) {

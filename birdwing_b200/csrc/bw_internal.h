@@ -28,16 +28,11 @@ struct bw_plan {
     int log_n = 0, log_r = 0, log_c = 0, log_cb = 0, lo = 0;
     int log_cb1 = 0;     // forward column pass tile width (its own shared-memory budget)
     int tw_smem_r = 0;   // column stage twiddles staged in shared memory
-    int rlog_row = 4;    // radix of the row kernel's rounds (2^3 or 2^4)
-    int rlog_col = 4;    // radix of the column kernels' rounds (single products, 64-bit path)
     int log_r2 = 0;      // three-pass schedule: middle column length (0: two passes)
     int log_cb2 = 0, lo_out = 0;
     int small = 0;       // single-pass plan: the whole n-point transform in one CTA
     int w64 = 0;         // 64-bit coefficients (two words each): K = 3 on the 64-bit
                          // path, K = 6 on the 32-bit path
-    int tma_cols = 0;    // inverse column tiles by tensor copies (BW_PLAN_TMA_COLS)
-    int shfl_rows = 0;   // row pass exchange through warp shuffles (BW_PLAN_SHFL_ROWS)
-    int k1_pp = 0;       // 32-bit path, 64-bit coefficients: one prime per forward-pass CTA
     int coef_half = 0;   // ... prime loop: both operands in the low half, half the u64 copy
     int device = 0;
     bool zt_a = false, zt_b = false;
@@ -89,7 +84,6 @@ struct bw_group_launch {
     uint32_t* d_err;    // bit 0: look-back wait timed out; bit 1: check failed
     int spin_limit;
     bool inject_wait_fault = false;  // test hook: every look-back wait runs out
-    int rlog = 0;       // row-pass radix log2 (0: radix 8 on the 64-bit path, 16 on the 32-bit)
 };
 int bw_enqueue_group(const bw_group_launch& g, cudaStream_t s);
 // ... of one arithmetic (bw_group_*.cu).
@@ -148,7 +142,6 @@ struct bw_ctx {
     size_t out_tiles_per = 0;      // carry tiles per K4 launch
     int spin_limit = 1 << 22;
     bool inject_wait_fault = false;
-    CUtensorMap tmap_res;          // residues of A as [prime][row][column] (tma_cols)
 };
 
 // Stage order of one host-pointer product (bw_stage_order): begin(i, s)

@@ -26,45 +26,24 @@ int bw_set_transform_attrs() {
                                                  kMaxDynSmem);
             if (e != cudaSuccess) st = e;
         };
-        if constexpr (!Ar::kF64) {
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false>);
+        if constexpr (sizeof(typename Ar::T) == 8) {
+            if constexpr (!Ar::kF64) {
+                set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, false, true>);
+                set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, false, true>);
+            }
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, true>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, true>);
+        } else {
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, !SPLIT16>);
+            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, !SPLIT16>);
         }
         set((const void*)k_inv_col<Ar, 4, true>);
         set((const void*)k_inv_col<Ar, 4, false>);
         set((const void*)k_row<Ar, 64, 4>);
-        set((const void*)k_row<Ar, 128, 4>);
         set((const void*)k_row<Ar, 256, 4>);
         set((const void*)k_row<Ar, 512, 4>);
-        set((const void*)k_row<Ar, 64, 3>);
-        set((const void*)k_row<Ar, 128, 3>);
-        set((const void*)k_row<Ar, 256, 3>);
-        set((const void*)k_row<Ar, 512, 3>);
-        if constexpr (sizeof(typename Ar::T) == 4) set((const void*)k_row<Ar, 256, 4, true>);
-        if constexpr (sizeof(typename Ar::T) == 4 && !SPLIT16) {
-            // 64-bit coefficients on the 32-bit path
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, false>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, false>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, true>);
-        }
         set((const void*)k_mid_col<Ar, false>);
         set((const void*)k_mid_col<Ar, true>);
-        set((const void*)k_inv_col_tma<Ar, 4>);
-        if constexpr (sizeof(typename Ar::T) == 8) {
-            if constexpr (!Ar::kF64) {
-                set((const void*)k_fwd_col<Ar, SPLIT16, 3, true, false, true>);
-                set((const void*)k_fwd_col<Ar, SPLIT16, 3, false, false, true>);
-                set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, false, true>);
-                set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, false, true>);
-            }
-            set((const void*)k_fwd_col<Ar, SPLIT16, 3, true, true, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 3, false, true, true>);
-            set((const void*)k_inv_col<Ar, 3, true>);
-            set((const void*)k_inv_col<Ar, 3, false>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, true, true, true>);
-            set((const void*)k_fwd_col<Ar, SPLIT16, 4, false, true, true>);
-        }
     });
     if (st != cudaSuccess) return bw_fail(BW_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(st));
     return BW_OK;
@@ -164,28 +143,21 @@ cudaError_t launch_mid2(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T
     });
 }
 
-template <class Ar, int RLOG>
+// The any-length row pass: rows shorter than 2^5 or longer than 2^13 points, or
+// past the 58-bit primes' room.
+template <class Ar>
 void launch_row(const bw_plan* pl, const PlanDev<Ar>& pd, typename Ar::T* ra,
                 const typename Ar::T* rb, int sq, size_t smem, cudaStream_t s) {
-    dim3 g(1u << (pl->log_r + pl->log_r2), pl->K);
-    // one thread per sub-problem of a round, 64..512 threads (radix-8 rounds,
-    // and radix-16 rounds on the 32-bit path: at most 256, each thread taking
-    // several sub-problems, so that the CTA's registers leave room for more
-    // than one CTA per SM; 2^13-point rows on the 32-bit path ran one 512-thread
-    // CTA per SM at 70 registers)
-    const int cap = (RLOG == 3 || sizeof(typename Ar::T) == 4) ? 256 : 512;
-    const int want = std::min(cap, std::max(64, 1 << (pl->log_c - RLOG)));
-    if constexpr (sizeof(typename Ar::T) == 4 && RLOG == 4) {
-        if (pl->shfl_rows && want == 256) {
-            k_row<Ar, 256, 4, true><<<g, 256, smem, s>>>(pd, ra, rb, sq);
-            return;
-        }
-    }
-    switch (want) {
-        case 512: k_row<Ar, 512, RLOG><<<g, 512, smem, s>>>(pd, ra, rb, sq); break;
-        case 256: k_row<Ar, 256, RLOG><<<g, 256, smem, s>>>(pd, ra, rb, sq); break;
-        case 128: k_row<Ar, 128, RLOG><<<g, 128, smem, s>>>(pd, ra, rb, sq); break;
-        default: k_row<Ar, 64, RLOG><<<g, 64, smem, s>>>(pd, ra, rb, sq); break;
+    const dim3 g(1u << (pl->log_r + pl->log_r2), pl->K);
+    // one thread per sub-problem of a round, 64 to 512 threads (at most 256 on
+    // the 32-bit path, so that more than one CTA fits an SM)
+    const int want = 1 << (pl->log_c > 4 ? pl->log_c - 4 : 0);
+    if (want <= 64) {
+        k_row<Ar, 64, 4><<<g, 64, smem, s>>>(pd, ra, rb, sq);
+    } else if (want <= 256 || sizeof(typename Ar::T) == 4) {
+        k_row<Ar, 256, 4><<<g, 256, smem, s>>>(pd, ra, rb, sq);
+    } else {
+        k_row<Ar, 512, 4><<<g, 512, smem, s>>>(pd, ra, rb, sq);
     }
 }
 
@@ -225,18 +197,16 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const size_t tw_bytes = ts ? (size_t)R * sizeof(Tw<T>) : 0;
 
     const int CB1 = 1 << pl->log_cb1;
-    // the 64-bit path stages the coefficients inside the residue tile and
-    // runs one prime per CTA (grid.x = tile * K + prime); so does the 32-bit
-    // path with 64-bit coefficients when asked (BW_PLAN_K1_ONE_PRIME); the
+    // the any-length pass: the 64-bit path stages the coefficients inside the
+    // residue tile and runs one prime per CTA (grid.x = tile * K + prime); the
     // 32-bit path keeps a u16 (16-bit) or u64 (64-bit coefficients) copy
     constexpr bool PP = sizeof(T) == 8;
-    const bool pp32 = W64 && sizeof(T) == 4 && pl->k1_pp;
     // (64-bit coefficients on the 32-bit path: the u64 copy holds the loaded
     // rows only, half the tile when both operands fill at most half of it)
     const size_t coef_rows = (W64 && sizeof(T) == 4 && pl->coef_half) ? (size_t)R / 2 : R;
     const size_t smem1 = tw_bytes + tile_elems((size_t)R * CB1) * sizeof(T) +
-                         coef_rows * CB1 * ((PP || pp32) ? 0 : SPLIT16 ? 2 : W64 ? 8 : 4) +
-                         (W64 && sizeof(T) == 4 && !pp32 ? 16 : 0);
+                         coef_rows * CB1 * (PP ? 0 : SPLIT16 ? 2 : W64 ? 8 : 4) +
+                         (W64 && sizeof(T) == 4 ? 16 : 0);
     // K1 takes coefficient counts, or word counts for 64-bit coefficients
     const size_t in_a = W64 ? pl->la : pl->nca, in_b = W64 ? pl->lb : pl->ncb;
     const int cols_outer = 1 << (pl->log_c + pl->log_r2);
@@ -244,41 +214,12 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const unsigned zt = (pl->zt_a ? 1u : 0u) | (pl->zt_b ? 2u : 0u);
     cudaError_t ke = cudaSuccess;  // a fixed-length launch's status
     auto k1 = [&](int tile0, int ntiles) {
-        {
-            if (pl->v2_cols) {
-                ke = launch_fwd_col2<Ar, W64 ? 64 : SPLIT16 ? 16 : 32>(
-                    pl, pd, a, in_a, b, in_b, ra, rb, zt, tile0, ntiles, square, c->stream);
-                return;
-            }
+        if (pl->v2_cols) {
+            ke = launch_fwd_col2<Ar, W64 ? 64 : SPLIT16 ? 16 : 32>(
+                pl, pd, a, in_a, b, in_b, ra, rb, zt, tile0, ntiles, square, c->stream);
+            return;
         }
-        dim3 g1(ntiles * ((PP || pp32) ? pl->K : 1), 1, square ? 1 : 2);
-        if constexpr (W64 && sizeof(T) == 4) {
-            if (pp32) {
-                if (ts) {
-                    k_fwd_col<Ar, SPLIT16, 4, true, true, true>
-                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
-                                                                tile0);
-                } else {
-                    k_fwd_col<Ar, SPLIT16, 4, false, true, true>
-                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
-                                                                tile0);
-                }
-                return;
-            }
-        }
-        if constexpr (PP) {
-            if (pl->rlog_col == 3) {
-                if (ts) {
-                    k_fwd_col<Ar, SPLIT16, 3, true, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
-                        pd, a, in_a, b, in_b, ra, rb, zt, tile0);
-                } else {
-                    k_fwd_col<Ar, SPLIT16, 3, false, W64, PP>
-                        <<<g1, kColThreads, smem1, c->stream>>>(pd, a, in_a, b, in_b, ra, rb, zt,
-                                                                tile0);
-                }
-                return;
-            }
-        }
+        dim3 g1(ntiles * (PP ? pl->K : 1), 1, square ? 1 : 2);
         if (ts) {
             k_fwd_col<Ar, SPLIT16, 4, true, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
                 pd, a, in_a, b, in_b, ra, rb, zt, tile0);
@@ -318,15 +259,10 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const int CB2 = 1 << pl->log_cb2;
     const size_t smem_mid = (((size_t)1 << pl->log_r2) + CB2) * sizeof(Tw<T>) +
                             tile_elems((size_t)CB2 << pl->log_r2) * sizeof(T);
-    bool mid2 = false;
-    {
-        if (pl->v2_mid) {
-            mid2 = true;
-            BW_CUDA(ke);
-            BW_CUDA((launch_mid2<Ar, false>(pl, pd, ra, rb, square ? 1 : 2, c->stream)));
-        }
-    }
-    if (pl->log_r2 && !mid2) {
+    if (pl->v2_mid) {
+        BW_CUDA(ke);
+        BW_CUDA((launch_mid2<Ar, false>(pl, pd, ra, rb, square ? 1 : 2, c->stream)));
+    } else if (pl->log_r2) {
         dim3 gm(C / CB2, R, pl->K * (square ? 1 : 2));
         k_mid_col<Ar, false><<<gm, kColThreads, smem_mid, c->stream>>>(pd, ra, rb);
     }
@@ -337,58 +273,28 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const size_t smem2 = ntab * sizeof(Tw<T>) + tile_elems(C) * sizeof(T) * (square ? 1 : 2);
     const T* rbs = square ? ra : rb;
     const int sq = square ? 1 : 0;
-    bool row_done = false;
     BW_CUDA(ke);
     if (pl->v2_rows) {
         BW_CUDA(launch_row2<Ar>(pl, pd, ra, rbs, sq, !timing, c->stream));
-        row_done = true;
-    }
-    if (row_done) {
-    } else if (pl->rlog_row == 3) {
-        launch_row<Ar, 3>(pl, pd, ra, rbs, sq, smem2, c->stream);
     } else {
-        launch_row<Ar, 4>(pl, pd, ra, rbs, sq, smem2, c->stream);
+        launch_row<Ar>(pl, pd, ra, rbs, sq, smem2, c->stream);
     }
     if (timing) cudaEventRecord(c->ev[3], c->stream);
 
-    {
-        if (pl->v2_mid) BW_CUDA((launch_mid2<Ar, true>(pl, pd, ra, ra, 1, c->stream)));
-    }
-    if (pl->log_r2 && !mid2) {
+    if (pl->v2_mid) {
+        BW_CUDA((launch_mid2<Ar, true>(pl, pd, ra, ra, 1, c->stream)));
+    } else if (pl->log_r2) {
         dim3 gm(C / CB2, R, pl->K);
         k_mid_col<Ar, true><<<gm, kColThreads, smem_mid, c->stream>>>(pd, ra, ra);
     }
     const size_t smem3 = tw_bytes + tile_elems((size_t)R * CB) * sizeof(T);
     dim3 g3(cols_outer / CB, pl->K);
-    bool inv_done = false;
-    {
-        if (pl->v2_cols) {
-            BW_CUDA(launch_inv_col2<Ar>(pl, pd, ra, c->cst, cols_outer / CB, !timing,
-                                        c->stream));
-            inv_done = true;
-        }
-    }
-    if (pl->tma_cols) {
-        k_inv_col_tma<Ar, 4><<<g3, kColThreads, (size_t)R * CB * sizeof(T) + 128, c->stream>>>(
-            pd, ra, c->cst, c->tmap_res, c->err, c->spin_limit);
-        inv_done = true;
-    }
-    if constexpr (PP) {
-        if (!inv_done && pl->rlog_col == 3) {
-            if (ts) {
-                k_inv_col<Ar, 3, true><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
-            } else {
-                k_inv_col<Ar, 3, false><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
-            }
-            inv_done = true;
-        }
-    }
-    if (!inv_done) {
-        if (ts) {
-            k_inv_col<Ar, 4, true><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
-        } else {
-            k_inv_col<Ar, 4, false><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
-        }
+    if (pl->v2_cols) {
+        BW_CUDA(launch_inv_col2<Ar>(pl, pd, ra, c->cst, cols_outer / CB, !timing, c->stream));
+    } else if (ts) {
+        k_inv_col<Ar, 4, true><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
+    } else {
+        k_inv_col<Ar, 4, false><<<g3, kColThreads, smem3, c->stream>>>(pd, ra, c->cst);
     }
     if (timing) cudaEventRecord(c->ev[4], c->stream);
     BW_CUDA(cudaGetLastError());

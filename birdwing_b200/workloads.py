@@ -144,6 +144,7 @@ OTHER_EXPECT = dict(path=32, coeff_bits=64, num_primes=6)
 
 def algorithm_of(info):
     """One-line description of what a plan runs, from bw_plan_info fields."""
-    prime_bits = 58 if info["path"] == 64 else 30
+    primes = info.get("primes") or [(1 << 58) - 1 if info["path"] == 64 else (1 << 30) - 1]
+    prime_bits = max(p.bit_length() for p in primes)
     return (f"{info['coeff_bits']}-bit coefficients, n=2^{info['log_n']}, "
             f"{info['num_primes']} x {prime_bits}-bit primes ({info['path']}-bit prime path)")

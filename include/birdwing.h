@@ -16,10 +16,10 @@
  *                 transform length is twice the limb count).
  *   BW_PATH_P64 : 32-bit coefficients, 58-bit primes of the form c*2^32+1,
  *                 64-bit modular arithmetic; with 64-bit coefficients
- *                 (BW_PLAN_COEF64) primes of 51 and 52 bits in exact
- *                 double-precision modular arithmetic (58-bit ones when the
- *                 shorter operand has more than 2^28 words) (the reference's LIMB_BITS=64
- *                 "hybrid" and NATIVE_HOST_LIMBS pipelines; a u64 limb array
+ *                 (BW_PLAN_COEF64), and in batches and the server, primes of
+ *                 51 and 52 bits in exact double-precision modular arithmetic
+ *                 (58-bit ones when the shorter operand has more than 2^28
+ *                 words).  (The reference's LIMB_BITS=64 "hybrid" and NATIVE_HOST_LIMBS pipelines; a u64 limb array
  *                 is passed as twice as many u32 words).
  *
  * Everything crossing this boundary is a plain pointer, size or POD struct.
@@ -77,15 +77,20 @@ extern "C" {
 /* Split the transform into rows x 2^x columns for the 4-step schedule
  * (0 = automatic).  x <= 13 (64-bit path) or 14 (32-bit path). */
 #define BW_PLAN_LOG_COLS(x) (((unsigned)(x) & 0x1fu) << 8)
-/* Tuning switches: radix-8 instead of radix-16 rounds in the row pass;
- * stage the column stage twiddles in shared memory (when <= 32 KiB) instead
- * of reading them through L1; use the three-pass schedule (n = R * R2 * C)
- * even where two passes fit (it is used anyway beyond n = 2^26). */
+/* Tuning switches.  The passes run with compile-time lengths and fixed radix
+ * (16) and tile widths wherever the split allows (columns of 2^3 to 2^12 or
+ * 2^13 points, rows of 2^5 to 2^13), and these choose among what is left:
+ * BW_PLAN_TW_SMEM stages the column stage twiddles in shared memory (when <=
+ * 32 KiB), in the any-length column passes; BW_PLAN_THREE_PASS uses the
+ * three-pass schedule (n = R * R2 * C) even where two passes fit (it is used
+ * anyway beyond n = 2^26, with 64-bit coefficients on the 64-bit path from n =
+ * 2^24).  BW_PLAN_RADIX8, _RADIX16, _COL_RADIX8, _WIDE_COLS (but for the
+ * any-length columns' tile), _TMA_COLS, _NO_TMA_COLS, _SHFL_ROWS and
+ * _K1_ONE_PRIME are accepted and change nothing: the forms they chose measured
+ * slower than the fixed-length passes and are gone. */
 #define BW_PLAN_RADIX8      (1u << 16)
 #define BW_PLAN_TW_SMEM     (1u << 17)
 #define BW_PLAN_THREE_PASS  (1u << 18)
-/* Column-pass tiles of up to 128 KiB of residues instead of 64 KiB (twice
- * the columns per CTA: longer contiguous row segments, fewer CTAs per SM). */
 #define BW_PLAN_WIDE_COLS   (1u << 19)
 /* 64-bit coefficients (two words each).  On the 64-bit path: three primes,
  * all three carrying the coefficients (no redundant prime), half the
@@ -97,28 +102,12 @@ extern "C" {
  * path) or 6 (32-bit path).  The reference splits operands into 32-bit
  * coefficients only (src/zero_pad.cu:3-57); the product is the same. */
 #define BW_PLAN_COEF64      (1u << 20)
-/* Radix-16 rounds in the row pass where radix 8 is the default (single
- * products on the 64-bit path with rows of at most 2^12 points). */
+/* (see above) */
 #define BW_PLAN_RADIX16     (1u << 21)
-/* Radix-8 rounds in the column passes (single products on the 64-bit path). */
 #define BW_PLAN_COL_RADIX8  (1u << 22)
-/* Single products, two-pass schedule: the inverse column pass brings its tile
- * into shared memory with tensor-memory-accelerator box copies
- * (cp.async.bulk.tensor, one mbarrier) instead of per-element cp.async, and
- * runs its rounds on the dense tile.  On by default from transforms of 2^20
- * points (measured faster there, slower below); BW_PLAN_TMA_COLS forces it
- * on, BW_PLAN_NO_TMA_COLS off. */
 #define BW_PLAN_TMA_COLS    (1u << 23)
 #define BW_PLAN_NO_TMA_COLS (1u << 24)
-/* Single products on the 32-bit path with 2^12-point rows: the row pass hands
- * one round's outputs to the next through warp shuffles (a 16 x 16 transpose
- * inside each half-warp) instead of shared memory.  A measured alternative,
- * off by default. */
 #define BW_PLAN_SHFL_ROWS   (1u << 25)
-/* 32-bit path with 64-bit coefficients: the forward column pass runs one
- * prime per CTA, reducing the coefficients straight into its residue tile,
- * instead of looping over the six primes in one CTA with a u64 copy of the
- * tile's coefficients beside its residues (the default, measured faster). */
 #define BW_PLAN_K1_ONE_PRIME (1u << 26)
 
 /* ---- flags for bw_multiply ------------------------------------------------ */

@@ -178,3 +178,17 @@ def test_middle_lengths_exact(log_r2, path, K, flags):
             assert (c.multiply(a, b) == gmp_ref.mul(a, b)).all(), (la, lb)
         with bw.Plan(la, la, path, K, flags=flags | L.BW_PLAN_THREE_PASS) as p, bw.Context(p) as c:
             assert (c.square(a) == gmp_ref.mul(a, a)).all(), la
+
+
+@pytest.mark.parametrize("path,K,flags", [f[:3] for f in FORMS])
+def test_any_length_passes_exact(path, K, flags):
+    # the passes for any length, which BW_PLAN_TW_SMEM selects for the columns
+    # (two and three passes), beside the fixed-length rows
+    rng = np.random.default_rng(97)
+    for la, lb in ((3001, 2500), (70001, 65536)):
+        a, b = (rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32) for n in (la, lb))
+        want = gmp_ref.mul(a, b)
+        for fl in (L.BW_PLAN_TW_SMEM, L.BW_PLAN_TW_SMEM | L.BW_PLAN_THREE_PASS,
+                   L.BW_PLAN_TW_SMEM | L.BW_PLAN_WIDE_COLS):
+            with bw.Plan(la, lb, path, K, flags=flags | fl) as p, bw.Context(p) as c:
+                assert (c.multiply(a, b) == want).all(), (la, lb, hex(fl))
