@@ -452,8 +452,8 @@ int bw_check_size(int path, int K, size_t la, size_t lb, int* log_n_out) {
 
 // 64-bit path with 64-bit coefficients and three primes: ceil(l / 2)
 // coefficients per operand; every coefficient of the product is below
-// min(na, nb) 2^128, far under p0 p1 p2 (2^184.9) for any size the
-// transform reaches, and all three primes carry it (none is redundant).
+// min(na, nb) 2^128, under p0 p1 p2 of the set choose_f64 picks for it, and all
+// three primes carry it (none is redundant).
 // On the 32-bit path (six primes, v2(p - 1) >= 23) the transform reaches 2^23
 // points, 2^23-word operands; the six primes' product (2^177) bounds every
 // coefficient there (min(na, nb) 2^128 <= 2^150).
@@ -478,9 +478,9 @@ int bw_check_size_w64(size_t la, size_t lb, int* log_n_out, int path = BW_PATH_P
 // num_primes 0 on the 64-bit path: 64-bit coefficients with three primes
 // (3 primes x n/2 points instead of 2 x n) where they halve the transform
 // and their own transform has at least 2^19 points.  On a B200 they measured
-// faster from there (2^20-word operands: 0.245 vs 0.324 ms; 2^23: 1.93 vs
-// 2.58 ms); below, the three-prime Garner and fixed costs make them slower
-// (2^18 words: 0.124 vs 0.100 ms).  Every product that BW_PATH_AUTO moves off
+// faster from there (2^20-word operands, on integers: 0.245 vs 0.324 ms; 2^23
+// words now 0.76 vs 1.84 ms); below, the three-prime Garner and fixed costs
+// made them slower (2^18 words: 0.124 vs 0.100 ms).  Every product that BW_PATH_AUTO moves off
 // the 32-bit path (more than 2^21 of its points) has at least 2^19 of them.
 constexpr int kW64MinLogN = 19;
 
@@ -528,10 +528,12 @@ static int resolve_plan(int path, int num_primes, size_t la, size_t lb, unsigned
         path = force64 ? BW_PATH_P64
                        : bw_choose_path(K < 2 || K > 3 ? 2 : K, la, lb, num_primes == 0);
         // a single product the 16-bit split leaves: 64-bit coefficients on
-        // the 32-bit path (six primes) while their transform fits (n <= 2^23);
-        // on a B200 they measured faster than the 64-bit path's from 2^20-word
-        // operands (0.206 vs 0.213 ms; 2^21 words 0.347 vs 0.387, 2^22 0.690
-        // vs 0.760, 2^23 1.356 vs 1.514 ms)
+        // the 32-bit path (six primes) while their transform fits (n <= 2^23).
+        // The line was drawn when the 64-bit path's three primes ran on
+        // integers (2^23 words 1.36 vs 1.51 ms); in double precision they are
+        // now the faster ones (three products in flight: 2^20 words 77 vs 88
+        // us, 2^21 168 vs 185, 2^22 351 vs 381, 2^23 750 vs 811), but which
+        // plan AUTO resolves to is part of the interface
         if (!force64 && num_primes == 0 && path == BW_PATH_P64) {
             if (bw_check_size_w64(la, lb, nullptr, BW_PATH_P32) == BW_OK) {
                 path = BW_PATH_P32;
