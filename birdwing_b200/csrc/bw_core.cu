@@ -1017,8 +1017,9 @@ int enqueue_carry(bw_ctx* c, uint32_t* out, bool timing, int pieces = 1) {
                              reinterpret_cast<const T*>(c->d_res_a), out, M, NL, c->rec_s,
                              &c->cst->any, c->err));
         if (c->ntiles > 1)
-            BW_CUDA(launch_after(!timing, k_carry_fix, dim3(1), kFixThreads, 0, c->stream,
-                                 c->rec_s, (uint32_t)c->ntiles, out, M, &c->cst->any));
+            BW_CUDA(launch_after(!timing, k_carry_fix, dim3(fix_ctas(c->ntiles)), kFixThreads, 0,
+                                 c->stream, c->rec_s, (uint32_t)c->ntiles, out, M,
+                                 &c->cst->any));
         c->out_pieces = 1;
         return BW_OK;
     }

@@ -127,7 +127,7 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
         kb_carry_words<Ar, SPLIT16><<<dim3((unsigned)g.ntiles, np), kWordsThreads, 0, s>>>(
             P, g.d_desc, ra, g.d_err);
         if (g.ntiles > 1)
-            kb_carry_fix<<<np, kBatchFixThreads, 0, s>>>(
+            kb_carry_fix<<<dim3(fix_ctas(g.ntiles), np), kFixThreads, 0, s>>>(
                 g.d_desc, ((size_t)1 << pl.log_n) / (SPLIT16 ? 2 : 1));
     }
     return cudaGetLastError();

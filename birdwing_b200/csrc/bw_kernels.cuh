@@ -108,7 +108,7 @@ struct PlanDev {
 // Carry look-back state of one context.
 struct CarryState {
     uint32_t counter;   // dynamic tile ticket (reset by K3 before every K4)
-    uint32_t any;       // some tile's kind is not kill (k_carry_words, cleared by k_carry_fix)
+    uint32_t any;       // some tile's kind is not kill (k_carry_words; reset by K3)
     uint32_t pad[2];
 };
 
@@ -982,7 +982,7 @@ __device__ __forceinline__ void inv_col_body(const PlanDev<Ar>& P, typename Ar::
                                              CarryState* cst, int tile, int kp,
                                              unsigned char* smem_raw) {
     using T = typename Ar::T;
-    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = 0;
+    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = 0;
     const int log_r = P.log_r, log_c = P.log_c + P.log_r2, log_cb = P.log_cb;
     const int R = 1 << log_r;
     const size_t C = (size_t)1 << log_c;
@@ -1610,68 +1610,98 @@ __device__ __forceinline__ void garner_carry_body(
 // 72 -> 92 us at 2^24 words, and no gain in a graph at 2^16.)
 constexpr int kWordsThreads = kCarryThreads + 32;
 
-// One CTA of NT threads: each thread takes a contiguous run of tiles; a run
-// passes on a constant (its last non-propagating tile's carry) or its own
-// carry-in, and a scan over the runs in shared memory gives each run its
-// carry-in.
-constexpr int kFixThreads = 1024;
-template <int NT>
+// The fix runs on up to one CTA per SM, each with a contiguous share of the
+// tiles.  The carry into a share comes from the latest tile before it that does
+// not propagate; inside it, 256 tiles at a time get their carry-ins by ballots,
+// and the tiles whose carry-in is 1 are then taken by warps, 32 words a step.
+// All-ones operands, whose product's low half is one long chain, are the worst
+// case: 2^23 words 0.78 ms against 0.76 for random ones (8.2 with one thread per
+// run of tiles, word by word).  A CTA per 64 tiles, eight to a warp; without
+// chains every CTA returns at once.
+constexpr int kFixThreads = 256;
+inline unsigned fix_ctas(size_t ntiles) {
+    return ntiles < 128 ? 1u : ntiles < 64 * 148 ? (unsigned)(ntiles / 64) : 148u;
+}
+
+// +1 at the first word of tile t, by one warp; ones: the tile propagates (its
+// words are all ones and become zero).
+__device__ __forceinline__ void carry_fix_tile(uint32_t t, bool ones, uint32_t* __restrict__ out,
+                                               size_t M) {
+    const int lane = threadIdx.x & 31;
+    const size_t beg = (size_t)t * kCarryTileWords;
+    const size_t end = min(M, beg + kCarryTileWords);
+    if (ones) {
+        for (size_t i = beg + lane; i < end; i += 32) out[i] = 0u;
+        return;
+    }
+    for (size_t i = beg; i < end; i += 32) {
+        const size_t j = i + lane;
+        const uint32_t v = j < end ? __ldcg(out + j) : 0xffffffffu;
+        const uint32_t stop = __ballot_sync(0xffffffffu, v != 0xffffffffu);
+        const int f = stop ? __ffs((int)stop) - 1 : 32;
+        if (j < end && lane <= f) out[j] = lane == f ? v + 1u : 0u;
+        if (stop) break;
+    }
+}
+
 __device__ __forceinline__ void carry_fix_body(const uint32_t* __restrict__ kinds,
                                                uint32_t ntiles, uint32_t* __restrict__ out,
-                                               size_t M, uint32_t* __restrict__ any) {
+                                               size_t M, const uint32_t* __restrict__ any,
+                                               uint32_t part, uint32_t parts) {
     if (__ldcg(any) == 0u) return;  // every tile kills
-    __shared__ uint32_t s_f[NT];    // 0, 1: constant carry out; 2: passes carry-in
-    const int tid = threadIdx.x;
-    const uint32_t per = (ntiles + NT - 1) / NT;
-    const uint32_t t0 = min(ntiles, (uint32_t)tid * per), t1 = min(ntiles, t0 + per);
-    uint32_t f = 2;
-    for (uint32_t t = t0; t < t1; ++t) {
-        const uint32_t k = __ldcg(kinds + t);
-        if (k == 0u || k == 3u) f = k & 1u;  // kill / generate: a constant
-    }
-    s_f[tid] = f;
-    __syncthreads();
-    if (tid == 0) *any = 0u;  // for the next product (every thread has read it)
-    // inclusive scan of "the latest constant": combine(a, b) = b unless b
-    // passes its carry-in
-    for (int d = 1; d < NT; d <<= 1) {
-        const uint32_t a = tid >= d ? s_f[tid - d] : 2u;
+    constexpr uint32_t NT = kFixThreads, NW = NT / 32;
+    __shared__ uint32_t s_pos, s_n, s_last[NW], s_list[NT];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t share = (ntiles + parts - 1) / parts;
+    const uint32_t r0 = min(ntiles, part * share), r1 = min(ntiles, r0 + share);
+    // the carry into the share (0 into the first tile)
+    uint32_t cin = 0;
+    for (uint32_t e = r0; e > 0; e -= min(e, NT)) {
         __syncthreads();
-        if (s_f[tid] == 2u) s_f[tid] = a;
+        if (tid == 0) s_pos = NT;
         __syncthreads();
-    }
-    uint32_t eps = tid > 0 ? s_f[tid - 1] : 0u;
-    if (eps == 2u) eps = 0u;  // nothing before this run sets it: carry-in 0
-    for (uint32_t t = t0; t < t1; ++t) {
-        const uint32_t k = __ldcg(kinds + t);
-        if (eps) {
-            const size_t beg = (size_t)t * kCarryTileWords;
-            const size_t end = min(M, beg + kCarryTileWords);
-            if (k == 2u) {
-                // a propagating tile's words are all ones: with the carry in
-                // they all become zero (and the carry passes on)
-                for (size_t i = beg; i < end; ++i) out[i] = 0u;
-            } else {
-                for (size_t i = beg; i < end; ++i) {
-                    const uint32_t v = out[i] + 1u;
-                    out[i] = v;
-                    if (v != 0u) break;
-                }
-            }
+        if (tid < e && __ldcg(kinds + (e - 1 - tid)) != 2u) atomicMin(&s_pos, tid);
+        __syncthreads();
+        if (s_pos < NT) {
+            cin = __ldcg(kinds + (e - 1 - s_pos)) & 1u;
+            break;
         }
-        eps = (k >> eps) & 1u;
+    }
+    for (uint32_t c0 = r0; c0 < r1; c0 += NT) {
+        const uint32_t t = c0 + tid;
+        const uint32_t k = t < r1 ? __ldcg(kinds + t) : 2u;
+        // kill and generate pass on a constant, 0 and 1
+        const uint32_t con = __ballot_sync(0xffffffffu, k != 2u);
+        const uint32_t val = __ballot_sync(0xffffffffu, k == 3u);
+        if (lane == 0) s_last[warp] = con ? (val >> (31 - __clz(con))) & 1u : 2u;
+        if (tid == 0) s_n = 0;
+        __syncthreads();
+        uint32_t eps = cin, cout = cin;
+        for (uint32_t w = 0; w < NW; ++w)
+            if (s_last[w] != 2u) {
+                cout = s_last[w];
+                if (w < warp) eps = cout;
+            }
+        const uint32_t below = con & ((1u << lane) - 1u);
+        if (below) eps = (val >> (31 - __clz(below))) & 1u;
+        if (eps && t < r1) s_list[atomicAdd(&s_n, 1u)] = 2u * t + (k == 2u ? 1u : 0u);
+        __syncthreads();
+        for (uint32_t i = warp; i < s_n; i += NW)
+            carry_fix_tile(s_list[i] >> 1, (s_list[i] & 1u) != 0, out, M);
+        cin = cout;
+        __syncthreads();
     }
 }
 
 static __global__ void __launch_bounds__(kFixThreads)
 k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __restrict__ out,
-            size_t M, uint32_t* __restrict__ any) {
+            size_t M, const uint32_t* __restrict__ any) {
     grid_release();
     grid_wait();
-    carry_fix_body<kFixThreads>(kinds, ntiles, out, M, any);
+    carry_fix_body(kinds, ntiles, out, M, any, blockIdx.x, gridDim.x);
 }
 
-// any: set when a tile's kind is not kill (zero between products).
+// any: set when a tile's kind is not kill (zero before).
 // Four CTAs per SM with 64-bit coefficients (56 registers; 2^23 coefficients
 // 78 -> 71 us, double precision, 83 -> 77 six primes), three otherwise (at four
 // the digit sums spill: 2^20 points 47 -> 50 us for the product).
@@ -1782,14 +1812,13 @@ kb_carry_words(const PlanDev<Ar> P, const BatchProd* __restrict__ D,
     carry_words_body<Ar, SPLIT16, false>(P, res_a + d.res_off, d.out, M, NL, d.rec_s, &d.cst->any,
                                          err);
 }
-constexpr int kBatchFixThreads = 64;
-static __global__ void __launch_bounds__(kBatchFixThreads)
+// blockIdx.y = product
+static __global__ void __launch_bounds__(kFixThreads)
 kb_carry_fix(const BatchProd* __restrict__ D, size_t NL) {
-    const BatchProd d = D[blockIdx.x];
+    const BatchProd d = D[blockIdx.y];
     const size_t M = (size_t)d.la + d.lb, words = NL > M ? NL : M;
-    carry_fix_body<kBatchFixThreads>(d.rec_s,
-                                     (uint32_t)((words + kCarryTileWords - 1) / kCarryTileWords),
-                                     d.out, M, &d.cst->any);
+    carry_fix_body(d.rec_s, (uint32_t)((words + kCarryTileWords - 1) / kCarryTileWords), d.out, M,
+                   &d.cst->any, blockIdx.x, gridDim.x);
 }
 
 // Carry words of the last thread of every tile but the last (its 8 words'

@@ -647,7 +647,7 @@ __device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar:
     using Cfg = ColCfg<Ar, LOGR>;
     constexpr int LCB = Cfg::LCB;
     constexpr int RL0 = first_rl(LOGR), NT = Cfg::NT, CB = 1 << LCB;
-    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = 0;
+    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = 0;
     const int log_c = P.log_c + P.log_r2;
     const PrimeDev<Ar>& pr = P.pr[kp];
     const Ar ar = pr.ar;
