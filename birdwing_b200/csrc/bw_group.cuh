@@ -116,10 +116,7 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
     } else {
         kb_inv_col<Ar, 4><<<dim3(C / CB, pl.K, np), kColThreads, smem3, s>>>(P, g.d_desc, ra);
     }
-    // Few tiles (at most the chip holds at once): the look-back form, one launch,
-    // whose waits are short there -- a serving group's cost is its launches on
-    // the host.  Also for the test hook that makes the waits run out.
-    if (g.inject_wait_fault || np * g.ntiles <= 3 * 148) {
+    if (bw_group_lookback(g)) {
         kb_garner_carry<Ar, SPLIT16><<<dim3((unsigned)g.ntiles, np), kCarryThreads, 0, s>>>(
             P, g.d_desc, ra, 1u, g.inject_wait_fault ? 1u + (1u << 27) : 1u, g.d_err,
             g.spin_limit);

@@ -86,6 +86,18 @@ struct bw_group_launch {
     bool inject_wait_fault = false;  // test hook: every look-back wait runs out
 };
 int bw_enqueue_group(const bw_group_launch& g, cudaStream_t s);
+// Carry form of a 4-step group.  Few tiles (at most the chip holds at once): the
+// look-back form, one launch, whose waits are short there -- a serving group's
+// cost is its launches on the host.  Also for the test hook that makes the
+// waits run out.
+inline bool bw_group_lookback(const bw_group_launch& g) {
+    return g.inject_wait_fault || g.np * g.ntiles <= 3 * 148;
+}
+// Kernels bw_enqueue_group launches for a group.
+inline int bw_group_kernels(const bw_group_launch& g) {
+    if (g.plan->small) return 1;
+    return bw_group_lookback(g) || g.ntiles <= 1 ? 4 : 5;
+}
 // ... of one arithmetic (bw_group_*.cu).
 template <class Ar, bool SPLIT16>
 cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s);

@@ -425,7 +425,7 @@ int launch_group(bw_server* s, Group* g) {
     if (e != cudaSuccess) return bw_fail(BW_ECUDA, "launch: %s", cudaGetErrorString(e));
     {
         std::lock_guard<std::mutex> lk(s->mu);
-        s->launches += small ? 1 : ntiles > 1 ? 5 : 4;
+        s->launches += bw_group_kernels(gl);
     }
     return BW_OK;
 }
