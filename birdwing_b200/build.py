@@ -16,7 +16,7 @@ SOURCES = ["bw_core.cu", "bw_tr_p32.cu", "bw_tr_p32w.cu", "bw_tr_p64.cu", "bw_tr
            "bw_group_p32.cu", "bw_group_f64.cu", "bw_one.cu",
            "bw_server.cu", "bw_probe.cu"]
 HEADERS = ["bw_arith.cuh", "bw_kernels.cuh", "bw_ntt.cuh", "bw_host.h", "bw_internal.h", "bw_transform.cuh",
-           "bw_group.cuh"]
+           "bw_group.cuh", "bw_staging.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -34,6 +34,7 @@
 #include "bw_host.h"
 #include "bw_internal.h"
 #include "bw_kernels.cuh"
+#include "bw_staging.h"
 
 using namespace bw;
 
@@ -105,79 +106,6 @@ struct Bucket {
     unsigned char* d_state = nullptr;
     size_t ntiles = 0;
 };
-
-// Host staging copies of a batch (operands into pinned memory, results out of
-// it) run on a few threads, in chunks that overlap the DMA.  One set of threads
-// per direction works through the chunks: they were started anew for each of
-// four chunks, at most eight of them, and the upload of 137 MB took 5.6-7.3 ms
-// where its DMA takes 2.6.
-constexpr size_t kStageChunks = 8;
-constexpr size_t kStageThreads = 16;
-
-// A helper thread's part of every chunk: part t of T, by words (off(i): word
-// offset of product i, off(count) the end).
-template <class Off>
-size_t part_begin(size_t lo, size_t hi, size_t t, size_t T, Off off) {
-    const size_t w = off(lo) + (off(hi) - off(lo)) * t / T;
-    while (lo < hi) {
-        const size_t mid = (lo + hi) / 2;
-        if (off(mid) < w) {
-            lo = mid + 1;
-        } else {
-            hi = mid;
-        }
-    }
-    return lo;
-}
-
-// copy(i) for every product, chunk by chunk (chunk c: products [chunk(c),
-// chunk(c + 1))), on T threads.  before(c) runs on the caller's thread before
-// chunk c may be copied, after(c) once it has been; a non-zero result of either
-// ends the walk and is returned.  Threads that cannot be started are done
-// without.
-template <class Chunk, class Off, class Copy, class Before, class After>
-int staged_copy(size_t bytes, Chunk chunk, Off off, Copy copy, Before before, After after) {
-    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t T = std::min<size_t>({kStageThreads, hw, std::max<size_t>(1, bytes >> 21)});
-    std::atomic<size_t> ready{0}, parts[kStageChunks];
-    for (auto& p : parts) p.store(0);
-    std::atomic<bool> stop{false};
-    auto part = [&](size_t c, size_t t) {
-        const size_t lo = chunk(c), hi = chunk(c + 1);
-        const size_t end = part_begin(lo, hi, t + 1, T, off);
-        for (size_t i = part_begin(lo, hi, t, T, off); i < (t + 1 == T ? hi : end); ++i) copy(i);
-        parts[c].fetch_add(1, std::memory_order_release);
-    };
-    std::vector<std::thread> th;
-    size_t started = 1;  // the caller's thread takes part 0 and those not started
-    try {
-        th.reserve(T);
-        for (; started < T; ++started)
-            th.emplace_back([&, t = started] {
-                for (size_t c = 0; c < kStageChunks; ++c) {
-                    while (ready.load(std::memory_order_acquire) <= c) {
-                        if (stop.load(std::memory_order_relaxed)) return;
-                        std::this_thread::yield();
-                    }
-                    part(c, t);
-                }
-            });
-    } catch (...) {
-    }
-    int rc = 0;
-    for (size_t c = 0; c < kStageChunks && !rc; ++c) {
-        rc = before(c);
-        if (rc) break;
-        ready.store(c + 1, std::memory_order_release);
-        part(c, 0);
-        for (size_t t = started; t < T; ++t) part(c, t);
-        while (parts[c].load(std::memory_order_acquire) < T) std::this_thread::yield();
-        rc = after(c);
-    }
-    stop.store(true);
-    for (auto& x : th) x.join();
-    return rc;
-}
 
 void free_bucket(Bucket& b) {
     cudaFree(b.d_desc);
