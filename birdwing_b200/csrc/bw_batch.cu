@@ -573,10 +573,12 @@ extern "C" int bw_batch_run(bw_batch* bt, unsigned what, bw_timing* tm) {
         what |= BW_BATCH_UPLOAD;  // the staging arenas were (re)built
     }
     const size_t np = bt->prods.size();
-    auto chunk = [&](size_t c) { return c * np / kStageChunks; };
+    // first product of chunk c of n
+    auto split = [np](size_t n) { return [=](size_t c) { return c * np / n; }; };
     cudaEventRecord(bt->ev[0], bt->stream);
     if (what & BW_BATCH_UPLOAD) {
         // chunk c's DMA runs while the host stages chunk c + 1
+        const auto chunk = split(stage_chunks(bt->in_words * 4));
         const int rc = staged_copy(
             bt->in_words * 4, chunk,
             [&](size_t i) { return i < np ? bt->prods[i].in_a : bt->in_words; },
@@ -600,8 +602,10 @@ extern "C" int bw_batch_run(bw_batch* bt, unsigned what, bw_timing* tm) {
     cudaEventRecord(bt->ev[1], bt->stream);
     if (what & BW_BATCH_COMPUTE) BW_TRY(cudaGraphLaunch(bt->exec, bt->stream));
     cudaEventRecord(bt->ev[2], bt->stream);
+    const size_t down = stage_chunks(bt->out_words * 4);
+    const auto chunk = split(down);
     if (what & BW_BATCH_DOWNLOAD) {
-        for (size_t c = 0; c < kStageChunks; ++c) {
+        for (size_t c = 0; c < down; ++c) {
             const size_t lo = chunk(c), hi = chunk(c + 1);
             if (lo == hi) continue;
             const size_t w_lo = bt->prods[lo].out;

@@ -10,8 +10,15 @@
 
 namespace bw {
 
-constexpr size_t kStageChunks = 8;
+constexpr size_t kStageChunks = 8;  // most chunks
 constexpr size_t kStageThreads = 16;
+
+// Chunks of a copy: one per 256 KiB.  Each costs a copy, an event and a wait
+// (16 products of 64 words: 97 us with eight chunks whatever the size, 50 in
+// one; 16 of 1000 words 113, 68).
+inline size_t stage_chunks(size_t bytes) {
+    return std::min(kStageChunks, std::max<size_t>(1, bytes >> 18));
+}
 
 // A thread's part of every chunk: part t of T, by words (off(i): word offset of
 // product i, off(count) the end).
@@ -29,8 +36,8 @@ size_t part_begin(size_t lo, size_t hi, size_t t, size_t T, Off off) {
     return lo;
 }
 
-// copy(i) for every product, chunk by chunk (chunk c: products [chunk(c),
-// chunk(c + 1))), on T threads: one set of them works through the chunks
+// copy(i) for every product, chunk by chunk (chunk c of stage_chunks(bytes):
+// products [chunk(c), chunk(c + 1))), on T threads: one set of them works through the chunks
 // (started anew for each of four chunks, at most eight, the upload of 137 MB
 // took 5.6-7.3 ms where its DMA takes 2.6).  before(c) runs on the caller's
 // thread before chunk c may be copied, after(c) once it has been; a non-zero
@@ -49,6 +56,7 @@ template <class Chunk, class Off, class Copy, class Before, class After>
 int staged_copy(size_t bytes, Chunk chunk, Off off, Copy copy, Before before, After after) {
     using Clock = std::chrono::steady_clock;
     const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t chunks = stage_chunks(bytes);
     const size_t T = std::min<size_t>({kStageThreads, hw, std::max<size_t>(1, bytes >> 21)});
     std::atomic<size_t> ready{0}, parts[kStageChunks];
     for (auto& p : parts) p.store(0);
@@ -65,7 +73,7 @@ int staged_copy(size_t bytes, Chunk chunk, Off off, Copy copy, Before before, Af
         th.reserve(T);
         for (; started < T; ++started)
             th.emplace_back([&, t = started] {
-                for (size_t c = 0; c < kStageChunks; ++c) {
+                for (size_t c = 0; c < chunks; ++c) {
                     const auto t0 = Clock::now();
                     while (ready.load(std::memory_order_acquire) <= c) {
                         if (stop.load(std::memory_order_relaxed)) return;
@@ -83,7 +91,7 @@ int staged_copy(size_t bytes, Chunk chunk, Off off, Copy copy, Before before, Af
     } catch (...) {
     }
     int rc = 0;
-    for (size_t c = 0; c < kStageChunks && !rc; ++c) {
+    for (size_t c = 0; c < chunks && !rc; ++c) {
         rc = before(c);
         if (rc) break;
         ready.store(c + 1, std::memory_order_release);

@@ -1,6 +1,6 @@
 """The batch's host staging copies (csrc/bw_staging.h), compiled for the host:
-every product copied exactly once whatever the sizes, errors end the walk, and
-threads that wait sleep -- a caller that waits 0.4 s for its DMA costs next to
+every product copied exactly once whatever the sizes, in chunks that follow the
+bytes, errors end the walk, and threads that wait sleep -- a caller that waits 0.4 s for its DMA costs next to
 no processor time."""
 import os
 import subprocess
@@ -35,7 +35,7 @@ int main(int, char** v) {
     std::vector<std::atomic<int>> seen(np);
     for (auto& x : seen) x = 0;
     const double c0 = cpu();
-    auto chunk = [&](size_t c) { return c * np / bw::kStageChunks; };
+    auto chunk = [&](size_t c) { return c * np / bw::stage_chunks(bytes); };
     auto offs = [&](size_t i) { return off[i]; };
     auto copy = [&](size_t i) { ++seen[i]; };
     int befores = 0, afters = 0;
@@ -82,6 +82,13 @@ def staging(tmp_path_factory):
 def test_every_product_once(staging, products, nbytes):
     rc, once, befores, afters, early, late, _ = staging(products, nbytes, 0, -1, 0)
     assert (rc, once, early, late) == (0, products, 0, 0) and befores == afters
+
+
+@pytest.mark.parametrize("nbytes,chunks", [(0, 1), (8192, 1), ((1 << 18) - 4, 1), (3 << 18, 3),
+                                           (1 << 21, 8), (1 << 30, 8)])
+def test_chunks_follow_bytes(staging, nbytes, chunks):
+    # a chunk costs a copy, an event and a wait: small batches take one
+    assert staging(64, nbytes, 0, -1, 0)[2:4] == [chunks, chunks]
 
 
 @pytest.mark.parametrize("mode,rc", [(0, 7), (1, 9)])
