@@ -24,12 +24,30 @@ cudaError_t group_attrs() {
     return st;
 }
 
+// A kernel is loaded at its first use, or here (once) by a query that needs it
+// on the device.
+template <auto KERN>
+cudaError_t load_kernel() {
+    static const cudaError_t st = [] {
+        cudaFuncAttributes at;
+        return cudaFuncGetAttributes(&at, (const void*)KERN);
+    }();
+    return st;
+}
+template <auto KERN>
+cudaError_t group_kernel(bool load) {
+    const cudaError_t e = allow_smem<KERN>();
+    return e == cudaSuccess && load ? load_kernel<KERN>() : e;
+}
+
+// np = 0: the kernels of the plan's groups are loaded and nothing is launched.
 template <class Ar, bool SPLIT16>
 cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
     using T = typename Ar::T;
     const bw_plan& pl = *g.plan;
     const PlanDev<Ar>& P = plan_dev<Ar>(&pl);
     const unsigned np = g.np;
+    const bool load = np == 0;
     T* ra = static_cast<T*>(g.res_a);
     T* rb = static_cast<T*>(g.res_b);
     constexpr int CW = SPLIT16 ? 16 : 32;
@@ -40,15 +58,15 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
             // one round of both operands of one prime at a time, at most 256
             // threads
             constexpr int TH = 2 * Cfg::G < 32 ? 32 : 2 * Cfg::G > 256 ? 256 : 2 * Cfg::G;
-            const cudaError_t e = allow_smem<&kb_one<Ar, LN, CW, TH>>();
-            if (e != cudaSuccess) return e;
+            const cudaError_t e = group_kernel<&kb_one<Ar, LN, CW, TH>>(load);
+            if (e != cudaSuccess || load) return e;
             kb_one<Ar, LN, CW, TH><<<np, TH, Cfg::smem(pl.K, 1), s>>>(P, g.d_desc, g.d_err);
             return cudaGetLastError();
         });
     }
     if (pl.small) {
         const cudaError_t ea = group_attrs<Ar, SPLIT16>();
-        if (ea != cudaSuccess) return ea;
+        if (ea != cudaSuccess || load) return ea;
         const int n = 1 << pl.log_n;
         const size_t smem = 2 * tile_elems(n) * sizeof(T);
         const int want = std::min(256, std::max(64, n >> 4));
@@ -72,14 +90,14 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
         const cudaError_t e = with_columns<Ar>(pl.log_r, [&](auto lr) {
             constexpr int LR = decltype(lr)::value;
             using Cfg = ColCfg<Ar, LR>;
-            const cudaError_t e1 = allow_smem<&kb_fwd_col2<Ar, LR, CW>>();
-            if (e1 != cudaSuccess) return e1;
+            const cudaError_t e1 = group_kernel<&kb_fwd_col2<Ar, LR, CW>>(load);
+            if (e1 != cudaSuccess || load) return e1;
             kb_fwd_col2<Ar, LR, CW><<<dim3(C / CB1 * pl.K, 1, 2 * np), Cfg::NT, Cfg::smem, s>>>(
                 P, g.d_desc, ra, rb);
             return cudaSuccess;
         });
         if (e != cudaSuccess) return e;
-    } else {
+    } else if (!load) {
         kb_fwd_col<Ar, SPLIT16, 4><<<dim3(C / CB1, 1, 2 * np), kColThreads, smem1, s>>>(
             P, g.d_desc, ra, rb);
     }
@@ -91,15 +109,15 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
         const cudaError_t e = with_length<kRow2MinLog, kRow2MaxLog>(pl.log_c, [&](auto lc) {
             constexpr int LC = decltype(lc)::value;
             using Cfg = RowCfg<Ar, LC>;
-            const cudaError_t e1 = allow_smem<&kb_row2<Ar, LC>>();
-            if (e1 != cudaSuccess) return e1;
+            const cudaError_t e1 = group_kernel<&kb_row2<Ar, LC>>(load);
+            if (e1 != cudaSuccess || load) return e1;
             kb_row2<Ar, LC><<<g2, Cfg::NT, Cfg::smem(false), s>>>(P, g.d_desc, ra, rb);
             return cudaSuccess;
         });
         if (e != cudaSuccess) return e;
-    } else if (C <= 1024) {
+    } else if (!load && C <= 1024) {
         kb_row<Ar, 64, 4><<<g2, 64, smem2, s>>>(P, g.d_desc, ra, rb);
-    } else {
+    } else if (!load) {
         kb_row<Ar, 512, 4><<<g2, 512, smem2, s>>>(P, g.d_desc, ra, rb);
     }
     const size_t smem3 = tile_elems((size_t)R * CB) * sizeof(T);
@@ -107,14 +125,19 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
         const cudaError_t e = with_columns<Ar>(pl.log_r, [&](auto lr) {
             constexpr int LR = decltype(lr)::value;
             using Cfg = ColCfg<Ar, LR>;
-            const cudaError_t e1 = allow_smem<&kb_inv_col2<Ar, LR>>();
-            if (e1 != cudaSuccess) return e1;
+            const cudaError_t e1 = group_kernel<&kb_inv_col2<Ar, LR>>(load);
+            if (e1 != cudaSuccess || load) return e1;
             kb_inv_col2<Ar, LR><<<dim3(C / CB, pl.K, np), Cfg::NT, Cfg::smem, s>>>(P, g.d_desc, ra);
             return cudaSuccess;
         });
         if (e != cudaSuccess) return e;
-    } else {
+    } else if (!load) {
         kb_inv_col<Ar, 4><<<dim3(C / CB, pl.K, np), kColThreads, smem3, s>>>(P, g.d_desc, ra);
+    }
+    if (load) {
+        cudaError_t e = load_kernel<&kb_garner_carry<Ar, SPLIT16>>();
+        if (e == cudaSuccess) e = load_kernel<&kb_carry_words<Ar, SPLIT16>>();
+        return e == cudaSuccess ? load_kernel<&kb_carry_fix>() : e;
     }
     if (bw_group_lookback(g)) {
         kb_garner_carry<Ar, SPLIT16><<<dim3((unsigned)g.ntiles, np), kCarryThreads, 0, s>>>(

@@ -85,6 +85,7 @@ struct bw_group_launch {
     int spin_limit;
     bool inject_wait_fault = false;  // test hook: every look-back wait runs out
 };
+// np 0: nothing is launched, the kernels that the plan's groups run are loaded.
 int bw_enqueue_group(const bw_group_launch& g, cudaStream_t s);
 // Carry form of a 4-step group.  Few tiles (at most the chip holds at once): the
 // look-back form, one launch, whose waits are short there -- a serving group's

@@ -700,7 +700,13 @@ extern "C" int bw_server_prewarm(bw_server* s, int path, int max_log_n) {
         int top = std::min(max_log_n, std::min(kMaxGroupLogN, bw_path_max_log_n(pth, s->K)));
         for (int ln = 4; ln <= top; ++ln) {
             bw_plan* pl = nullptr;
-            const int rc = get_plan(s, pth, ln, &pl);
+            int rc = get_plan(s, pth, ln, &pl);
+            if (rc) return rc;
+            // the passes are kernels of their own per length: loaded here, not
+            // in the first request of each length
+            bw_group_launch load{};
+            load.plan = pl;
+            rc = bw_enqueue_group(load, nullptr);
             if (rc) return rc;
         }
     }

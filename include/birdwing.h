@@ -444,7 +444,8 @@ typedef struct bw_server_stats {
 int bw_server_create(bw_server** out, const bw_server_config* cfg);
 /* Waiting requests fail with BW_EBUSY; admitted ones finish first. */
 int bw_server_destroy(bw_server* server);
-/* Build the resident tables for every transform length up to 2^max_log_n. */
+/* Build the resident tables and load the kernels for every transform length up
+ * to 2^max_log_n. */
 int bw_server_prewarm(bw_server* server, int path, int max_log_n);
 /* Queue c[0 .. la+lb) = a * b.  a, b and c must stay valid until the
  * request finishes.  a == b with la == lb squares.  BW_EREJECT when the
