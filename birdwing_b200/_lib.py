@@ -137,6 +137,7 @@ SIGNATURES = {
     "bw_ctx_set_wait_limit": (_I, [_P, _I]),
     "bw_ctx_set_copy_chunks": (_I, [_P, _I]),
     "bw_ctx_inject_wait_fault": (_I, [_P, _I]),
+    "bw_ctx_inject_residue_fault": (_I, [_P, _I, _SZ]),
     "bw_multiply_host_once": (_I, [_P, _SZ, _P, _SZ, _P, _SZ, _I,
                                    ctypes.POINTER(ctypes.c_float)]),
     "bw_host_once_cache_limit": (_I, [_SZ]),

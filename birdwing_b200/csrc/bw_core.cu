@@ -790,12 +790,14 @@ static size_t coef_words(const bw_plan* pl) {
     return pl->w64 ? 2 * n : pl->path == BW_PATH_P32 ? n / 2 : n;
 }
 
+constexpr size_t kSumBytes = 3 * kSumSlots * sizeof(Sum);
+
 static size_t ctx_bytes(const bw_plan* pl) {
     const size_t n = (size_t)1 << pl->log_n;
     const int w = pl->path == BW_PATH_P64 ? 8 : 4;
     const size_t nl = std::max(coef_words(pl), pl->la + pl->lb);
     const size_t ntiles = (nl + kCarryTileWords - 1) / kCarryTileWords;
-    return 2 * (size_t)pl->K * n * w + (pl->la + pl->lb) * 4 * 2 + 64 + ntiles * 20;
+    return 2 * (size_t)pl->K * n * w + (pl->la + pl->lb) * 4 * 2 + 64 + kSumBytes + ntiles * 20;
 }
 
 extern "C" int bw_plan_get_info(const bw_plan* pl, bw_plan_info* o) {
@@ -850,15 +852,18 @@ extern "C" int bw_ctx_create(bw_ctx** out, const bw_plan* pl, void* stream) {
     // power of two)
     const size_t words = std::max(coef_words(pl), pl->la + pl->lb);
     c->ntiles = (words + kCarryTileWords - 1) / kCarryTileWords;
-    c->state_bytes = 32 + c->ntiles * 16 + c->ntiles * 4;
+    // carry state, error word, word sums, records
+    constexpr size_t rec = 32 + kSumBytes;
+    c->state_bytes = rec + c->ntiles * 16 + c->ntiles * 4;
     if ((e = cudaMalloc(&c->d_state, c->state_bytes)) != cudaSuccess)
         return fail(bw_fail(BW_ENOMEM, "carry state: %s", cudaGetErrorString(e)));
     if ((e = cudaMemset(c->d_state, 0, c->state_bytes)) != cudaSuccess)
         return fail(bw_fail(BW_ECUDA, "memset: %s", cudaGetErrorString(e)));
     c->cst = reinterpret_cast<CarryState*>(c->d_state);
     c->err = reinterpret_cast<uint32_t*>(c->d_state + 16);
-    c->rec_x = reinterpret_cast<uint4*>(c->d_state + 32);
-    c->rec_s = reinterpret_cast<uint32_t*>(c->d_state + 32 + c->ntiles * 16);
+    c->sums = reinterpret_cast<Sum*>(c->d_state + 32);
+    c->rec_x = reinterpret_cast<uint4*>(c->d_state + rec);
+    c->rec_s = reinterpret_cast<uint32_t*>(c->d_state + rec + c->ntiles * 16);
     if ((e = cudaMallocHost(&c->h_err, 16)) != cudaSuccess)
         return fail(bw_fail(BW_ENOMEM, "pinned: %s", cudaGetErrorString(e)));
     for (auto& ev : c->ev)
@@ -935,7 +940,7 @@ static int read_device_errors(bw_ctx* c) {
         BW_CUDA(cudaStreamSynchronize(c->stream));
         if (e & 1u)
             return bw_fail(BW_ETIMEOUT, "carry look-back wait exceeded its bound (err=0x%x)", e);
-        return bw_fail(BW_ECHECK, "redundant-prime reconstruction check failed (err=0x%x)", e);
+        return bw_fail(BW_ECHECK, "the product's consistency check failed (err=0x%x)", e);
     }
     return BW_OK;
 }
@@ -951,6 +956,15 @@ extern "C" int bw_ctx_inject_wait_fault(bw_ctx* c, int enable) {
     bw_clear_error();
     if (!c) return bw_fail(BW_EINVAL, "NULL ctx");
     c->inject_wait_fault = enable != 0;
+    return BW_OK;
+}
+
+extern "C" int bw_ctx_inject_residue_fault(bw_ctx* c, int enable, size_t at) {
+    bw_clear_error();
+    if (!c) return bw_fail(BW_EINVAL, "NULL ctx");
+    if (at >> c->plan->log_n) return bw_fail(BW_EINVAL, "residue %zu beyond the transform", at);
+    c->inject_residue_fault = enable != 0;
+    c->fault_at = at;
     return BW_OK;
 }
 
@@ -1000,7 +1014,7 @@ int copy_chunks_for(const bw_ctx* c, bool ordered) {
 }
 
 template <class Ar, bool SPLIT16, bool W64 = false>
-int enqueue_carry(bw_ctx* c, uint32_t* out, bool timing, int pieces = 1) {
+int enqueue_carry(bw_ctx* c, uint32_t* out, bool square, bool timing, int pieces = 1) {
     using T = typename Ar::T;
     const bw_plan* pl = c->plan;
     const PlanDev<Ar>& pd = plan_dev<Ar>(pl);
@@ -1015,17 +1029,17 @@ int enqueue_carry(bw_ctx* c, uint32_t* out, bool timing, int pieces = 1) {
         BW_CUDA(launch_after(!timing, k_carry_words<Ar, SPLIT16, W64>,
                              dim3((unsigned)c->ntiles), kWordsThreads, 0, c->stream, pd,
                              reinterpret_cast<const T*>(c->d_res_a), out, M, NL, c->rec_s,
-                             &c->cst->any, c->err));
-        if (c->ntiles > 1)
-            BW_CUDA(launch_after(!timing, k_carry_fix, dim3(fix_ctas(c->ntiles)), kFixThreads, 0,
-                                 c->stream, c->rec_s, (uint32_t)c->ntiles, out, M,
-                                 &c->cst->any));
+                             &c->cst->any, c->err, c->sums + 2 * kSumSlots));
+        if (W64 || c->ntiles > 1)
+            BW_CUDA(launch_after(!timing, k_carry_fix<W64>, dim3(fix_ctas(c->ntiles)), kFixThreads,
+                                 0, c->stream, c->rec_s, (uint32_t)c->ntiles, out, M, c->cst,
+                                 c->sums, square ? 1 : 0, c->err));
         c->out_pieces = 1;
         return BW_OK;
     }
     if (++c->epoch >= (1u << 28)) {
         c->epoch = 2;
-        BW_CUDA(cudaMemsetAsync(c->d_state + 32, 0, c->state_bytes - 32, c->stream));
+        BW_CUDA(cudaMemsetAsync(c->rec_x, 0, c->ntiles * 20, c->stream));
     }
     const uint32_t epoch = c->epoch;
     if (c->ntiles > 1) {
@@ -1045,44 +1059,48 @@ int enqueue_carry(bw_ctx* c, uint32_t* out, bool timing, int pieces = 1) {
         k_garner_carry<Ar, SPLIT16, W64><<<nb, kCarryThreads, 0, c->stream>>>(
             pd, reinterpret_cast<const T*>(c->d_res_a), out, M, NL, c->cst, c->rec_x, c->rec_s,
             epoch, c->inject_wait_fault ? epoch + (1u << 27) : epoch, c->err,
-            c->spin_limit);
+            c->spin_limit, c->sums + 2 * kSumSlots);
         if (pieces > 1) BW_CUDA(cudaEventRecord(c->out_ev[c->out_pieces], c->stream));
         c->out_pieces++;
     }
+    if (W64) k_check_sums<<<1, 32, 0, c->stream>>>(c->sums, square ? 1 : 0, c->err);
     BW_CUDA(cudaGetLastError());
     return BW_OK;
+}
+
+// K1..K4 of one product in its plan's arithmetic.
+template <class Ar, bool SPLIT16, bool W64>
+int enqueue_stages(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_t* out, bool square,
+                   bool timing, const HostIO* io) {
+    int rc = bw_enqueue_transform<Ar, SPLIT16, W64>(c, a, b, square, timing, io);
+    if (!rc && c->inject_residue_fault) {
+        using T = typename Ar::T;
+        T* r = reinterpret_cast<T*>(c->d_res_a);
+        BW_CUDA(cudaMemcpyAsync(r + c->fault_at, r + (c->fault_at ^ 1), sizeof(T),
+                                cudaMemcpyDeviceToDevice, c->stream));
+    }
+    if (!rc) rc = enqueue_carry<Ar, SPLIT16, W64>(c, out, square, timing, io ? io->chunks : 1);
+    // a product that was not enqueued to its end leaves no sums behind
+    if (rc && W64) cudaMemsetAsync(c->sums, 0, kSumBytes, c->stream);
+    return rc;
 }
 
 int enqueue_product(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_t* out,
                     bool square, bool timing, const HostIO* io = nullptr) {
     const bw_plan* pl = c->plan;
     const int pieces = io ? io->chunks : 1;
-    int rc;
-    if (pl->one && !timing && pieces == 1 && !c->inject_wait_fault) {
+    if (pl->one && !timing && pieces == 1 && !c->inject_wait_fault && !c->inject_residue_fault) {
         BW_CUDA(bw_launch_one(pl, a, square ? a : b, out, square, c->err, c->stream));
         c->out_pieces = 1;
         return BW_OK;
     }
-    if (pl->w64 && pl->path == BW_PATH_P32) {
-        rc = bw_enqueue_transform<Ar32, false, true>(c, a, b, square, timing, io);
-        if (!rc) rc = enqueue_carry<Ar32, false, true>(c, out, timing, pieces);
-    } else if (pl->w64) {
-        rc = pl->f64 == 1 ? bw_enqueue_transform<ArD<0>, false, true>(c, a, b, square, timing, io)
-             : pl->f64 == 2
-                 ? bw_enqueue_transform<ArD<1>, false, true>(c, a, b, square, timing, io)
-                 : bw_enqueue_transform<Ar64, false, true>(c, a, b, square, timing, io);
-        if (!rc)
-            rc = pl->f64 == 1   ? enqueue_carry<ArD<0>, false, true>(c, out, timing, pieces)
-                 : pl->f64 == 2 ? enqueue_carry<ArD<1>, false, true>(c, out, timing, pieces)
-                                : enqueue_carry<Ar64, false, true>(c, out, timing, pieces);
-    } else if (pl->path == BW_PATH_P64) {
-        rc = bw_enqueue_transform<Ar64, false>(c, a, b, square, timing, io);
-        if (!rc) rc = enqueue_carry<Ar64, false>(c, out, timing, pieces);
-    } else {
-        rc = bw_enqueue_transform<Ar32, true>(c, a, b, square, timing, io);
-        if (!rc) rc = enqueue_carry<Ar32, true>(c, out, timing, pieces);
-    }
-    return rc;
+    auto go = pl->w64 && pl->path == BW_PATH_P32 ? enqueue_stages<Ar32, false, true>
+              : pl->f64 == 1                     ? enqueue_stages<ArD<0>, false, true>
+              : pl->f64 == 2                     ? enqueue_stages<ArD<1>, false, true>
+              : pl->w64                          ? enqueue_stages<Ar64, false, true>
+              : pl->path == BW_PATH_P64          ? enqueue_stages<Ar64, false, false>
+                                                 : enqueue_stages<Ar32, true, false>;
+    return go(c, a, b, out, square, timing, io);
 }
 
 float ev_ms(cudaEvent_t a, cudaEvent_t b) {
@@ -1154,7 +1172,7 @@ static int do_multiply(bw_ctx* c, const uint32_t* a, size_t la, const uint32_t* 
     if (timing) cudaEventRecord(c->ev[0], c->stream);
     int rc;
     if (flags & BW_PTR_DEVICE) {
-        if (!timing && !c->inject_wait_fault && !pl->one) {
+        if (!timing && !c->inject_wait_fault && !c->inject_residue_fault && !pl->one) {
             rc = launch_graph(c, a, b, out, sq);
             if (rc <= 0) return rc;  // 1: fall back to direct launches
         }

@@ -132,6 +132,7 @@ struct bw_ctx {
     uint32_t* err = nullptr;
     uint4* rec_x = nullptr;
     uint32_t* rec_s = nullptr;
+    bw::Sum* sums = nullptr;    // word sums (64-bit coefficients)
     size_t ntiles = 0;
     // look-back record tag of the last product.  Direct launches use 2, 3, ..;
     // the replayable graph clears the records and always uses 1.
@@ -155,6 +156,8 @@ struct bw_ctx {
     size_t out_tiles_per = 0;      // carry tiles per K4 launch
     int spin_limit = 1 << 22;
     bool inject_wait_fault = false;
+    bool inject_residue_fault = false;  // residue fault_at of prime 0 is its neighbour's
+    size_t fault_at = 0;
 };
 
 // Stage order of one host-pointer product (bw_stage_order): begin(i, s)

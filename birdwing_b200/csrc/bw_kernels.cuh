@@ -109,7 +109,8 @@ struct PlanDev {
 struct CarryState {
     uint32_t counter;   // dynamic tile ticket (reset by K3 before every K4)
     uint32_t any;       // some tile's kind is not kill (k_carry_words; reset by K3)
-    uint32_t pad[2];
+    uint32_t done;      // fix CTAs that have finished (reset by K3)
+    uint32_t pad;
 };
 
 // One product of a batch (device memory).  Residues of product i live at
@@ -191,6 +192,54 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Sums of 32-bit words modulo 2^32 - 1, where a number is congruent to the sum
+// of its words: the check of products with 64-bit coefficients, whose primes
+// leave no room to see a wrong residue.  K1 sums the operands' words as it loads
+// them, K4 the product's, and the last kernel compares (k_carry_fix): a product
+// that went wrong in between passes with probability 2^-32.  (By its size alone
+// 98% of wrong coefficients of 2^22-coefficient operands pass: three 51-bit
+// primes hold 2^150.03, the coefficients reach 2^150.)  Three sums (a, b, c) of
+// kSumSlots partial ones each, which the comparison clears.  Cost, 2^23 words:
+// 752 -> 757 us (double precision), 805 -> 808 (six primes, 8.0 M words).
+// A word enters seven times (prime to 2^32 - 1): one wide multiply-add each, on
+// a pipe that these kernels leave idle, where a 64-bit addition takes two of the
+// instructions that they are short of.
+constexpr int kSumSlots = 16;
+constexpr uint32_t kSumWeight = 7;
+using Sum = unsigned long long;
+__device__ __forceinline__ void add_word(uint64_t& acc, uint32_t w) {
+    asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(acc) : "r"(w), "n"(kSumWeight));
+}
+
+// A warp's partial sums into a slot (every lane calls it; acc: of add_word).
+__device__ __forceinline__ void sum_words(Sum* slots, uint32_t slot, uint64_t acc) {
+    const uint64_t v = (acc & 0xffffffffu) + (acc >> 32);
+    const uint32_t x = (uint32_t)v + (uint32_t)(v >> 32);
+    const uint32_t lo = __reduce_add_sync(0xffffffffu, x & 0xffffu);
+    const uint32_t hi = __reduce_add_sync(0xffffffffu, x >> 16);
+    if ((threadIdx.x & 31) == 0)
+        atomicAdd(slots + (slot & (kSumSlots - 1)), (Sum)lo + ((Sum)hi << 16));
+}
+
+// Compares and clears the sums of one product; by one warp.
+__device__ __forceinline__ void check_sums(Sum* sums, bool square, uint32_t* err) {
+    constexpr Sum m = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    Sum v[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (lane < kSumSlots) {
+            v[k] = __ldcg(sums + k * kSumSlots + lane) % m;
+            sums[k * kSumSlots + lane] = 0;
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], d);
+        v[k] %= m;
+    }
+    // (7 a) (7 b) = 7 (7 c)
+    if (lane == 0 && v[0] * (square ? v[0] : v[1]) % m != kSumWeight * v[2] % m) atomicOr(err, 2u);
 }
 
 // Asynchronous global -> shared copy of one element (cp.async): a tile's
@@ -712,6 +761,16 @@ kb_fwd_col(const PlanDev<Ar> P, const BatchProd* __restrict__ D, typename Ar::T*
                                            blockIdx.x, smem_raw);
 }
 
+// Sum of an operand's words, beside the any-length K1 (the fixed-length one
+// sums as it loads).
+static __global__ void __launch_bounds__(256)
+k_sum_words(const uint32_t* __restrict__ w, size_t n, Sum* slots) {
+    uint64_t acc = 0;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
+        add_word(acc, __ldg(w + i));
+    sum_words(slots, blockIdx.x, acc);
+}
+
 // ------------------------------------------------------------------ K2
 // Per-row twiddle tables: F[i] = w^(i k1), G[j] = w^(j 2^a k1) (forward) and
 // the inverse pair with n^-1 2^bits folded into Gi.  w^e comes from the
@@ -982,7 +1041,7 @@ __device__ __forceinline__ void inv_col_body(const PlanDev<Ar>& P, typename Ar::
                                              CarryState* cst, int tile, int kp,
                                              unsigned char* smem_raw) {
     using T = typename Ar::T;
-    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = 0;
+    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = cst->done = 0;
     const int log_r = P.log_r, log_c = P.log_c + P.log_r2, log_cb = P.log_cb;
     const int R = 1 << log_r;
     const size_t C = (size_t)1 << log_c;
@@ -1392,11 +1451,13 @@ struct CarryShared {
 // predecessor's, resolve the 1-bit carry chain inside the tile, publish the
 // tile status and look back across tiles, then write the final words.  Every
 // thread of the CTA calls it; it returns after its last barrier.
+// sum: where the product's words are summed (SUM).
+template <bool SUM>
 __device__ __forceinline__ void carry_finish_tile(
     uint32_t t, size_t j0, const uint32_t (&l)[kCarryWordsPerThread], const uint32_t (&X)[3],
     uint32_t* __restrict__ out, size_t M, uint4* __restrict__ rec_x,
     uint32_t* __restrict__ rec_s, uint32_t epoch, uint32_t wait_epoch,
-    uint32_t* __restrict__ err, int spin_limit, CarryShared& sh) {
+    uint32_t* __restrict__ err, int spin_limit, CarryShared& sh, Sum* sum) {
     constexpr int E = kCarryWordsPerThread;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -1528,6 +1589,12 @@ __device__ __forceinline__ void carry_finish_tile(
         for (int e = 0; e < E; ++e)
             if (j0 + e < M) out[j0 + e] = w[e];
     }
+    if constexpr (SUM) {
+        uint64_t acc = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) add_word(acc, j0 + e < M ? w[e] : 0u);
+        sum_words(sum, t, acc);
+    }
 }
 
 // Words l and carry-out X of E = 8 output words from digit sums (16- and
@@ -1571,7 +1638,7 @@ __device__ __forceinline__ void garner_carry_body(
     const PlanDev<Ar>& P, const typename Ar::T* __restrict__ res, uint32_t* __restrict__ out,
     size_t M, size_t NL, CarryState* cst, uint4* __restrict__ rec_x,
     uint32_t* __restrict__ rec_s, uint32_t epoch, uint32_t wait_epoch,
-    uint32_t* __restrict__ err, int spin_limit) {
+    uint32_t* __restrict__ err, int spin_limit, Sum* sum) {
     constexpr int E = kCarryWordsPerThread;
     constexpr int TL = kCarryTileWords;
     __shared__ uint32_t s_tile;
@@ -1590,7 +1657,8 @@ __device__ __forceinline__ void garner_carry_body(
     garner_local<Ar, SPLIT16, W64, true>(P, res + j0 * elems_per_word2<SPLIT16, W64>() / 2, n,
                                          j0 < NL, l, X, &bad);
     if (bad) atomicOr(err, 2u);
-    carry_finish_tile(t, j0, l, X, out, M, rec_x, rec_s, epoch, wait_epoch, err, spin_limit, sh);
+    carry_finish_tile<W64>(t, j0, l, X, out, M, rec_x, rec_s, epoch, wait_epoch, err, spin_limit,
+                           sh, sum);
 }
 
 // K4 without waits (single products).  The look-back form above keeps every
@@ -1644,13 +1712,22 @@ __device__ __forceinline__ void carry_fix_tile(uint32_t t, bool ones, uint32_t* 
     }
 }
 
+// SUM: the last CTA to finish checks the product's word sums, to which each CTA
+// adds what it changed: 1 for every tile whose carry-in is 1, but for those that
+// propagate (words 2^32 - 1 and 0 are both 0).
+template <bool SUM>
 __device__ __forceinline__ void carry_fix_body(const uint32_t* __restrict__ kinds,
                                                uint32_t ntiles, uint32_t* __restrict__ out,
-                                               size_t M, const uint32_t* __restrict__ any,
-                                               uint32_t part, uint32_t parts) {
-    if (__ldcg(any) == 0u) return;  // every tile kills
+                                               size_t M, CarryState* cst, uint32_t part,
+                                               uint32_t parts, Sum* sums, bool square,
+                                               uint32_t* err) {
+    if (__ldcg(&cst->any) == 0u) {  // every tile kills
+        if (SUM && part == 0 && threadIdx.x < 32) check_sums(sums, square, err);
+        return;
+    }
     constexpr uint32_t NT = kFixThreads, NW = NT / 32;
     __shared__ uint32_t s_pos, s_n, s_last[NW], s_list[NT];
+    uint32_t added = 0;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t share = (ntiles + parts - 1) / parts;
     const uint32_t r0 = min(ntiles, part * share), r1 = min(ntiles, r0 + share);
@@ -1684,21 +1761,41 @@ __device__ __forceinline__ void carry_fix_body(const uint32_t* __restrict__ kind
             }
         const uint32_t below = con & ((1u << lane) - 1u);
         if (below) eps = (val >> (31 - __clz(below))) & 1u;
-        if (eps && t < r1) s_list[atomicAdd(&s_n, 1u)] = 2u * t + (k == 2u ? 1u : 0u);
+        if (eps && t < r1) {
+            s_list[atomicAdd(&s_n, 1u)] = 2u * t + (k == 2u ? 1u : 0u);
+            added += k == 2u ? 0u : 1u;
+        }
         __syncthreads();
         for (uint32_t i = warp; i < s_n; i += NW)
             carry_fix_tile(s_list[i] >> 1, (s_list[i] & 1u) != 0, out, M);
         cin = cout;
         __syncthreads();
     }
+    if constexpr (SUM) {
+        sum_words(sums + 2 * kSumSlots, part, kSumWeight * added);
+        __shared__ uint32_t s_done;
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_done = atomicAdd(&cst->done, 1u);
+        __syncthreads();
+        if (s_done == parts - 1 && tid < 32) check_sums(sums, square, err);
+    }
 }
 
+template <bool SUM>
 static __global__ void __launch_bounds__(kFixThreads)
 k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __restrict__ out,
-            size_t M, const uint32_t* __restrict__ any) {
+            size_t M, CarryState* cst, Sum* __restrict__ sums, int square,
+            uint32_t* __restrict__ err) {
     grid_release();
     grid_wait();
-    carry_fix_body(kinds, ntiles, out, M, any, blockIdx.x, gridDim.x);
+    carry_fix_body<SUM>(kinds, ntiles, out, M, cst, blockIdx.x, gridDim.x, sums, square != 0, err);
+}
+
+// The check alone, behind the look-back form's pieces.
+static __global__ void __launch_bounds__(32)
+k_check_sums(Sum* sums, int square, uint32_t* err) {
+    check_sums(sums, square != 0, err);
 }
 
 // any: set when a tile's kind is not kill (zero before).
@@ -1711,7 +1808,7 @@ __device__ __forceinline__ void carry_words_body(const PlanDev<Ar>& P,
                                                  uint32_t* __restrict__ out, size_t M, size_t NL,
                                                  uint32_t* __restrict__ kinds,
                                                  uint32_t* __restrict__ any,
-                                                 uint32_t* __restrict__ err) {
+                                                 uint32_t* __restrict__ err, Sum* sum) {
     constexpr int E = kCarryWordsPerThread;
     constexpr int TL = kCarryTileWords;
     __shared__ CarryShared sh;
@@ -1779,6 +1876,12 @@ __device__ __forceinline__ void carry_words_body(const PlanDev<Ar>& P,
             for (int e = 0; e < E; ++e)
                 if (j0 + e < M) out[j0 + e] = w[e];
         }
+        if constexpr (W64) {
+            uint64_t acc = 0;
+#pragma unroll
+            for (int e = 0; e < E; ++e) add_word(acc, j0 + e < M ? w[e] : 0u);
+            sum_words(sum, t, acc);
+        }
     }
     if (tid == 0 && gridDim.x > 1) {
         const uint32_t kind = chain_out(sh.w, 0u, kCarryThreads / 32) |
@@ -1792,10 +1895,10 @@ template <class Ar, bool SPLIT16, bool W64 = false>
 __global__ void __launch_bounds__(kWordsThreads, W64 ? 4 : 3)
 k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
               uint32_t* __restrict__ out, size_t M, size_t NL, uint32_t* __restrict__ kinds,
-              uint32_t* __restrict__ any, uint32_t* __restrict__ err) {
+              uint32_t* __restrict__ any, uint32_t* __restrict__ err, Sum* __restrict__ sum) {
     grid_release();
     grid_wait();
-    carry_words_body<Ar, SPLIT16, W64>(P, res, out, M, NL, kinds, any, err);
+    carry_words_body<Ar, SPLIT16, W64>(P, res, out, M, NL, kinds, any, err, sum);
 }
 
 // batched: blockIdx.y = product; the look-back kernel's 22-34% of issue slots
@@ -1810,15 +1913,15 @@ kb_carry_words(const PlanDev<Ar> P, const BatchProd* __restrict__ D,
     const size_t M = (size_t)d.la + d.lb;
     if ((size_t)blockIdx.x * kCarryTileWords >= (NL > M ? NL : M)) return;
     carry_words_body<Ar, SPLIT16, false>(P, res_a + d.res_off, d.out, M, NL, d.rec_s, &d.cst->any,
-                                         err);
+                                         err, nullptr);
 }
 // blockIdx.y = product
 static __global__ void __launch_bounds__(kFixThreads)
 kb_carry_fix(const BatchProd* __restrict__ D, size_t NL) {
     const BatchProd d = D[blockIdx.y];
     const size_t M = (size_t)d.la + d.lb, words = NL > M ? NL : M;
-    carry_fix_body(d.rec_s, (uint32_t)((words + kCarryTileWords - 1) / kCarryTileWords), d.out, M,
-                   &d.cst->any, blockIdx.x, gridDim.x);
+    carry_fix_body<false>(d.rec_s, (uint32_t)((words + kCarryTileWords - 1) / kCarryTileWords),
+                          d.out, M, d.cst, blockIdx.x, gridDim.x, nullptr, false, nullptr);
 }
 
 // Carry words of the last thread of every tile but the last (its 8 words'
@@ -1864,9 +1967,10 @@ __global__ void __launch_bounds__(kCarryThreads, 4)
 k_garner_carry(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
                uint32_t* __restrict__ out, size_t M, size_t NL, CarryState* cst,
                uint4* __restrict__ rec_x, uint32_t* __restrict__ rec_s, uint32_t epoch,
-               uint32_t wait_epoch, uint32_t* __restrict__ err, int spin_limit) {
+               uint32_t wait_epoch, uint32_t* __restrict__ err, int spin_limit,
+               Sum* __restrict__ sum) {
     garner_carry_body<Ar, SPLIT16, W64>(P, res, out, M, NL, cst, rec_x, rec_s, epoch,
-                                        wait_epoch, err, spin_limit);
+                                        wait_epoch, err, spin_limit, sum);
 }
 
 // batched: blockIdx.y = product
@@ -1878,7 +1982,7 @@ kb_garner_carry(const PlanDev<Ar> P, const BatchProd* __restrict__ D,
     const BatchProd d = D[blockIdx.y];
     const size_t NL = ((size_t)1 << P.log_n) / (SPLIT16 ? 2 : 1);
     garner_carry_body<Ar, SPLIT16>(P, res_a + d.res_off, d.out, (size_t)d.la + d.lb, NL, d.cst,
-                                   d.rec_x, d.rec_s, epoch, wait_epoch, err, spin_limit);
+                                   d.rec_x, d.rec_s, epoch, wait_epoch, err, spin_limit, nullptr);
 }
 
 // ------------------------------------------------------------------ small products

@@ -146,7 +146,7 @@ int run(int path, int K, const void* residues, size_t n, int log_n, uint32_t* ou
         pd, static_cast<const T*>(residues), out, out_words, NL,
         reinterpret_cast<CarryState*>(sb), reinterpret_cast<uint4*>(sb + 32),
         reinterpret_cast<uint32_t*>(sb + 32 + ntiles * 16), 1u, 1u,
-        reinterpret_cast<uint32_t*>(sb + 16), 1 << 22);
+        reinterpret_cast<uint32_t*>(sb + 16), 1 << 22, nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return bw_fail(BW_ECUDA, "launch: %s", cudaGetErrorString(e));
     uint32_t err = 0;

@@ -525,12 +525,13 @@ __device__ __forceinline__ void st_off(T* base, uint32_t o, T v) {
 }
 
 // Forward column pass of one tile, operand and prime.  zt: the upper half of
-// the rows is zero pad.
+// the rows is zero pad.  sum: where prime 0's CTAs sum the operand's words
+// (64-bit coefficients).
 template <class Ar, int LOGR, int CW>
 __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
                                               const uint32_t* __restrict__ limbs, size_t ncoef,
                                               typename Ar::T* res, bool zt, int tile, int kp,
-                                              unsigned char* smem_raw) {
+                                              unsigned char* smem_raw, Sum* sum) {
     using T = typename Ar::T;
     using L = LayCol<T>;
     using Cfg = ColCfg<Ar, LOGR>;
@@ -566,6 +567,7 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
 #pragma unroll
             for (int k = 0; k < NL; ++k) raw[k] = coef.load(o + k * step);
         };
+        uint64_t acc = 0;  // the words' sum
         if constexpr (AHEAD) load(threadIdx.x);
 #pragma unroll 1
         for (int sp = threadIdx.x; sp < N; sp += NT) {
@@ -576,6 +578,15 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
             T x[1 << RL];
             if constexpr (FIRST) {
                 if constexpr (!AHEAD) load(sp);
+                if constexpr (CW == 64) {
+                    if (kp == 0) {
+#pragma unroll
+                        for (int k = 0; k < NL; ++k) {
+                            add_word(acc, (uint32_t)raw[k]);
+                            add_word(acc, (uint32_t)(raw[k] >> 32));
+                        }
+                    }
+                }
 #pragma unroll
                 for (int k = 0; k < NL; ++k) x[k] = CoefLoad<Ar, CW>::residue(ar, raw[k]);
                 if constexpr (AHEAD) {
@@ -597,6 +608,9 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
                     buf[p0 + L::template off<false>(k, DS, 0)] = x[k];
                 }
             }
+        }
+        if constexpr (FIRST && CW == 64) {
+            if (kp == 0) sum_words(sum, (uint32_t)tile, acc);
         }
     };
     using std::false_type;
@@ -628,13 +642,14 @@ template <class Ar, int LOGR, int CW>
 __global__ void __launch_bounds__(ColCfg<Ar, LOGR>::NT, ColCfg<Ar, LOGR>::kMinCtas)
 k_fwd_col2(const PlanDev<Ar> P, const uint32_t* __restrict__ limbs_a, size_t ncoef_a,
            const uint32_t* __restrict__ limbs_b, size_t ncoef_b, typename Ar::T* res_a,
-           typename Ar::T* res_b, unsigned zt_mask, int tile0) {
+           typename Ar::T* res_b, unsigned zt_mask, int tile0, Sum* __restrict__ sums) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     grid_release();
     const int op = blockIdx.z;
     fwd_col2_body<Ar, LOGR, CW>(P, op ? limbs_b : limbs_a, op ? ncoef_b : ncoef_a,
                                      op ? res_b : res_a, (zt_mask >> op) & 1u,
-                                     tile0 + (int)(blockIdx.x / P.K), blockIdx.x % P.K, smem_raw);
+                                     tile0 + (int)(blockIdx.x / P.K), blockIdx.x % P.K, smem_raw,
+                                     sums + op * kSumSlots);
 }
 
 // Inverse column pass of one tile and prime, in place, residues fully reduced.
@@ -647,7 +662,7 @@ __device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar:
     using Cfg = ColCfg<Ar, LOGR>;
     constexpr int LCB = Cfg::LCB;
     constexpr int RL0 = first_rl(LOGR), NT = Cfg::NT, CB = 1 << LCB;
-    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = 0;
+    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = cst->done = 0;
     const int log_c = P.log_c + P.log_r2;
     const PrimeDev<Ar>& pr = P.pr[kp];
     const Ar ar = pr.ar;
@@ -858,7 +873,8 @@ kb_fwd_col2(const PlanDev<Ar> P, const BatchProd* __restrict__ D, typename Ar::T
     const size_t ncoef = (size_t)(op ? d.lb : d.la) * (CW == 16 ? 2 : 1);
     const size_t n = (size_t)1 << P.log_n;
     fwd_col2_body<Ar, LOGR, CW>(P, op ? d.b : d.a, ncoef, (op ? res_b : res_a) + d.res_off,
-                                ncoef <= n / 2, blockIdx.x / P.K, blockIdx.x % P.K, smem_raw);
+                                ncoef <= n / 2, blockIdx.x / P.K, blockIdx.x % P.K, smem_raw,
+                                nullptr);
 }
 
 // blockIdx.x = row, .y = prime, .z = product

@@ -102,14 +102,15 @@ template <class Ar, int CW>
 cudaError_t launch_fwd_col2(const bw_plan* pl, const PlanDev<Ar>& pd, const uint32_t* a,
                             size_t na, const uint32_t* b, size_t nb, typename Ar::T* ra,
                             typename Ar::T* rb, unsigned zt, int tile0, int ntiles, bool square,
-                            cudaStream_t s) {
+                            Sum* sums, cudaStream_t s) {
     return with_columns<Ar>(pl->log_r, [&](auto lr) {
         constexpr int LR = decltype(lr)::value;
         using Cfg = ColCfg<Ar, LR>;
         const cudaError_t e = allow_smem<&k_fwd_col2<Ar, LR, CW>>();
         if (e != cudaSuccess) return e;
         const dim3 g((unsigned)ntiles * pl->K, 1, square ? 1 : 2);
-        k_fwd_col2<Ar, LR, CW><<<g, Cfg::NT, Cfg::smem, s>>>(pd, a, na, b, nb, ra, rb, zt, tile0);
+        k_fwd_col2<Ar, LR, CW><<<g, Cfg::NT, Cfg::smem, s>>>(pd, a, na, b, nb, ra, rb, zt, tile0,
+                                                               sums);
         return cudaSuccess;
     });
 }
@@ -216,7 +217,7 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     auto k1 = [&](int tile0, int ntiles) {
         if (pl->v2_cols) {
             ke = launch_fwd_col2<Ar, W64 ? 64 : SPLIT16 ? 16 : 32>(
-                pl, pd, a, in_a, b, in_b, ra, rb, zt, tile0, ntiles, square, c->stream);
+                pl, pd, a, in_a, b, in_b, ra, rb, zt, tile0, ntiles, square, c->sums, c->stream);
             return;
         }
         dim3 g1(ntiles * (PP ? pl->K : 1), 1, square ? 1 : 2);
@@ -254,6 +255,11 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
             BW_CUDA(cudaStreamWaitEvent(c->stream, c->in_ev[k], 0));
             k1(k * per, per);
         }
+    }
+    if (W64 && !pl->v2_cols) {
+        const unsigned nb = 4 * 148;
+        k_sum_words<<<nb, 256, 0, c->stream>>>(a, pl->la, c->sums);
+        if (!square) k_sum_words<<<nb, 256, 0, c->stream>>>(b, pl->lb, c->sums + kSumSlots);
     }
     // three passes: middle column pass with the outer twiddle
     const int CB2 = 1 << pl->log_cb2;

@@ -65,7 +65,7 @@ extern "C" {
 #define BW_ETIMEOUT    (-4)  /* a bounded device-side wait gave up            */
 #define BW_EREJECT     (-5)  /* admission rejected (memory budget)            */
 #define BW_ESIZE       (-6)  /* product size outside the supported limits     */
-#define BW_ECHECK      (-7)  /* redundant-prime consistency check failed      */
+#define BW_ECHECK      (-7)  /* a product's consistency check failed          */
 #define BW_EBUSY       (-8)  /* resource still in use                         */
 
 /* ---- prime paths --------------------------------------------------------- */
@@ -226,7 +226,13 @@ int bw_ctx_set_copy_chunks(bw_ctx* ctx, int chunks);
 /* The cudaStream_t the context issues work on. */
 void* bw_ctx_stream(const bw_ctx* ctx);
 /* Wait for the context's stream and report device-side errors raised by
- * earlier BW_PTR_DEVICE calls (BW_ETIMEOUT, BW_ECHECK). */
+ * earlier BW_PTR_DEVICE calls (BW_ETIMEOUT, BW_ECHECK).
+ * BW_ECHECK: with 64-bit coefficients the product's words are compared with the
+ * operands' modulo 2^32 - 1, which one wrong residue passes with probability
+ * 2^-32.  With three primes and 16- or 32-bit coefficients the third prime must
+ * agree with the first two.  With two primes a wrong coefficient is seen only
+ * where it is out of bounds: on the 64-bit path all but one in 2^20, on the
+ * 32-bit path none. */
 int bw_ctx_sync(bw_ctx* ctx);
 
 /* c[0 .. la+lb) = a[0 .. la) * b[0 .. lb).  lc must be >= la + lb; words of
@@ -258,6 +264,10 @@ int bw_multiply_coeffs(bw_ctx* ctx, const uint32_t* a, size_t la,
  * No counterpart in the reference (it checks no CUDA errors at all). */
 int bw_ctx_set_wait_limit(bw_ctx* ctx, int polls);
 int bw_ctx_inject_wait_fault(bw_ctx* ctx, int enable);
+/* Test hook for the consistency checks (BW_ECHECK): the next products
+ * reconstruct with residue `at` of the first prime replaced by its neighbour's
+ * (at ^ 1), a valid residue in the wrong place. */
+int bw_ctx_inject_residue_fault(bw_ctx* ctx, int enable, size_t at);
 
 /* Largest number of 2048-word carry tiles bw_garner_carry_noalloc handles:
  * up to 2^26 output words (products of up to 2^31 bits). */
