@@ -145,7 +145,7 @@ struct bw_batch {
     size_t graph_nodes = 0;
     size_t kernel_nodes = 0;
     int spin_limit = 1 << 22;
-    bool inject_wait_fault = false;
+    bool inject_wait_fault = false, inject_residue_fault = false;
     // BW_BATCH_PERSISTENT: per prime path (0: 64-bit, 1: 32-bit), the small
     // buckets' device table, their work items and the queue head
     bool persistent = false;
@@ -430,7 +430,7 @@ int build_layout(bw_batch* bt) {
         if (bt->persistent && bk.small) continue;
         bw_group_launch g{&bk.plan, bk.d_desc, (unsigned)bk.prods.size(), bk.d_res_a,
                           bk.d_res_b, bk.ntiles, bt->d_err, bt->spin_limit,
-                          bt->inject_wait_fault};
+                          bt->inject_wait_fault, bt->inject_residue_fault};
         rc = bw_enqueue_group(g, bt->side[branch++ % nside]);
     }
     for (int s = 0; s < nside; ++s) {
@@ -644,7 +644,7 @@ extern "C" int bw_batch_run(bw_batch* bt, unsigned what, bw_timing* tm) {
     }
     const uint32_t err = *bt->h_err;
     if (err & 1u) return bw_fail(BW_ETIMEOUT, "carry look-back wait exceeded its bound");
-    if (err) return bw_fail(BW_ECHECK, "redundant-prime reconstruction check failed");
+    if (err) return bw_fail(BW_ECHECK, "the products' consistency check failed");
     return BW_OK;
 }
 
@@ -661,6 +661,14 @@ extern "C" int bw_batch_inject_wait_fault(bw_batch* bt, int enable) {
     if (!bt) return bw_fail(BW_EINVAL, "NULL batch");
     bt->inject_wait_fault = enable != 0;
     bt->dirty = true;
+    return BW_OK;
+}
+
+extern "C" int bw_batch_inject_residue_fault(bw_batch* bt, int enable) {
+    bw_clear_error();
+    if (!bt) return bw_fail(BW_EINVAL, "NULL batch");
+    bt->inject_residue_fault = enable != 0;
+    bt->dirty = true;  // part of the captured graph
     return BW_OK;
 }
 

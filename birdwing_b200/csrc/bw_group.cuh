@@ -139,6 +139,10 @@ cudaError_t bw_enqueue_group_of(const bw_group_launch& g, cudaStream_t s) {
         if (e == cudaSuccess) e = load_kernel<&kb_carry_words<Ar, SPLIT16>>();
         return e == cudaSuccess ? load_kernel<&kb_carry_fix>() : e;
     }
+    if (g.inject_residue_fault) {
+        const cudaError_t e = cudaMemcpyAsync(ra, ra + 1, sizeof(T), cudaMemcpyDeviceToDevice, s);
+        if (e != cudaSuccess) return e;
+    }
     if (bw_group_lookback(g)) {
         kb_garner_carry<Ar, SPLIT16><<<dim3((unsigned)g.ntiles, np), kCarryThreads, 0, s>>>(
             P, g.d_desc, ra, 1u, g.inject_wait_fault ? 1u + (1u << 27) : 1u, g.d_err,

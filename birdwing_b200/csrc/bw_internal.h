@@ -84,6 +84,7 @@ struct bw_group_launch {
     uint32_t* d_err;    // bit 0: look-back wait timed out; bit 1: check failed
     int spin_limit;
     bool inject_wait_fault = false;  // test hook: every look-back wait runs out
+    bool inject_residue_fault = false;  // test hook (4-step): residue 0 of product 0 is residue 1
 };
 // np 0: nothing is launched, the kernels that the plan's groups run are loaded.
 int bw_enqueue_group(const bw_group_launch& g, cudaStream_t s);

@@ -1170,7 +1170,7 @@ __device__ __forceinline__ unsigned __int128 garner_one(const PlanDev<Ar>& P, ty
 
 // Digit sums D[e] < 2^96 of E output words from their coefficients' residues
 // r[k] (one coefficient per word, or two 16-bit ones).  Sets *bad when the
-// redundant third prime disagrees or a value reaches 2^96.
+// redundant third prime disagrees or a value reaches its bound.
 template <class Ar, bool SPLIT16, int E>
 __device__ __forceinline__ void garner_combine(
     const PlanDev<Ar>& P, const typename Ar::T (&r)[kDigitPrimes][E * (SPLIT16 ? 2 : 1)],
@@ -1185,7 +1185,14 @@ __device__ __forceinline__ void garner_combine(
         } else {
             D[e] = garner_one(P, r[0][e], r[1][e], r[2][e], bad);
         }
-        bad |= (uint32_t)((D[e] >> 96) != 0);
+        // (double precision: the coefficient's own bound, n/2 2^64 -- two 50-bit
+        // primes hold 2^100, so the 2^96 that two 58-bit ones leave far behind
+        // would let one wrong coefficient in 16 pass)
+        if constexpr (Ar::kF64) {
+            bad |= (uint32_t)(((uint64_t)(D[e] >> 64) >> (P.log_n - 1)) != 0);
+        } else {
+            bad |= (uint32_t)((D[e] >> 96) != 0);
+        }
     }
     *bad_out |= bad;
 }

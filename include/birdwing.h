@@ -231,8 +231,8 @@ void* bw_ctx_stream(const bw_ctx* ctx);
  * operands' modulo 2^32 - 1, which one wrong residue passes with probability
  * 2^-32.  With three primes and 16- or 32-bit coefficients the third prime must
  * agree with the first two.  With two primes a wrong coefficient is seen only
- * where it is out of bounds: on the 64-bit path all but one in 2^20, on the
- * 32-bit path none. */
+ * where it is out of bounds: on the 64-bit path all but one in 2^20 (in groups,
+ * all but n in 2^37, n the transform length), on the 32-bit path none. */
 int bw_ctx_sync(bw_ctx* ctx);
 
 /* c[0 .. la+lb) = a[0 .. la) * b[0 .. lb).  lc must be >= la + lb; words of
@@ -390,6 +390,9 @@ int bw_batch_get_info(const bw_batch* batch, bw_batch_info* info);
  * it is switched off.  Both rebuild the captured graph at the next run. */
 int bw_batch_set_wait_limit(bw_batch* batch, int polls);
 int bw_batch_inject_wait_fault(bw_batch* batch, int enable);
+/* As bw_ctx_inject_residue_fault: residue 0 of each 4-step group's first
+ * product. */
+int bw_batch_inject_residue_fault(bw_batch* batch, int enable);
 
 /* Time each candidate form of each group (one CTA per product where the
  * transform fits shared memory; 4-step with each column/row split from

@@ -1,4 +1,4 @@
-"""BW_ECHECK on products with 64-bit coefficients: no prime is redundant there,
+"""BW_ECHECK.  On products with 64-bit coefficients no prime is redundant,
 so the product's words are checked against the operands' modulo 2^32 - 1.  One
 residue in the wrong place (data only: a valid residue copied from its
 neighbour) is reported however little room the primes leave, in every form of
@@ -82,3 +82,26 @@ def test_carry_chains_pass_the_check(la, lb, path):
             c.set_copy_chunks(chunks)
             check_reports(c, lambda: c.multiply(a, b), want, spots)
         check_reports(c, lambda: device_product(c, a, b), want, spots)
+
+
+@pytest.mark.parametrize("K", [2, 3])
+@pytest.mark.parametrize("words", [3000, 100000])
+def test_groups_report_a_wrong_residue(words, K):
+    # the 64-bit path's groups: with two primes by the coefficient's bound (a
+    # wrong one passes with probability n 2^-37), with three by the third.
+    # 64 products, one at a time: by the bound 2^96 alone some would pass.
+    rng = np.random.default_rng(words)
+    a, b = (np.zeros(words, dtype=np.uint32) for _ in range(2))
+    with bw.Batch(num_primes=K) as bt:
+        out = bt.add(a, b, path=64)
+        for on in [1] * 64 + [0]:
+            a[:] = rng.integers(0, 1 << 32, words, dtype=np.uint64)
+            b[:] = rng.integers(0, 1 << 32, words, dtype=np.uint64)
+            bw._lib.check(bw.lib.bw_batch_inject_residue_fault(bt._h, on))
+            if on:
+                with pytest.raises(bw.BwError) as e:
+                    bt.run()
+                assert e.value.code == L.BW_ECHECK
+            else:
+                bt.run()
+                assert (out == gmp_ref.mul(a, b)).all()
