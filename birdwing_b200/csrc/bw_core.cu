@@ -713,8 +713,10 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
                 }
             }
             const int top = w == 8 ? kCol2MaxLog64 : kCol2MaxLog32;
-            // (their addresses are 32-bit byte offsets into one prime's residues)
-            if (pl->log_r >= kCol2MinLog && pl->log_r <= top && !pl->tw_smem_r &&
+            // (their addresses are 32-bit byte offsets into one prime's residues;
+            // 64-bit coefficients come to the 58-bit primes only beyond that)
+            const bool long_only = pl->w64 && path == BW_PATH_P64 && !pl->f64;
+            if (!long_only && pl->log_r >= kCol2MinLog && pl->log_r <= top && !pl->tw_smem_r &&
                 ((size_t)w << log_n) < (size_t)1 << 32) {
                 pl->v2_cols = 1;
                 const int cb = w == 8 ? col_log_cb<8>(pl->log_r) : col_log_cb<4>(pl->log_r);
@@ -741,8 +743,10 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
     return rc;
 }
 
-extern "C" int bw_plan_create(bw_plan** out, int path, size_t la, size_t lb, int num_primes,
-                              unsigned flags) {
+// arith: double-precision prime set (0: integers) of 64-bit coefficients on the
+// 64-bit path; -1: by the operands.
+extern "C" int bw_plan_create_arith(bw_plan** out, int path, size_t la, size_t lb, int num_primes,
+                                    unsigned flags, int arith) {
     bw_clear_error();
     if (!out) return bw_fail(BW_EINVAL, "out is NULL");
     *out = nullptr;
@@ -761,6 +765,16 @@ extern "C" int bw_plan_create(bw_plan** out, int path, size_t la, size_t lb, int
     pl->nca = w64 ? (la + 1) / 2 : la * cpw;
     pl->ncb = w64 ? (lb + 1) / 2 : lb * cpw;
     if (w64 && path == BW_PATH_P64) pl->f64 = choose_f64(pl->nca, pl->ncb);
+    if (arith >= 0 && arith != pl->f64) {
+        // only where the set's product holds the coefficients
+        const bool holds = pl->w64 && path == BW_PATH_P64 &&
+                           (arith == 0 || (arith == 2 && pl->f64 == 1));
+        if (!holds) {
+            delete pl;
+            return bw_fail(BW_EINVAL, "arithmetic %d does not hold the product", arith);
+        }
+        pl->f64 = arith;
+    }
     const size_t half = ((size_t)1 << log_n) / 2;
     pl->zt_a = pl->nca <= half;
     pl->zt_b = pl->ncb <= half;
@@ -773,6 +787,11 @@ extern "C" int bw_plan_create(bw_plan** out, int path, size_t la, size_t lb, int
     pl->order = new bw_stage_order();
     *out = pl;
     return BW_OK;
+}
+
+extern "C" int bw_plan_create(bw_plan** out, int path, size_t la, size_t lb, int num_primes,
+                              unsigned flags) {
+    return bw_plan_create_arith(out, path, la, lb, num_primes, flags, -1);
 }
 
 extern "C" int bw_plan_destroy(bw_plan* pl) {

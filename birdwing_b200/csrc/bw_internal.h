@@ -65,6 +65,13 @@ struct bw_plan {
 // column tiles narrowed for small n so that the column passes fill the SMs.
 int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int mode);
 
+// bw_plan_create with the arithmetic of 64-bit coefficients on the 64-bit path
+// named (0: 58-bit integer primes, 2: the second double-precision set, -1: by
+// the operands), for tests: left to itself a plan takes the integers above 2^27
+// coefficients of the shorter operand and the second set above 2^22.
+extern "C" int bw_plan_create_arith(bw_plan** out, int path, size_t la, size_t lb, int num_primes,
+                                    unsigned flags, int arith);
+
 // Largest transform of a launch group: the two-pass schedule.
 constexpr int kMaxGroupLogN = 26;
 

@@ -215,10 +215,14 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
     const unsigned zt = (pl->zt_a ? 1u : 0u) | (pl->zt_b ? 2u : 0u);
     cudaError_t ke = cudaSuccess;  // a fixed-length launch's status
     auto k1 = [&](int tile0, int ntiles) {
-        if (pl->v2_cols) {
-            ke = launch_fwd_col2<Ar, W64 ? 64 : SPLIT16 ? 16 : 32>(
-                pl, pd, a, in_a, b, in_b, ra, rb, zt, tile0, ntiles, square, c->sums, c->stream);
-            return;
+        // (bw_plan_setup: no fixed columns for 64-bit coefficients in 58-bit primes)
+        if constexpr (!W64 || !std::is_same<Ar, Ar64>::value) {
+            if (pl->v2_cols) {
+                ke = launch_fwd_col2<Ar, W64 ? 64 : SPLIT16 ? 16 : 32>(
+                    pl, pd, a, in_a, b, in_b, ra, rb, zt, tile0, ntiles, square, c->sums,
+                    c->stream);
+                return;
+            }
         }
         dim3 g1(ntiles * (PP ? pl->K : 1), 1, square ? 1 : 2);
         if (ts) {
