@@ -1048,11 +1048,11 @@ int enqueue_carry(bw_ctx* c, uint32_t* out, bool square, bool timing, int pieces
         BW_CUDA(launch_after(!timing, k_carry_words<Ar, SPLIT16, W64>,
                              dim3((unsigned)c->ntiles), kWordsThreads, 0, c->stream, pd,
                              reinterpret_cast<const T*>(c->d_res_a), out, M, NL, c->rec_s,
-                             &c->cst->any, c->err, c->sums + 2 * kSumSlots));
-        if (W64 || c->ntiles > 1)
+                             &c->cst->any, c->err, c->sums, square ? 1 : 0));
+        if (c->ntiles > 1)
             BW_CUDA(launch_after(!timing, k_carry_fix<W64>, dim3(fix_ctas(c->ntiles)), kFixThreads,
-                                 0, c->stream, c->rec_s, (uint32_t)c->ntiles, out, M, c->cst,
-                                 c->sums, square ? 1 : 0, c->err));
+                                 0, c->stream, c->rec_s, (uint32_t)c->ntiles, out, M,
+                                 &c->cst->any, c->sums, square ? 1 : 0, c->err));
         c->out_pieces = 1;
         return BW_OK;
     }

@@ -109,8 +109,7 @@ struct PlanDev {
 struct CarryState {
     uint32_t counter;   // dynamic tile ticket (reset by K3 before every K4)
     uint32_t any;       // some tile's kind is not kill (k_carry_words; reset by K3)
-    uint32_t done;      // fix CTAs that have finished (reset by K3)
-    uint32_t pad;
+    uint32_t pad[2];
 };
 
 // One product of a batch (device memory).  Residues of product i live at
@@ -197,12 +196,13 @@ __device__ __forceinline__ void grid_release() {
 // Sums of 32-bit words modulo 2^32 - 1, where a number is congruent to the sum
 // of its words: the check of products with 64-bit coefficients, whose primes
 // leave no room to see a wrong residue.  K1 sums the operands' words as it loads
-// them, K4 the product's, and the last kernel compares (k_carry_fix): a product
-// that went wrong in between passes with probability 2^-32.  (By its size alone
-// 98% of wrong coefficients of 2^22-coefficient operands pass: three 51-bit
-// primes hold 2^150.03, the coefficients reach 2^150.)  Three sums (a, b, c) of
-// kSumSlots partial ones each, which the comparison clears.  Cost, 2^23 words:
-// 752 -> 757 us (double precision), 805 -> 808 (six primes, 8.0 M words).
+// them, K4 the product's digits before the carry is resolved, and the last kernel
+// compares: a product that went wrong in between passes with probability 2^-32.
+// (By its size alone 98% of wrong coefficients of 2^22-coefficient operands
+// pass: three 51-bit primes hold 2^150.03, the coefficients reach 2^150.)  Three
+// sums (a, b, c) of kSumSlots partial ones each, which the comparison clears.
+// Cost: 2^23 words 754 -> 756 us, 2^21 words (six primes) 184.5 -> 185.5, others
+// within the noise.
 // A word enters seven times (prime to 2^32 - 1): one wide multiply-add each, on
 // a pipe that these kernels leave idle, where a 64-bit addition takes two of the
 // instructions that they are short of.
@@ -213,33 +213,55 @@ __device__ __forceinline__ void add_word(uint64_t& acc, uint32_t w) {
     asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(acc) : "r"(w), "n"(kSumWeight));
 }
 
-// A warp's partial sums into a slot (every lane calls it; acc: of add_word).
-__device__ __forceinline__ void sum_words(Sum* slots, uint32_t slot, uint64_t acc) {
+// A CTA's partial sum, of up to 8 warps: each warp leaves its own (acc: of
+// add_word), and after a barrier one warp adds them to a slot.  (One atomic a
+// warp on the slots' line took K4 from 0.24 to 0.42 ms at 2^25 words.)
+struct SumParts {
+    uint2 w[8];
+};
+__device__ __forceinline__ void sum_part(SumParts& s, uint64_t acc) {
     const uint64_t v = (acc & 0xffffffffu) + (acc >> 32);
     const uint32_t x = (uint32_t)v + (uint32_t)(v >> 32);
     const uint32_t lo = __reduce_add_sync(0xffffffffu, x & 0xffffu);
     const uint32_t hi = __reduce_add_sync(0xffffffffu, x >> 16);
-    if ((threadIdx.x & 31) == 0)
-        atomicAdd(slots + (slot & (kSumSlots - 1)), (Sum)lo + ((Sum)hi << 16));
+    if ((threadIdx.x & 31) == 0) s.w[threadIdx.x >> 5] = make_uint2(lo, hi);
+}
+__device__ __forceinline__ void sum_parts(Sum* slots, uint32_t slot, const SumParts& s,
+                                          int warps) {
+    const int lane = threadIdx.x & 31;
+    const uint2 p = lane < warps ? s.w[lane] : make_uint2(0, 0);
+    const uint32_t lo = __reduce_add_sync(0xffffffffu, p.x);
+    const uint32_t hi = __reduce_add_sync(0xffffffffu, p.y);
+    if (lane == 0) atomicAdd(slots + (slot & (kSumSlots - 1)), (Sum)lo + ((Sum)hi << 16));
 }
 
-// Compares and clears the sums of one product; by one warp.
-__device__ __forceinline__ void check_sums(Sum* sums, bool square, uint32_t* err) {
+// Compares and clears the sums of one product, by one warp; load: what each lane
+// reads of them.
+struct SumLanes {
+    Sum v[3] = {0, 0, 0};
+};
+__device__ __forceinline__ SumLanes load_sums(const Sum* sums) {
+    SumLanes r;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        if (lane < kSumSlots) r.v[k] = __ldcg(sums + k * kSumSlots + lane);
+    return r;
+}
+__device__ __forceinline__ void check_sums(Sum* sums, SumLanes s, bool square, uint32_t* err) {
     constexpr Sum m = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    Sum v[3] = {0, 0, 0};
+    // (partial sums stay below 2^59, sixteen of them below 2^63)
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        if (lane < kSumSlots) {
-            v[k] = __ldcg(sums + k * kSumSlots + lane) % m;
-            sums[k * kSumSlots + lane] = 0;
-        }
+        if (lane < kSumSlots) sums[k * kSumSlots + lane] = 0;
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], d);
-        v[k] %= m;
+        for (int d = kSumSlots / 2; d > 0; d >>= 1) s.v[k] += __shfl_xor_sync(0xffffffffu, s.v[k], d);
+        s.v[k] %= m;
     }
     // (7 a) (7 b) = 7 (7 c)
-    if (lane == 0 && v[0] * (square ? v[0] : v[1]) % m != kSumWeight * v[2] % m) atomicOr(err, 2u);
+    if (lane == 0 && s.v[0] * (square ? s.v[0] : s.v[1]) % m != kSumWeight * s.v[2] % m)
+        atomicOr(err, 2u);
 }
 
 // Asynchronous global -> shared copy of one element (cp.async): a tile's
@@ -551,7 +573,8 @@ template <class Ar, bool SPLIT16, int RLOG, bool TS, bool W64 = false, bool PP =
 __device__ __forceinline__ void fwd_col_body(const PlanDev<Ar>& P,
                                              const uint32_t* __restrict__ limbs, size_t ncoef,
                                              typename Ar::T* res, bool zt_in, int tile,
-                                             unsigned char* smem_raw, int kp0 = 0) {
+                                             unsigned char* smem_raw, int kp0 = 0,
+                                             Sum* sum = nullptr) {
     static_assert(!PP || (!SPLIT16 && sizeof(typename Ar::T) == 8), "PP: 64-bit path");
     using T = typename Ar::T;
     const bool zt = zt_in && P.log_r > 0;
@@ -664,6 +687,22 @@ __device__ __forceinline__ void fwd_col_body(const PlanDev<Ar>& P,
         }
     }
     cp_async_wait();
+    if constexpr (W64) {
+        // the words this thread staged, once per operand
+        if (!PP || kp0 == 0) {
+            uint64_t acc = 0;
+            for (int e = threadIdx.x; e < (rows_loaded << log_cb); e += blockDim.x) {
+                const uint32_t* w = PP ? reinterpret_cast<const uint32_t*>(buf + LayCol<T>::p(e))
+                                       : reinterpret_cast<const uint32_t*>(coef + e);
+                add_word(acc, w[0]);
+                add_word(acc, w[1]);
+            }
+            __shared__ SumParts sp;
+            sum_part(sp, acc);
+            __syncthreads();
+            if (threadIdx.x < 32) sum_parts(sum, (uint32_t)tile, sp, kColThreads / 32);
+        }
+    }
 
     const int nr = sched_rounds<RLOG>(log_r);
     for (int kp = PP ? kp0 : 0; kp < (PP ? kp0 + 1 : P.K); ++kp) {
@@ -735,14 +774,15 @@ template <class Ar, bool SPLIT16, int RLOG, bool TS, bool W64 = false, bool PP =
 __global__ void __launch_bounds__(kColThreads, 3)
 k_fwd_col(const PlanDev<Ar> P, const uint32_t* __restrict__ limbs_a, size_t ncoef_a,
           const uint32_t* __restrict__ limbs_b, size_t ncoef_b, typename Ar::T* res_a,
-          typename Ar::T* res_b, unsigned zt_mask, int tile0) {
+          typename Ar::T* res_b, unsigned zt_mask, int tile0, Sum* __restrict__ sums) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int op = blockIdx.z;
     fwd_col_body<Ar, SPLIT16, RLOG, TS, W64, PP>(P, op ? limbs_b : limbs_a,
                                                  op ? ncoef_b : ncoef_a, op ? res_b : res_a,
                                                  (zt_mask >> op) & 1u,
                                                  tile0 + (int)(PP ? blockIdx.x / P.K : blockIdx.x),
-                                                 smem_raw, PP ? (int)(blockIdx.x % P.K) : 0);
+                                                 smem_raw, PP ? (int)(blockIdx.x % P.K) : 0,
+                                                 sums + op * kSumSlots);
 }
 
 // batched: blockIdx.z = 2 * product + operand
@@ -759,16 +799,6 @@ kb_fwd_col(const PlanDev<Ar> P, const BatchProd* __restrict__ D, typename Ar::T*
     fwd_col_body<Ar, SPLIT16, RLOG, false>(P, op ? d.b : d.a, ncoef,
                                            (op ? res_b : res_a) + d.res_off, ncoef <= n / 2,
                                            blockIdx.x, smem_raw);
-}
-
-// Sum of an operand's words, beside the any-length K1 (the fixed-length one
-// sums as it loads).
-static __global__ void __launch_bounds__(256)
-k_sum_words(const uint32_t* __restrict__ w, size_t n, Sum* slots) {
-    uint64_t acc = 0;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
-        add_word(acc, __ldg(w + i));
-    sum_words(slots, blockIdx.x, acc);
 }
 
 // ------------------------------------------------------------------ K2
@@ -1041,7 +1071,7 @@ __device__ __forceinline__ void inv_col_body(const PlanDev<Ar>& P, typename Ar::
                                              CarryState* cst, int tile, int kp,
                                              unsigned char* smem_raw) {
     using T = typename Ar::T;
-    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = cst->done = 0;
+    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = 0;
     const int log_r = P.log_r, log_c = P.log_c + P.log_r2, log_cb = P.log_cb;
     const int R = 1 << log_r;
     const size_t C = (size_t)1 << log_c;
@@ -1451,7 +1481,20 @@ struct CarryShared {
     uint32_t lastx[kCarryThreads / 32][3];
     uint32_t cin[3];
     uint32_t eps;
+    SumParts sum;
 };
+
+// A thread's share of the product's word sum: its digits S and the carry c out of
+// them.  Before the 1-bit carries are resolved, which move a 1 from a word to a
+// carry and so leave the sum as it is.
+__device__ __forceinline__ uint64_t digit_sum(const uint32_t (&S)[kCarryWordsPerThread],
+                                              uint32_t c) {
+    uint64_t acc = 0;
+#pragma unroll
+    for (int e = 0; e < kCarryWordsPerThread; ++e) add_word(acc, S[e]);
+    add_word(acc, c);
+    return acc;
+}
 
 // Tile t's carry, given every thread's 8 words l (digit sums added with
 // carry-in zero) and carry-out X: publish the tile's carry words, take the
@@ -1530,10 +1573,14 @@ __device__ __forceinline__ void carry_finish_tile(
             all &= S[e];
         }
         st = c ? 2 : (all == 0xffffffffu ? 1 : 0);
+        if constexpr (SUM) sum_part(sh.sum, digit_sum(S, (uint32_t)c));
     }
 
     const ChainMasks cm = chain_prepare(st, sh.w);
     __syncthreads();
+    if constexpr (SUM) {
+        if (warp == kCarryThreads / 32 - 1) sum_parts(sum, t, sh.sum, kCarryThreads / 32);
+    }
 
     // ---- tile status, publish, look back (thread 0)
     if (tid == 0) {
@@ -1595,12 +1642,6 @@ __device__ __forceinline__ void carry_finish_tile(
 #pragma unroll
         for (int e = 0; e < E; ++e)
             if (j0 + e < M) out[j0 + e] = w[e];
-    }
-    if constexpr (SUM) {
-        uint64_t acc = 0;
-#pragma unroll
-        for (int e = 0; e < E; ++e) add_word(acc, j0 + e < M ? w[e] : 0u);
-        sum_words(sum, t, acc);
     }
 }
 
@@ -1719,22 +1760,13 @@ __device__ __forceinline__ void carry_fix_tile(uint32_t t, bool ones, uint32_t* 
     }
 }
 
-// SUM: the last CTA to finish checks the product's word sums, to which each CTA
-// adds what it changed: 1 for every tile whose carry-in is 1, but for those that
-// propagate (words 2^32 - 1 and 0 are both 0).
-template <bool SUM>
 __device__ __forceinline__ void carry_fix_body(const uint32_t* __restrict__ kinds,
                                                uint32_t ntiles, uint32_t* __restrict__ out,
-                                               size_t M, CarryState* cst, uint32_t part,
-                                               uint32_t parts, Sum* sums, bool square,
-                                               uint32_t* err) {
-    if (__ldcg(&cst->any) == 0u) {  // every tile kills
-        if (SUM && part == 0 && threadIdx.x < 32) check_sums(sums, square, err);
-        return;
-    }
+                                               size_t M, const uint32_t* __restrict__ any,
+                                               uint32_t part, uint32_t parts) {
+    if (__ldcg(any) == 0u) return;  // every tile kills
     constexpr uint32_t NT = kFixThreads, NW = NT / 32;
     __shared__ uint32_t s_pos, s_n, s_last[NW], s_list[NT];
-    uint32_t added = 0;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t share = (ntiles + parts - 1) / parts;
     const uint32_t r0 = min(ntiles, part * share), r1 = min(ntiles, r0 + share);
@@ -1768,41 +1800,34 @@ __device__ __forceinline__ void carry_fix_body(const uint32_t* __restrict__ kind
             }
         const uint32_t below = con & ((1u << lane) - 1u);
         if (below) eps = (val >> (31 - __clz(below))) & 1u;
-        if (eps && t < r1) {
-            s_list[atomicAdd(&s_n, 1u)] = 2u * t + (k == 2u ? 1u : 0u);
-            added += k == 2u ? 0u : 1u;
-        }
+        if (eps && t < r1) s_list[atomicAdd(&s_n, 1u)] = 2u * t + (k == 2u ? 1u : 0u);
         __syncthreads();
         for (uint32_t i = warp; i < s_n; i += NW)
             carry_fix_tile(s_list[i] >> 1, (s_list[i] & 1u) != 0, out, M);
         cin = cout;
         __syncthreads();
     }
-    if constexpr (SUM) {
-        sum_words(sums + 2 * kSumSlots, part, kSumWeight * added);
-        __shared__ uint32_t s_done;
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) s_done = atomicAdd(&cst->done, 1u);
-        __syncthreads();
-        if (s_done == parts - 1 && tid < 32) check_sums(sums, square, err);
-    }
 }
 
+// SUM: the first CTA also compares the product's word sums.
 template <bool SUM>
 static __global__ void __launch_bounds__(kFixThreads)
 k_carry_fix(const uint32_t* __restrict__ kinds, uint32_t ntiles, uint32_t* __restrict__ out,
-            size_t M, CarryState* cst, Sum* __restrict__ sums, int square,
+            size_t M, const uint32_t* __restrict__ any, Sum* __restrict__ sums, int square,
             uint32_t* __restrict__ err) {
     grid_release();
     grid_wait();
-    carry_fix_body<SUM>(kinds, ntiles, out, M, cst, blockIdx.x, gridDim.x, sums, square != 0, err);
+    if constexpr (SUM) {
+        if (blockIdx.x == 0 && threadIdx.x < 32)
+            check_sums(sums, load_sums(sums), square != 0, err);
+    }
+    carry_fix_body(kinds, ntiles, out, M, any, blockIdx.x, gridDim.x);
 }
 
 // The check alone, behind the look-back form's pieces.
 static __global__ void __launch_bounds__(32)
 k_check_sums(Sum* sums, int square, uint32_t* err) {
-    check_sums(sums, square != 0, err);
+    check_sums(sums, load_sums(sums), square != 0, err);
 }
 
 // any: set when a tile's kind is not kill (zero before).
@@ -1815,7 +1840,8 @@ __device__ __forceinline__ void carry_words_body(const PlanDev<Ar>& P,
                                                  uint32_t* __restrict__ out, size_t M, size_t NL,
                                                  uint32_t* __restrict__ kinds,
                                                  uint32_t* __restrict__ any,
-                                                 uint32_t* __restrict__ err, Sum* sum) {
+                                                 uint32_t* __restrict__ err, Sum* sums,
+                                                 bool square) {
     constexpr int E = kCarryWordsPerThread;
     constexpr int TL = kCarryTileWords;
     __shared__ CarryShared sh;
@@ -1860,10 +1886,24 @@ __device__ __forceinline__ void carry_words_body(const PlanDev<Ar>& P,
             all &= S[e];
         }
         st = c ? 2 : (all == 0xffffffffu ? 1 : 0);
+        if constexpr (W64) {
+            if (own) sum_part(sh.sum, digit_sum(S, (uint32_t)c));
+        }
     }
     ChainMasks cm{0, 0};
     if (own) cm = chain_prepare(st, sh.w);
     __syncthreads();
+    if constexpr (W64) {
+        if (!own) {
+            sum_parts(sums + 2 * kSumSlots, t, sh.sum, kCarryThreads / 32);
+            // a product of one tile has no fix to compare the sums
+            if (gridDim.x == 1) {
+                __threadfence();
+                __syncwarp();
+                check_sums(sums, load_sums(sums), square, err);
+            }
+        }
+    }
     if (own) {
         const uint32_t mc = chain_mine(cm, sh.w, 0u);
         uint32_t w[E];
@@ -1883,12 +1923,6 @@ __device__ __forceinline__ void carry_words_body(const PlanDev<Ar>& P,
             for (int e = 0; e < E; ++e)
                 if (j0 + e < M) out[j0 + e] = w[e];
         }
-        if constexpr (W64) {
-            uint64_t acc = 0;
-#pragma unroll
-            for (int e = 0; e < E; ++e) add_word(acc, j0 + e < M ? w[e] : 0u);
-            sum_words(sum, t, acc);
-        }
     }
     if (tid == 0 && gridDim.x > 1) {
         const uint32_t kind = chain_out(sh.w, 0u, kCarryThreads / 32) |
@@ -1902,10 +1936,11 @@ template <class Ar, bool SPLIT16, bool W64 = false>
 __global__ void __launch_bounds__(kWordsThreads, W64 ? 4 : 3)
 k_carry_words(const PlanDev<Ar> P, const typename Ar::T* __restrict__ res,
               uint32_t* __restrict__ out, size_t M, size_t NL, uint32_t* __restrict__ kinds,
-              uint32_t* __restrict__ any, uint32_t* __restrict__ err, Sum* __restrict__ sum) {
+              uint32_t* __restrict__ any, uint32_t* __restrict__ err, Sum* __restrict__ sums,
+              int square) {
     grid_release();
     grid_wait();
-    carry_words_body<Ar, SPLIT16, W64>(P, res, out, M, NL, kinds, any, err, sum);
+    carry_words_body<Ar, SPLIT16, W64>(P, res, out, M, NL, kinds, any, err, sums, square != 0);
 }
 
 // batched: blockIdx.y = product; the look-back kernel's 22-34% of issue slots
@@ -1920,15 +1955,15 @@ kb_carry_words(const PlanDev<Ar> P, const BatchProd* __restrict__ D,
     const size_t M = (size_t)d.la + d.lb;
     if ((size_t)blockIdx.x * kCarryTileWords >= (NL > M ? NL : M)) return;
     carry_words_body<Ar, SPLIT16, false>(P, res_a + d.res_off, d.out, M, NL, d.rec_s, &d.cst->any,
-                                         err, nullptr);
+                                         err, nullptr, false);
 }
 // blockIdx.y = product
 static __global__ void __launch_bounds__(kFixThreads)
 kb_carry_fix(const BatchProd* __restrict__ D, size_t NL) {
     const BatchProd d = D[blockIdx.y];
     const size_t M = (size_t)d.la + d.lb, words = NL > M ? NL : M;
-    carry_fix_body<false>(d.rec_s, (uint32_t)((words + kCarryTileWords - 1) / kCarryTileWords),
-                          d.out, M, d.cst, blockIdx.x, gridDim.x, nullptr, false, nullptr);
+    carry_fix_body(d.rec_s, (uint32_t)((words + kCarryTileWords - 1) / kCarryTileWords), d.out, M,
+                   &d.cst->any, blockIdx.x, gridDim.x);
 }
 
 // Carry words of the last thread of every tile but the last (its 8 words'

@@ -544,6 +544,8 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
     T* gout = res + ((size_t)kp << P.log_n) + c0;
     T* buf = reinterpret_cast<T*>(smem_raw);
     const CoefLoad<Ar, CW> coef(limbs, ncoef);
+    uint64_t acc = 0;  // the words' sum (prime 0's CTAs)
+    __shared__ SumParts parts;
 
     auto round = [&](auto s0_, auto rl_, auto zt_) {
         constexpr int S0 = decltype(s0_)::value, RL = decltype(rl_)::value;
@@ -567,7 +569,6 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
 #pragma unroll
             for (int k = 0; k < NL; ++k) raw[k] = coef.load(o + k * step);
         };
-        uint64_t acc = 0;  // the words' sum
         if constexpr (AHEAD) load(threadIdx.x);
 #pragma unroll 1
         for (int sp = threadIdx.x; sp < N; sp += NT) {
@@ -609,9 +610,6 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
                 }
             }
         }
-        if constexpr (FIRST && CW == 64) {
-            if (kp == 0) sum_words(sum, (uint32_t)tile, acc);
-        }
     };
     using std::false_type;
     using std::true_type;
@@ -620,8 +618,14 @@ __device__ __forceinline__ void fwd_col2_body(const PlanDev<Ar>& P,
     } else {
         round(std::integral_constant<int, 0>{}, std::integral_constant<int, RL0>{}, false_type{});
     }
+    if constexpr (CW == 64) {
+        if (kp == 0) sum_part(parts, acc);
+    }
+    if constexpr (LOGR > RL0 || CW == 64) __syncthreads();
+    if constexpr (CW == 64) {
+        if (kp == 0 && threadIdx.x < 32) sum_parts(sum, (uint32_t)tile, parts, NT / 32);
+    }
     if constexpr (LOGR > RL0) {
-        __syncthreads();
         round(std::integral_constant<int, RL0>{}, std::integral_constant<int, 4>{}, false_type{});
     }
     if constexpr (LOGR > RL0 + 4) {
@@ -662,7 +666,7 @@ __device__ __forceinline__ void inv_col2_body(const PlanDev<Ar>& P, typename Ar:
     using Cfg = ColCfg<Ar, LOGR>;
     constexpr int LCB = Cfg::LCB;
     constexpr int RL0 = first_rl(LOGR), NT = Cfg::NT, CB = 1 << LCB;
-    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = cst->done = 0;
+    if (tile == 0 && kp == 0 && threadIdx.x == 0) cst->counter = cst->any = 0;
     const int log_c = P.log_c + P.log_r2;
     const PrimeDev<Ar>& pr = P.pr[kp];
     const Ar ar = pr.ar;

@@ -227,10 +227,10 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
         dim3 g1(ntiles * (PP ? pl->K : 1), 1, square ? 1 : 2);
         if (ts) {
             k_fwd_col<Ar, SPLIT16, 4, true, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
-                pd, a, in_a, b, in_b, ra, rb, zt, tile0);
+                pd, a, in_a, b, in_b, ra, rb, zt, tile0, c->sums);
         } else {
             k_fwd_col<Ar, SPLIT16, 4, false, W64, PP><<<g1, kColThreads, smem1, c->stream>>>(
-                pd, a, in_a, b, in_b, ra, rb, zt, tile0);
+                pd, a, in_a, b, in_b, ra, rb, zt, tile0, c->sums);
         }
     };
     if (!io || io->chunks <= 1) {
@@ -259,11 +259,6 @@ int bw_enqueue_transform(bw_ctx* c, const uint32_t* a, const uint32_t* b, bool s
             BW_CUDA(cudaStreamWaitEvent(c->stream, c->in_ev[k], 0));
             k1(k * per, per);
         }
-    }
-    if (W64 && !pl->v2_cols) {
-        const unsigned nb = 4 * 148;
-        k_sum_words<<<nb, 256, 0, c->stream>>>(a, pl->la, c->sums);
-        if (!square) k_sum_words<<<nb, 256, 0, c->stream>>>(b, pl->lb, c->sums + kSumSlots);
     }
     // three passes: middle column pass with the outer twiddle
     const int CB2 = 1 << pl->log_cb2;
