@@ -615,7 +615,12 @@ int bw_plan_setup(bw_plan* pl, int path, int K, int log_n, unsigned flags, int m
             // -> 28.1 (two primes), 2^19 49 -> 40 and 2^20 94 -> 88 (six), 44
             // -> 35 and 83 -> 77 (double precision); equal or slower elsewhere
             const int square = (log_n + 1) / 2;
-            const int single_c = log_n >= 17 && log_n <= 20 ? (log_n + 4) / 2 : square;
+            // 58-bit integers up to 2^9 points: rows of 4 and long columns, the
+            // rows' any-length pass being one thread's work otherwise (2^7
+            // points 22.7 -> 17.2 us, 2^8 24.7 -> 18.6, 2^9 22.7 -> 18.6)
+            const int single_c = log_n >= 17 && log_n <= 20              ? (log_n + 4) / 2
+                                 : path == BW_PATH_P64 && !pl->f64 && log_n <= 9 ? 2
+                                                                                 : square;
             const int group_c = log_n <= 14   ? std::max(log_n - 3, square)
                                 : log_n <= 16 ? log_n - 4
                                               : std::max(10, square);
