@@ -337,8 +337,8 @@ def tune_table():
 
 def set_tune_entry(path, num_primes, log_n, small, log_cols=0, row_radix=0):
     """One tune-table entry: one CTA per product (small), or the 4-step
-    kernels with 2^log_cols columns (0: automatic) and row rounds of radix
-    row_radix (8 or 16; 0: the path's default)."""
+    kernels with 2^log_cols columns (0: automatic).  row_radix (0, 8 or 16) is
+    kept with the entry and has no effect: rows run in radix 16."""
     check(lib.bw_tune_table_set(path, num_primes, log_n, 1 if small else 0, log_cols,
                                 row_radix))
 

@@ -783,6 +783,9 @@ extern "C" int bw_plan_create_arith(bw_plan** out, int path, size_t la, size_t l
     const size_t half = ((size_t)1 << log_n) / 2;
     pl->zt_a = pl->nca <= half;
     pl->zt_b = pl->ncb <= half;
+    // (switches whose forms are gone)
+    flags &= ~(BW_PLAN_RADIX8 | BW_PLAN_RADIX16 | BW_PLAN_COL_RADIX8 | BW_PLAN_TMA_COLS |
+               BW_PLAN_NO_TMA_COLS | BW_PLAN_SHFL_ROWS | BW_PLAN_K1_ONE_PRIME);
     pl->one = path == BW_PATH_P32 && !w64 && log_n <= kOneMaxLogSingle && flags == 0;
     rc = bw_plan_setup(pl, path, K, log_n, flags, 2);
     if (rc) {

@@ -404,8 +404,8 @@ int bw_batch_autotune(bw_batch* batch, int reps);
  * log_cols, row_radix, ms}.  Writes at most len bytes including the
  * terminating NUL; *needed gets the full size. */
 int bw_tune_table_export(char* buf, size_t len, size_t* needed);
-/* Set one tune-table entry (log_cols 0 = automatic split; row_radix 8 or 16,
- * or 0 for the path's default: 8 on the 64-bit path, 16 on the 32-bit). */
+/* Set one tune-table entry (log_cols 0 = automatic split).  row_radix 0, 8 or
+ * 16 is kept with the entry and has no effect: rows run in radix 16. */
 int bw_tune_table_set(int path, int num_primes, int log_n, int small, int log_cols,
                       int row_radix);
 
