@@ -5,7 +5,7 @@ Default workload (configuration 2): one plain 2^28-bit x 2^28-bit product
 coefficients, n = 2^24, two 58-bit primes (64-bit prime path); the library's
 plan for it runs 64-bit coefficients over three primes of 51 bits.  A "step" is
 one full product.  Metric: products/s (whole job), with the per-stage times,
-the HBM roofline of the dominant kernel and the product-level algorithmic
+the roofline of the dominant kernel and the product-level algorithmic
 byte model (12*K*n*w + in + out) beside it.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
@@ -135,6 +135,24 @@ def model_bytes(la, lb, n, K, w, square):
     inv = 2 * knw                                               # INV pass 2
     carry = knw + 4 * (la + lb)                                 # Garner + carry
     return {"fwd_ms": fwd, "mul_ms": row, "intt_ms": inv, "crt_carry_ms": carry}
+
+
+def moved_bytes(la, lb, n, K, w, square):
+    """Bytes each kernel has to move: what it reads and writes once, the row pass
+    fused (both operands' rows in, the product's rows out)."""
+    knw = K * n * w
+    ops = 1 if square else 2
+    return {"fwd_ms": 4 * (la + (0 if square else lb)) + ops * knw, "mul_ms": (ops + 1) * knw,
+            "intt_ms": 2 * knw, "crt_carry_ms": knw + 4 * (la + lb)}
+
+
+def kernel_butterflies(info, square):
+    """Butterflies of each kernel: (n/2) per stage, prime and transform."""
+    per = info["num_primes"] * (1 << (info["log_n"] - 1))
+    ops = 1 if square else 2
+    outer = info["log_n"] - info["log_cols"]
+    return {"fwd_ms": ops * per * outer, "mul_ms": (ops + 1) * per * info["log_cols"],
+            "intt_ms": per * outer, "crt_carry_ms": 0}
 
 
 def load_peaks():
@@ -1347,8 +1365,34 @@ def bench_plain(args):
         kernel_names = {"fwd_ms": "k_fwd_col", "mul_ms": "k_row", "intt_ms": "k_inv_col",
                         "crt_carry_ms": "k_garner_carry"}
         peak, peak_kind = load_peaks()
-        achieved = mb[dom] / (stage[dom] * 1e-3) / 1e9
         own_model = sum(mb.values())
+        # the dominant kernel against both ceilings; the nearer one bounds it
+        moved = moved_bytes(la, lb, n, K, w, square)[dom]
+        gbs = moved / (stage[dom] * 1e-3) / 1e9
+        roofline = {"bound": "hbm", "kernel": kernel_names[dom], "achieved": gbs, "peak": peak,
+                    "unit": "GB/s", "frac": gbs / peak, "peak_source": peak_kind}
+        # arithmetic ceiling: butterflies at the rate they reach with nothing
+        # else running -- integer butterflies as measured, or, in double
+        # precision (primes of at most 52 bits on the 64-bit path), 8 FP64
+        # operations each at 64 per SM-cycle
+        if path == 64 and max(info["primes"]).bit_length() <= 52:
+            import torch
+            pipe = "fp64"
+            bfly_rate = (64 / 8 * torch.cuda.get_device_properties(0).multi_processor_count *
+                         1e6 * ((clocks or {}).get("sm_max_mhz") or 1965))
+            how = "8 FP64 operations per butterfly at 64 per SM-cycle, maximum SM clock"
+        else:
+            pipe = "int"
+            bfly_rate, _ = butterfly_rate(path)
+            how = ("bw_butterfly_rate: the path's own forward and inverse butterflies from "
+                   "registers, best over 2/4/8 CTAs per SM (bench.py --config intpeak)")
+        done = kernel_butterflies(info, square)[dom] / (stage[dom] * 1e-3)
+        if done / bfly_rate > gbs / peak:
+            roofline.update(bound=pipe, achieved=done / 1e9, peak=bfly_rate / 1e9,
+                            unit="Gbutterflies/s", frac=done / bfly_rate, peak_source=how)
+        roofline.update(hbm_gbs=gbs, hbm_frac=gbs / peak,
+                        traffic=load_traffic(cfg, kernel_names[dom]), algorithmic_bytes=moved,
+                        bytes_model="what the kernel reads and writes once")
         fixed, fk, fn, fw = fixed_model(cfg)
         line = {
             "metric": "products/s", "value": job_throughput(args.steps, world, total_ms),
@@ -1365,12 +1409,7 @@ def bench_plain(args):
             "correctness_check": check,
             "hbm_footprint_bytes": device_bytes,
             "stage_ms": stage,
-            "roofline": {"bound": "hbm", "kernel": kernel_names[dom], "achieved": achieved,
-                         "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "peak_source": peak_kind,
-                         "traffic": load_traffic(cfg, kernel_names[dom]),
-                         "algorithmic_bytes": mb[dom],
-                         "bytes_model": "the chosen algorithm's K*n*w per kernel"},
+            "roofline": roofline,
             "product_roofline": {
                 "fixed_model_bytes": fixed,
                 "fixed_model": f"12*K*n*w + in + out at the workload's stated K={fk}, "
@@ -1406,20 +1445,8 @@ def bench_plain(args):
             other["int_floor_frac"] = ofloor / other["ms_per_step"]
             line["other_path"] = other
         if world == 1:
-            # arithmetic floor: the plan's butterflies at the rate they reach
-            # with nothing else running -- integer butterflies as measured, or,
-            # in double precision (primes of at most 52 bits on the 64-bit
-            # path), 8 FP64 operations each at 64 per SM-cycle
-            bfly = plan_butterflies(info, square)
-            if path == 64 and max(info["primes"]).bit_length() <= 52:
-                import torch
-                rate = (64 / 8 * torch.cuda.get_device_properties(0).multi_processor_count *
-                        1e6 * ((clocks or {}).get("sm_max_mhz") or 1965))
-                how = "8 FP64 operations per butterfly at 64 per SM-cycle, maximum SM clock"
-            else:
-                rate, _ = butterfly_rate(path)
-                how = ("bw_butterfly_rate: the path's own forward and inverse butterflies from "
-                       "registers, best over 2/4/8 CTAs per SM (bench.py --config intpeak)")
+            # arithmetic floor: the plan's butterflies at that rate
+            bfly, rate = plan_butterflies(info, square), bfly_rate
             floor_ms = bfly / rate * 1e3
             line["int_floor"] = {"butterflies": bfly, "butterflies_per_s": rate,
                                  "floor_ms": floor_ms, "frac": floor_ms / ms, "how": how}

@@ -131,8 +131,10 @@ struct Ar32 {
 // be 2 short, so the product lies in [0, 3p)).  The forward (CT) butterfly
 // adds without reducing: from inputs below 3p its stage-0 sums stay below 6p
 // and every later stage adds less than 3p, so s stages stay below 3p (s + 1)
-// -- below 64p for the at most 13 stages one pass runs (the headroom the
-// 58-bit primes buy: with primes near 2^62 every butterfly reduced its input).
+// -- below 64p for 20 stages, as many as the fixed-length row pass reaches when
+// it continues the column pass's values up to its first multiplication of each
+// (bw_plan_setup keeps longer sums on the any-length rows).  It is the headroom
+// the 58-bit primes buy: with primes near 2^62 every butterfly reduced its input.
 // The inverse (GS) transform keeps values in [0, 3p): sums are reduced by one
 // conditional subtraction of 3p, differences are offset by 3p (6p < 2^64).
 // A forward output enters the pointwise product reduced to [0, 2p) by an
@@ -325,9 +327,11 @@ struct Ar64 {
 // POL 0: primes within 1% above 2^50: q needs X <= 3.96, |r| <= p (1/2 + 0.066
 //   X).  Forward: a round reduces the half it does not multiply in its first
 //   stage and then adds four stages: from X = 3.1 at most 1.21, 1.79, 2.41,
-//   3.07.  Inverse: the sums of every second stage, and of a round's last, are
-//   reduced: from E a difference of 4 E and an output of 1/2 + 0.27 E, so E
-//   stays below 0.69 and differences below 2.8.
+//   3.07.  A row's last round starts from products instead (0.71) and ends at
+//   3.12, an any-length row, whose first stage has no multiplication, at 3.31.
+//   Inverse: the sums of every second stage, and of a round's last, are reduced:
+//   from E a difference of 4 E and an output of 1/2 + 0.27 E, so from the
+//   pointwise product's 0.72 E stays below that, and differences below 2.9.
 // POL 1: primes just above 2^51.67 (X <= 1.24 for q, 2.4 for exact sums, |r| <=
 //   p (1/2 + 0.21 X)), for transforms whose coefficients need three such
 //   primes: a forward round reduces all its values before its first and third
@@ -356,7 +360,7 @@ struct ArD {
         return __dadd_rn(__fma_rn(-q, p, h), l);
     }
     // the pointwise product: a any forward output, b reduced (POL 0: |a b| <=
-    // 3.1 p * p/2, so |q| < 2^51 and the result is below 0.61 p)
+    // 3.31 p * p/2, so |q| < 2^51 and the result is below 0.72 p)
     __device__ __forceinline__ T pointwise(T a, T b) const {
         return POL ? red(mul(red(a), b)) : mul(a, b);
     }

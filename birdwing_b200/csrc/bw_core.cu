@@ -515,11 +515,14 @@ int bw_check_size_w64(size_t la, size_t lb, int* log_n_out, int path = BW_PATH_P
 
 // num_primes 0 on the 64-bit path: 64-bit coefficients with three primes
 // (3 primes x n/2 points instead of 2 x n) where they halve the transform
-// and their own transform has at least 2^19 points.  On a B200 they measured
-// faster from there (2^20-word operands, on integers: 0.245 vs 0.324 ms; 2^23
-// words now 0.76 vs 1.84 ms); below, the three-prime Garner and fixed costs
-// made them slower (2^18 words: 0.124 vs 0.100 ms).  Every product that BW_PATH_AUTO moves off
-// the 32-bit path (more than 2^21 of its points) has at least 2^19 of them.
+// and their own transform has at least 2^19 points.  The line was drawn on
+// integer transforms (2^18 words: 0.124 vs 0.100 ms).  In double precision they
+// are faster everywhere (three products in flight, 64- vs 32-bit coefficients:
+// 2^14 words 6.7 vs 12.5 us, 2^16 10.6 vs 16.9, 2^18 19.7 vs 45.5, 2^20 77 vs
+// 208), but the plan that num_primes 0 resolves to is part of the interface
+// (include/birdwing.h); BW_PLAN_COEF64 asks for them at any size.  Every product
+// that BW_PATH_AUTO moves off the 32-bit path (more than 2^21 of its points) has
+// at least 2^19 points of them.
 constexpr int kW64MinLogN = 19;
 
 bool bw_w64_pays(size_t la, size_t lb) {
@@ -535,16 +538,15 @@ bool bw_w64_pays(size_t la, size_t lb) {
     return l64 >= kW64MinLogN && l64 < l32;
 }
 
-// BW_PATH_AUTO: the 32-bit path while its transform has at most 2^24 points
-// (its 32-bit butterflies are about four times cheaper than the 64-bit ones,
-// which more than pays for its doubled transform length against 32-bit
-// coefficients on the 64-bit path: on a B200 it measured 10-30% faster from
-// 2^14- to 2^27-bit operands, equal at 2^28), the 64-bit path beyond and
-// wherever the 32-bit path cannot hold the product.  Where the 64-bit path
-// would use 64-bit coefficients (w64_ok: single products with num_primes 0)
-// the crossover is at 2^21 points of the 32-bit path: 2^20-word operands
-// measured 0.245 ms against 0.282 ms, 2^22 words 1.00 against 1.13 ms, 2^18
-// words 0.124 against 0.091 ms.
+// BW_PATH_AUTO: the 32-bit path while its transform has at most 2^24 points,
+// the 64-bit path beyond and wherever the 32-bit path cannot hold the product
+// (32-bit coefficients, three products in flight, 32- vs 64-bit path: 2^16 words
+// 10.6 vs 16.9 us, 2^20 129 vs 208, 2^22 681 vs 803, 2^23 1826 vs 1803).  Where
+// the 64-bit path would use 64-bit coefficients (w64_ok: single products with
+// num_primes 0) the line is at 2^21 points of the 32-bit path.  It too was drawn
+// on integer transforms (2^18 words 0.124 vs 0.091 ms); they are now ahead from
+// 2^17 words (13.0 vs 15.6 us; 2^18 19.7 vs 28.1, 2^19 35 vs 59, 2^16 10.6
+// both), and the line stays for the interface's sake.
 constexpr int kAutoP32MaxLogN = 24;
 constexpr int kAutoP32MaxLogNW64 = 21;
 
@@ -569,8 +571,8 @@ static int resolve_plan(int path, int num_primes, size_t la, size_t lb, unsigned
         // the 32-bit path (six primes) while their transform fits (n <= 2^23).
         // The line was drawn when the 64-bit path's three primes ran on
         // integers (2^23 words 1.36 vs 1.51 ms); in double precision they are
-        // now the faster ones (three products in flight: 2^20 words 77 vs 88
-        // us, 2^21 168 vs 185, 2^22 351 vs 381, 2^23 750 vs 811), but which
+        // now the faster ones (three products in flight: 2^20 words 77 vs 87
+        // us, 2^21 169 vs 184, 2^22 352 vs 379, 2^23 735 vs 805), but which
         // plan AUTO resolves to is part of the interface
         if (!force64 && num_primes == 0 && path == BW_PATH_P64) {
             if (bw_check_size_w64(la, lb, nullptr, BW_PATH_P32) == BW_OK) {
@@ -1176,10 +1178,10 @@ float ev_ms(cudaEvent_t a, cudaEvent_t b) {
 
 }  // namespace
 
-// Device-pointer product through a CUDA graph of the whole pipeline (look-back
-// records cleared, K1..K4), captured on first use and replayed while a, b,
-// out and the squaring choice stay the same.  Returns 1 when a graph cannot
-// be used (the stream is already being captured by the caller).
+// Device-pointer product through a CUDA graph of the whole pipeline (K1..K4),
+// captured on first use and replayed while a, b, out and the squaring choice
+// stay the same.  Returns 1 when a graph cannot be used (the stream is already
+// being captured by the caller).
 static int launch_graph(bw_ctx* c, const uint32_t* a, const uint32_t* b, uint32_t* out, bool sq) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)

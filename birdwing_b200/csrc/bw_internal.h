@@ -77,10 +77,11 @@ constexpr int kMaxGroupLogN = 26;
 
 // One launch group: np products of one plan (equal path, K and transform
 // length), product q described by d_desc[q].  A single-pass plan (small)
-// runs ks_product, one CTA per product, with residue scratch res_a
-// (np * K * n elements); a 4-step plan runs kb_fwd_col, kb_row, kb_inv_col
-// and kb_garner_carry over residue arenas res_a and res_b of the same size,
-// with per-product look-back state (zeroed before the launch, epoch 1).
+// runs kb_one, one CTA per product (beyond 2^12 points ks_product, with residue
+// scratch res_a, np * K * n elements); a 4-step plan runs kb_fwd_col2, kb_row2,
+// kb_inv_col2 (or their any-length forms) and a carry over residue arenas res_a
+// and res_b of the same size, with per-product carry state (zeroed before the
+// launch, epoch 1).
 struct bw_group_launch {
     const bw_plan* plan;
     const bw::BatchProd* d_desc;
@@ -142,8 +143,7 @@ struct bw_ctx {
     uint32_t* rec_s = nullptr;
     bw::Sum* sums = nullptr;    // word sums (64-bit coefficients)
     size_t ntiles = 0;
-    // look-back record tag of the last product.  Direct launches use 2, 3, ..;
-    // the replayable graph clears the records and always uses 1.
+    // look-back record tag of the last product that used the look-back carry
     uint32_t epoch = 1;
     cudaGraphExec_t gexec = nullptr;  // device-pointer product, replayed while
     const void* g_a = nullptr;        // the pointers stay the same

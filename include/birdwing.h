@@ -141,7 +141,11 @@ typedef struct bw_ctx bw_ctx;
  * Field meanings follow the reference's NTTTiming (include/gpu_ntt.h:87-99):
  * fwd_ms covers limb split + zero pad + forward column pass for both operands;
  * mul_ms the fused row pass (forward rows, pointwise product, inverse rows);
- * intt_ms the inverse column pass; crt_carry_ms the fused Garner + carry. */
+ * intt_ms the inverse column pass; crt_carry_ms the fused Garner + carry.
+ * Products of at most 2^11 points with 16-bit coefficients otherwise run in one
+ * kernel, which has no such stages: with timing they run these, and take longer
+ * than without.  Calls with timing also wait between kernels where others start
+ * the next one early. */
 typedef struct bw_timing {
     float h2d_ms;
     float fwd_ms;
@@ -197,7 +201,11 @@ int bw_size_supported(int path, int num_primes, size_t la, size_t lb);
  * (BW_PLAN_COEF64) where they halve the transform and it has at least 2^19
  * points, else 32-bit coefficients with K = 2.  num_primes 2 or 3 keeps the
  * reference's 16- or 32-bit coefficients (and then AUTO takes the 32-bit path
- * up to 2^24 points).  The plan is bound to the current CUDA device. */
+ * up to 2^24 points).  These choices are kept from version to version, so that
+ * a size keeps its primes and coefficients; where another plan measures faster
+ * (64-bit coefficients on the 64-bit path, from about 2^17 words) BW_PATH_P64
+ * with BW_PLAN_COEF64 asks for it.  The plan is bound to the current CUDA
+ * device. */
 int bw_plan_create(bw_plan** out, int path, size_t la, size_t lb,
                    int num_primes, unsigned flags);
 int bw_plan_destroy(bw_plan* plan);
