@@ -924,7 +924,15 @@ extern "C" int bw_ctx_create(bw_ctx** out, const bw_plan* pl, void* stream) {
     c->state_bytes = rec + c->ntiles * 16 + c->ntiles * 4;
     if ((e = cudaMalloc(&c->d_state, c->state_bytes)) != cudaSuccess)
         return fail(bw_fail(BW_ENOMEM, "carry state: %s", cudaGetErrorString(e)));
-    if ((e = cudaMemset(c->d_state, 0, c->state_bytes)) != cudaSuccess)
+    // (on the context's stream: a clear on the default stream may come after work
+    // that is queued there, and so into the first products)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    e = cudaStreamIsCapturing(c->stream, &cap);
+    if (e == cudaSuccess)
+        e = cap == cudaStreamCaptureStatusNone
+                ? cudaMemsetAsync(c->d_state, 0, c->state_bytes, c->stream)
+                : cudaMemset(c->d_state, 0, c->state_bytes);
+    if (e != cudaSuccess)
         return fail(bw_fail(BW_ECUDA, "memset: %s", cudaGetErrorString(e)));
     c->cst = reinterpret_cast<CarryState*>(c->d_state);
     c->err = reinterpret_cast<uint32_t*>(c->d_state + 16);

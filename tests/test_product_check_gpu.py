@@ -105,3 +105,25 @@ def test_groups_report_a_wrong_residue(words, K):
             else:
                 bt.run()
                 assert (out == gmp_ref.mul(a, b)).all()
+
+
+def test_context_made_beside_a_busy_default_stream():
+    # the carry state and the sums are clear before the first product, whatever
+    # is queued on the default stream when the context is made
+    import torch
+    n = 1 << 16
+    a, b = operands(n, n, "ones")
+    want = torch.from_numpy(gmp_ref.mul(a, b).view(np.int32)).cuda()
+    d = [torch.from_numpy(x.view(np.int32)).cuda() for x in (a, b)]
+    out = torch.empty(2 * n, dtype=torch.int32, device="cuda")
+    with bw.Plan(n, n, 64, flags=C64) as p:
+        torch.cuda.synchronize()
+        for _ in range(5):
+            torch.cuda._sleep(4_000_000)  # about 2 ms
+            with bw.Context(p) as c:
+                for _ in range(200):
+                    c.multiply_device(d[0].data_ptr(), n, d[1].data_ptr(), n, out.data_ptr(),
+                                      2 * n)
+                c.sync()
+            torch.cuda.synchronize()
+            assert torch.equal(out, want)
