@@ -84,10 +84,11 @@ extern "C" {
  * 32 KiB), in the any-length column passes; BW_PLAN_THREE_PASS uses the
  * three-pass schedule (n = R * R2 * C) even where two passes fit (it is used
  * anyway beyond n = 2^26, with 64-bit coefficients on the 64-bit path from n =
- * 2^24).  BW_PLAN_RADIX8, _RADIX16, _COL_RADIX8, _WIDE_COLS (but for the
- * any-length columns' tile), _TMA_COLS, _NO_TMA_COLS, _SHFL_ROWS and
- * _K1_ONE_PRIME are accepted and change nothing: the forms they chose measured
- * slower than the fixed-length passes and are gone. */
+ * 2^24); BW_PLAN_WIDE_COLS widens the any-length columns' tile.  A product of at
+ * most 2^11 points with 16-bit coefficients runs in one kernel without them and
+ * in these passes with any.  BW_PLAN_RADIX8, _RADIX16, _COL_RADIX8, _TMA_COLS,
+ * _NO_TMA_COLS, _SHFL_ROWS and _K1_ONE_PRIME are accepted and change nothing: the
+ * forms they chose measured slower than the fixed-length passes and are gone. */
 #define BW_PLAN_RADIX8      (1u << 16)
 #define BW_PLAN_TW_SMEM     (1u << 17)
 #define BW_PLAN_THREE_PASS  (1u << 18)
